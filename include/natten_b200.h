@@ -149,13 +149,18 @@ unsigned long long natten_launch_count(void); /* kernels launched by this librar
 /* Bounded waits.  Every barrier wait inside the tensor-core kernels has a cycle budget; a
  * kernel whose wait runs out raises a status word on its device, stops touching data, frees
  * what it holds and returns, and kernels launched afterwards on that device return at once
- * without computing until the word is cleared.  The three calls below act on the current device.
+ * without computing until the word is cleared.  The calls below act on the current device
+ * (natten_host_status: on the named one).
  *   natten_device_status  synchronises the device; NATTEN_OK or NATTEN_E_DEVICE.
  *   natten_clear_status   synchronises, resets the word; 0 or a cudaError_t value.
+ *   natten_host_status    non-zero once a kernel of `device` has given up: the kernel itself writes a
+ *                         word in mapped host memory, so this is a plain read (no CUDA call), to be
+ *                         made before the next launch or after the stream was synchronised.
  *   natten_status_async   enqueues a 4-byte copy of the word into caller-owned pinned host
  *                         memory on `stream` (no synchronisation, no allocation): non-zero there
  *                         after the stream has passed that point means a kernel gave up.       */
 int natten_device_status(void);
+int natten_host_status(int device);
 int natten_clear_status(void);
 int natten_status_async(int32_t* pinned_host_word, void* stream);
 /* Test hook: cycle budget of those waits (<= 0 restores the default of about two seconds) and a

@@ -1,4 +1,5 @@
-"""Build the CUDA library in-tree: ``natten_mps_b200/libnatten_b200.so``.
+"""Build the native code in-tree: ``natten_mps_b200/libnatten_b200.so`` (the CUDA library behind the C ABI, no
+torch in it) and ``natten_mps_b200/_native.so`` (the PyTorch operators on top of it, host code only).
 
 nvcc cross-compiles for sm_100a without a GPU.  Each ``.cu`` file is compiled to
 an object in ``csrc/build/`` (in parallel, skipped when the object is newer than
@@ -14,6 +15,7 @@ import subprocess
 _PKG = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_PKG, "csrc")
 LIB_PATH = os.path.join(_PKG, "libnatten_b200.so")
+NATIVE_PATH = os.path.join(_PKG, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -26,6 +28,28 @@ def _nvcc() -> str:
         if cand and (os.path.isabs(cand) and os.path.exists(cand) or not os.path.isabs(cand)):
             return cand
     return "nvcc"
+
+
+def build_native(headers, force: bool = False) -> str:
+    """Compile csrc/torch_ops.cpp against the running interpreter's torch and link it to the CUDA library."""
+    import sysconfig
+
+    import torch
+
+    src = os.path.join(_CSRC, "torch_ops.cpp")
+    newest = max([os.path.getmtime(src)] + [os.path.getmtime(h) for h in headers if h.endswith(".h")])
+    if not force and os.path.exists(NATIVE_PATH) and os.path.getmtime(NATIVE_PATH) >= newest:
+        return NATIVE_PATH
+    troot = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    subprocess.check_call([
+        "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        *[f"-I{d}" for d in (os.path.join(troot, "include"), os.path.join(troot, "include", "torch", "csrc", "api", "include"),
+                             os.path.join(cuda, "include"), sysconfig.get_paths()["include"])],
+        src, "-o", NATIVE_PATH, f"-L{_PKG}", "-l:libnatten_b200.so", "-Wl,-rpath,$ORIGIN",
+        f"-L{os.path.join(troot, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"])
+    return NATIVE_PATH
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -53,6 +77,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             os.path.getmtime(o) > os.path.getmtime(LIB_PATH) for o in objects):
         subprocess.check_call([_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared",
                                "-o", LIB_PATH, *objects, "-lcuda"])
+    build_native(headers, force)
     return LIB_PATH
 
 

@@ -1,7 +1,7 @@
-"""ctypes binding of ``libnatten_b200.so`` (declared in ``include/natten_b200.h``).
+"""ctypes binding of ``libnatten_b200.so`` (declared in ``include/natten_b200.h``): what ``HostStep``, the
+benchmark and the tests use.  The operators reach the same library from ``csrc/torch_ops.cpp``.
 
-This is the only place the Python package touches native code.  There is no
-CPU or PyTorch fallback: if the library is missing, importing an op raises.
+There is no CPU or PyTorch fallback: if the library is missing, calling an op raises.
 """
 from __future__ import annotations
 
@@ -23,7 +23,7 @@ EXPORTS = (
     "natten_fused_fwd", "natten_fused_bwd", "natten_workspace_bytes", "natten_qk_fwd",
     "natten_qk_bwd", "natten_qk_rpb_fwd", "natten_qk_rpb_bwd", "natten_av_fwd", "natten_av_bwd", "natten_strerror",
     "natten_abi_version", "natten_last_path", "natten_launch_count", "natten_device_status",
-    "natten_clear_status", "natten_status_async", "natten_debug_wait",
+    "natten_clear_status", "natten_status_async", "natten_host_status", "natten_debug_wait",
     "natten_fused_bwd_static", "natten_static_scratch_bytes",
 )
 
@@ -89,7 +89,9 @@ def lib():
 def set_force(path: Optional[str]) -> None:
     """Testing aid: force ``"simt"`` or ``"tc"`` kernels (``None`` = automatic)."""
     global _force_flags
+    from ._torch_ops import native
     _force_flags = {None: 0, "auto": 0, "simt": FLAG_FORCE_SIMT, "tc": FLAG_FORCE_TC}[path]
+    native.set_flags(_force_flags)
 
 
 def last_path() -> str:
@@ -104,42 +106,18 @@ def device_status() -> int:
 def clear_status() -> None:
     """Reset the current device's status word after a kernel gave up on a wait (synchronises)."""
     rc = int(lib().natten_clear_status())
-    for w in _status_words.values():
-        w.zero_()
     if rc:
         raise RuntimeError(f"natten_clear_status: CUDA error {rc}")
 
 
-# One pinned host word per device.  After every launch the library copies the device's status
-# word into it on the launching stream; the word is looked at (a plain host read) at the next
-# call and by ``poll_status``, so a kernel that gave up surfaces as a RuntimeError instead of
-# silently empty results.
-_status_words = {}
-
-
-def _status_word(device: torch.device) -> torch.Tensor:
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    w = _status_words.get(idx)
-    if w is None:
-        w = torch.zeros(1, dtype=torch.int32).pin_memory()
-        _status_words[idx] = w
-    return w
-
-
 def poll_status(device: torch.device) -> None:
-    """Raise if a kernel on ``device`` reported a timed-out wait (no synchronisation: sees what
-    the stream has copied back so far)."""
-    if int(_status_word(device)[0]) != 0:
+    """Raise if a kernel on ``device`` reported a timed-out wait (no synchronisation, nothing queued: such a
+    kernel has written the device's word in host memory itself)."""
+    idx = device.index if device.index is not None else torch.cuda.current_device()
+    if lib().natten_host_status(idx) != 0:
         raise RuntimeError(
             "natten_b200: a tensor-core kernel gave up on a bounded wait (results since then are "
             "invalid); call natten_mps_b200._cabi.clear_status() to re-arm the device")
-
-
-def track_status(t: torch.Tensor) -> None:
-    """Enqueue the status copy behind the kernels just launched on ``t``'s current stream."""
-    w = _status_word(t.device)
-    with torch.cuda.device(t.device):
-        lib().natten_status_async(ctypes.c_void_p(w.data_ptr()), stream_of(t))
 
 
 def launch_count() -> int:

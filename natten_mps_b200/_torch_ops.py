@@ -13,30 +13,24 @@ They are thin compositions of four rank-generic ops that own the kernels:
 
     na_fused      -> (out, lse)   fused forward; GQA, additional tokens, extents
     na_fused_bwd  -> (dq, dk, dv, d_extra_k, d_extra_v)
-    na_qk / na_qk_bwd,  na_av / na_av_bwd
+    na_qk / na_qk_bwd,  na_qk_rpb / na_qk_rpb_bwd,  na_av / na_av_bwd
 
-Only a ``CUDA`` implementation (plus ``Meta`` shape functions) is registered:
-calling an op with CPU tensors fails in the dispatcher instead of silently
-running something else.
+Schemas and ``Meta`` shape functions are here; the ``CUDA`` and autograd kernels are
+native (``csrc/torch_ops.cpp``).  Nothing is registered for other devices: calling an op
+with CPU tensors fails in the dispatcher instead of silently running something else.
 """
 from __future__ import annotations
 
-from typing import List, Optional, Sequence, Tuple
+import os
+from typing import List, Sequence
 
 import torch
 
-from . import _backend
-
 LIB = torch.library.Library("natten_b200", "DEF")
-NS = "natten_b200"
 
 
 def _strided(spatial: Sequence[int], stride: Sequence[int]) -> List[int]:
     return [(n - 1) // s + 1 for n, s in zip(spatial, stride)]
-
-
-def _opt(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    return None if t is None or t.numel() == 0 else t
 
 
 # ---------------------------------------------------------------------------
@@ -53,14 +47,6 @@ LIB.define(
     "-> (Tensor, Tensor, Tensor, Tensor, Tensor)")
 
 
-@torch.library.impl(LIB, "na_fused", "CUDA")
-def _na_fused_cuda(query, key, value, extra_k, extra_v, extents, kernel_size, stride, dilation,
-                   is_causal, scale):
-    return _backend.fused_forward(query, key, value, tuple(kernel_size), tuple(stride),
-                                  tuple(dilation), tuple(is_causal), float(scale),
-                                  extra_k, extra_v, extents)
-
-
 @torch.library.impl(LIB, "na_fused", "Meta")
 def _na_fused_meta(query, key, value, extra_k, extra_v, extents, kernel_size, stride, dilation,
                    is_causal, scale):
@@ -72,18 +58,6 @@ def _na_fused_meta(query, key, value, extra_k, extra_v, extents, kernel_size, st
     return out, lse
 
 
-@torch.library.impl(LIB, "na_fused_bwd", "CUDA")
-def _na_fused_bwd_cuda(query, key, value, extra_k, extra_v, extents, out, lse, dout, dlse,
-                       kernel_size, stride, dilation, is_causal, scale):
-    dq, dk, dv, dek, dev = _backend.fused_backward(
-        query, key, value, out, lse, dout, tuple(kernel_size), tuple(stride), tuple(dilation),
-        tuple(is_causal), float(scale), extra_k, extra_v, extents, dlse)
-    if dek is None:
-        dek = query.new_empty(0)
-        dev = query.new_empty(0)
-    return dq, dk, dv, dek, dev
-
-
 @torch.library.impl(LIB, "na_fused_bwd", "Meta")
 def _na_fused_bwd_meta(query, key, value, extra_k, extra_v, extents, out, lse, dout, dlse,
                        kernel_size, stride, dilation, is_causal, scale):
@@ -91,42 +65,6 @@ def _na_fused_bwd_meta(query, key, value, extra_k, extra_v, extents, out, lse, d
     dev = torch.empty_like(extra_v) if extra_v is not None else query.new_empty(0)
     return (query.new_empty(query.shape), key.new_empty(key.shape), value.new_empty(value.shape),
             dek, dev)
-
-
-def _fused_setup(ctx, inputs, output):
-    (q, k, v, ek, ev, extents, kernel_size, stride, dilation, is_causal, scale) = inputs
-    out, lse = output
-    ctx.geometry = (list(kernel_size), list(stride), list(dilation), list(is_causal), float(scale))
-    ctx.has_extra = ek is not None
-    ctx.has_extents = extents is not None
-    saved = [q, k, v, out, lse]
-    if ek is not None:
-        saved += [ek, ev]
-    if extents is not None:
-        saved.append(extents)
-    ctx.save_for_backward(*saved)
-
-
-def _fused_backward(ctx, grad_out, grad_lse):
-    saved = list(ctx.saved_tensors)
-    q, k, v, out, lse = saved[:5]
-    rest = saved[5:]
-    ek = ev = extents = None
-    if ctx.has_extra:
-        ek, ev = rest[0], rest[1]
-        rest = rest[2:]
-    if ctx.has_extents:
-        extents = rest[0]
-    ks, st, dil, causal, scale = ctx.geometry
-    if grad_out is None:
-        grad_out = torch.zeros_like(out)
-    dq, dk, dv, dek, dev = torch.ops.natten_b200.na_fused_bwd(
-        q, k, v, ek, ev, extents, out, lse, grad_out, grad_lse, ks, st, dil, causal, scale)
-    return (dq, dk, dv, dek if ctx.has_extra else None, dev if ctx.has_extra else None, None,
-            None, None, None, None, None)
-
-
-torch.library.register_autograd(f"{NS}::na_fused", _fused_backward, setup_context=_fused_setup)
 
 
 # ---------------------------------------------------------------------------
@@ -140,12 +78,9 @@ LIB.define("na_av(Tensor attn, Tensor value, int[] kernel_size, int[] dilation, 
            "bool[] is_causal) -> Tensor")
 LIB.define("na_av_bwd(Tensor dout, Tensor attn, Tensor value, int[] kernel_size, int[] dilation, "
            "int[] stride, bool[] is_causal) -> (Tensor, Tensor)")
-
-
-@torch.library.impl(LIB, "na_qk", "CUDA")
-def _na_qk_cuda(query, key, kernel_size, dilation, stride, is_causal, scale):
-    return _backend.qk_forward(query, key, tuple(kernel_size), tuple(dilation), tuple(stride),
-                               tuple(is_causal), scale)
+LIB.define("na_qk_rpb(Tensor query, Tensor key, Tensor rpb, int[] kernel_size, int[] dilation, float? scale) -> Tensor")
+LIB.define("na_qk_rpb_bwd(Tensor dlogits, Tensor query, Tensor key, int[] rpb_shape, int[] kernel_size, "
+           "int[] dilation, float? scale) -> (Tensor, Tensor, Tensor)")
 
 
 @torch.library.impl(LIB, "na_qk", "Meta")
@@ -158,37 +93,9 @@ def _na_qk_meta(query, key, kernel_size, dilation, stride, is_causal, scale):
                             query.shape[-2], ktot))
 
 
-@torch.library.impl(LIB, "na_qk_bwd", "CUDA")
-def _na_qk_bwd_cuda(dlogits, query, key, kernel_size, dilation, stride, is_causal, scale):
-    return _backend.qk_backward(dlogits, query, key, tuple(kernel_size), tuple(dilation),
-                                tuple(stride), tuple(is_causal), scale)
-
-
 @torch.library.impl(LIB, "na_qk_bwd", "Meta")
 def _na_qk_bwd_meta(dlogits, query, key, kernel_size, dilation, stride, is_causal, scale):
     return query.new_empty(query.shape), key.new_empty(key.shape)
-
-
-def _qk_setup(ctx, inputs, output):
-    q, k, kernel_size, dilation, stride, is_causal, scale = inputs
-    ctx.geometry = (list(kernel_size), list(dilation), list(stride), list(is_causal), scale)
-    ctx.save_for_backward(q, k)
-
-
-def _qk_backward(ctx, grad_logits):
-    q, k = ctx.saved_tensors
-    ks, dil, st, causal, scale = ctx.geometry
-    dq, dk = torch.ops.natten_b200.na_qk_bwd(grad_logits, q, k, ks, dil, st, causal, scale)
-    return dq, dk, None, None, None, None, None
-
-
-torch.library.register_autograd(f"{NS}::na_qk", _qk_backward, setup_context=_qk_setup)
-
-
-@torch.library.impl(LIB, "na_av", "CUDA")
-def _na_av_cuda(attn, value, kernel_size, dilation, stride, is_causal):
-    return _backend.av_forward(attn, value, tuple(kernel_size), tuple(dilation), tuple(stride),
-                               tuple(is_causal))
 
 
 @torch.library.impl(LIB, "na_av", "Meta")
@@ -196,32 +103,22 @@ def _na_av_meta(attn, value, kernel_size, dilation, stride, is_causal):
     return value.new_empty((*attn.shape[:-1], value.shape[-1]))
 
 
-@torch.library.impl(LIB, "na_av_bwd", "CUDA")
-def _na_av_bwd_cuda(dout, attn, value, kernel_size, dilation, stride, is_causal):
-    return _backend.av_backward(dout, attn, value, tuple(kernel_size), tuple(dilation),
-                                tuple(stride), tuple(is_causal))
-
-
 @torch.library.impl(LIB, "na_av_bwd", "Meta")
 def _na_av_bwd_meta(dout, attn, value, kernel_size, dilation, stride, is_causal):
     return attn.new_empty(attn.shape, dtype=value.dtype), value.new_empty(value.shape)
 
 
-def _av_setup(ctx, inputs, output):
-    attn, v, kernel_size, dilation, stride, is_causal = inputs
-    ctx.geometry = (list(kernel_size), list(dilation), list(stride), list(is_causal))
-    ctx.attn_dtype = attn.dtype
-    ctx.save_for_backward(attn, v)
+@torch.library.impl(LIB, "na_qk_rpb", "Meta")
+def _na_qk_rpb_meta(query, key, rpb, kernel_size, dilation, scale):
+    ktot = 1
+    for x in kernel_size:
+        ktot *= x
+    return query.new_empty((*query.shape[:-1], ktot))
 
 
-def _av_backward(ctx, grad_out):
-    attn, v = ctx.saved_tensors
-    ks, dil, st, causal = ctx.geometry
-    dattn, dv = torch.ops.natten_b200.na_av_bwd(grad_out, attn, v, ks, dil, st, causal)
-    return dattn.to(ctx.attn_dtype), dv, None, None, None, None
-
-
-torch.library.register_autograd(f"{NS}::na_av", _av_backward, setup_context=_av_setup)
+@torch.library.impl(LIB, "na_qk_rpb_bwd", "Meta")
+def _na_qk_rpb_bwd_meta(dlogits, query, key, rpb_shape, kernel_size, dilation, scale):
+    return query.new_empty(query.shape), key.new_empty(key.shape), query.new_empty(rpb_shape)
 
 
 # ---------------------------------------------------------------------------
@@ -270,5 +167,28 @@ def _define_rank_ops(rank: int) -> None:
 for _rank in (1, 2, 3):
     _define_rank_ops(_rank)
 
-OP_NAMES = ("na_fused", "na_fused_bwd", "na_qk", "na_qk_bwd", "na_av", "na_av_bwd") + tuple(
+OP_NAMES = ("na_fused", "na_fused_bwd", "na_qk", "na_qk_bwd", "na_qk_rpb", "na_qk_rpb_bwd", "na_av", "na_av_bwd") + tuple(
     f"na{r}d_{s}" for r in (1, 2, 3) for s in ("qk", "av", "fwd", "varlen_fwd"))
+
+
+# ---------------------------------------------------------------------------
+# native kernels of the ops, and the functional API's native entry points
+# ---------------------------------------------------------------------------
+class _NotBuilt:
+    """Stands in for the native module in a tree that has not been built: shapes (Meta) still work, calls with
+    CUDA tensors fail."""
+
+    def __getattr__(self, name):
+        def call(*args):
+            if any(isinstance(a, torch.Tensor) and a.is_cuda for a in args):
+                raise RuntimeError(f"{_NATIVE_PATH} is missing: build it with `python -m natten_mps_b200._build` "
+                                   "(there is no fallback implementation)")
+            return NotImplemented
+        return call
+
+
+_NATIVE_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_native.so")
+if os.path.exists(_NATIVE_PATH):
+    from . import _native as native      # registers the CUDA and autograd kernels
+else:
+    native = _NotBuilt()

@@ -300,6 +300,7 @@ int natten_last_path(void) { return t_last_path; }
 unsigned long long natten_launch_count(void) { return simt_launch_count() + tc_launch_count(); }
 int natten_device_status(void) { return tc_device_status() == 0 ? NATTEN_OK : NATTEN_E_DEVICE; }
 int natten_clear_status(void) { return tc_clear_status(); }
+int natten_host_status(int device) { return tc_host_status(device); }
 int natten_status_async(int32_t* pinned_host_word, void* stream)
 {
     return tc_status_async(reinterpret_cast<int*>(pinned_host_word), (cudaStream_t)stream);

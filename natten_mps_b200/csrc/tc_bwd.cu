@@ -743,7 +743,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
     if (warp == kComputeWarps) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
-        if (lane == 0 && *abort_flag) atomicExch(P.status, 1);
+        if (lane == 0 && *abort_flag) raise_status(P);
     }
 }
 
@@ -984,8 +984,6 @@ int tc_fused_bwd(int dtype, const Geo& g_in, const void* q, const void* k, const
     }
     Plan plan;
     if (!make_plan(g, plan, kCols, /*with_stride=*/false, /*interleave=*/true)) return -2;
-    plan.p.status = status_ptr();
-    if (!plan.p.status) return -2;
     if (g.B == 0) return 0;
     if (g.Hq > 65535 || g.B > 65535) return -2;
     float* delta = reinterpret_cast<float*>(workspace);

@@ -692,7 +692,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (warp == 4) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
-        if (lane == 0 && *abort_flag) atomicExch(P.status, 1);
+        if (lane == 0 && *abort_flag) raise_status(P);
     }
 }
 
@@ -716,8 +716,6 @@ int tc_fused_fwd_small(int dtype, const Geo& g, const void* q, const void* k, co
     if (g.n_extra > 0 && (!encode_extra_map(&mek, ek, bf16, g.B, g.n_extra, g.Hkv, g.D, kKeys, plan.p.split_heads) ||
                           !encode_extra_map(&mev, ev, bf16, g.B, g.n_extra, g.Hkv, g.Dv, kKeys, plan.p.split_heads)))
         return -2;
-    plan.p.status = status_ptr();
-    if (!plan.p.status) return -2;
     if (plan.p.work_q == 0 || g.B == 0) return 0;
     cudaError_t err = cudaSuccess;
     auto launch = [&](auto dh, auto bf, auto inner) {

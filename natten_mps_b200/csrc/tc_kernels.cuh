@@ -34,6 +34,8 @@ unsigned long long tc_launch_count();
 int tc_device_status();
 // Reset the status word of the current device (synchronises); returns a cudaError_t value.
 int tc_clear_status();
+// What the kernels of a device that gave up have written into host memory so far (no synchronisation, no CUDA call).
+int tc_host_status(int device);
 // Enqueue a copy of the current device's status word into `host_word` (pinned host memory) on stream s.
 int tc_status_async(int* host_word, cudaStream_t s);
 // Test hooks: cycle budget of the barrier waits (<= 0 restores the default) and a fault to inject

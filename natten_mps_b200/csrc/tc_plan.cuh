@@ -34,7 +34,8 @@ struct TcParams {
     float scale_log2, scale;
     const int* extents;
     long long ltot;
-    int* status;
+    int* status;           // device word: kernels that start after a failed wait drain at once
+    int* status_host;      // the same for the host (mapped pinned memory), see raise_status
     // Interleaved chunks (forward only): along an axis with il > 1 chunk ci holds the box columns
     // ci, ci + il, ci + 2*il, ... instead of a contiguous block, so that every chunk carries a share of
     // every row's window.  il == 1: blocked (chunk ci = columns [ci*cb, (ci+1)*cb)).
@@ -57,9 +58,19 @@ struct TcParams {
     long long otot;
 };
 
+int* status_host_ptr();   // the current device's word in mapped host memory
 int* status_ptr();   // device address of the library's status word on the current device (tc_status.cu)
 long long debug_wait_budget();   // barrier-wait budget in cycles (test hook; default kWaitBudgetCycles)
 int debug_inject();              // test hook, see TcParams::inject
+
+// A wait ran out: tell the kernels that follow (device word) and the host (its word in mapped memory, so that no
+// copy has to be queued behind every launch).  One thread.
+__device__ __forceinline__ void raise_status(const TcParams& P)
+{
+    atomicExch(P.status, 1);
+    *static_cast<volatile int*>(P.status_host) = 1;
+    __threadfence_system();
+}
 
 // n / d with a precomputed multiplier; exact while n * d < 2^32 (checked on the host).
 __device__ __forceinline__ unsigned fast_div(unsigned n, unsigned mul) { return mul ? __umulhi(n, mul) : n; }
@@ -453,7 +464,9 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
     p.ltot = g.ltot;
     p.wait_budget = debug_wait_budget();
     p.inject = debug_inject();
-    return true;
+    p.status = status_ptr();
+    p.status_host = status_host_ptr();
+    return p.status && p.status_host;
 }
 
 // 5-D map over [B, X0, X1, X2, heads*D] (innermost first in the arrays below).

@@ -368,7 +368,7 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     if (warp == 8) {
         tc_fence_after();
         tmem_dealloc(tmem, 128);
-        if (lane == 0 && *abort_flag) atomicExch(P.status, 1);
+        if (lane == 0 && *abort_flag) raise_status(P);
     }
 }
 
@@ -628,7 +628,7 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
     if (warp == 8) {
         tc_fence_after();
         tmem_dealloc(tmem, SM::kTmemCols);
-        if (lane == 0 && *abort_flag) atomicExch(P.status, 1);
+        if (lane == 0 && *abort_flag) raise_status(P);
     }
 }
 
@@ -894,7 +894,7 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     if (warp == 8) {
         tc_fence_after();
         tmem_dealloc(tmem, SM::kTmemCols);
-        if (lane == 0 && *abort_flag) atomicExch(P.status, 1);
+        if (lane == 0 && *abort_flag) raise_status(P);
     }
 }
 
@@ -953,8 +953,6 @@ int tc_scores(int dtype, const Geo& g, const void* x, const long long xs[3], con
     if (!encode_map(&mx, x, bf16, plan.p, g.Hq, g.D, xs, plan.box_q, /*query_lattice=*/true) ||
         !encode_map(&my, y, bf16, plan.p, g.Hkv, g.D, ys, plan.box_kv))
         return -2;
-    plan.p.status = status_ptr();
-    if (!plan.p.status) return -2;
     if (plan.p.work_q == 0) return 0;
     if (g.D == 64)
         return bf16 ? launch_scores<64, true>(plan, mx, my, g, out, scale, neg_inf, s, rpb, rpb_table)
@@ -986,8 +984,6 @@ int tc_apply(int dtype, const Geo& g, const void* w, const void* y, const long l
     const bool bf16 = dtype == 2;
     CUtensorMap my;
     if (!encode_map(&my, y, bf16, plan.p, g.Hkv, g.D, ys, plan.box_kv)) return -2;
-    plan.p.status = status_ptr();
-    if (!plan.p.status) return -2;
     if (plan.p.work_q == 0) return 0;
     if (g.D == 64)
         return bf16 ? launch_apply<64, true>(plan, my, g, w, out, scale, out_by_position, s)
@@ -1014,8 +1010,6 @@ int tc_gather(int dtype, const Geo& g, const void* w, const void* x, const long 
     const bool bf16 = dtype == 2;
     CUtensorMap mx;
     if (!encode_map(&mx, x, bf16, plan.p, g.Hq, g.D, xs, plan.box_kv)) return -2;
-    plan.p.status = status_ptr();
-    if (!plan.p.status) return -2;
     if (plan.p.work_kv == 0) return 0;
     if (g.D == 64)
         return bf16 ? launch_gather<64, true>(plan, mx, g, w, dst, scale, s) : launch_gather<64, false>(plan, mx, g, w, dst, scale, s);

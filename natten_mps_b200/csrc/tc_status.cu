@@ -17,6 +17,7 @@ __device__ int g_tc_status = 0;
 namespace {
 std::mutex g_status_mutex;
 int* g_status_addr[64] = {nullptr};
+std::atomic<int*> g_status_host[64] = {};    // pinned, mapped: a kernel that gives up writes it itself
 std::atomic<long long> g_wait_budget{tc::kWaitBudgetCycles};
 std::atomic<int> g_inject{0};
 } // namespace
@@ -36,6 +37,23 @@ int* status_ptr()
     return g_status_addr[dev];
 }
 
+int* status_host_ptr()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    if (int* w = g_status_host[dev].load(std::memory_order_acquire)) return w;
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    int* w = g_status_host[dev].load(std::memory_order_acquire);
+    if (!w) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return nullptr;
+        w = static_cast<int*>(p);
+        *w = 0;
+        g_status_host[dev].store(w, std::memory_order_release);
+    }
+    return w;
+}
+
 long long debug_wait_budget() { return g_wait_budget.load(); }
 int debug_inject() { return g_inject.load(); }
 
@@ -51,6 +69,9 @@ int tc_device_status()
 int tc_clear_status()
 {
     const int zero = 0;
+    int dev = 0;
+    if (cudaDeviceSynchronize() == cudaSuccess && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64)
+        if (int* w = g_status_host[dev].load(std::memory_order_acquire)) *static_cast<volatile int*>(w) = 0;
     return (int)cudaMemcpyToSymbol(g_tc_status, &zero, sizeof(int));
 }
 
@@ -59,6 +80,13 @@ int tc_status_async(int* host_word, cudaStream_t s)
     int* p = tcplan::status_ptr();
     if (!p || !host_word) return (int)cudaErrorInvalidValue;
     return (int)cudaMemcpyAsync(host_word, p, sizeof(int), cudaMemcpyDeviceToHost, s);
+}
+
+int tc_host_status(int device)
+{
+    if (device < 0 || device >= 64) return 0;
+    int* w = g_status_host[device].load(std::memory_order_acquire);
+    return w ? *static_cast<volatile int*>(w) : 0;
 }
 
 void tc_debug_wait(long long budget_cycles, int inject)

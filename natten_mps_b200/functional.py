@@ -18,7 +18,7 @@ from typing import Optional, Tuple, Union
 import torch
 import torch.nn.functional as F
 
-from . import _torch_ops  # noqa: F401  (registers torch.ops.natten_b200.*)
+from ._torch_ops import native      # registers torch.ops.natten_b200.*
 from .utils.params import (
     check_dilation_kernel_vs_input,
     check_kernel_size_vs_input,
@@ -104,8 +104,16 @@ def _global_attention(query, key, value, scale, return_lse, extra_k, extra_v):
     return out, lse.transpose(1, 2).reshape(B, *spatial, Hq)
 
 
+# Every entry point first hands its arguments to the native parser, which checks them, calls the operator and
+# returns its result -- or NotImplemented for anything out of the ordinary.  What follows here then raises the
+# error, serves the rare form, or (under the compiler) is what gets traced.
 def _na(rank, query, key, value, kernel_size, stride, dilation, is_causal, scale, return_lse,
         additional_keys, additional_values):
+    if not torch.compiler.is_compiling():
+        result = native.na(rank, query, key, value, kernel_size, stride, dilation, is_causal, scale, return_lse,
+                           additional_keys, additional_values)
+        if result is not NotImplemented:
+            return result
     _check_qkv(query, key, value, rank)
     has_extra = _check_additional(query, key, additional_keys, additional_values)
     ks = normalize_kernel_size(kernel_size, rank)
@@ -167,6 +175,10 @@ def na3d(query, key, value, kernel_size: IntOrTuple, stride: IntOrTuple = 1,
 # split ops
 # ---------------------------------------------------------------------------
 def _na_qk(rank, query, key, kernel_size, dilation, stride, is_causal, scale):
+    if not torch.compiler.is_compiling():
+        result = native.na_qk(rank, query, key, None, kernel_size, dilation, stride, is_causal, scale)
+        if result is not NotImplemented:
+            return result
     if query.ndim != rank + 3 or key.ndim != rank + 3:
         raise ValueError(f"na{rank}d_qk expects query/key with shape {_LAYOUT[rank]}.")
     if query.shape != key.shape:
@@ -183,6 +195,10 @@ def _na_qk(rank, query, key, kernel_size, dilation, stride, is_causal, scale):
 
 
 def _na_av(rank, attn, value, kernel_size, dilation, stride, is_causal):
+    if not torch.compiler.is_compiling():
+        result = native.na_av(rank, attn, value, kernel_size, dilation, stride, is_causal)
+        if result is not NotImplemented:
+            return result
     names = {1: "[B, L, H, K]", 2: "[B, H, W, heads, K]", 3: "[B, D, H, W, heads, K]"}
     if attn.ndim != rank + 3:
         raise ValueError(f"na{rank}d_av expects attn with shape {names[rank]}.")
@@ -230,26 +246,12 @@ def na3d_qk(query, key, kernel_size: IntOrTuple, dilation: IntOrTuple = 1, *,
     return _na_qk(3, query, key, kernel_size, dilation, stride, is_causal, scale)
 
 
-class _QKRPB(torch.autograd.Function):
-    """Split QK with a relative position bias (``src/natten_mps/compat/v014.py:66-183``)."""
-
-    @staticmethod
-    def forward(ctx, query, key, rpb, ks, dil, scale):
-        from . import _backend
-        ctx.save_for_backward(query, key)
-        ctx.geo = (ks, dil, scale, tuple(rpb.shape), rpb.dtype)
-        return _backend.qk_rpb_forward(query, key, rpb, ks, dil, scale)
-
-    @staticmethod
-    def backward(ctx, grad_logits):
-        from . import _backend
-        query, key = ctx.saved_tensors
-        ks, dil, scale, rpb_shape, rpb_dtype = ctx.geo
-        dq, dk, drpb = _backend.qk_rpb_backward(grad_logits, query, key, rpb_shape, ks, dil, scale)
-        return dq, dk, drpb.to(rpb_dtype), None, None, None
-
-
 def _na_qk_rpb(rank, query, key, rpb, kernel_size, dilation, scale):
+    """Split QK with a relative position bias (``src/natten_mps/compat/v014.py:66-183``)."""
+    if not torch.compiler.is_compiling() and rpb is not None:
+        result = native.na_qk(rank, query, key, rpb, kernel_size, dilation, 1, False, scale)
+        if result is not NotImplemented:
+            return result
     if query.ndim != rank + 3 or key.ndim != rank + 3:
         raise ValueError(f"na{rank}d_qk_rpb expects query/key with shape {_LAYOUT[rank]}.")
     if query.shape != key.shape:
@@ -266,7 +268,7 @@ def _na_qk_rpb(rank, query, key, rpb, kernel_size, dilation, scale):
     want = (query.shape[-2], *[2 * x - 1 for x in ks])
     if tuple(rpb.shape) != want:
         raise ValueError(f"rpb must have shape {list(want)} for {rank}D.")
-    return _QKRPB.apply(query, key, rpb, ks, dil, None if scale is None else float(scale))
+    return torch.ops.natten_b200.na_qk_rpb(query, key, rpb, list(ks), list(dil), None if scale is None else float(scale))
 
 
 def na1d_qk_rpb(query, key, rpb, kernel_size: IntOrTuple, dilation: IntOrTuple = 1, *,
@@ -345,6 +347,11 @@ def _check_sizes(sizes: torch.Tensor, batch: int, max_spatial, ks, rank: int) ->
 
 def _na_varlen(rank, query, key, value, sizes, kernel_size, dilation, scale, additional_keys,
                additional_values):
+    if not torch.compiler.is_compiling():
+        result = native.na_varlen(rank, query, key, value, sizes, kernel_size, dilation, scale, additional_keys,
+                                  additional_values)
+        if result is not NotImplemented:
+            return result
     if query.ndim != rank + 3 or key.ndim != rank + 3 or value.ndim != rank + 3:
         raise ValueError(f"na{rank}d_varlen expects query/key/value with shape {_LAYOUT[rank]}.")
     if query.shape[:-2] != key.shape[:-2] or key.shape != value.shape or query.shape[-1] != key.shape[-1] \

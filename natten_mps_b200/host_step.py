@@ -192,8 +192,6 @@ class HostStep:
                                       _cabi.ptr(lse), _cabi.ptr(go), None, _cabi.ptr(dq), _cabi.ptr(dk), _cabi.ptr(dv),
                                       None, None, _cabi.ptr(self._ws), self._ws.numel(), stream)
             _cabi.check(rc, "natten_fused_bwd")
-        if i == len(self._params) - 1:         # once per step: status word -> pinned host word
-            _cabi.track_status(q)
 
     def wait(self):
         """Make the caller's current stream wait for everything queued so far (the copies out included)."""

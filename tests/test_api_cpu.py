@@ -193,3 +193,16 @@ def test_module_state_dict_names_and_shapes_match_the_reference_fixture():
         state = {k[2:]: torch.as_tensor(v) for k, v in a.items() if k.startswith("p.")}
         assert {k: tuple(v.shape) for k, v in state.items()} == {k: tuple(v.shape) for k, v in m.state_dict().items()}
         m.load_state_dict(state)
+
+
+@pytest.mark.parametrize("kernel,native", [(3, True), ((3, 5), True), ([3, 5], True), (type("I", (int,), {})(3), False)],
+                         ids=["int", "tuple", "list", "int_subclass"])
+def test_native_parser_serves_plain_arguments_and_leaves_the_rest(kernel, native):
+    from natten_mps_b200._torch_ops import native as N
+    q = _meta(1, 9, 10, 2, 16)
+    got = N.na(2, q, q, q, kernel, 1, 1, False, None, False, None, None)
+    assert (got is not NotImplemented) == native
+    assert F.na2d(q, q, q, kernel).shape == q.shape          # the Python path serves what the parser declined
+    for bad in (dict(stride=6), dict(dilation=4), dict(is_causal=1), dict(kernel_size=(3, 3, 3)), dict(kernel_size=0)):
+        a = {**dict(kernel_size=5, stride=1, dilation=1, is_causal=False), **bad}
+        assert N.na(2, q, q, q, a["kernel_size"], a["stride"], a["dilation"], a["is_causal"], None, False, None, None) is NotImplemented
