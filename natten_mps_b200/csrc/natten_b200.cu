@@ -103,6 +103,10 @@ int natten_fused_fwd(const natten_params_t* p, const void* q, const void* k, con
     }
     if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
     t_last_path = NATTEN_PATH_SIMT;
+    if (!(p->flags & NATTEN_FLAG_FORCE_SIMT)) {
+        rc = fma_fused_fwd(p->dtype, g, q, k, v, out, lse, s);
+        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+    }
     return from_cuda(simt_fused_fwd(p->dtype, g, q, k, v, extra_k, extra_v, out, lse, s));
 }
 
@@ -143,6 +147,10 @@ int natten_fused_bwd(const natten_params_t* p, const void* q, const void* k, con
     }
     if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
     t_last_path = NATTEN_PATH_SIMT;
+    if (!(p->flags & NATTEN_FLAG_FORCE_SIMT)) {
+        rc = fma_fused_bwd(p->dtype, g, q, k, v, out, lse, dout, dlse, dq, dk, dv, workspace, s);
+        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+    }
     return from_cuda(simt_fused_bwd(p->dtype, g, q, k, v, extra_k, extra_v, out, lse, dout, dlse, dq, dk,
                                     dv, dextra_k, dextra_v, workspace, s));
 }

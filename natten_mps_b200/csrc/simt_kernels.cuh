@@ -23,6 +23,11 @@ cudaError_t simt_qk_bwd(int dtype, const Geo& g, const void* q, const void* k, c
 cudaError_t simt_av_fwd(int dtype, const Geo& g, const void* attn, const void* v, void* out, cudaStream_t s);
 cudaError_t simt_av_bwd(int dtype, const Geo& g, const void* attn, const void* v, const void* dout,
                         void* dattn, void* dv, cudaStream_t s);
+// Window kernels in fp32 arithmetic (win_fma.cu): head dims 32 / 64 / 128, unit stride, no additional tokens, no
+// per-sample extents, rows readable 16 bytes at a time; -2 for anything else.  The workspace starts with delta.
+int fma_fused_fwd(int dtype, const Geo& g, const void* q, const void* k, const void* v, void* out, void* lse, cudaStream_t s);
+int fma_fused_bwd(int dtype, const Geo& g, const void* q, const void* k, const void* v, const void* out, const void* lse,
+                  const void* dout, const void* dlse, void* dq, void* dk, void* dv, void* workspace, cudaStream_t s);
 unsigned long long simt_launch_count();
 void simt_count_launch(int n);
 

@@ -65,7 +65,8 @@ int debug_inject();              // test hook, see TcParams::inject
 
 // A wait ran out: tell the kernels that follow (device word) and the host (its word in mapped memory, so that no
 // copy has to be queued behind every launch).  One thread.
-__device__ __forceinline__ void raise_status(const TcParams& P)
+template <typename Params>
+__device__ __forceinline__ void raise_status(const Params& P)
 {
     atomicExch(P.status, 1);
     *static_cast<volatile int*>(P.status_host) = 1;

@@ -1,0 +1,685 @@
+// Window kernels in full fp32 arithmetic: fused attention for float32 tensors and the split operators for every type
+// whose head dim the tensor-core kernels do not take (sums always in fp32; 16-bit tensors are widened when they are
+// staged).
+//
+// Bound: the multiply-adds and the shared-memory reads that feed them.  A warp of the general SIMT kernels reads a whole
+// row from memory for every (query, key) pair; here four queries share every key row that is read, from shared memory:
+//   * a query (or key) row is spread over LPQ = D / 8 lanes, 8 channels each; a group of LPQ lanes holds FOUR rows that
+//     are neighbours along a1 (rank 1: along a2), 32 / LPQ groups sit next to each other along a2;
+//   * the column box of the CTA's rows is staged in shared memory in chunks, fp32, 16-byte pieces swizzled so that the
+//     eight lanes of a phase touch different banks;
+//   * per column a lane reads its 8 channels (two 16-byte reads), multiplies them with its four rows (packed fp32 pairs),
+//     the four partial sums are reduced over the group so that lane i ends up with row i's (3 shuffles for 4 lanes), it
+//     alone does the scalar work of that row (mask, exponential), and four shuffles hand the results back.
+// A pass over the columns of K = 7 x 7 costs 23 shared-memory cycles for 32 pairs of which 70 % are needed.
+//
+// Rows are queries and columns keys, or the other way round (key side: dK, dV; columns = the queries that attend to a key,
+// a contiguous range per axis).  Fixed order of summation everywhere, no atomics.
+#include "simt_kernels.cuh"
+
+#include "tc_kernels.cuh"
+#include "tc_plan.cuh"
+
+#include <algorithm>
+#include <type_traits>
+
+namespace natten {
+namespace {
+
+using tcplan::fast_div;
+using tcplan::fast_exp2;
+using tcplan::fma2;
+using tcplan::hi_of;
+using tcplan::inverse_range;
+using tcplan::kernel_axis_ok;
+using tcplan::lo_of;
+using tcplan::mul2;
+using tcplan::pack2;
+
+constexpr int kWarpsF = 4;
+constexpr int kThreadsF = 32 * kWarpsF;
+constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+
+// A tensor as the kernels see it: element strides of batch, token, head.
+struct TensorF {
+    const void* p;
+    long long bs, ts, hs;
+};
+
+struct FmaParams {
+    int L[3], K[3], dil[3], causal[3];
+    int tile1, tile2, ww;                // rows of a CTA along a1 and a2; warps along a2 (the others along a1)
+    int ntile[3];                        // CTA tiles per axis and dilation group
+    int chunk_rows, chunk_cols;          // columns staged at a time
+    int rank, B, Hq, Hkv, group;
+    long long ltot;
+    int ktot;
+    float scale, scale_log2;
+    TensorF row1, row2, col1, col2;      // row tensors (queries | keys), column tensors (keys | queries)
+};
+
+template <bool kKeySide>
+__device__ __forceinline__ void range_of(const FmaParams& P, int a, int x, int Lp, int& f, int& e, bool exact = true)
+{
+    if (kKeySide) {
+        int lo, hi;
+        inverse_range(x, Lp, P.K[a], P.causal[a], lo, hi, exact);
+        f = lo;
+        e = hi + 1;
+    } else {
+        const int first = P.causal[a] ? x - (P.K[a] - 1) : window_start(x, Lp, P.K[a], 1);
+        f = first > 0 ? first : 0;
+        e = first + P.K[a] < Lp ? first + P.K[a] : Lp;
+    }
+}
+
+// A CTA's rows and column box.
+struct TileF {
+    int rg[3], o[3], Lp[3], lo[3], n[3];
+};
+template <bool kKeySide>
+__device__ __forceinline__ bool tile_of(const FmaParams& P, unsigned bx, TileF& T)
+{
+    const int tile[3] = {1, P.tile1, P.tile2};
+    bool active = true;
+#pragma unroll
+    for (int a = 2; a >= 0; --a) {
+        const unsigned q = bx / (unsigned)P.ntile[a];
+        T.o[a] = (int)(bx - q * P.ntile[a]) * tile[a];
+        bx = q;
+    }
+#pragma unroll
+    for (int a = 2; a >= 0; --a) {
+        const unsigned q = bx / (unsigned)P.dil[a];
+        T.rg[a] = (int)(bx - q * P.dil[a]);
+        bx = q;
+        T.Lp[a] = (P.L[a] - T.rg[a] + P.dil[a] - 1) / P.dil[a];
+        if (T.o[a] >= T.Lp[a]) active = false;
+    }
+    if (!active) return false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int last = min(T.o[a] + tile[a], T.Lp[a]) - 1;
+        int t, hi;
+        range_of<kKeySide>(P, a, T.o[a], T.Lp[a], T.lo[a], t, false);
+        range_of<kKeySide>(P, a, last, T.Lp[a], t, hi, false);
+        T.n[a] = hi - T.lo[a];
+    }
+    return true;
+}
+__device__ __forceinline__ long long flat_of(const FmaParams& P, const TileF& T, int x0, int x1, int x2)
+{
+    return ((long long)(T.rg[0] + P.dil[0] * x0) * P.L[1] + (T.rg[1] + P.dil[1] * x1)) * P.L[2] + (T.rg[2] + P.dil[2] * x2);
+}
+
+// Eight values of a tensor row as four packed pairs.
+template <typename T> __device__ __forceinline__ void load8(const T* p, uint64_t (&x)[4])
+{
+    if constexpr (std::is_same<T, float>::value) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(p), b = *reinterpret_cast<const ulonglong2*>(p + 4);
+        x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+    } else {
+        const uint4 r = *reinterpret_cast<const uint4*>(p);
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float2 f;
+            if constexpr (std::is_same<T, __half>::value) f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+            else f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+            x[i] = pack2(f.x, f.y);
+        }
+    }
+}
+template <typename T> __device__ __forceinline__ void store8(T* p, const uint64_t (&x)[4])
+{
+    if constexpr (std::is_same<T, float>::value) {
+        *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(x[0], x[1]);
+        *reinterpret_cast<ulonglong2*>(p + 4) = make_ulonglong2(x[2], x[3]);
+    } else {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = tcplan::cvt_pack<std::is_same<T, __nv_bfloat16>::value>(lo_of(x[i]), hi_of(x[i]));
+        *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+template <typename T> __device__ __forceinline__ float widen(T v)
+{
+    if constexpr (std::is_same<T, float>::value) return v;
+    else if constexpr (std::is_same<T, __half>::value) return __half2float(v);
+    else return __bfloat162float(v);
+}
+template <typename T> __device__ __forceinline__ T narrow(float v)
+{
+    if constexpr (std::is_same<T, float>::value) return v;
+    else if constexpr (std::is_same<T, __half>::value) return __float2half_rn(v);
+    else return __float2bfloat16_rn(v);
+}
+
+// Lane layout and shared-memory layout for head dim D.
+template <int D, bool LINE> struct LaneF {
+    static constexpr int LPQ = D / 8, GP = 32 / LPQ;     // lanes per row, groups of four rows per warp
+    static constexpr int kPieces = D / 4;                // 16-byte pieces of a column
+    // physical piece of logical piece j of the column with chunk-relative index x along a2: neighbouring groups (columns one
+    // apart; rank 1: four) or, for longer rows, the two halves of a 256-byte span read from different halves of the banks
+    static __device__ __forceinline__ int piece(int j, int x) { return D == 32 ? j ^ ((LINE ? x >> 2 : x) & 1) : j ^ ((j >> 3) & 1); }
+};
+
+// Stage columns [y0, y1) x [s0, s1) (box-relative) at a0 position x0 of one tensor: [row][col][D] fp32.
+template <typename T, int D, bool LINE>
+__device__ __forceinline__ void stage_cols(const FmaParams& P, const TileF& Ti, const TensorF& t, int b, int h, int x0, int y0, int y1,
+                                           int s0, int s1, float* dst)
+{
+    using LF = LaneF<D, LINE>;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nc = s1 - s0;
+    const T* base = static_cast<const T*>(t.p) + b * t.bs + h * t.hs;
+    constexpr int V = std::is_same<T, float>::value ? 4 : 8;             // channels per 16-byte load
+    constexpr int kLoads = D / V;
+    for (int y = y0 + warp; y < y1; y += kWarpsF) {
+        const long long pos = flat_of(P, Ti, x0, Ti.lo[1] + y, Ti.lo[2] + s0);
+        const T* src = base + pos * t.ts;
+        float* row = dst + (size_t)(y - y0) * P.chunk_cols * D;
+        for (int i = lane; i < nc * kLoads; i += 32) {
+            const int x = i / kLoads, j = i % kLoads;
+            const T* s = src + (long long)x * P.dil[2] * t.ts + V * j;
+            float* d = row + x * D;
+            if constexpr (V == 4) {
+                const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(d + 4 * LF::piece(j, x)));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(s) : "memory");
+            } else {
+                uint64_t v[4];
+                load8<T>(s, v);
+                *reinterpret_cast<ulonglong2*>(d + 4 * LF::piece(2 * j, x)) = make_ulonglong2(v[0], v[1]);
+                *reinterpret_cast<ulonglong2*>(d + 4 * LF::piece(2 * j + 1, x)) = make_ulonglong2(v[2], v[3]);
+            }
+        }
+    }
+}
+__device__ __forceinline__ void staged()
+{
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+}
+
+// This lane's 8 channels (logical pieces 2c, 2c + 1) of staged column x of a row.
+template <int D, bool LINE>
+__device__ __forceinline__ void read_col(const float* row, int x, int c, uint64_t (&v)[4])
+{
+    using LF = LaneF<D, LINE>;
+    const float* p = row + x * D;
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(p + 4 * LF::piece(2 * c, x));
+    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(p + 4 * LF::piece(2 * c + 1, x));
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ float dot8(const uint64_t (&a)[4], const uint64_t (&b)[4])
+{
+    uint64_t s = mul2(a[0], b[0]);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) s = fma2(a[i], b[i], s);
+    return lo_of(s) + hi_of(s);
+}
+// Partial sums of four rows over the group's lanes -> lane c gets the total of row c & 3.
+template <int LPQ> __device__ __forceinline__ float reduce4(float s0, float s1, float s2, float s3, int c)
+{
+    const bool b0 = c & 1, b1 = c & 2;
+    float k0 = b0 ? s1 : s0, k1 = b0 ? s3 : s2;
+    k0 += __shfl_xor_sync(0xffffffffu, b0 ? s0 : s1, 1);
+    k1 += __shfl_xor_sync(0xffffffffu, b0 ? s2 : s3, 1);
+    float k = b1 ? k1 : k0;
+    k += __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2);
+#pragma unroll
+    for (int m = 4; m < LPQ; m <<= 1) k += __shfl_xor_sync(0xffffffffu, k, m);
+    return k;
+}
+// The value of row j, from the lane that has it.
+__device__ __forceinline__ float row_value(float v, int lane, int c, int j) { return __shfl_sync(0xffffffffu, v, (lane - c) | j); }
+__device__ __forceinline__ uint64_t twice(float v) { return pack2(v, v); }
+
+// A lane's view of its group's four rows.
+template <int D, bool LINE, bool kKeySide> struct RowsF {
+    using LF = LaneF<D, LINE>;
+    int lane, c, g, x1, x2;              // first row of the group
+    int f1, f2;                          // own row (c & 3): its columns, box-relative ...
+    unsigned n1, n2;
+    int r0, r1, c0, c1;                  // the group's: rows of columns (warp-uniform) and columns; empty: none
+    int nmax;                            // most columns of any group of the warp
+
+    __device__ __forceinline__ void init(const FmaParams& P, const TileF& T)
+    {
+        const int warp = threadIdx.x >> 5;
+        lane = threadIdx.x & 31;
+        c = lane % LF::LPQ;
+        g = lane / LF::LPQ;
+        const int wx = warp % P.ww, wy = warp / P.ww;
+        x1 = T.o[1] + (LINE ? 0 : 4 * wy);
+        x2 = T.o[2] + (LINE ? 4 : 1) * (LF::GP * wx + g);
+        const int j = c & 3;
+        f1 = f2 = 0;
+        n1 = n2 = 0u;
+        if (exists(T, j)) {
+            int e;
+            range_of<kKeySide>(P, 1, row1(j), T.Lp[1], f1, e);
+            n1 = e > f1 ? (unsigned)(e - f1) : 0u;
+            range_of<kKeySide>(P, 2, row2(j), T.Lp[2], f2, e);
+            n2 = e > f2 ? (unsigned)(e - f2) : 0u;
+            f1 -= T.lo[1];
+            f2 -= T.lo[2];
+        }
+        // unions over the rows that exist (bounds never decrease with the row)
+        r0 = r1 = c0 = c1 = 0;
+        if (x1 < T.Lp[1]) {
+            int t;
+            range_of<kKeySide>(P, 1, x1, T.Lp[1], r0, t, false);
+            range_of<kKeySide>(P, 1, min(row1(3), T.Lp[1] - 1), T.Lp[1], t, r1, false);
+            r0 -= T.lo[1];
+            r1 -= T.lo[1];
+        }
+        if (x2 < T.Lp[2]) {
+            int t;
+            range_of<kKeySide>(P, 2, x2, T.Lp[2], c0, t, false);
+            range_of<kKeySide>(P, 2, min(row2(3), T.Lp[2] - 1), T.Lp[2], t, c1, false);
+            c0 -= T.lo[2];
+            c1 -= T.lo[2];
+        }
+    }
+    __device__ __forceinline__ int row1(int j) const { return x1 + (LINE ? 0 : j); }
+    __device__ __forceinline__ int row2(int j) const { return x2 + (LINE ? j : 0); }
+    __device__ __forceinline__ bool exists(const TileF& T, int j) const { return row1(j) < T.Lp[1] && row2(j) < T.Lp[2]; }
+    __device__ __forceinline__ long long flat(const FmaParams& P, const TileF& T, int j) const { return flat_of(P, T, T.o[0], row1(j), row2(j)); }
+
+    // this lane's 8 channels of the four rows (zero where there is no row)
+    template <typename T> __device__ __forceinline__ void load_rows(const FmaParams& P, const TileF& Ti, const TensorF& t, int b, int h,
+                                                                    uint64_t (&x)[4][4]) const
+    {
+        const T* base = static_cast<const T*>(t.p) + b * t.bs + h * t.hs + 8 * c;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[j][i] = 0ull;
+            if (exists(Ti, j)) load8<T>(base + flat(P, Ti, j) * t.ts, x[j]);
+        }
+    }
+    // Walk the staged chunk [y0, y1) x [s0, s1): body(row of shared memory columns, chunk-relative column, own row's column valid,
+    // box-relative row and column)
+    template <typename F> __device__ __forceinline__ void walk(int y0, int y1, int s0, int s1, F&& body) const
+    {
+        const int a = max(c0, s0), n = min(c1, s1) - a;
+        int most = n > 0 ? n : 0;
+#pragma unroll
+        for (int m = 16; m >= LF::LPQ; m >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, m));
+        const int from = max(r0, y0), to = min(r1, y1);
+        for (int y = from; y < to; ++y) {
+            const bool row_ok = (unsigned)(y - f1) < n1;
+#pragma unroll 2
+            for (int t = 0; t < most; ++t) {
+                const int x = a + t;
+                const bool ok = row_ok && t < n && (unsigned)(x - f2) < n2;
+                body(y - y0, min(x, s1 - 1) - s0, ok, y, x);
+            }
+        }
+    }
+};
+
+// Walks the CTA's column box in chunks: before(x0, y0, y1, s0, s1) stages one, then every warp visits it.
+template <typename Stage, typename Visit>
+__device__ __forceinline__ void for_chunks(const FmaParams& P, const TileF& T, Stage&& stage, Visit&& visit)
+{
+    for (int i0 = 0; i0 < T.n[0]; ++i0)
+        for (int y0 = 0; y0 < T.n[1]; y0 += P.chunk_rows)
+            for (int s0 = 0; s0 < T.n[2]; s0 += P.chunk_cols) {
+                const int y1 = min(y0 + P.chunk_rows, T.n[1]), s1 = min(s0 + P.chunk_cols, T.n[2]);
+                __syncthreads();
+                stage(T.lo[0] + i0, y0, y1, s0, s1);
+                staged();
+                visit(T.lo[0] + i0, y0, y1, s0, s1);
+            }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// fused forward.  Row i's stabiliser lives in lane i of its group: the first score it meets; moved (everything
+// accumulated so far is rescaled, a warp-uniform branch) only when a score exceeds it by 2^30.
+// ---------------------------------------------------------------------------------------------------------------
+template <typename T, int D, bool LINE>
+__global__ void __launch_bounds__(kThreadsF, 4)
+fma_fwd_kernel(const __grid_constant__ FmaParams P, T* __restrict__ out, float* __restrict__ lse)
+{
+    using LF = LaneF<D, LINE>;
+    extern __shared__ __align__(16) float sm[];
+    const int h = blockIdx.y, b = blockIdx.z, hk = h / P.group;
+    TileF Ti;
+    if (!tile_of<false>(P, blockIdx.x, Ti)) return;
+    RowsF<D, LINE, false> R;
+    R.init(P, Ti);
+    uint64_t q[4][4], acc[4][4];
+    R.template load_rows<T>(P, Ti, P.row1, b, h, q);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
+    float m = -INFINITY, l = 0.f;
+    float* vs = sm + P.chunk_rows * P.chunk_cols * D;
+    for_chunks(P, Ti,
+        [&](int x0, int y0, int y1, int s0, int s1) {
+            stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm);
+            stage_cols<T, D, LINE>(P, Ti, P.col2, b, hk, x0, y0, y1, s0, s1, vs);
+        },
+        [&](int, int y0, int y1, int s0, int s1) {
+            R.walk(y0, y1, s0, s1, [&](int y, int x, bool ok, int, int) {
+                const int row = y * P.chunk_cols * D;
+                uint64_t k[4], v[4];
+                read_col<D, LINE>(sm + row, x, R.c, k);
+                const float s = reduce4<LF::LPQ>(dot8(q[0], k), dot8(q[1], k), dot8(q[2], k), dot8(q[3], k), R.c) * P.scale_log2;
+                read_col<D, LINE>(vs + row, x, R.c, v);
+                const bool grow = ok && s > m + 30.f;
+                if (__any_sync(0xffffffffu, grow)) {
+                    const float fac = grow ? fast_exp2(m - s) : 1.f;
+                    if (grow) m = s;
+                    l *= fac;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint64_t f2 = twice(row_value(fac, R.lane, R.c, j));
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[j][i] = mul2(acc[j][i], f2);
+                    }
+                }
+                const float p = ok ? fast_exp2(s - m) : 0.f;
+                l += p;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint64_t p2 = twice(row_value(p, R.lane, R.c, j));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[j][i] = fma2(p2, v[i], acc[j][i]);
+                }
+            });
+        });
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint64_t f2 = twice(row_value(inv, R.lane, R.c, j));
+        if (!R.exists(Ti, j)) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] = mul2(acc[j][i], f2);
+        store8<T>(out + (((long long)b * P.ltot + R.flat(P, Ti, j)) * P.Hq + h) * D + 8 * R.c, acc[j]);
+    }
+    if (R.c < 4 && R.exists(Ti, R.c))
+        lse[((long long)b * P.ltot + R.flat(P, Ti, R.c)) * P.Hq + h] = l > 0.f ? (m + log2f(l)) * kLn2 : 0.f;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// fused backward, query side: dQ, and delta = rowsum(out * dout) - dlse for the key side
+// ---------------------------------------------------------------------------------------------------------------
+template <typename T, int D, bool LINE>
+__global__ void __launch_bounds__(kThreadsF, 3)
+fma_bwd_q_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ out, const float* __restrict__ lse,
+                 const float* __restrict__ dlse, float* __restrict__ delta, T* __restrict__ dq)
+{
+    using LF = LaneF<D, LINE>;
+    extern __shared__ __align__(16) float sm[];
+    const int h = blockIdx.y, b = blockIdx.z, hk = h / P.group;
+    TileF Ti;
+    if (!tile_of<false>(P, blockIdx.x, Ti)) return;
+    RowsF<D, LINE, false> R;
+    R.init(P, Ti);
+    uint64_t q[4][4], go[4][4], acc[4][4];
+    float lse2 = 0.f, dl = 0.f;
+    {
+        const TensorF ot{out, P.ltot * P.Hq * D, (long long)P.Hq * D, D};
+        R.template load_rows<T>(P, Ti, ot, b, h, q);
+        R.template load_rows<T>(P, Ti, P.row2, b, h, go);
+        dl = reduce4<LF::LPQ>(dot8(q[0], go[0]), dot8(q[1], go[1]), dot8(q[2], go[2]), dot8(q[3], go[3]), R.c);
+        const int j = R.c & 3;
+        if (R.exists(Ti, j)) {
+            const long long row = ((long long)b * P.ltot + R.flat(P, Ti, j)) * P.Hq + h;
+            lse2 = lse[row] * kLog2e;
+            if (dlse) dl -= dlse[row];
+            if (R.c < 4) delta[row] = dl;
+        }
+    }
+    R.template load_rows<T>(P, Ti, P.row1, b, h, q);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
+    float* vs = sm + P.chunk_rows * P.chunk_cols * D;
+    for_chunks(P, Ti,
+        [&](int x0, int y0, int y1, int s0, int s1) {
+            stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm);
+            stage_cols<T, D, LINE>(P, Ti, P.col2, b, hk, x0, y0, y1, s0, s1, vs);
+        },
+        [&](int, int y0, int y1, int s0, int s1) {
+            R.walk(y0, y1, s0, s1, [&](int y, int x, bool ok, int, int) {
+                const int row = y * P.chunk_cols * D;
+                uint64_t k[4], v[4];
+                read_col<D, LINE>(sm + row, x, R.c, k);
+                read_col<D, LINE>(vs + row, x, R.c, v);
+                const float s = reduce4<LF::LPQ>(dot8(q[0], k), dot8(q[1], k), dot8(q[2], k), dot8(q[3], k), R.c);
+                const float dp = reduce4<LF::LPQ>(dot8(go[0], v), dot8(go[1], v), dot8(go[2], v), dot8(go[3], v), R.c);
+                const float p = ok ? fast_exp2(fmaf(s, P.scale_log2, -lse2)) : 0.f;
+                const float ds = ok ? p * (dp - dl) * P.scale : 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint64_t d2 = twice(row_value(ds, R.lane, R.c, j));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[j][i] = fma2(d2, k[i], acc[j][i]);
+                }
+            });
+        });
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (R.exists(Ti, j)) store8<T>(dq + (((long long)b * P.ltot + R.flat(P, Ti, j)) * P.Hq + h) * D + 8 * R.c, acc[j]);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// fused backward, key side: dK and dV over the queries that attend to the keys, one query head of the group at a time
+// ---------------------------------------------------------------------------------------------------------------
+template <typename T, int D, bool LINE>
+__global__ void __launch_bounds__(kThreadsF, 2)
+fma_bwd_k_kernel(const __grid_constant__ FmaParams P, const float* __restrict__ lse, const float* __restrict__ delta,
+                 T* __restrict__ dk, T* __restrict__ dv)
+{
+    using LF = LaneF<D, LINE>;
+    extern __shared__ __align__(16) float sm[];
+    const int hk = blockIdx.y, b = blockIdx.z;
+    TileF Ti;
+    if (!tile_of<true>(P, blockIdx.x, Ti)) return;
+    RowsF<D, LINE, true> R;
+    R.init(P, Ti);
+    uint64_t k[4][4], v[4][4], ak[4][4], av[4][4];
+    R.template load_rows<T>(P, Ti, P.row1, b, hk, k);
+    R.template load_rows<T>(P, Ti, P.row2, b, hk, v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ak[j][i] = av[j][i] = 0ull;
+    const int cells = P.chunk_rows * P.chunk_cols;
+    float* gs = sm + cells * D;
+    float2* stats = reinterpret_cast<float2*>(gs + cells * D);       // lse * log2(e), delta of the chunk's queries
+    for (int h = hk * P.group; h < (hk + 1) * P.group; ++h)
+        for_chunks(P, Ti,
+            [&](int x0, int y0, int y1, int s0, int s1) {
+                stage_cols<T, D, LINE>(P, Ti, P.col1, b, h, x0, y0, y1, s0, s1, sm);
+                stage_cols<T, D, LINE>(P, Ti, P.col2, b, h, x0, y0, y1, s0, s1, gs);
+                for (int y = y0 + (threadIdx.x >> 5); y < y1; y += kWarpsF)
+                    for (int x = s0 + (threadIdx.x & 31); x < s1; x += 32) {
+                        const long long row = ((long long)b * P.ltot + flat_of(P, Ti, x0, Ti.lo[1] + y, Ti.lo[2] + x)) * P.Hq + h;
+                        stats[(y - y0) * P.chunk_cols + (x - s0)] = make_float2(lse[row] * kLog2e, delta[row]);
+                    }
+            },
+            [&](int, int y0, int y1, int s0, int s1) {
+                R.walk(y0, y1, s0, s1, [&](int y, int x, bool ok, int, int) {
+                    const int row = y * P.chunk_cols * D;
+                    uint64_t q[4], go[4];
+                    read_col<D, LINE>(sm + row, x, R.c, q);
+                    read_col<D, LINE>(gs + row, x, R.c, go);
+                    const float2 st = stats[y * P.chunk_cols + x];
+                    const float s = reduce4<LF::LPQ>(dot8(k[0], q), dot8(k[1], q), dot8(k[2], q), dot8(k[3], q), R.c);
+                    const float dp = reduce4<LF::LPQ>(dot8(v[0], go), dot8(v[1], go), dot8(v[2], go), dot8(v[3], go), R.c);
+                    const float p = ok ? fast_exp2(fmaf(s, P.scale_log2, -st.x)) : 0.f;
+                    const float ds = ok ? p * (dp - st.y) * P.scale : 0.f;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint64_t p2 = twice(row_value(p, R.lane, R.c, j)), d2 = twice(row_value(ds, R.lane, R.c, j));
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            av[j][i] = fma2(p2, go[i], av[j][i]);
+                            ak[j][i] = fma2(d2, q[i], ak[j][i]);
+                        }
+                    }
+                });
+            });
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (R.exists(Ti, j)) {
+            const long long o = (((long long)b * P.ltot + R.flat(P, Ti, j)) * P.Hkv + hk) * D + 8 * R.c;
+            store8<T>(dk + o, ak[j]);
+            store8<T>(dv + o, av[j]);
+        }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------------------------
+// Rows of a warp are 4 x (256 / D) (rank 1: one row of 1024 / D).  `tensors`: column tensors staged side by side,
+// `extra`: further shared-memory bytes per staged column.
+bool make_fma(const Geo& g, FmaParams& p, bool key_side, int tensors, int extra, size_t fixed, dim3& grid, size_t& smem)
+{
+    if ((g.D != 32 && g.D != 64 && g.D != 128) || g.n_extra || g.extents || g.B == 0) return false;
+    const int pad = 3 - g.rank;
+    for (int a = 0; a < 3; ++a) {
+        const int s = a - pad;
+        p.L[a] = s >= 0 ? g.L[s] : 1;
+        p.K[a] = s >= 0 ? g.K[s] : 1;
+        p.dil[a] = s >= 0 ? g.dil[s] : 1;
+        p.causal[a] = s >= 0 ? g.causal[s] : 0;
+        if (s >= 0 && (g.st[s] != 1 || !kernel_axis_ok(g, s))) return false;
+    }
+    p.rank = g.rank; p.B = g.B; p.Hq = g.Hq; p.Hkv = g.Hkv; p.group = g.group;
+    p.ltot = g.ltot; p.ktot = g.ktot;
+    p.scale = (float)g.scale;
+    p.scale_log2 = (float)(g.scale * 1.4426950408889634);
+    const int gp = 256 / g.D, inverse = key_side ? 1 : 0;
+    if (g.rank == 1) {
+        p.ww = kWarpsF;
+        p.tile1 = 1;
+        p.tile2 = 4 * gp * kWarpsF;
+    } else {
+        // warps side by side or stacked: fewest columns staged and rows of columns walked over the whole grid
+        const int lp1 = (p.L[1] + p.dil[1] - 1) / p.dil[1], lp2 = (p.L[2] + p.dil[2] - 1) / p.dil[2];
+        long long best = -1;
+        for (int ww = kWarpsF; ww >= 1; ww /= 2) {
+            const int t1 = 4 * (kWarpsF / ww), t2 = gp * ww;
+            const long long n = (long long)((lp1 + t1 - 1) / t1) * ((lp2 + t2 - 1) / t2) *
+                                ((t1 - 1 + p.K[1]) * (long long)(t2 - 1 + p.K[2]) + 2LL * kWarpsF * (3 + p.K[1]) * p.K[2]);
+            if (best < 0 || n < best) { best = n; p.ww = ww; p.tile1 = t1; p.tile2 = t2; }
+        }
+    }
+    long long tiles = 1;
+    const int tile[3] = {1, p.tile1, p.tile2};
+    for (int a = 0; a < 3; ++a) {
+        p.ntile[a] = ((p.L[a] + p.dil[a] - 1) / p.dil[a] + tile[a] - 1) / tile[a];
+        tiles *= (long long)p.ntile[a] * p.dil[a];
+    }
+    const int heads = key_side ? g.Hkv : g.Hq;
+    if (tiles > 0x7fffffffll || heads > 65535 || g.B > 65535) return false;
+    grid = dim3((unsigned)tiles, (unsigned)heads, (unsigned)g.B);
+    // Chunk: whole rows of the box where two of them fit in 40 KB (four CTAs share an SM's 227), else pieces of one row.
+    const int cell = g.D * 4 * tensors + extra, budget = 40 * 1024;
+    auto longest = [&](int a) {                              // of a CTA's box along axis a, clamped edges included
+        const int lp = (p.L[a] + p.dil[a] - 1) / p.dil[a];
+        return std::min(lp, tile[a] - 1 + p.K[a] + inverse * (p.causal[a] ? 0 : p.K[a]));
+    };
+    p.chunk_cols = longest(2);
+    if (p.chunk_cols * cell > budget / 2) p.chunk_cols = std::max(8, std::min(p.chunk_cols, budget / cell / 8 * 8));
+    p.chunk_rows = std::max(1, std::min(longest(1), budget / (p.chunk_cols * cell)));
+    smem = (size_t)p.chunk_rows * p.chunk_cols * cell + fixed;
+    return smem <= kMaxDynamicSmem;
+}
+
+// Rows readable 16 bytes at a time.
+bool vec_rows(const void* p, const long long s[3], int elt)
+{
+    return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && s[0] * elt % 16 == 0 && s[1] * elt % 16 == 0 && s[2] * elt % 16 == 0;
+}
+TensorF tensor_of(const void* p, const long long s[3]) { return TensorF{p, s[0], s[1], s[2]}; }
+TensorF dense(const void* p, const Geo& g, int heads, int D)
+{
+    return TensorF{p, g.ltot * heads * (long long)D, (long long)heads * D, D};
+}
+template <typename F> void with_dim(int D, F&& f)
+{
+    if (D == 32) f(std::integral_constant<int, 32>{});
+    else if (D == 64) f(std::integral_constant<int, 64>{});
+    else f(std::integral_constant<int, 128>{});
+}
+template <typename F> void with_line(const Geo& g, F&& f)
+{
+    if (g.rank == 1) f(std::true_type{});
+    else f(std::false_type{});
+}
+template <typename K> cudaError_t prepare_kernel(K kernel, size_t smem)
+{
+    return smem > 48 * 1024 ? ensure_dynamic_smem((const void*)kernel, kMaxDynamicSmem) : cudaSuccess;
+}
+
+} // namespace
+
+int fma_fused_fwd(int dtype, const Geo& g, const void* q, const void* k, const void* v, void* out, void* lse, cudaStream_t s)
+{
+    if (dtype != 0 || g.Dv != g.D || !vec_rows(q, g.qs, 4) || !vec_rows(k, g.ks, 4) || !vec_rows(v, g.vs, 4) ||
+        (reinterpret_cast<uintptr_t>(out) & 15u))
+        return -2;
+    FmaParams p;
+    dim3 grid;
+    size_t smem;
+    if (!make_fma(g, p, false, 2, 0, 0, grid, smem)) return -2;
+    p.row1 = tensor_of(q, g.qs);
+    p.col1 = tensor_of(k, g.ks);
+    p.col2 = tensor_of(v, g.vs);
+    cudaError_t err = cudaSuccess;
+    with_dim(g.D, [&](auto dim) {
+        with_line(g, [&](auto line) {
+            auto* kernel = fma_fwd_kernel<float, decltype(dim)::value, decltype(line)::value>;
+            if ((err = prepare_kernel(kernel, smem)) != cudaSuccess) return;
+            kernel<<<grid, kThreadsF, smem, s>>>(p, (float*)out, (float*)lse);
+            err = cudaGetLastError();
+        });
+    });
+    simt_count_launch(1);
+    return (int)err;
+}
+
+int fma_fused_bwd(int dtype, const Geo& g, const void* q, const void* k, const void* v, const void* out, const void* lse,
+                  const void* dout, const void* dlse, void* dq, void* dk, void* dv, void* workspace, cudaStream_t s)
+{
+    if (dtype != 0 || g.Dv != g.D || !vec_rows(q, g.qs, 4) || !vec_rows(k, g.ks, 4) || !vec_rows(v, g.vs, 4)) return -2;
+    for (const void* p : {out, dout, (const void*)dq, (const void*)dk, (const void*)dv})
+        if (reinterpret_cast<uintptr_t>(p) & 15u) return -2;
+    FmaParams pq, pk;
+    dim3 gq, gk;
+    size_t sq, sk;
+    if (!make_fma(g, pq, false, 2, 0, 0, gq, sq) || !make_fma(g, pk, true, 2, 8, 0, gk, sk)) return -2;
+    float* delta = static_cast<float*>(workspace);
+    pq.row1 = tensor_of(q, g.qs);
+    pq.row2 = dense(dout, g, g.Hq, g.D);
+    pq.col1 = tensor_of(k, g.ks);
+    pq.col2 = tensor_of(v, g.vs);
+    pk.row1 = pq.col1;
+    pk.row2 = pq.col2;
+    pk.col1 = pq.row1;
+    pk.col2 = pq.row2;
+    cudaError_t err = cudaSuccess;
+    with_dim(g.D, [&](auto dim) {
+        with_line(g, [&](auto line) {
+            constexpr int D = decltype(dim)::value;
+            auto* kq = fma_bwd_q_kernel<float, D, decltype(line)::value>;
+            auto* kk = fma_bwd_k_kernel<float, D, decltype(line)::value>;
+            if ((err = prepare_kernel(kq, sq)) != cudaSuccess || (err = prepare_kernel(kk, sk)) != cudaSuccess) return;
+            kq<<<gq, kThreadsF, sq, s>>>(pq, (const float*)out, (const float*)lse, (const float*)dlse, delta, (float*)dq);
+            kk<<<gk, kThreadsF, sk, s>>>(pk, (const float*)lse, delta, (float*)dk, (float*)dv);
+            err = cudaGetLastError();
+        });
+    });
+    simt_count_launch(2);
+    return (int)err;
+}
+
+} // namespace natten
