@@ -171,6 +171,10 @@ int natten_qk_fwd(const natten_params_t* p, const void* q, const void* k, void* 
         if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
     }
     t_last_path = NATTEN_PATH_SIMT;
+    if (!(p->flags & NATTEN_FLAG_FORCE_SIMT)) {
+        rc = fma_scores(p->dtype, g, q, g.qs, k, g.ks, g.has_scale ? (float)g.scale : 1.f, true, logits, (cudaStream_t)stream);
+        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+    }
     return from_cuda(simt_qk_fwd(p->dtype, g, q, k, logits, (cudaStream_t)stream));
 }
 
@@ -196,6 +200,16 @@ int natten_qk_bwd(const natten_params_t* p, const void* q, const void* k, const 
         dk_done = rc == 0;
         if (dq_done || dk_done) t_last_path = NATTEN_PATH_TCGEN05;
         if ((p->flags & NATTEN_FLAG_FORCE_TC) && !(dq_done && dk_done)) return NATTEN_E_UNSUPPORTED;
+        if (!dq_done) {
+            rc = fma_apply(p->dtype, g, dlogits, k, g.ks, sc, dq, (cudaStream_t)stream);
+            if (rc > 0) return rc;
+            dq_done = rc == 0;
+        }
+        if (!dk_done) {
+            rc = fma_gather(p->dtype, g, dlogits, q, g.qs, sc, dk, (cudaStream_t)stream);
+            if (rc > 0) return rc;
+            dk_done = rc == 0;
+        }
         if (dq_done && dk_done) return NATTEN_OK;
     }
     return from_cuda(simt_qk_bwd(p->dtype, g, q, k, dlogits, dq_done ? nullptr : dq, dk_done ? nullptr : dk,
@@ -216,6 +230,8 @@ int natten_qk_rpb_fwd(const natten_params_t* p, const void* q, const void* k, co
                        (cudaStream_t)stream, rpb);
         if (rc == 0) { t_last_path = NATTEN_PATH_TCGEN05; return NATTEN_OK; }
         if (rc > 0) return rc;
+        rc = fma_scores(p->dtype, g, q, g.qs, k, g.ks, g.has_scale ? (float)g.scale : 1.f, true, logits, (cudaStream_t)stream, rpb);
+        if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_SIMT; return rc; }
     }
     // otherwise the logits first, then the bias in a second pass
     rc = natten_qk_fwd(p, q, k, logits, stream);
@@ -253,6 +269,12 @@ int natten_av_fwd(const natten_params_t* p, const void* attn, const void* v, voi
         if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
     }
     t_last_path = NATTEN_PATH_SIMT;
+    if (!(p->flags & NATTEN_FLAG_FORCE_SIMT)) {
+        Geo gv = g;
+        gv.D = g.Dv;
+        rc = fma_apply(p->dtype, gv, attn, v, g.vs, 1.f, out, (cudaStream_t)stream);
+        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+    }
     return from_cuda(simt_av_fwd(p->dtype, g, attn, v, out, (cudaStream_t)stream));
 }
 
@@ -283,8 +305,20 @@ int natten_av_bwd(const natten_params_t* p, const void* attn, const void* v, con
         dv_done = rc == 0;
         if (da_done || dv_done) t_last_path = NATTEN_PATH_TCGEN05;
         if (da_done && dv_done) return NATTEN_OK;
+        if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
+        if (!da_done) {
+            rc = fma_scores(p->dtype, gv, dout, dos, v, g.vs, 1.f, false, dattn, (cudaStream_t)stream);
+            if (rc > 0) return rc;
+            da_done = rc == 0;
+        }
+        if (!dv_done) {
+            rc = fma_gather(p->dtype, gv, attn, dout, dos, 1.f, dv, (cudaStream_t)stream);
+            if (rc > 0) return rc;
+            dv_done = rc == 0;
+        }
+        if (da_done && dv_done) return NATTEN_OK;
     }
-    if ((p->flags & NATTEN_FLAG_FORCE_TC) && !(da_done && dv_done)) return NATTEN_E_UNSUPPORTED;
+    if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
     return from_cuda(simt_av_bwd(p->dtype, g, attn, v, dout, da_done ? nullptr : dattn, dv_done ? nullptr : dv,
                                  (cudaStream_t)stream));
 }

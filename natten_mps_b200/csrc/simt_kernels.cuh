@@ -28,6 +28,11 @@ cudaError_t simt_av_bwd(int dtype, const Geo& g, const void* attn, const void* v
 int fma_fused_fwd(int dtype, const Geo& g, const void* q, const void* k, const void* v, void* out, void* lse, cudaStream_t s);
 int fma_fused_bwd(int dtype, const Geo& g, const void* q, const void* k, const void* v, const void* out, const void* lse,
                   const void* dout, const void* dlse, void* dq, void* dk, void* dv, void* workspace, cudaStream_t s);
+// The split operators' three products (see tc_kernels.cuh) by the same kernels, every type but float64; unit stride.
+int fma_scores(int dtype, const Geo& g, const void* x, const long long xs[3], const void* y, const long long ys[3], float scale,
+               bool neg_inf, void* out, cudaStream_t s, const void* rpb = nullptr);
+int fma_apply(int dtype, const Geo& g, const void* w, const void* y, const long long ys[3], float scale, void* out, cudaStream_t s);
+int fma_gather(int dtype, const Geo& g, const void* w, const void* x, const long long xs[3], float scale, void* dst, cudaStream_t s);
 unsigned long long simt_launch_count();
 void simt_count_launch(int n);
 

@@ -1,0 +1,88 @@
+"""The fp32-arithmetic window kernels (four rows per lane group over a staged column box) and the one-pass bias gradient,
+against the CPU oracle: ragged tiles, remainders of rows and columns, boxes larger than a chunk, clamped edges, causal axes,
+dilation with uneven groups, GQA and the three ranks.  The split cases are as large as the kernels' size rule asks for."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from natten_mps_b200 import _cabi
+from natten_mps_b200 import functional as F
+from tests._gpu_util import TOL, check, run_fused, rounded
+
+pytestmark = pytest.mark.gpu
+
+# name, spatial, B, Hq, Hkv, kernel, dilation, causal, D
+FUSED_CASES = [
+    ("1d_smallest", (3,), 1, 1, 1, (2,), (1,), (False,), 32),
+    ("1d_remainders", (515,), 2, 2, 1, (63,), (2,), (True,), 64),
+    ("2d_tiles_plus_one", (17, 33), 1, 2, 2, (7, 7), (1, 1), (False, False), 32),
+    ("2d_even_causal_dil", (23, 30), 1, 4, 2, (4, 6), (3, 2), (True, False), 32),
+    ("2d_window_is_all", (9, 11), 2, 1, 1, (9, 11), (1, 1), (False, False), 128),
+    ("2d_box_past_a_chunk", (40, 44), 1, 1, 1, (21, 19), (1, 1), (False, True), 128),
+    ("3d_ragged", (5, 9, 14), 1, 2, 1, (3, 5, 7), (1, 1, 2), (True, False, False), 32),
+]
+
+
+@pytest.mark.parametrize("case", FUSED_CASES, ids=lambda c: c[0])
+def test_fused_float32(case):
+    _, sp, B, Hq, Hkv, K, dil, causal, D = case
+    rng = np.random.default_rng(7)
+    r = lambda h: rng.standard_normal((B, *sp, h, D))
+    got, want = run_fused(len(sp), torch.float32, r(Hq), r(Hkv), r(Hkv), r(Hq),
+                          dict(kernel_size=K, dilation=dil, is_causal=causal, return_lse=True))
+    for name in ("out", "lse", "dq", "dk", "dv"):
+        check(name, got[name], want[name], torch.float32)
+
+
+SPLIT_CASES = [
+    ("2d_d32_ragged", (57, 61), 2, 4, 4, (7, 9), (1, 1), (False, False), 32),
+    ("2d_d32_even_causal_dil", (66, 45), 2, 4, 4, (6, 12), (2, 3), (False, True), 32),
+    ("1d_d32", (3001,), 3, 4, 4, (43,), (1,), (False,), 32),
+    ("3d_d32", (6, 23, 25), 2, 4, 4, (3, 5, 5), (1, 1, 2), (True, False, False), 32),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16], ids=["f32", "bf16", "f16"])
+@pytest.mark.parametrize("case", SPLIT_CASES, ids=lambda c: c[0])
+def test_split(case, dtype):
+    _, sp, B, Hq, Hkv, K, dil, causal, D = case
+    rank = len(sp)
+    g = torch.Generator().manual_seed(5)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype)
+    q, k, v, do = r(B, *sp, Hq, D), r(B, *sp, Hkv, D), r(B, *sp, Hkv, D), r(B, *sp, Hq, D)
+    kw = dict(kernel_size=K, dilation=dil, is_causal=causal)
+    w, gl = r(B, *sp, Hq, int(np.prod(K))), r(B, *sp, Hq, int(np.prod(K)))
+    qk, av = {1: (F.na1d_qk, F.na1d_av), 2: (F.na2d_qk, F.na2d_av), 3: (F.na3d_qk, F.na3d_av)}[rank]
+    leaf = lambda t: t.cuda().requires_grad_(True)
+    qd, kd, vd, wd = leaf(q), leaf(k), leaf(v), leaf(w)
+    logits, out = qk(qd, kd, **kw), av(wd, vd, **kw)
+    dq, dk = torch.autograd.grad(logits, [qd, kd], gl.cuda())
+    dw, dv = torch.autograd.grad(out, [wd, vd], do.cuda())
+    n = lambda t: t.float().numpy()
+    want = dict(logits=oracle.na_qk(n(q), n(k), **kw), out=oracle.na_av(n(w), n(v), **kw))
+    want["dq"], want["dk"] = oracle.na_qk_backward(n(q), n(k), n(gl), **kw)
+    want["dw"], want["dv"] = oracle.na_av_backward(n(w), n(v), n(do), **kw)
+    for name, got in dict(logits=logits, out=out, dq=dq, dk=dk, dw=dw, dv=dv).items():
+        check(name, got, want[name], dtype, scale_rel=True)
+
+
+# the register part (interior positions), the table part (clamped edges, slots past the registers) and both cluster sizes
+BIAS_CASES = [((95,), 12, 8, (13,), (1,)), ((40, 17), 2, 4, (7, 5), (1, 3)), ((29, 31), 1, 2, (17, 17), (1, 1)),
+              ((30, 33), 1, 1, (23, 25), (1, 1)), ((5, 12, 14), 2, 2, (3, 5, 3), (1, 2, 1))]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("case", BIAS_CASES, ids=lambda c: "x".join(map(str, c[0])))
+def test_bias_gradient_in_one_pass(case, dtype):
+    sp, B, H, K, dil = case
+    g = torch.Generator().manual_seed(11)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype)
+    q, k, rpb = r(B, *sp, H, 32), r(B, *sp, H, 32), r(H, *[2 * x - 1 for x in K])
+    gl = r(B, *sp, H, int(np.prod(K)))
+    rd = rpb.cuda().requires_grad_(True)
+    fn = {1: F.na1d_qk_rpb, 2: F.na2d_qk_rpb, 3: F.na3d_qk_rpb}[len(sp)]
+    (got,) = torch.autograd.grad(fn(q.cuda(), k.cuda(), rd, K, dil), [rd], gl.cuda())
+    n = lambda t: t.float().numpy()
+    _, _, want = oracle.na_qk_rpb_backward(n(q), n(k), n(rpb), n(gl), kernel_size=K, dilation=dil)
+    check("drpb", got, want, dtype, scale_rel=True)
