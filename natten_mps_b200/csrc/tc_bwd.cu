@@ -31,31 +31,11 @@
 
 #include <type_traits>
 
-#ifndef NATTEN_ABL
-#define NATTEN_ABL 0
-#endif
-
 namespace natten {
 
 using namespace tc;
 using namespace tcplan;
 using namespace rowtile;
-
-// Optional clock stamps of one CTA's pipeline events (development builds only: -DNATTEN_TRACE).
-#ifdef NATTEN_TRACE
-__device__ long long g_trace_bwd[2 * 16 * 512];
-#define STAMP(id)                                                                                   \
-    do {                                                                                            \
-        if (blockIdx.x == 7 && lane == 0 && tn < 255) {                                             \
-            long long* tr_ = g_trace_bwd + (kKeySide ? 16 * 512 : 0) + warp * 512;                  \
-            tr_[2 * tn] = (id);                                                                     \
-            tr_[2 * tn + 1] = clock64();                                                            \
-            ++tn;                                                                                   \
-        }                                                                                           \
-    } while (0)
-#else
-#define STAMP(id) do { } while (0)
-#endif
 
 namespace {
 
@@ -105,9 +85,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
     constexpr uint32_t kTmemCols = Smem::kTmemCols, kColA2 = Smem::kColA2;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#ifdef NATTEN_TRACE
-    int tn = 0;
-#endif
     const int quad = warp & 3, piece = (warp >> 2) & 1;      // compute warps: TMEM lane quadrant, 32-column piece
     const int prior_abort = *reinterpret_cast<volatile int*>(P.status);   // loaded early, used at barrier set-up
     const unsigned nwork = kKeySide ? P.work_kv : P.work_q;
@@ -242,15 +219,11 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 __syncwarp();                    // every lane has read the head
                 if (leader) mbar_arrive(bar_tab_empty + 8 * slot);
                 if (!T.active) continue;
-                STAMP(190);
                 ok = mbar_wait(bar_row, tileno & 1, abort_flag, P.wait_budget);
-                STAMP(191);
                 ok = ok && mbar_wait(bar_col + 8 * (g % kStages), (g / kStages) & 1, abort_flag, P.wait_budget);
                 if (!ok) break;
-                STAMP(192);
                 issue_s_dp(g, 0, T);
                 for (int cc = 0; cc < T.total && ok; ++cc, ++g) {
-                    STAMP(200 + cc);
                     if (kTwoBuf && cc + 1 < T.total) {
                         // two buffers: the next chunk's products go into the other buffer, whose P / dS were read
                         // by products this warp issued earlier, so they need not wait for the threads
@@ -260,16 +233,12 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     }
                     ok = mbar_wait(bar_sp_of(g), par_of(g), abort_flag, P.wait_budget);               // S/dP consumed, P/dS stored
                     if (!ok) break;
-                    STAMP(210);
                     issue_acc(g, cc > 0);                                    // reads P/dS ...
-                    STAMP(215);
                     if (!kTwoBuf && cc + 1 < T.total) {
                         ok = mbar_wait(bar_col + 8 * ((g + 1) % kStages), ((g + 1) / kStages) & 1, abort_flag, P.wait_budget);
                         if (!ok) break;
-                        STAMP(216);
                         issue_s_dp(g + 1, cc + 1, T);                                // ... before the next S/dP overwrite them
                     }
-                    STAMP(220);
                 }
                 ++tileno;
             }
@@ -350,23 +319,19 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
         }
         for (unsigned work = blockIdx.x; work < nwork; work += gridDim.x, ++item) {
             const unsigned wn = work + gridDim.x;
-            STAMP(390);
             if (wn < nwork) {                    // the next item's table first: it is needed before this tile ends
                 bwd_tile_setup<kKeySide>(P, wn, Tn);
                 write_table(wn, item + 1, Tn);
             }
-            STAMP(395);
             if (T.active) {
                 // the row tiles are free once the previous tile's last S / dP products have finished
                 if (tiles > 0) ok = ok && mbar_wait(bar_rowfree, (tiles - 1) & 1, abort_flag, P.wait_budget);
-                STAMP(398);
                 if (lane == 0 && ok) issue_rows(T);
                 ++tiles;
                 int ci[3] = {0, 0, 0}, hc = T.hy * P.group;
                 const int head_kv = kKeySide ? T.hy : T.hy / P.group;
                 for (int cc = 0; cc < T.total; ++cc, ++g) {
                     const int s = g % kStages;
-                    STAMP(400 + cc);
                     // key side: the chunk's column statistics are fetched before the wait for the stage, so that
                     // their latency is not part of what follows it
                     float raw_lse[kCols / 32], raw_delta[kCols / 32];
@@ -393,7 +358,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                         }
                     }
                     if (g >= (unsigned)kStages) ok = ok && mbar_wait(bar_free + 8 * s, ((g / kStages) - 1) & 1, abort_flag, P.wait_budget);
-                    STAMP(410);
                     if (lane == 0 && ok) {
                         const uint32_t bar = bar_col + 8 * s;
                         mbar_expect_tx(bar, 2 * kColTile);
@@ -448,7 +412,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             const unsigned slot = item & 1;
             ok = mbar_wait(bar_tab_full + 8 * slot, (item >> 1) & 1, abort_flag, P.wait_budget) && ok;
             const uint8_t* tab = smem + Smem::kTab + slot * Smem::kTabBytes;
-            STAMP(300);
             const TileHead T = *reinterpret_cast<const TileHead*>(tab + kAxisEntries * 16);
             int f[3], e[3];
             bool valid_row = true, in_tensor = true;
@@ -470,7 +433,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 }
             }
             mbar_arrive(bar_tab_empty + 8 * slot);
-            STAMP(301);
             if (!valid_row) { e[0] = f[0]; e[1] = f[1]; e[2] = f[2]; }
             const long long out_row = ((long long)T.b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + T.hy;
             // query side: the row's lse and delta; scaled where they are first used, so that the loads' latency
@@ -480,7 +442,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 raw_lse = lse[out_row];
                 raw_delta = delta[out_row];
             }
-            STAMP(302);
             if (!T.active) {                     // padding rows get zero gradients
                 if (in_tensor) {
 #pragma unroll
@@ -586,19 +547,13 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     mine[0] = (word & 0xFFFFu) != 0u;
                     mine[1] = (word >> 16) != 0u;
                 }
-#if NATTEN_ABL == 2
-                const bool any[2] = {false, false};
-#else
                 const bool any[2] = {__any_sync(0xffffffffu, mine[0]) != 0, __any_sync(0xffffffffu, mine[1]) != 0};
-#endif
                 const bool separable = kInner > 0 && !extra;
                 const bool full = !separable && __all_sync(0xffffffffu, word == 0xffffffffu);
-                STAMP(310 + ((any[0] || any[1]) ? 1 : 0));
                 ok = ok && mbar_wait(bar_s_of(g), par_of(g), abort_flag, P.wait_budget);      // also: the P/dS this buffer held were consumed
                 const uint32_t tbuf = trow + buf_cols(g);
                 if (kKeySide) ok = ok && mbar_wait(bar_stats + 8 * (g % kStages), (g / kStages) & 1, abort_flag, P.wait_budget);
                 tc_fence_after();
-                STAMP(320);
                 const float row_lse2 = -raw_lse * 1.4426950408889634f, row_delta = -raw_delta * P.scale;   // negated, pre-scaled addends
                 const uint64_t scale_log2_2 = pack2(P.scale_log2, P.scale_log2), scale_2 = pack2(P.scale, P.scale);
 #pragma unroll
@@ -673,7 +628,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(bar_sp_of(g));
-                STAMP(330);
                 // next chunk (innermost axis fastest; wraps to the next query head on the key side)
                 if (mapped) {
                     if (++cl == T.nchunks) cl = 0;
@@ -687,10 +641,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             }
 
             // ---- accumulators -> global: this warp owns 32 of the 64 channels ----
-            STAMP(340);
             ok = ok && mbar_wait(bar_free + 8 * ((g - 1) % kStages), ((g - 1) / kStages) & 1, abort_flag, P.wait_budget);   // the last chunk's accumulating products
             tc_fence_after();
-            STAMP(350);
             // The accumulators leave through shared memory and a bulk tensor store: every thread converts its
             // 32 channels of its row and writes them into a [128 x DH] tile laid out like the row tiles the loads
             // bring in (128-byte rows, 16-byte chunks swizzled by the row); one thread then hands the tile to the
@@ -721,7 +673,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 }
                 fence_async_smem();                                          // the TMA unit reads through the async proxy
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (warp == 0 && lane == 0 && ok && NATTEN_ABL != 1) {
+                if (warp == 0 && lane == 0 && ok) {
                     const CUtensorMap* map = which == 0 ? &tmO1 : &tmO2;
 #pragma unroll
                     for (int hf = 0; hf < Smem::kHalves; ++hf)
@@ -732,7 +684,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             }
             // the next tile's first accumulating MMA is issued only after every thread has passed here
             tc_fence_before();
-            STAMP(360);
         }
     }
 
@@ -1003,17 +954,5 @@ size_t tc_bwd_workspace_bytes(int dtype, const Geo& g)
     const size_t rows_full = (size_t)g.B * (size_t)g.ltot * (size_t)g.Hq;
     return 2 * align256(rows_full * 4) + align256(rows_full * (size_t)g.D * 2);
 }
-
-#ifdef NATTEN_TRACE
-extern "C" int natten_trace_read_bwd(long long* host, int clear)
-{
-    cudaError_t e = cudaMemcpyFromSymbol(host, g_trace_bwd, sizeof(g_trace_bwd));
-    if (e == cudaSuccess && clear) {
-        static long long zeros[2 * 16 * 512] = {0};
-        e = cudaMemcpyToSymbol(g_trace_bwd, zeros, sizeof(g_trace_bwd));
-    }
-    return (int)e;
-}
-#endif
 
 } // namespace natten

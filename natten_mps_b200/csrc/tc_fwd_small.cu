@@ -27,29 +27,11 @@
 
 #include <type_traits>
 
-#ifndef NATTEN_ABL
-#define NATTEN_ABL 0
-#endif
-
 namespace natten {
 
 using namespace tc;
 using namespace tcplan;
 using namespace fwdgeom;
-
-#ifdef NATTEN_TRACE
-__device__ long long g_trace_small[8 * 512];
-#define STAMP(id)                                                                                   \
-    do {                                                                                            \
-        if (blockIdx.x == 9 && lane == 0 && tn < 255) {       \
-            g_trace_small[warp * 512 + 2 * tn] = (id);                                              \
-            g_trace_small[warp * 512 + 2 * tn + 1] = clock64();                                     \
-            ++tn;                                                                                   \
-        }                                                                                           \
-    } while (0)
-#else
-#define STAMP(id) do { } while (0)
-#endif
 
 namespace {
 
@@ -83,6 +65,25 @@ struct FwdSmall {
     static constexpr uint32_t kColO = kTwoS ? 128 : 64;
 };
 
+// 4 x 4 transpose of 16-byte pieces among four adjacent lanes: w[i] of lane j <-> w[j] of lane i (j = lane & 3).
+__device__ __forceinline__ void transpose4(uint32_t (&w)[4][4], int j)
+{
+#pragma unroll
+    for (int m = 1; m <= 2; m *= 2) {
+        const bool up = j & m;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i & m) continue;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[i][k] : w[i | m][k], m);
+                if (up) w[i][k] = got;
+                else w[i | m][k] = got;
+            }
+        }
+    }
+}
+
 template <int DH, bool BF16, int kInner>
 __global__ void __launch_bounds__(kThreads, FwdSmall<DH>::kPerSm)
 tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -97,9 +98,6 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     constexpr bool kTwoS = FS::kTwoS;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#ifdef NATTEN_TRACE
-    int tn = 0;
-#endif
     const int prior_abort = *reinterpret_cast<volatile int*>(P.status);
 
     const uint32_t sbase = smem_u32(smem);
@@ -304,7 +302,6 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 if (nch == 0) break;
                 ok = mbar_wait(bar_q, ti & 1, abort_flag, P.wait_budget);
                 issue_qk(H, 0);
-                STAMP(200);
                 discover();                      // the next tile's geometry, while the threads work on this chunk
                 while (refill()) {}
                 for (int c = 0; c < nch && ok; ++c) {
@@ -314,10 +311,8 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     if (!ok) break;
                     ok = mbar_wait(bar_p_of(n_pv), par_of(n_pv), abort_flag, P.wait_budget);      // P(c) stored over S(c)
                     if (!ok) break;
-                    STAMP(210);
                     issue_pv(c, c + 1 == nch);       // reads P(c) ...
                     if (!kTwoS && c + 1 < nch) issue_qk(H, c + 1);   // ... before the next scores overwrite it (issue order)
-                    STAMP(220);
                     while (refill()) {}
                 }
             }
@@ -401,7 +396,6 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (!ok) break;
         const FwdTile T = *hdr_slot(t);
         if (T.nch == 0) break;
-        STAMP(290);
         // ---- this thread's query row ----
         int f[3], e[3];
         bool valid_q, in_tensor;
@@ -479,11 +473,9 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const bool fast = kRows16 && !extra;
             if (fast && colbits != add_cols) refresh_add(colbits);
 
-            STAMP(300 + c);
             scol = trow + kColS + s_cols(n);
             ok = ok && mbar_wait(bar_s_of(n), par_of(n), abort_flag, P.wait_budget);     // one score buffer: every earlier product has finished, too
             tc_fence_after();
-            STAMP(310);
             if (!ok) { words[0] = 0u; words[1] = 0u; rowbits = 0u; dirty = 7u; }
 
             uint32_t stored = 0u;            // pieces of this chunk that hold probabilities (bit per piece)
@@ -555,20 +547,11 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             for (int pc = 0; pc < 4; ++pc) {
                 uint32_t pk[8];
                 if (fast) {
-#if NATTEN_ABL == 2
-                    const bool rowok = false;
-#else
                     const bool rowok = ((rowbits >> pc) & 1u) && colbits != 0u;
-#endif
                     if (__any_sync(0xffffffffu, rowok)) {
                         uint32_t s[16];
                         tmem_ld16(scol + 16 * pc, s);
                         tmem_ld_wait();
-#if NATTEN_ABL == 3
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) pk[i] = s[2 * i] & 1u;
-                        stored |= 1u << pc;
-#else
                         if (m == -INFINITY && rowok) {           // first valid columns of this row: fix the stabiliser
                             float mm = -INFINITY;
 #pragma unroll
@@ -616,7 +599,6 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         }
                         if (rowok) l += lo_of(rr) + hi_of(rr);
                         stored |= 1u << pc;
-#endif
                     } else {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) pk[i] = 0u;
@@ -639,7 +621,6 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(bar_p_of(n));
-            STAMP(330);
             if (!mapped) {
                 ++ci[2];
                 dirty = 4u;
@@ -653,28 +634,33 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // ---- normalise and write out ----
         ok = mbar_wait(bar_o, t & 1, abort_flag, P.wait_budget) && ok;
         tc_fence_after();
-        STAMP(340);
         {
             const bool live = valid_q && ok;
             const float inv = (live && l > 0.f) ? 1.f / l : 0.f;
-            uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
+            // A thread holds a row, but 32 rows written 16 bytes at a time are 32 lines per store instruction (the stores of
+            // the tile kept the load / store unit busy for 4200 cycles, 15 % of the kernel).  Four lanes exchange their
+            // 16-byte pieces of 32 channels, so that a store writes 64 bytes of each of eight rows.
+            const long long my_row = in_tensor ? out_row : -1;
+            long long rows4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) rows4[i] = __shfl_sync(0xffffffffu, my_row, (lane & ~3) | i);
+            const int piece = lane & 3;
 #pragma unroll
             for (int part = 0; part < DH / 32; ++part) {
                 if (32 * part >= P.dreal) break;             // padded channels are not part of the output
-                uint32_t o[32];
+                uint32_t o[32], w[4][4];
                 tmem_ld32(trow + kColO + 32 * part, o);
                 tmem_ld_wait();
-                if (in_tensor && NATTEN_ABL != 1) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        if (32 * part + 8 * i >= P.dreal) break;
-                        uint32_t wv[4];
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            wv[j] = live ? cvt_pack<BF16>(__uint_as_float(o[8 * i + 2 * j]) * inv, __uint_as_float(o[8 * i + 2 * j + 1]) * inv) : 0u;
-                        o4[4 * part + i] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-                    }
-                }
+                    for (int j = 0; j < 4; ++j)
+                        w[i][j] = live ? cvt_pack<BF16>(__uint_as_float(o[8 * i + 2 * j]) * inv, __uint_as_float(o[8 * i + 2 * j + 1]) * inv) : 0u;
+                transpose4(w, piece);                        // w[i]: this lane's piece of row i of the four
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (rows4[i] >= 0 && 32 * part + 8 * piece < P.dreal)
+                        reinterpret_cast<uint4*>(out + rows4[i] * P.dreal)[4 * part + piece] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
             }
             // natural-log lse of scale * logits
             if (in_tensor)
@@ -682,7 +668,6 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         // the next tile's first P V is issued only after this thread has stored its next P
         tc_fence_before();
-        STAMP(350);
         }
     }
 
@@ -748,17 +733,5 @@ int tc_fused_fwd_small(int dtype, const Geo& g, const void* q, const void* k, co
 static unsigned long long g_tc_launches = 0;
 void tc_count_launch() { ++g_tc_launches; }
 unsigned long long tc_launch_count() { return g_tc_launches; }
-
-#ifdef NATTEN_TRACE
-extern "C" int natten_trace_read_small(long long* host, int clear)
-{
-    cudaError_t e = cudaMemcpyFromSymbol(host, g_trace_small, sizeof(g_trace_small));
-    if (e == cudaSuccess && clear) {
-        static long long zeros[8 * 512] = {0};
-        e = cudaMemcpyToSymbol(g_trace_small, zeros, sizeof(g_trace_small));
-    }
-    return (int)e;
-}
-#endif
 
 } // namespace natten
