@@ -71,7 +71,8 @@ struct SmemB {
 // written out.  Barrier phases run on across tiles (g = chunks processed so far).
 // kInner: innermost chunk extent when it is 16 or 32 (separable row / column masks, packed
 // 16-bit arithmetic), 0 = any geometry (per-column validity words).
-template <int DH, bool BF16, bool kKeySide, int kInner>
+// kShort: the last 32 of the DH channels are padding.
+template <int DH, bool BF16, bool kKeySide, int kInner, bool kShort>
 __global__ void __launch_bounds__(kThreads, (DH == 64 ? 2 : 1))
 tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ CUtensorMap tmR2,
               const __grid_constant__ CUtensorMap tmC1, const __grid_constant__ CUtensorMap tmC2,
@@ -185,9 +186,10 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 tc_fence_after();
                 // 32 bytes per k-step inside a 64-channel block; blocks are kRowHalf / kColHalf apart
 #pragma unroll
-                for (int ks = 0; ks < DH / 16; ++ks)
+                for (int ks = 0; ks < (kShort ? DH / 16 - 2 : DH / 16); ++ks) {
                     mma_ss_e(tmem + col_out + buf_cols(g), dR + (((ks / 4) * kRowHalf + (ks % 4) * 32) >> 4),
                              dC + (((ks / 4) * kColHalf + (ks % 4) * 32) >> 4), idesc_kk, ks > 0, leader);
+                }
                 mma_commit_e(bar_s_of(g), leader);
                 if (cc + 1 == X.total) mma_commit_e(bar_rowfree, leader);      // the tile's last read of this stream's row tile
             };
@@ -301,13 +303,13 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             mbar_arrive(bar_tab_full + 8 * slot);
         };
         auto issue_rows = [&](const BwdTile& X) {
-            const int hx = X.hy * DH;
+            const int hx = X.hy;
             mbar_expect_tx(bar_row, 2 * kTile);
 #pragma unroll
             for (int hf = 0; hf < Smem::kHalves; ++hf) {
-                tma_load_heads(sbase + Smem::kR1 + hf * kRowHalf, &tmR1, bar_row, P, DH, hx + 64 * hf, X.rg[2] + P.dil[2] * X.origin[2],
+                tma_load_heads(sbase + Smem::kR1 + hf * kRowHalf, &tmR1, bar_row, P, hx, 64 * hf, X.rg[2] + P.dil[2] * X.origin[2],
                             X.rg[1] + P.dil[1] * X.origin[1], X.rg[0] + P.dil[0] * X.origin[0], X.b);
-                tma_load_heads(sbase + Smem::kR2 + hf * kRowHalf, &tmR2, bar_row, P, DH, hx + 64 * hf, X.rg[2] + P.dil[2] * X.origin[2],
+                tma_load_heads(sbase + Smem::kR2 + hf * kRowHalf, &tmR2, bar_row, P, hx, 64 * hf, X.rg[2] + P.dil[2] * X.origin[2],
                             X.rg[1] + P.dil[1] * X.origin[1], X.rg[0] + P.dil[0] * X.origin[0], X.b);
             }
         };
@@ -366,18 +368,18 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
 #pragma unroll
                             for (int a = 0; a < 3; ++a) X[a] = T.rg[a] + P.dil[a] * (T.boxlo[a] + chunk_coord(P, a, ci[a], 0));
                             // query side: columns are keys (kv head); key side: columns are queries (query head)
-                            const int hx = (kKeySide ? hc : head_kv) * DH;
+                            const int hx = kKeySide ? hc : head_kv;
 #pragma unroll
                             for (int hf = 0; hf < Smem::kHalves; ++hf) {
-                                tma_load_heads(sbase + Smem::kC1 + s * kColTile + hf * kColHalf, &tmC1, bar, P, DH, hx + 64 * hf, X[2], X[1], X[0], T.b);
-                                tma_load_heads(sbase + Smem::kC2 + s * kColTile + hf * kColHalf, &tmC2, bar, P, DH, hx + 64 * hf, X[2], X[1], X[0], T.b);
+                                tma_load_heads(sbase + Smem::kC1 + s * kColTile + hf * kColHalf, &tmC1, bar, P, hx, 64 * hf, X[2], X[1], X[0], T.b);
+                                tma_load_heads(sbase + Smem::kC2 + s * kColTile + hf * kColHalf, &tmC2, bar, P, hx, 64 * hf, X[2], X[1], X[0], T.b);
                             }
                         } else {                             // additional tokens (rows past n_extra are zero-filled)
                             const int e0 = (cc - T.nbox) * kCols;
 #pragma unroll
                             for (int hf = 0; hf < Smem::kHalves; ++hf) {
-                                tma_load_heads(sbase + Smem::kC1 + s * kColTile + hf * kColHalf, &tmE1, bar, P, DH, head_kv * DH + 64 * hf, e0, 0, 0, T.b);
-                                tma_load_heads(sbase + Smem::kC2 + s * kColTile + hf * kColHalf, &tmE2, bar, P, DH, head_kv * DH + 64 * hf, e0, 0, 0, T.b);
+                                tma_load_heads(sbase + Smem::kC1 + s * kColTile + hf * kColHalf, &tmE1, bar, P, head_kv, 64 * hf, e0, 0, 0, T.b);
+                                tma_load_heads(sbase + Smem::kC2 + s * kColTile + hf * kColHalf, &tmE2, bar, P, head_kv, 64 * hf, e0, 0, 0, T.b);
                             }
                         }
                     }
@@ -652,6 +654,31 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             const int row = quad * 32 + lane;
 #pragma unroll
             for (int which = 0; which < (kKeySide ? 2 : 1); ++which) {
+                if (kShort && P.shared_box) {               // a 64-channel box would write into the next head: 64-byte pieces of a row instead
+                    const long long my_row = in_tensor ? out_row : -1;
+                    uint16_t* dst = which == 0 ? out1 : out2;
+#pragma unroll 1
+                    for (int part = 0; part < CH / 32; ++part) {
+                        const int ch = CH * piece + 32 * part;
+                        if (ch >= P.dreal) break;
+                        uint32_t a[32], w[4][4];
+                        tmem_ld32(trow + (which == 0 ? kColA1 : kColA2) + ch, a);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                w[i][j] = live ? pack16(__uint_as_float(a[8 * i + 2 * j]), __uint_as_float(a[8 * i + 2 * j + 1]), BF16) : 0u;
+                        transpose4(w, lane & 3);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const long long r4 = __shfl_sync(0xffffffffu, my_row, (lane & ~3) | i);
+                            const int c8 = ch + 8 * (lane & 3);
+                            if (r4 >= 0 && c8 < P.dreal) *reinterpret_cast<uint4*>(dst + r4 * P.dreal + c8) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+                        }
+                    }
+                    continue;
+                }
                 if (warp == 0 && lane == 0) tma_store_wait_read();               // the previous store has let go of the tile
                 asm volatile("bar.sync 1, 256;" ::: "memory");
 #pragma unroll
@@ -876,20 +903,25 @@ int launch_bwd(int dtype, const Geo& g, const Plan& plan, const void* q, const v
     for (int a = 0; a < 3; ++a) ngroups *= p.dil[a];
     const dim3 grid_q(persistent_grid(p.work_q, DH == 64 ? 2 : 1));
     const dim3 grid_k(persistent_grid(p.work_kv, DH == 64 ? 2 : 1));
-    auto launch = [&](auto inner) {
+    auto launch = [&](auto inner, auto shorter) {
         constexpr int kInner = decltype(inner)::value;
-        ensure_dynamic_smem((const void*)tc_bwd_kernel<DH, BF16, false, kInner>, Smem::kTotal);
-        ensure_dynamic_smem((const void*)tc_bwd_kernel<DH, BF16, true, kInner>, Smem::kTotal);
-        tc_bwd_kernel<DH, BF16, false, kInner><<<grid_q, kThreads, Smem::kTotal, s>>>(
+        constexpr bool kShort = decltype(shorter)::value;
+        ensure_dynamic_smem((const void*)tc_bwd_kernel<DH, BF16, false, kInner, kShort>, Smem::kTotal);
+        ensure_dynamic_smem((const void*)tc_bwd_kernel<DH, BF16, true, kInner, kShort>, Smem::kTotal);
+        tc_bwd_kernel<DH, BF16, false, kInner, kShort><<<grid_q, kThreads, Smem::kTotal, s>>>(
             q_tile, do_tile, k_chunk, v_chunk, ek_chunk, ev_chunk, dq_tile, dq_tile, p, lse_k, delta_k, (uint16_t*)dq, nullptr);
         tc_count_launch();
-        tc_bwd_kernel<DH, BF16, true, kInner><<<grid_k, kThreads, Smem::kTotal, s>>>(
+        tc_bwd_kernel<DH, BF16, true, kInner, kShort><<<grid_k, kThreads, Smem::kTotal, s>>>(
             k_tile, v_tile, q_chunk, do_chunk, ek_chunk, ev_chunk, dk_tile, dv_tile, p, lse_k, delta_k, (uint16_t*)dk, (uint16_t*)dv);
         tc_count_launch();
     };
-    if (p.cb[2] == 16) launch(std::integral_constant<int, 16>{});
-    else if (p.cb[2] == 32) launch(std::integral_constant<int, 32>{});
-    else launch(std::integral_constant<int, 0>{});
+    auto by_short = [&](auto inner) {
+        if (g.D <= DH - 32) launch(inner, std::true_type{});
+        else launch(inner, std::false_type{});
+    };
+    if (p.cb[2] == 16) by_short(std::integral_constant<int, 16>{});
+    else if (p.cb[2] == 32) by_short(std::integral_constant<int, 32>{});
+    else by_short(std::integral_constant<int, 0>{});
     cudaError_t err = cudaGetLastError();
     // The additional tokens' own gradients sum over every query of the sample: SIMT kernel.
     if (err == cudaSuccess && g.n_extra > 0)

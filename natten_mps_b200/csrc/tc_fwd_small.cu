@@ -65,26 +65,8 @@ struct FwdSmall {
     static constexpr uint32_t kColO = kTwoS ? 128 : 64;
 };
 
-// 4 x 4 transpose of 16-byte pieces among four adjacent lanes: w[i] of lane j <-> w[j] of lane i (j = lane & 3).
-__device__ __forceinline__ void transpose4(uint32_t (&w)[4][4], int j)
-{
-#pragma unroll
-    for (int m = 1; m <= 2; m *= 2) {
-        const bool up = j & m;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (i & m) continue;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[i][k] : w[i | m][k], m);
-                if (up) w[i][k] = got;
-                else w[i | m][k] = got;
-            }
-        }
-    }
-}
-
-template <int DH, bool BF16, int kInner>
+// kShort: the last 32 of the DH channels are padding.
+template <int DH, bool BF16, int kInner, bool kShort>
 __global__ void __launch_bounds__(kThreads, FwdSmall<DH>::kPerSm)
 tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmEK,
@@ -212,7 +194,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         mbar_expect_tx(bar_q, kQBytes + ((P.inject == 1 && tl == 0) ? 16u : 0u));
 #pragma unroll
                         for (int hf = 0; hf < kHalves; ++hf)
-                            tma_load_heads(sbase + kOffQ + hf * kQHalf, &tmQ, bar_q, P, DH, H->h * DH + 64 * hf,
+                            tma_load_heads(sbase + kOffQ + hf * kQHalf, &tmQ, bar_q, P, H->h, 64 * hf,
                                         H->rg[2] + P.dil[2] * (H->x0[2] + H->sx[2] * H->origin[2]),
                                         H->rg[1] + P.dil[1] * (H->x0[1] + H->sx[1] * H->origin[1]),
                                         H->rg[0] + P.dil[0] * (H->x0[0] + H->sx[0] * H->origin[0]), H->b);
@@ -234,15 +216,15 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         const int X2 = H->rg[2] + P.dil[2] * (H->lo[2] + chunk_coord(P, 2, ldc[2], 0));
 #pragma unroll
                         for (int hf = 0; hf < kHalves; ++hf) {
-                            tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, &tmK, bar, P, DH, H->hk * DH + 64 * hf, X2, X1, X0, H->b);
-                            tma_load_heads(sbase + kOffV + s * kKVBytes + hf * kKVHalf, &tmV, bar, P, DH, H->hk * DH + 64 * hf, X2, X1, X0, H->b);
+                            tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, &tmK, bar, P, H->hk, 64 * hf, X2, X1, X0, H->b);
+                            tma_load_heads(sbase + kOffV + s * kKVBytes + hf * kKVHalf, &tmV, bar, P, H->hk, 64 * hf, X2, X1, X0, H->b);
                         }
                     } else {                     // additional tokens (rows past n_extra are zero-filled)
                         const int e0 = (cl - H->nnb) * kKeys;
 #pragma unroll
                         for (int hf = 0; hf < kHalves; ++hf) {
-                            tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, &tmEK, bar, P, DH, H->hk * DH + 64 * hf, e0, 0, 0, H->b);
-                            tma_load_heads(sbase + kOffV + s * kKVBytes + hf * kKVHalf, &tmEV, bar, P, DH, H->hk * DH + 64 * hf, e0, 0, 0, H->b);
+                            tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, &tmEK, bar, P, H->hk, 64 * hf, e0, 0, 0, H->b);
+                            tma_load_heads(sbase + kOffV + s * kKVBytes + hf * kKVHalf, &tmEV, bar, P, H->hk, 64 * hf, e0, 0, 0, H->b);
                         }
                     }
                 }
@@ -268,9 +250,10 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     const uint64_t dk0 = smem_desc(sbase + kOffK + s * kKVBytes, 16, 1024);
                     tc_fence_after();
 #pragma unroll
-                    for (int ks = 0; ks < DH / 16; ++ks)            // 32 bytes per k-step inside a 64-channel block
+                    for (int ks = 0; ks < (kShort ? DH / 16 - 2 : DH / 16); ++ks) {     // 32 bytes per k-step inside a 64-channel block
                         mma_ss_e(tmem + kColS + s_cols(n_qk), dq0 + ((((ks / 4) * kQHalf) + (ks % 4) * 32) >> 4),
                                  dk0 + ((((ks / 4) * kKVHalf) + (ks % 4) * 32) >> 4), idesc_qk, ks > 0, leader);
+                    }
                     mma_commit_e(bar_s_of(n_qk), leader);
                     if (c + 1 == H->nch) mma_commit_e(bar_qfree, leader);     // last scores of the tile: Q may go once they are done
                 }
@@ -703,20 +686,24 @@ int tc_fused_fwd_small(int dtype, const Geo& g, const void* q, const void* k, co
         return -2;
     if (plan.p.work_q == 0 || g.B == 0) return 0;
     cudaError_t err = cudaSuccess;
-    auto launch = [&](auto dh, auto bf, auto inner) {
+    auto launch = [&](auto dh, auto bf, auto inner, auto shorter) {
         constexpr int kDh = decltype(dh)::value;
         constexpr bool kBf = decltype(bf)::value;
         constexpr int kInner = decltype(inner)::value;
         using FS = FwdSmall<kDh>;
         const unsigned grid = persistent_grid(plan.p.work_q, FS::kPerSm);
-        err = ensure_dynamic_smem((const void*)tc_fwd_small_kernel<kDh, kBf, kInner>, FS::kSmemTotal);
+        err = ensure_dynamic_smem((const void*)tc_fwd_small_kernel<kDh, kBf, kInner, decltype(shorter)::value>, FS::kSmemTotal);
         if (err != cudaSuccess) return;
-        tc_fwd_small_kernel<kDh, kBf, kInner><<<grid, kThreads, FS::kSmemTotal, s>>>(mq, mk, mv, mek, mev, plan.p, (uint16_t*)out, (float*)lse);
+        tc_fwd_small_kernel<kDh, kBf, kInner, decltype(shorter)::value><<<grid, kThreads, FS::kSmemTotal, s>>>(mq, mk, mv, mek, mev, plan.p, (uint16_t*)out, (float*)lse);
+    };
+    auto by_short = [&](auto dh, auto bf, auto inner) {
+        if (g.D <= decltype(dh)::value - 32) launch(dh, bf, inner, std::true_type{});
+        else launch(dh, bf, inner, std::false_type{});
     };
     auto by_inner = [&](auto dh, auto bf) {
-        if (plan.p.cb[2] == 16) launch(dh, bf, std::integral_constant<int, 16>{});
-        else if (plan.p.cb[2] == 32) launch(dh, bf, std::integral_constant<int, 32>{});
-        else launch(dh, bf, std::integral_constant<int, 0>{});
+        if (plan.p.cb[2] == 16) by_short(dh, bf, std::integral_constant<int, 16>{});
+        else if (plan.p.cb[2] == 32) by_short(dh, bf, std::integral_constant<int, 32>{});
+        else by_short(dh, bf, std::integral_constant<int, 0>{});
     };
     auto by_type = [&](auto dh) {
         if (bf16) by_inner(dh, std::true_type{});

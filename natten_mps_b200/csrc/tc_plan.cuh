@@ -45,6 +45,12 @@ struct TcParams {
     // maps then carry the head as an axis of its own ([D, H, X2, X1, B]; ranks 1 and 2) and a 64-channel
     // box reads zeros past the real head dim `dreal`.  Outputs are written `dreal` channels wide.
     int dreal, split_heads;
+    // Rank 3 has no map axis left for the head.  There a 64-channel box of a head dim of 32 or 96 reads 32 channels of the
+    // next head: the score products leave them out (the kernels' kShort: they end 32 channels early, which saves the
+    // padded steps of the other ranks, too), and the accumulated columns past dreal are not written out.  shared_box:
+    // such maps are in use.  hpitch: channels from head to head.  (8 x 28 x 28, 3 x 5 x 5, 6 heads of 32, batch 2, bf16, against the
+    // general kernels that took these before: forward 351 -> 33 us, backward 888 -> 140.)
+    int shared_box, hpitch;
     long long wait_budget; // cycles a barrier wait may take before the CTA gives up
     int inject;            // test hook: 1 = the forward's first query barrier expects bytes that never arrive
     // Output stride (forward only).  Inside dilation group r of an axis the queries sit at the
@@ -102,14 +108,14 @@ __device__ __forceinline__ bool cta_geometry(const TcParams& P, unsigned bx, int
     return active;
 }
 
-// Tile load whose first coordinate is head * dh + channel block: with a head axis of its own in the map
-// (split_heads) the two are separated again.  dh is the kernel's (padded) head dim, a power of two.
+// Tile load of channels ch .. ch + 63 of head h: one coordinate, or two where the map has a head axis of its own.
 __device__ __forceinline__ void tma_load_heads(uint32_t dst, const CUtensorMap* map, uint32_t bar, const TcParams& P,
-                                               int dh, int c0, int c1, int c2, int c3, int c4)
+                                               int h, int ch, int c1, int c2, int c3, int c4)
 {
-    if (P.split_heads) tma_load_5d(dst, map, bar, c0 & (dh - 1), c0 / dh, c1, c2, c4);
-    else tma_load_5d(dst, map, bar, c0, c1, c2, c3, c4);
+    if (P.split_heads) tma_load_5d(dst, map, bar, ch, h, c1, c2, c4);
+    else tma_load_5d(dst, map, bar, h * P.hpitch + ch, c1, c2, c3, c4);
 }
+// Tile store at head * dh + channel block, dh the kernel's (padded) head dim, a power of two.
 __device__ __forceinline__ void tma_store_heads(const CUtensorMap* map, uint32_t src, const TcParams& P, int dh, int c0,
                                                 int c1, int c2, int c3, int c4)
 {
@@ -258,6 +264,25 @@ __device__ __forceinline__ uint32_t piece_word_ranges(const TcParams& P, int pc,
         }
     }
     return w;
+}
+
+// 4 x 4 transpose of 16-byte pieces among four adjacent lanes: w[i] of lane j <-> w[j] of lane i (j = lane & 3).
+__device__ __forceinline__ void transpose4(uint32_t (&w)[4][4], int j)
+{
+#pragma unroll
+    for (int m = 1; m <= 2; m *= 2) {
+        const bool up = j & m;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i & m) continue;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[i][k] : w[i | m][k], m);
+                if (up) w[i][k] = got;
+                else w[i | m][k] = got;
+            }
+        }
+    }
 }
 
 // Packed 16-bit pair arithmetic (element 0 in the low half).
@@ -449,7 +474,9 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
         }
     }
     p.dreal = g.D;
-    p.split_heads = (g.D != 64 && g.D != 128) ? 1 : 0;
+    p.split_heads = (g.D != 64 && g.D != 128 && g.rank < 3) ? 1 : 0;
+    p.shared_box = g.D != 64 && g.D != 128 && !p.split_heads;
+    p.hpitch = g.D;
     p.group_mul = g.group >= 2 ? (unsigned)((0x100000000ull + g.group - 1) / g.group) : 0u;
     p.rank = g.rank; p.B = g.B; p.Hq = g.Hq; p.Hkv = g.Hkv; p.group = g.group;
     p.n_extra = g.n_extra;
@@ -564,16 +591,16 @@ inline bool tc_eligible(int dtype, const Geo& g, const void* q, const void* k, c
 {
     if (dtype != 1 && dtype != 2) return false;                 // f16 / bf16
     if (g.D < 8 || g.D > 128 || g.D % 8 != 0 || g.Dv != g.D) return false;
-    const bool padded = g.D != 64 && g.D != 128;              // zero-padded channels need the head as a map axis of its own
-    if (padded && g.rank > 2) return false;
+    const bool padded = g.D != 64 && g.D != 128;              // zero-padded channels need the head as a map axis of its own (rank 3: see TcParams::shared_box)
+    if (padded && g.rank > 2 && g.D != 32 && g.D != 96) return false;
     if (!(g.scale > 0.0)) return false;
     for (int a = 0; a < g.rank; ++a) {
         if (g.st[a] != 1 && !allow_stride) return false;
         if (!kernel_axis_ok(g, a)) return false;
     }
     // heads must be adjacent so that (head, channel) folds into one map dimension
-    if (!padded && (g.qs[2] != g.D || g.ks[2] != g.D || g.vs[2] != g.Dv)) return false;
-    if (padded && (g.qs[2] % 8 != 0 || g.ks[2] % 8 != 0 || g.vs[2] % 8 != 0)) return false;
+    if ((!padded || g.rank > 2) && (g.qs[2] != g.D || g.ks[2] != g.D || g.vs[2] != g.Dv)) return false;
+    if (padded && g.rank < 3 && (g.qs[2] % 8 != 0 || g.ks[2] % 8 != 0 || g.vs[2] % 8 != 0)) return false;
     const long long strs[6] = {g.qs[0], g.qs[1], g.ks[0], g.ks[1], g.vs[0], g.vs[1]};
     for (long long s : strs)
         if (s % 8 != 0) return false;                           // 16-byte global strides
