@@ -831,6 +831,8 @@ int launch_bwd(int dtype, const Geo& g, const Plan& plan, const void* q, const v
                void* dv, float* delta, cudaStream_t s, const Expanded* ex = nullptr)
 {
     const TcParams& p = plan.p;
+    Plan key_plan = plan;
+    fit_key_boxes(key_plan);
     // With an output stride the kernels run on the unit-stride geometry `g` over full-resolution copies of
     // dout / lse / delta (see expand_strided_kernel); the caller's arrays are only read to build them.
     const void* dout_k = ex ? ex->dout_full : dout;
@@ -846,8 +848,8 @@ int launch_bwd(int dtype, const Geo& g, const Plan& plan, const void* q, const v
         !encode_map(&v_chunk, v, bf, p, g.Hkv, g.D, g.vs, plan.box_kv, false, true) ||
         !encode_map(&k_tile, k, bf, p, g.Hkv, g.D, g.ks, plan.box_q) ||
         !encode_map(&v_tile, v, bf, p, g.Hkv, g.D, g.vs, plan.box_q) ||
-        !encode_map(&q_chunk, q, bf, p, g.Hq, g.D, g.qs, plan.box_kv, false, true) ||
-        !encode_map(&do_chunk, dout_k, bf, p, g.Hq, g.D, dos, plan.box_kv, false, true))
+        !encode_map(&q_chunk, q, bf, key_plan.p, g.Hq, g.D, g.qs, key_plan.box_kv, false, true) ||
+        !encode_map(&do_chunk, dout_k, bf, key_plan.p, g.Hq, g.D, dos, key_plan.box_kv, false, true))
         return -2;
     // outputs: contiguous [B, *L, H, D]; stored as row tiles
     CUtensorMap dq_tile, dk_tile, dv_tile;
@@ -912,7 +914,7 @@ int launch_bwd(int dtype, const Geo& g, const Plan& plan, const void* q, const v
             q_tile, do_tile, k_chunk, v_chunk, ek_chunk, ev_chunk, dq_tile, dq_tile, p, lse_k, delta_k, (uint16_t*)dq, nullptr);
         tc_count_launch();
         tc_bwd_kernel<DH, BF16, true, kInner, kShort><<<grid_k, kThreads, Smem::kTotal, s>>>(
-            k_tile, v_tile, q_chunk, do_chunk, ek_chunk, ev_chunk, dk_tile, dv_tile, p, lse_k, delta_k, (uint16_t*)dk, (uint16_t*)dv);
+            k_tile, v_tile, q_chunk, do_chunk, ek_chunk, ev_chunk, dk_tile, dv_tile, key_plan.p, lse_k, delta_k, (uint16_t*)dk, (uint16_t*)dv);
         tc_count_launch();
     };
     auto by_short = [&](auto inner) {

@@ -137,7 +137,7 @@ __device__ __forceinline__ int chunks_along(const TcParams& P, int a, int extent
 // reference's window arithmetic never reaches the last key with an even kernel).  `exact` = false
 // gives a range that is never empty (a superset, for bounding boxes); with `exact` a key that no query
 // attends to gets qhi < qlo.
-__device__ __forceinline__ void inverse_range(int n, int L, int K, int causal, int& qlo, int& qhi, bool exact = true)
+__host__ __device__ __forceinline__ void inverse_range(int n, int L, int K, int causal, int& qlo, int& qhi, bool exact = true)
 {
     if (causal) {
         qlo = n;
@@ -495,6 +495,35 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
     p.status = status_ptr();
     p.status_host = status_host_ptr();
     return p.status && p.status_host;
+}
+
+// Column count of an interleaved axis for key tiles.  A key next to a clamped edge is read by every query of the edge, so a
+// tile that starts (or ends) inside that range has a longer box than tile - 1 + K columns, and the il chunks of the axis
+// have to hold it: a wider interleave where the tensor map can express it, else blocked chunks.  No cost for the others.
+inline void fit_key_boxes(Plan& plan)
+{
+    TcParams& p = plan.p;
+    for (int a = 0; a < 3; ++a) {
+        if (p.il[a] <= 1) continue;
+        int longest = 0;
+        if (p.extents) longest = p.tile[a] + 2 * p.K[a];         // any length: no tile needs more
+        else
+            for (int rg = 0; rg < p.dil[a]; ++rg) {
+                const int len = (p.L[a] - rg + p.dil[a] - 1) / p.dil[a];
+                for (int o = 0; o < len; o += p.tile[a]) {
+                    int lo, hi, t;
+                    inverse_range(o, len, p.K[a], p.causal[a], lo, t, false);
+                    inverse_range(o + p.tile[a] < len ? o + p.tile[a] - 1 : len - 1, len, p.K[a], p.causal[a], t, hi, false);
+                    longest = hi - lo + 1 > longest ? hi - lo + 1 : longest;
+                }
+            }
+        int il = (longest + p.cb[a] - 1) / p.cb[a];
+        if (il <= p.il[a]) continue;
+        if (p.dil[a] * il > 8 || p.cb[a] * p.dil[a] * il > 256) il = 1;
+        p.il[a] = il;
+        p.il_mul[a] = il > 1 ? (unsigned)((0x100000000ull + il - 1) / il) : 0u;
+        plan.box_kv[a] = p.cb[a] * p.dil[a] * il;
+    }
 }
 
 // 5-D map over [B, X0, X1, X2, heads*D] (innermost first in the arrays below).
