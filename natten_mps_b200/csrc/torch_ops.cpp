@@ -18,6 +18,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <ATen/autocast_mode.h>
 #include <torch/library.h>
 
 #include <algorithm>
@@ -557,6 +558,90 @@ Tensor qk_rpb_autograd(const Tensor& q, const Tensor& k, const Tensor& rpb, IntA
     return QkRpbFn::apply(q, k, rpb, ks, dil, scale);
 }
 
+// The whole module, projections included, as one node of the autograd graph.  Built from the separate operators a training
+// pass of it took 330 us on the host (projections, views, unbind and their thirty backward operators) where the kernels
+// take 165: most of the host time goes into dispatching and into the engine's bookkeeping between small operators.  The
+// products are the ones the separate operators run; the three gradients of the packed projection are put side by side by
+// one copy instead of three.
+struct Projected { Tensor y1, y2, q, k, v; };
+Projected project(const Tensor& x, const Tensor& w1, const OptTensor& b1, const Tensor& w2, const OptTensor& b2, int64_t heads, int64_t kv)
+{
+    auto split = [&](const Tensor& y, int64_t n, int64_t h) {
+        std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end() - 1);
+        if (n > 1) shape.push_back(n);
+        shape.push_back(h);
+        shape.push_back(y.size(-1) / (n * h));
+        return y.view(shape);
+    };
+    Projected r;
+    r.y1 = at::linear(x, w1, b1);
+    if (w2.defined()) {
+        r.y2 = at::linear(x, w2, b2);
+        r.q = split(r.y1, 1, heads);
+        const Tensor t = split(r.y2, 2, kv);
+        r.k = t.select(-3, 0);
+        r.v = t.select(-3, 1);
+    } else {
+        const Tensor t = split(r.y1, 3, heads);
+        r.q = t.select(-3, 0);
+        r.k = t.select(-3, 1);
+        r.v = t.select(-3, 2);
+    }
+    return r;
+}
+Tensor rows_of(const Tensor& t) { return t.reshape({-1, t.size(-1)}); }
+Tensor joined_heads(const Tensor& out)
+{
+    std::vector<int64_t> shape(out.sizes().begin(), out.sizes().end() - 1);
+    shape.back() *= out.size(-1);
+    return out.reshape(shape);
+}
+
+struct ModuleFn : public torch::autograd::Function<ModuleFn> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1, const OptTensor& b1, const OptTensor& w2,
+                          const OptTensor& b2, const Tensor& wp, const OptTensor& bp, int64_t heads, int64_t kv, IntArrayRef ks, IntArrayRef st,
+                          IntArrayRef dil, const Bools& causal, double scale)
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const Projected r = project(x, w1, b1, w2.value_or(Tensor()), b2, heads, kv);
+        auto [out, lse] = call_fused(r.q, r.k, r.v, std::nullopt, std::nullopt, std::nullopt, ks, st, dil, causal, scale);
+        ctx->saved_data["g"] = pack({ks, st, dil}, causal);
+        ctx->saved_data["s"] = scale;
+        ctx->saved_data["m"] = (int64_t)((b1 ? 4 : 0) | (w2 ? 8 : 0) | (b2 ? 16 : 0) | (bp ? 64 : 0) | 35);     // arguments that are there
+        ctx->save_for_backward({x, w1, w2.value_or(Tensor()), wp, r.q, r.k, r.v, out, lse});
+        return at::linear(joined_heads(out), wp, bp);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads)
+    {
+        static const auto op = handle<decltype(fused_bwd_cuda)>("natten_b200::na_fused_bwd");
+        const auto s = ctx->get_saved_variables();
+        const Tensor &x = s[0], &w1 = s[1], &w2 = s[2], &wp = s[3];
+        const Unpacked u(ctx, 3);
+        variable_list r(14);
+        const int64_t there = ctx->saved_data.at("m").toInt();
+        bool needs[7];
+        for (int i = 0, edge = 0; i < 7; ++i) needs[i] = ((there >> i) & 1) && ctx->needs_input_grad(edge++);
+        const Tensor g = rows_of(grads[0]), x2 = rows_of(x);
+        if (needs[6]) r[6] = g.sum(0);           // (a kernel first: it makes the device's context current on the engine's thread)
+        if (needs[5]) r[5] = g.t().mm(rows_of(joined_heads(s[7])));
+        bool inner = false;
+        for (int i = 0; i < 5; ++i) inner = inner || needs[i];
+        if (!inner) return r;
+        auto [dq, dk, dv, dek, dev] = op.call(s[4], s[5], s[6], std::nullopt, std::nullopt, std::nullopt, s[7], s[8],
+                                              g.mm(wp).view(s[7].sizes()), std::nullopt, u.list(0), u.list(1), u.list(2), u.flags(3),
+                                              *saved_scale(ctx));
+        auto flat = [&](const Tensor& t) { return t.reshape({x2.size(0), -1}); };
+        const Tensor d1 = w2.defined() ? flat(dq) : at::cat({flat(dq), flat(dk), flat(dv)}, 1);
+        const Tensor d2 = w2.defined() ? at::cat({flat(dk), flat(dv)}, 1) : Tensor();
+        if (needs[0]) r[0] = (w2.defined() ? at::addmm(d1.mm(w1), d2, w2) : d1.mm(w1)).view(x.sizes());
+        if (needs[1]) r[1] = d1.t().mm(x2);
+        if (needs[2]) r[2] = d1.sum(0);
+        if (needs[3]) r[3] = d2.t().mm(x2);
+        if (needs[4]) r[4] = d2.sum(0);
+        return r;
+    }
+};
+
 // ----------------------------------------------------------------------------- argument parsing for functional.py
 // An integer per axis from an int or a tuple / list of ints; every value positive (bools are not integers here).
 bool ints(PyObject* o, int rank, int64_t (&out)[3])
@@ -692,6 +777,68 @@ PyObject* py_na(PyObject*, PyObject* const* args, Py_ssize_t n)
     END_HANDLE_TH_ERRORS
 }
 
+// na_module(rank, x, w1, b1 | None, w2 | None, b2 | None, proj weight, proj bias | None, heads, kv heads, kernel_size, stride,
+// dilation, is_causal, scale): the packed (w1) or separate (w1, w2) projections, attention and the output projection
+PyObject* py_module(PyObject*, PyObject* const* args, Py_ssize_t n)
+{
+    HANDLE_TH_ERRORS
+    const int rank = n == 15 ? (int)PyLong_AsLong(args[0]) : 0;
+    if (rank < 1 || rank > 3 || at::impl::torch_function_mode_enabled() || c10::impl::dispatch_mode_enabled() ||
+        at::autocast::is_autocast_enabled(at::kCUDA) || PyLong_AsLong(args[8]) < 1 || PyLong_AsLong(args[9]) < 1)
+        return not_handled();
+    // anything that wraps tensors or records them (functorch, functionalisation, subclasses) takes the separate operators
+    const c10::DispatchKeySet plain({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
+                                     c10::DispatchKey::AutocastCUDA});
+    const c10::DispatchKeySet modes({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::FuncTorchDynamicLayerBackMode,
+                                     c10::DispatchKey::Functionalize, c10::DispatchKey::Python});
+    if (!(c10::impl::tls_local_dispatch_key_set().included_ & modes).empty()) return not_handled();
+    const int64_t heads = PyLong_AsLong(args[8]), kv = PyLong_AsLong(args[9]);
+    Tensor t[7];
+    for (int i = 0; i < 7; ++i) {
+        if (args[1 + i] == Py_None) continue;
+        const Tensor* p = tensor(args[1 + i], i == 0 ? rank + 2 : i % 2 ? 2 : 1);
+        if (!p || (p->key_set() - plain).highestFunctionalityKey() != c10::DispatchKey::Undefined || p->layout() != at::kStrided || p->numel() == 0) return not_handled();
+        t[i] = *p;
+        if (!t[0].defined() || p->scalar_type() != t[0].scalar_type() || p->device() != t[0].device()) return not_handled();
+    }
+    const Tensor &x = t[0], &w1 = t[1], &b1 = t[2], &w2 = t[3], &b2 = t[4], &wp = t[5], &bp = t[6];
+    if (!x.defined() || !w1.defined() || !wp.defined() || !x.is_cuda() || (b2.defined() && !w2.defined())) return not_handled();
+    const int64_t C = x.size(-1), D = C / heads;
+    if (D * heads != C || heads % kv != 0 || w1.size(0) != (w2.defined() ? C : 3 * C) || w1.size(1) != C || wp.size(0) != C ||
+        wp.size(1) != C || (w2.defined() ? w2.size(0) != 2 * kv * D || w2.size(1) != C : kv != heads) ||
+        (b1.defined() && b1.size(0) != w1.size(0)) || (b2.defined() && b2.size(0) != w2.size(0)) || (bp.defined() && bp.size(0) != C))
+        return not_handled();
+    int64_t ks[3], st[3], dil[3];
+    Bools causal;
+    bool any_causal = false;
+    std::optional<double> scale;
+    if (!ints(args[10], rank, ks) || !ints(args[11], rank, st) || !ints(args[12], rank, dil) || !flags(args[13], rank, causal, any_causal) ||
+        !number(args[14], scale) || !scale || !kernel_fits(x, rank, ks, dil))
+        return not_handled();
+    bool covers = !any_causal;               // global attention, not ours
+    for (int a = 0; a < rank; ++a) {
+        if (st[a] > ks[a]) return not_handled();
+        covers = covers && ks[a] >= x.size(1 + a) && st[a] == 1;
+    }
+    if (covers) return not_handled();
+    Tensor out;
+    {
+        NoGil nogil;
+        const IntArrayRef ksr(ks, rank), str(st, rank), dilr(dil, rank);
+        auto opt = [](const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
+        if (wants_grad({&x, &w1, &b1, &w2, &b2, &wp, &bp})) {
+            out = ModuleFn::apply(x, w1, opt(b1), opt(w2), opt(b2), wp, opt(bp), heads, kv, ksr, str, dilr, causal, *scale);
+        } else {
+            at::AutoDispatchBelowADInplaceOrView below;
+            const Projected r = project(x, w1, opt(b1), w2, opt(b2), heads, kv);
+            out = at::linear(joined_heads(std::get<0>(call_fused(r.q, r.k, r.v, std::nullopt, std::nullopt, std::nullopt, ksr, str, dilr,
+                                                                 std::move(causal), *scale))), wp, opt(bp));
+        }
+    }
+    return wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
 // na_varlen(rank, query, key, value, sizes, kernel_size, dilation, scale, extra_k, extra_v)
 PyObject* py_varlen(PyObject*, PyObject* const* args, Py_ssize_t n)
 {
@@ -805,6 +952,7 @@ PyObject* py_set_flags(PyObject*, PyObject* o)
 
 PyMethodDef kMethods[] = {
     {"na", (PyCFunction)(void (*)(void))py_na, METH_FASTCALL, nullptr},
+    {"na_module", (PyCFunction)(void (*)(void))py_module, METH_FASTCALL, nullptr},
     {"na_varlen", (PyCFunction)(void (*)(void))py_varlen, METH_FASTCALL, nullptr},
     {"na_qk", (PyCFunction)(void (*)(void))py_qk, METH_FASTCALL, nullptr},
     {"na_av", (PyCFunction)(void (*)(void))py_av, METH_FASTCALL, nullptr},

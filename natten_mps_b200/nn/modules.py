@@ -14,13 +14,21 @@ from typing import Optional, Tuple, Union
 import torch
 
 from .. import functional as F
+from .._torch_ops import native
 from ..utils.params import normalize_tuple_param
 
 _FUSED = {1: F.na1d, 2: F.na2d, 3: F.na3d}
 _QK = {1: F.na1d_qk, 2: F.na2d_qk, 3: F.na3d_qk}
 _AV = {1: F.na1d_av, 2: F.na2d_av, 3: F.na3d_av}
 _VARLEN = {1: F.na1d_varlen, 2: F.na2d_varlen, 3: F.na3d_varlen}
+_NO_PARAMETERS: dict = {}
 _IN_LAYOUT = {1: "[B, L, C]", 2: "[B, H, W, C]", 3: "[B, D, H, W, C]"}
+
+
+def _plain_linear(m) -> bool:
+    """A Linear whose call does nothing but the product: no hooks, no patched forward, not a subclass."""
+    return (type(m) is torch.nn.Linear and not m._forward_hooks and not m._forward_pre_hooks and not m._backward_hooks
+            and not m._backward_pre_hooks and "forward" not in m.__dict__)
 
 
 class _NeighborhoodAttention(torch.nn.Module):
@@ -67,6 +75,22 @@ class _NeighborhoodAttention(torch.nn.Module):
             q, k, v = self.qkv(x).reshape(*lead, 3, self.num_heads, self.head_dim).unbind(dim=-3)
         return q, k, v
 
+    def _in_one_call(self, x):
+        """Projections and attention as one native call (one autograd node); NotImplemented where the sub-modules are not
+        the plain ones of ``__init__`` or the call needs the separate operators for another reason."""
+        sub = self._modules
+        proj, drop = sub["proj"], sub["proj_drop"]
+        first, second = (sub["q_proj"], sub["kv_proj"]) if self._use_gqa else (sub["qkv"], None)
+        if (type(drop) is not torch.nn.Dropout or (drop.training and drop.p > 0.0) or drop._forward_hooks or drop._forward_pre_hooks
+                or drop._backward_hooks or drop._backward_pre_hooks or not _plain_linear(proj) or not _plain_linear(first)
+                or (second is not None and not _plain_linear(second)) or torch.nn.modules.module._has_any_global_hook()
+                or type(self)._project is not _NeighborhoodAttention._project or torch.compiler.is_compiling()):
+            return NotImplemented
+        p1, p2, po = first._parameters, second._parameters if second is not None else _NO_PARAMETERS, proj._parameters
+        return native.na_module(self.rank, x, p1.get("weight"), p1.get("bias"), p2.get("weight"), p2.get("bias"), po.get("weight"),
+                                po.get("bias"), self.num_heads, self.num_kv_heads, self.kernel_size, self.stride, self.dilation,
+                                self.is_causal, self.scale)
+
     def forward(self, x: torch.Tensor, sizes: Optional[torch.Tensor] = None) -> torch.Tensor:
         r = self.rank
         if x.ndim != r + 2:
@@ -74,6 +98,10 @@ class _NeighborhoodAttention(torch.nn.Module):
         if x.shape[-1] != self.embed_dim:
             raise ValueError(
                 f"Input channel dim ({x.shape[-1]}) must equal embed_dim ({self.embed_dim}).")
+        if sizes is None and self.attn_drop_p <= 0.0:
+            out = self._in_one_call(x)
+            if out is not NotImplemented:
+                return out
         q, k, v = self._project(x)
         if sizes is not None:
             out = _VARLEN[r](q, k, v, sizes, kernel_size=self.kernel_size, dilation=self.dilation,

@@ -1,0 +1,44 @@
+"""The module as one native call against its separate operators (what it does with a hook in place): outputs and every
+gradient, packed and grouped projections, output stride, missing biases, frozen parameters, inference, a strided input."""
+import pytest
+import torch
+
+import natten_mps_b200 as nb
+
+pytestmark = pytest.mark.gpu
+
+CASES = [("2d", nb.NeighborhoodAttention2D, (13, 17), dict(kernel_size=5)),
+         ("2d_gqa", nb.NeighborhoodAttention2D, (12, 15), dict(kernel_size=(3, 5), dilation=(2, 1), num_kv_heads=2)),
+         ("1d_stride", nb.NeighborhoodAttention1D, (41,), dict(kernel_size=7, stride=2, qkv_bias=False)),
+         ("3d_causal", nb.NeighborhoodAttention3D, (3, 8, 9), dict(kernel_size=3, is_causal=(True, False, False), qk_scale=0.3))]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: c[0])
+def test_one_call_matches_the_separate_operators(case, dtype):
+    _, cls, size, kw = case
+    torch.manual_seed(1)
+    m = cls(128, 4, **kw).to("cuda", dtype)
+    base = torch.randn(2, *size, 160, device="cuda", dtype=dtype)
+    x = base[..., :128].requires_grad_(True)                     # rows are not adjacent
+    frozen = m.proj.weight
+    for step in ("all", "frozen", "inference"):
+        frozen.requires_grad_(step == "all")
+        leaves = [x] + [p for p in m.parameters() if p.requires_grad]
+        got = []
+        for hook in (False, True):
+            h = m.proj.register_forward_hook(lambda *a: None) if hook else None
+            with torch.set_grad_enabled(step != "inference"):
+                y = m(x)
+            assert y.requires_grad == (step != "inference")
+            if step != "inference":
+                names = y.grad_fn.name()
+                assert ("ModuleFn" in names) != hook, names
+                got.append([y, *torch.autograd.grad(y, leaves, torch.linspace(-1, 1, y.numel(), device="cuda").view_as(y).to(dtype))])
+            else:
+                got.append([y])
+            if h is not None:
+                h.remove()
+        for a, b in zip(*got):
+            tol = 1e-5 if dtype == torch.float32 else 1e-2
+            assert a.shape == b.shape and (a.float() - b.float()).norm() <= tol * b.float().norm().clamp_min(1e-3)
