@@ -252,6 +252,17 @@ template <int LPQ> __device__ __forceinline__ float reduce4(float s0, float s1, 
 // The value of row j, from the lane that has it.
 __device__ __forceinline__ float row_value(float v, int lane, int c, int j) { return __shfl_sync(0xffffffffu, v, (lane - c) | j); }
 __device__ __forceinline__ uint64_t twice(float v) { return pack2(v, v); }
+// Bits 0 .. 3: does the column at hand belong to rows 0 .. 3 of the group?  (ok: to the lane's own row.)
+__device__ __forceinline__ uint32_t rows_with(bool ok, int lane, int c) { return __ballot_sync(0xffffffffu, ok) >> (lane - c); }
+// acc += w * x where `on` is not zero
+__device__ __forceinline__ void add_if(uint32_t on, uint64_t (&acc)[4], uint64_t w, const uint64_t (&x)[4])
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %9, 0;\n\t"
+        "@p fma.rn.f32x2 %0, %8, %4, %0;\n\t@p fma.rn.f32x2 %1, %8, %5, %1;\n\t"
+        "@p fma.rn.f32x2 %2, %8, %6, %2;\n\t@p fma.rn.f32x2 %3, %8, %7, %3;\n\t}"
+        : "+l"(acc[0]), "+l"(acc[1]), "+l"(acc[2]), "+l"(acc[3])
+        : "l"(x[0]), "l"(x[1]), "l"(x[2]), "l"(x[3]), "l"(w), "r"(on));
+}
 
 // A lane's view of its group's four rows.
 template <int D, bool LINE, bool kKeySide> struct RowsF {
@@ -319,6 +330,27 @@ template <int D, bool LINE, bool kKeySide> struct RowsF {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) x[j][i] = 0ull;
     }
+    // acc[row] += a * xa + b * xb over the group's rows, a and b from the lane that has the row (zero where it does not attend
+    // to the column).  kExact: the columns that a row does not attend to are left out, whatever they hold; see exact_if_tainted.
+    template <bool kExact>
+    __device__ __forceinline__ void add_pair(uint64_t (&acc)[4][4], bool ok_a, float a, const uint64_t (&xa)[4], bool ok_b, float b,
+                                             const uint64_t (&xb)[4]) const
+    {
+        const uint32_t in_a = kExact ? rows_with(ok_a, lane, c) : 0u, in_b = kExact ? rows_with(ok_b, lane, c) : 0u;
+        a = ok_a ? a : 0.f;
+        b = ok_b ? b : 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t a2 = twice(row_value(a, lane, c, j)), b2 = twice(row_value(b, lane, c, j));
+            if constexpr (kExact) {
+                add_if(in_a & (1u << j), acc[j], a2, xa);
+                add_if(in_b & (1u << j), acc[j], b2, xb);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[j][i] = fma2(b2, xb[i], fma2(a2, xa[i], acc[j][i]));
+            }
+        }
+    }
     // Walk the staged chunk [y0, y1) x [s0, s1) two columns at a time (independent chains for the scheduler): neighbours along
     // a1 (rank 1: along a2), of which a group's union has an even number when the kernel size is odd.
     // body(shared-memory column of the first, of the second, whether each belongs to the lane's own row, box-relative row and column
@@ -379,6 +411,33 @@ __device__ __forceinline__ void for_chunks(const FmaParams& P, const TileF& T, S
             }
 }
 
+__device__ __forceinline__ void clear(uint64_t (&acc)[4][4])
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
+}
+// Not 0: some value is NaN or Inf.
+__device__ __forceinline__ int tainted(const uint64_t (&acc)[4][4])
+{
+    uint64_t t = 0ull;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t = fma2(acc[j][i], 0ull, t);
+    return lo_of(t) + hi_of(t) == 0.f ? 0 : 1;
+}
+// Runs pass(false), and pass(true) over it if that left a NaN or Inf in the CTA's sums (taint()).  Four rows share every column,
+// and the plain pass gives a row that does not attend to it a weight of zero, which a NaN or Inf turns into NaN; the exact pass
+// leaves it out.  Exact arithmetic throughout (a vote, and a predicate per row and column) took a float32 training step of
+// 56 x 56, 7 x 7, 4 heads of 32, batch 4 from 155 to 199 us; the test at the end takes it to 160.
+template <typename Pass, typename Taint> __device__ __forceinline__ void exact_if_tainted(Pass&& pass, Taint&& taint)
+{
+    pass(std::false_type{});
+    if (__syncthreads_or(taint())) pass(std::true_type{});
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // fused forward.  Row i's stabiliser lives in lane i of its group: the first score it meets; moved (everything
 // accumulated so far is rescaled, a warp-uniform branch) only when a score exceeds it by 2^30.
@@ -396,52 +455,49 @@ fma_fwd_kernel(const __grid_constant__ FmaParams P, T* __restrict__ out, float* 
     R.init(P, Ti);
     uint64_t q[4][4], acc[4][4];
     R.template load_rows<T>(P, Ti, P.row1, b, h, q);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
-    float m = -1e30f, l = 0.f;                                // finite: masked scores (-inf) minus it stay -inf
+    float m, l;
     float* vs = sm + P.chunk_rows * P.chunk_cols * D;
-    for_chunks(P, Ti,
-        [&](int x0, int y0, int y1, int s0, int s1) {
-            stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm);
-            stage_cols<T, D, LINE>(P, Ti, P.col2, b, hk, x0, y0, y1, s0, s1, vs);
-        },
-        [&](int, int y0, int y1, int s0, int s1) {
-            R.walk(P, y0, y1, s0, s1, [&](int xa, int xb, bool ok_a, bool ok_b, int, int) {
-                uint64_t ka[4], kb[4], va[4], vb[4];
-                read_col<D, LINE>(sm, xa, R.c, ka);
-                read_col<D, LINE>(sm, xb, R.c, kb);
-                float sa = reduce4<LF::LPQ>(dot8(q[0], ka), dot8(q[1], ka), dot8(q[2], ka), dot8(q[3], ka), R.c) * P.scale_log2;
-                float sb = reduce4<LF::LPQ>(dot8(q[0], kb), dot8(q[1], kb), dot8(q[2], kb), dot8(q[3], kb), R.c) * P.scale_log2;
-                read_col<D, LINE>(vs, xa, R.c, va);
-                read_col<D, LINE>(vs, xb, R.c, vb);
-                sa = ok_a ? sa : -INFINITY;
-                sb = ok_b ? sb : -INFINITY;
-                const float top = fmaxf(sa, sb);
-                if (__any_sync(0xffffffffu, top > m + 30.f)) {
-                    const bool grow = top > m + 30.f;
-                    const float fac = grow ? fast_exp2(m - top) : 1.f;
-                    if (grow) m = top;
-                    l *= fac;
+    exact_if_tainted([&](auto exact) {
+        constexpr bool kExact = decltype(exact)::value;
+        clear(acc);
+        m = -1e30f;                                          // finite: masked scores (-inf) minus it stay -inf
+        l = 0.f;
+        for_chunks(P, Ti,
+            [&](int x0, int y0, int y1, int s0, int s1) {
+                stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm);
+                stage_cols<T, D, LINE>(P, Ti, P.col2, b, hk, x0, y0, y1, s0, s1, vs);
+            },
+            [&](int, int y0, int y1, int s0, int s1) {
+                R.walk(P, y0, y1, s0, s1, [&](int xa, int xb, bool ok_a, bool ok_b, int, int) {
+                    uint64_t ka[4], kb[4], va[4], vb[4];
+                    read_col<D, LINE>(sm, xa, R.c, ka);
+                    read_col<D, LINE>(sm, xb, R.c, kb);
+                    float sa = reduce4<LF::LPQ>(dot8(q[0], ka), dot8(q[1], ka), dot8(q[2], ka), dot8(q[3], ka), R.c) * P.scale_log2;
+                    float sb = reduce4<LF::LPQ>(dot8(q[0], kb), dot8(q[1], kb), dot8(q[2], kb), dot8(q[3], kb), R.c) * P.scale_log2;
+                    read_col<D, LINE>(vs, xa, R.c, va);
+                    read_col<D, LINE>(vs, xb, R.c, vb);
+                    sa = ok_a ? sa : -INFINITY;
+                    sb = ok_b ? sb : -INFINITY;
+                    const float top = fmaxf(sa, sb);
+                    if (__any_sync(0xffffffffu, top > m + 30.f)) {
+                        const bool grow = top > m + 30.f;
+                        const float fac = grow ? fast_exp2(m - top) : 1.f;
+                        if (grow) m = top;
+                        l *= fac;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint64_t f2 = twice(row_value(fac, R.lane, R.c, j));
+                        for (int j = 0; j < 4; ++j) {
+                            const uint64_t f2 = twice(row_value(fac, R.lane, R.c, j));
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) acc[j][i] = mul2(acc[j][i], f2);
+                            for (int i = 0; i < 4; ++i) acc[j][i] = mul2(acc[j][i], f2);
+                        }
                     }
-                }
-                const float pa = fast_exp2(sa - m), pb = fast_exp2(sb - m);
-                l += pa + pb;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint64_t pa2 = twice(row_value(pa, R.lane, R.c, j)), pb2 = twice(row_value(pb, R.lane, R.c, j));
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[j][i] = fma2(pb2, vb[i], fma2(pa2, va[i], acc[j][i]));
-                }
+                    const float pa = fast_exp2(sa - m), pb = fast_exp2(sb - m);
+                    l += pa + pb;
+                    R.template add_pair<kExact>(acc, ok_a, pa, va, ok_b, pb, vb);
+                });
             });
-        });
-    const float inv = l > 0.f ? 1.f / l : 0.f;
+    }, [&] { return tainted(acc); });
+    const float inv = 1.f / l;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const uint64_t f2 = twice(row_value(inv, R.lane, R.c, j));
@@ -451,7 +507,7 @@ fma_fwd_kernel(const __grid_constant__ FmaParams P, T* __restrict__ out, float* 
         store8<T>(out + (((long long)b * P.ltot + R.flat(P, Ti, j)) * P.Hq + h) * D + 8 * R.c, acc[j]);
     }
     if (R.c < 4 && R.exists(Ti, R.c))
-        lse[((long long)b * P.ltot + R.flat(P, Ti, R.c)) * P.Hq + h] = l > 0.f ? (m + log2f(l)) * kLn2 : 0.f;
+        lse[((long long)b * P.ltot + R.flat(P, Ti, R.c)) * P.Hq + h] = (m + log2f(l)) * kLn2;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -485,37 +541,31 @@ fma_bwd_q_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ out,
         }
     }
     R.template load_rows<T>(P, Ti, P.row1, b, h, q);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
     float* vs = sm + P.chunk_rows * P.chunk_cols * D;
-    for_chunks(P, Ti,
-        [&](int x0, int y0, int y1, int s0, int s1) {
-            stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm);
-            stage_cols<T, D, LINE>(P, Ti, P.col2, b, hk, x0, y0, y1, s0, s1, vs);
-        },
-        [&](int, int y0, int y1, int s0, int s1) {
-            R.walk(P, y0, y1, s0, s1, [&](int xa, int xb, bool ok_a, bool ok_b, int, int) {
-                auto one = [&](int x, bool ok, uint64_t (&k)[4]) {
-                    uint64_t v[4];
-                    read_col<D, LINE>(sm, x, R.c, k);
-                    read_col<D, LINE>(vs, x, R.c, v);
-                    const float s = reduce4<LF::LPQ>(dot8(q[0], k), dot8(q[1], k), dot8(q[2], k), dot8(q[3], k), R.c);
-                    const float dp = reduce4<LF::LPQ>(dot8(go[0], v), dot8(go[1], v), dot8(go[2], v), dot8(go[3], v), R.c);
-                    const float ds = fast_exp2(fmaf(s, P.scale_log2, -lse2)) * (dp - dl) * P.scale;
-                    return ok ? ds : 0.f;
-                };
-                uint64_t ka[4], kb[4];
-                const float da = one(xa, ok_a, ka), db = one(xb, ok_b, kb);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint64_t da2 = twice(row_value(da, R.lane, R.c, j)), db2 = twice(row_value(db, R.lane, R.c, j));
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[j][i] = fma2(db2, kb[i], fma2(da2, ka[i], acc[j][i]));
-                }
+    exact_if_tainted([&](auto exact) {
+        constexpr bool kExact = decltype(exact)::value;
+        clear(acc);
+        for_chunks(P, Ti,
+            [&](int x0, int y0, int y1, int s0, int s1) {
+                stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm);
+                stage_cols<T, D, LINE>(P, Ti, P.col2, b, hk, x0, y0, y1, s0, s1, vs);
+            },
+            [&](int, int y0, int y1, int s0, int s1) {
+                R.walk(P, y0, y1, s0, s1, [&](int xa, int xb, bool ok_a, bool ok_b, int, int) {
+                    auto one = [&](int x, uint64_t (&k)[4]) {
+                        uint64_t v[4];
+                        read_col<D, LINE>(sm, x, R.c, k);
+                        read_col<D, LINE>(vs, x, R.c, v);
+                        const float s = reduce4<LF::LPQ>(dot8(q[0], k), dot8(q[1], k), dot8(q[2], k), dot8(q[3], k), R.c);
+                        const float dp = reduce4<LF::LPQ>(dot8(go[0], v), dot8(go[1], v), dot8(go[2], v), dot8(go[3], v), R.c);
+                        return fast_exp2(fmaf(s, P.scale_log2, -lse2)) * (dp - dl) * P.scale;
+                    };
+                    uint64_t ka[4], kb[4];
+                    const float da = one(xa, ka), db = one(xb, kb);
+                    R.template add_pair<kExact>(acc, ok_a, da, ka, ok_b, db, kb);
+                });
             });
-        });
+    }, [&] { return tainted(acc); });
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (R.exists(Ti, j)) store8<T>(dq + (((long long)b * P.ltot + R.flat(P, Ti, j)) * P.Hq + h) * D + 8 * R.c, acc[j]);
@@ -539,53 +589,44 @@ fma_bwd_k_kernel(const __grid_constant__ FmaParams P, const float* __restrict__ 
     uint64_t k[4][4], v[4][4], ak[4][4], av[4][4];
     R.template load_rows<T>(P, Ti, P.row1, b, hk, k);
     R.template load_rows<T>(P, Ti, P.row2, b, hk, v);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ak[j][i] = av[j][i] = 0ull;
     const int cells = P.chunk_rows * P.chunk_cols;
     float* gs = sm + cells * D;
     float2* stats = reinterpret_cast<float2*>(gs + cells * D);       // lse * log2(e), delta of the chunk's queries
-    for (int h = hk * P.group; h < (hk + 1) * P.group; ++h)
-        for_chunks(P, Ti,
-            [&](int x0, int y0, int y1, int s0, int s1) {
-                stage_cols<T, D, LINE>(P, Ti, P.col1, b, h, x0, y0, y1, s0, s1, sm);
-                stage_cols<T, D, LINE>(P, Ti, P.col2, b, h, x0, y0, y1, s0, s1, gs);
-                for (int y = y0 + (threadIdx.x >> 5); y < y1; y += kWarpsF)
-                    for (int x = s0 + (threadIdx.x & 31); x < s1; x += 32) {
-                        const long long row = ((long long)b * P.ltot + flat_of(P, Ti, x0, Ti.lo[1] + y, Ti.lo[2] + x)) * P.Hq + h;
-                        stats[(y - y0) * P.chunk_cols + (x - s0)] = make_float2(lse[row] * kLog2e, delta[row]);
-                    }
-            },
-            [&](int, int y0, int y1, int s0, int s1) {
-                R.walk(P, y0, y1, s0, s1, [&](int xa, int xb, bool ok_a, bool ok_b, int, int) {
-                    auto one = [&](int x, bool ok, uint64_t (&q)[4], uint64_t (&go)[4], float& p, float& ds) {
-                        read_col<D, LINE>(sm, x, R.c, q);
-                        read_col<D, LINE>(gs, x, R.c, go);
-                        const float2 st = stats[x];
-                        const float s = reduce4<LF::LPQ>(dot8(k[0], q), dot8(k[1], q), dot8(k[2], q), dot8(k[3], q), R.c);
-                        const float dp = reduce4<LF::LPQ>(dot8(v[0], go), dot8(v[1], go), dot8(v[2], go), dot8(v[3], go), R.c);
-                        p = fast_exp2(fmaf(s, P.scale_log2, -st.x));
-                        ds = p * (dp - st.y) * P.scale;
-                        p = ok ? p : 0.f;
-                        ds = ok ? ds : 0.f;
-                    };
-                    uint64_t qa[4], qb[4], ga[4], gb[4];
-                    float pa, pb, da, db;
-                    one(xa, ok_a, qa, ga, pa, da);
-                    one(xb, ok_b, qb, gb, pb, db);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint64_t pa2 = twice(row_value(pa, R.lane, R.c, j)), pb2 = twice(row_value(pb, R.lane, R.c, j));
-                        const uint64_t da2 = twice(row_value(da, R.lane, R.c, j)), db2 = twice(row_value(db, R.lane, R.c, j));
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            av[j][i] = fma2(pb2, gb[i], fma2(pa2, ga[i], av[j][i]));
-                            ak[j][i] = fma2(db2, qb[i], fma2(da2, qa[i], ak[j][i]));
+    exact_if_tainted([&](auto exact) {
+        constexpr bool kExact = decltype(exact)::value;
+        clear(ak);
+        clear(av);
+        for (int h = hk * P.group; h < (hk + 1) * P.group; ++h)
+            for_chunks(P, Ti,
+                [&](int x0, int y0, int y1, int s0, int s1) {
+                    stage_cols<T, D, LINE>(P, Ti, P.col1, b, h, x0, y0, y1, s0, s1, sm);
+                    stage_cols<T, D, LINE>(P, Ti, P.col2, b, h, x0, y0, y1, s0, s1, gs);
+                    for (int y = y0 + (threadIdx.x >> 5); y < y1; y += kWarpsF)
+                        for (int x = s0 + (threadIdx.x & 31); x < s1; x += 32) {
+                            const long long row = ((long long)b * P.ltot + flat_of(P, Ti, x0, Ti.lo[1] + y, Ti.lo[2] + x)) * P.Hq + h;
+                            stats[(y - y0) * P.chunk_cols + (x - s0)] = make_float2(lse[row] * kLog2e, delta[row]);
                         }
-                    }
+                },
+                [&](int, int y0, int y1, int s0, int s1) {
+                    R.walk(P, y0, y1, s0, s1, [&](int xa, int xb, bool ok_a, bool ok_b, int, int) {
+                        auto one = [&](int x, uint64_t (&q)[4], uint64_t (&go)[4], float& p, float& ds) {
+                            read_col<D, LINE>(sm, x, R.c, q);
+                            read_col<D, LINE>(gs, x, R.c, go);
+                            const float2 st = stats[x];
+                            const float s = reduce4<LF::LPQ>(dot8(k[0], q), dot8(k[1], q), dot8(k[2], q), dot8(k[3], q), R.c);
+                            const float dp = reduce4<LF::LPQ>(dot8(v[0], go), dot8(v[1], go), dot8(v[2], go), dot8(v[3], go), R.c);
+                            p = fast_exp2(fmaf(s, P.scale_log2, -st.x));
+                            ds = p * (dp - st.y) * P.scale;
+                        };
+                        uint64_t qa[4], qb[4], ga[4], gb[4];
+                        float pa, pb, da, db;
+                        one(xa, qa, ga, pa, da);
+                        one(xb, qb, gb, pb, db);
+                        R.template add_pair<kExact>(av, ok_a, pa, ga, ok_b, pb, gb);
+                        R.template add_pair<kExact>(ak, ok_a, da, qa, ok_b, db, qb);
+                    });
                 });
-            });
+    }, [&] { return tainted(ak) | tainted(av); });
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (R.exists(Ti, j)) {
@@ -732,32 +773,27 @@ fma_apply_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ w, T
     const int own = R.c & 3;
     const T* mine = w + (R.exists(Ti, own) ? (((long long)b * P.ltot + R.flat(P, Ti, own)) * P.Hq + h) * P.ktot : 0ll);
     uint64_t acc[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
-    for_chunks(P, Ti,
-        [&](int x0, int y0, int y1, int s0, int s1) { stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm); },
-        [&](int x0, int y0, int y1, int s0, int s1) {
-            const int at = S.at(x0);
-            T wa8[kAheadF], wb8[kAheadF];
-            R.template walk_ahead<kAheadF>(P, y0, y1, s0, s1, [&](int u, bool ok_a, bool ok_b, int y, int x) {
-                const int slot = at + y * P.K[2] + x;
-                wa8[u] = mine[ok_a ? slot : 0];
-                wb8[u] = mine[ok_b ? slot + (LINE ? 1 : P.K[2]) : 0];
-            }, [&](int u, int xa, int xb, bool ok_a, bool ok_b, int, int) {
-                const float wa = ok_a ? widen(wa8[u]) : 0.f, wb = ok_b ? widen(wb8[u]) : 0.f;
-                uint64_t va[4], vb[4];
-                read_col<D, LINE>(sm, xa, R.c, va);
-                read_col<D, LINE>(sm, xb, R.c, vb);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint64_t wa2 = twice(row_value(wa, R.lane, R.c, j)), wb2 = twice(row_value(wb, R.lane, R.c, j));
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[j][i] = fma2(wb2, vb[i], fma2(wa2, va[i], acc[j][i]));
-                }
+    exact_if_tainted([&](auto exact) {
+        constexpr bool kExact = decltype(exact)::value;
+        clear(acc);
+        for_chunks(P, Ti,
+            [&](int x0, int y0, int y1, int s0, int s1) { stage_cols<T, D, LINE>(P, Ti, P.col1, b, hk, x0, y0, y1, s0, s1, sm); },
+            [&](int x0, int y0, int y1, int s0, int s1) {
+                const int at = S.at(x0);
+                T wa8[kAheadF], wb8[kAheadF];
+                R.template walk_ahead<kAheadF>(P, y0, y1, s0, s1, [&](int u, bool ok_a, bool ok_b, int y, int x) {
+                    const int slot = at + y * P.K[2] + x;
+                    wa8[u] = mine[ok_a ? slot : 0];
+                    wb8[u] = mine[ok_b ? slot + (LINE ? 1 : P.K[2]) : 0];
+                }, [&](int u, int xa, int xb, bool ok_a, bool ok_b, int, int) {
+                    const float wa = widen(wa8[u]), wb = widen(wb8[u]);
+                    uint64_t va[4], vb[4];
+                    read_col<D, LINE>(sm, xa, R.c, va);
+                    read_col<D, LINE>(sm, xb, R.c, vb);
+                    R.template add_pair<kExact>(acc, ok_a, wa, va, ok_b, wb, vb);
+                });
             });
-        });
+    }, [&] { return tainted(acc); });
     const uint64_t sc2 = twice(P.scale);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -782,41 +818,36 @@ fma_gather_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ w, 
     R.init(P, Ti);
     const int n1 = R.row1(R.c & 3), n2 = R.row2(R.c & 3);
     uint64_t acc[4][4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
-    for (int h = hk * P.group; h < (hk + 1) * P.group; ++h)
-        for_chunks(P, Ti,
-            [&](int x0, int y0, int y1, int s0, int s1) { stage_cols<T, D, LINE>(P, Ti, P.col1, b, h, x0, y0, y1, s0, s1, sm); },
-            [&](int x0, int y0, int y1, int s0, int s1) {
-                // element of w: row of query (y, x), slot of the own key in its window (offsets within a sample fit 32 bits)
-                const int w2 = P.dil[2] * P.Hq * P.ktot, w1 = P.dil[1] * P.L[2] * P.Hq * P.ktot;
-                const T* base = w + (((long long)b * P.ltot + flat_of(P, Ti, x0, Ti.lo[1], Ti.lo[2])) * P.Hq + h) * P.ktot;
-                const int own = ((Ti.o[0] - first_of(P, 0, x0, Ti.Lp[0])) * P.K[1] + n1) * P.K[2] + n2;
-                T wa8[kAheadF], wb8[kAheadF];
-                R.template walk_ahead<kAheadF>(P, y0, y1, s0, s1, [&](int u, bool ok_a, bool ok_b, int y, int x) {
-                    const int at = own + x * w2 - first_of(P, 2, Ti.lo[2] + x, Ti.Lp[2]);
-                    if (LINE) {
-                        wa8[u] = base[ok_a ? at : 0];
-                        wb8[u] = base[ok_b ? own + (x + 1) * w2 - first_of(P, 2, Ti.lo[2] + x + 1, Ti.Lp[2]) : 0];
-                    } else {
-                        wa8[u] = base[ok_a ? at + y * w1 - P.K[2] * first_of(P, 1, Ti.lo[1] + y, Ti.Lp[1]) : 0];
-                        wb8[u] = base[ok_b ? at + (y + 1) * w1 - P.K[2] * first_of(P, 1, Ti.lo[1] + y + 1, Ti.Lp[1]) : 0];
-                    }
-                }, [&](int u, int xa, int xb, bool ok_a, bool ok_b, int, int) {
-                    const float wa = ok_a ? widen(wa8[u]) : 0.f, wb = ok_b ? widen(wb8[u]) : 0.f;
-                    uint64_t va[4], vb[4];
-                    read_col<D, LINE>(sm, xa, R.c, va);
-                    read_col<D, LINE>(sm, xb, R.c, vb);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint64_t wa2 = twice(row_value(wa, R.lane, R.c, j)), wb2 = twice(row_value(wb, R.lane, R.c, j));
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) acc[j][i] = fma2(wb2, vb[i], fma2(wa2, va[i], acc[j][i]));
-                    }
+    exact_if_tainted([&](auto exact) {
+        constexpr bool kExact = decltype(exact)::value;
+        clear(acc);
+        for (int h = hk * P.group; h < (hk + 1) * P.group; ++h)
+            for_chunks(P, Ti,
+                [&](int x0, int y0, int y1, int s0, int s1) { stage_cols<T, D, LINE>(P, Ti, P.col1, b, h, x0, y0, y1, s0, s1, sm); },
+                [&](int x0, int y0, int y1, int s0, int s1) {
+                    // element of w: row of query (y, x), slot of the own key in its window (offsets within a sample fit 32 bits)
+                    const int w2 = P.dil[2] * P.Hq * P.ktot, w1 = P.dil[1] * P.L[2] * P.Hq * P.ktot;
+                    const T* base = w + (((long long)b * P.ltot + flat_of(P, Ti, x0, Ti.lo[1], Ti.lo[2])) * P.Hq + h) * P.ktot;
+                    const int own = ((Ti.o[0] - first_of(P, 0, x0, Ti.Lp[0])) * P.K[1] + n1) * P.K[2] + n2;
+                    T wa8[kAheadF], wb8[kAheadF];
+                    R.template walk_ahead<kAheadF>(P, y0, y1, s0, s1, [&](int u, bool ok_a, bool ok_b, int y, int x) {
+                        const int at = own + x * w2 - first_of(P, 2, Ti.lo[2] + x, Ti.Lp[2]);
+                        if (LINE) {
+                            wa8[u] = base[ok_a ? at : 0];
+                            wb8[u] = base[ok_b ? own + (x + 1) * w2 - first_of(P, 2, Ti.lo[2] + x + 1, Ti.Lp[2]) : 0];
+                        } else {
+                            wa8[u] = base[ok_a ? at + y * w1 - P.K[2] * first_of(P, 1, Ti.lo[1] + y, Ti.Lp[1]) : 0];
+                            wb8[u] = base[ok_b ? at + (y + 1) * w1 - P.K[2] * first_of(P, 1, Ti.lo[1] + y + 1, Ti.Lp[1]) : 0];
+                        }
+                    }, [&](int u, int xa, int xb, bool ok_a, bool ok_b, int, int) {
+                        const float wa = widen(wa8[u]), wb = widen(wb8[u]);
+                        uint64_t va[4], vb[4];
+                        read_col<D, LINE>(sm, xa, R.c, va);
+                        read_col<D, LINE>(sm, xb, R.c, vb);
+                        R.template add_pair<kExact>(acc, ok_a, wa, va, ok_b, wb, vb);
+                    });
                 });
-            });
+    }, [&] { return tainted(acc); });
     const uint64_t sc2 = twice(P.scale);
 #pragma unroll
     for (int j = 0; j < 4; ++j)

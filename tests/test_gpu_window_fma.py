@@ -35,6 +35,38 @@ def test_fused_float32(case):
         check(name, got[name], want[name], torch.float32)
 
 
+def same_finite_values(name, got, want, dtype):
+    """`check` for results that hold NaN or Inf: the same elements finite, and those within its bounds."""
+    finite = np.isfinite(want)
+    assert finite.any()
+    assert np.array_equal(torch.isfinite(got).cpu().numpy(), finite), f"{name}: finite pattern differs"
+    check(name, torch.where(torch.isfinite(got), got, 0), np.where(finite, want, 0.), dtype, scale_rel=True)
+
+
+def poison(t, head, value, at):
+    """`value` in one token's head, `at` a fraction of every spatial extent (first sample)."""
+    t[(0, *[int(at * n) for n in t.shape[1:-2]], head)] = value
+
+
+POISON_CASES = [c for c in FUSED_CASES if c[0] in ("1d_remainders", "2d_tiles_plus_one", "2d_box_past_a_chunk", "3d_ragged")]
+POISON_CASES.append(("2d_even_causal", (23, 30), 1, 4, 2, (4, 6), (1, 1), (True, False), 64))
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")], ids=["nan", "inf"])
+@pytest.mark.parametrize("which", ["q", "k", "v", "dout"])
+@pytest.mark.parametrize("case", POISON_CASES, ids=lambda c: c[0])
+def test_fused_float32_reads_no_value_of_another_window(case, which, value):
+    """Four rows share every column that is read; a NaN or Inf reaches the rows whose window holds it and no others."""
+    _, sp, B, Hq, Hkv, K, dil, causal, D = case
+    rng = np.random.default_rng(17)
+    t = {n: rng.standard_normal((B, *sp, h, D)) for n, h in (("q", Hq), ("k", Hkv), ("v", Hkv), ("dout", Hq))}
+    poison(t[which], 0, value, 0.3)
+    got, want = run_fused(len(sp), torch.float32, t["q"], t["k"], t["v"], t["dout"],
+                          dict(kernel_size=K, dilation=dil, is_causal=causal, return_lse=True))
+    for name in ("out", "lse", "dq", "dk", "dv"):
+        same_finite_values(name, got[name], want[name], torch.float32)
+
+
 SPLIT_CASES = [
     ("2d_d32_ragged", (57, 61), 2, 4, 4, (7, 9), (1, 1), (False, False), 32),
     ("2d_d32_even_causal_dil", (66, 45), 2, 4, 4, (6, 12), (2, 3), (False, True), 32),
@@ -43,28 +75,48 @@ SPLIT_CASES = [
 ]
 
 
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16], ids=["f32", "bf16", "f16"])
-@pytest.mark.parametrize("case", SPLIT_CASES, ids=lambda c: c[0])
-def test_split(case, dtype):
-    _, sp, B, Hq, Hkv, K, dil, causal, D = case
-    rank = len(sp)
-    g = torch.Generator().manual_seed(5)
-    r = lambda *s: torch.randn(*s, generator=g).to(dtype)
-    q, k, v, do = r(B, *sp, Hq, D), r(B, *sp, Hkv, D), r(B, *sp, Hkv, D), r(B, *sp, Hq, D)
-    kw = dict(kernel_size=K, dilation=dil, is_causal=causal)
-    w, gl = r(B, *sp, Hq, int(np.prod(K))), r(B, *sp, Hq, int(np.prod(K)))
-    qk, av = {1: (F.na1d_qk, F.na1d_av), 2: (F.na2d_qk, F.na2d_av), 3: (F.na3d_qk, F.na3d_av)}[rank]
+def split_products(q, k, v, do, w, gl, kw):
+    """The six products of the split operators (logits and their gradients for `gl`, output and its for `do`), and the oracle's."""
+    qk, av = {1: (F.na1d_qk, F.na1d_av), 2: (F.na2d_qk, F.na2d_av), 3: (F.na3d_qk, F.na3d_av)}[q.ndim - 3]
     leaf = lambda t: t.cuda().requires_grad_(True)
     qd, kd, vd, wd = leaf(q), leaf(k), leaf(v), leaf(w)
     logits, out = qk(qd, kd, **kw), av(wd, vd, **kw)
-    dq, dk = torch.autograd.grad(logits, [qd, kd], gl.cuda())
-    dw, dv = torch.autograd.grad(out, [wd, vd], do.cuda())
+    got = dict(logits=logits.detach(), out=out.detach())
+    got["dq"], got["dk"] = torch.autograd.grad(logits, [qd, kd], gl.cuda())
+    got["dw"], got["dv"] = torch.autograd.grad(out, [wd, vd], do.cuda())
     n = lambda t: t.float().numpy()
     want = dict(logits=oracle.na_qk(n(q), n(k), **kw), out=oracle.na_av(n(w), n(v), **kw))
     want["dq"], want["dk"] = oracle.na_qk_backward(n(q), n(k), n(gl), **kw)
     want["dw"], want["dv"] = oracle.na_av_backward(n(w), n(v), n(do), **kw)
-    for name, got in dict(logits=logits, out=out, dq=dq, dk=dk, dw=dw, dv=dv).items():
-        check(name, got, want[name], dtype, scale_rel=True)
+    return got, want
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16], ids=["f32", "bf16", "f16"])
+@pytest.mark.parametrize("case", SPLIT_CASES, ids=lambda c: c[0])
+def test_split(case, dtype):
+    _, sp, B, Hq, Hkv, K, dil, causal, D = case
+    g = torch.Generator().manual_seed(5)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype)
+    q, k, v, do = r(B, *sp, Hq, D), r(B, *sp, Hkv, D), r(B, *sp, Hkv, D), r(B, *sp, Hq, D)
+    w, gl = r(B, *sp, Hq, int(np.prod(K))), r(B, *sp, Hq, int(np.prod(K)))
+    got, want = split_products(q, k, v, do, w, gl, dict(kernel_size=K, dilation=dil, is_causal=causal))
+    for name in want:
+        check(name, got[name], want[name], dtype, scale_rel=True)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")], ids=["nan", "inf"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("case", SPLIT_CASES, ids=lambda c: c[0])
+def test_split_reads_no_value_of_another_window(case, dtype, value):
+    _, sp, B, Hq, Hkv, K, dil, causal, D = case
+    g = torch.Generator().manual_seed(19)
+    r = lambda h, d: torch.randn(B, *sp, h, d, generator=g).to(dtype)
+    q, k, v, do, w, gl = r(Hq, D), r(Hkv, D), r(Hkv, D), r(Hq, D), r(Hq, int(np.prod(K))), r(Hq, int(np.prod(K)))
+    for head, (t, at) in enumerate(((q, 0.3), (k, 0.6), (v, 0.3), (do, 0.6))):
+        poison(t, head % 4, value, at)
+    got, want = split_products(q, k, v, do, w, gl, dict(kernel_size=K, dilation=dil, is_causal=causal))
+    for name in want:
+        same_finite_values(name, got[name], want[name], dtype)
 
 
 # the register part (interior positions), the table part (clamped edges, slots past the registers) and both cluster sizes
