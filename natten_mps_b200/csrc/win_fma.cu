@@ -25,6 +25,7 @@
 #include "tc_plan.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include <type_traits>
 
 namespace natten {
@@ -460,7 +461,7 @@ fma_fwd_kernel(const __grid_constant__ FmaParams P, T* __restrict__ out, float* 
     exact_if_tainted([&](auto exact) {
         constexpr bool kExact = decltype(exact)::value;
         clear(acc);
-        m = -1e30f;                                          // finite: masked scores (-inf) minus it stay -inf
+        m = -FLT_MAX;                                        // finite: masked scores (-inf) minus it stay -inf
         l = 0.f;
         for_chunks(P, Ti,
             [&](int x0, int y0, int y1, int s0, int s1) {

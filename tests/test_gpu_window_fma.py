@@ -138,3 +138,20 @@ def test_bias_gradient_in_one_pass(case, dtype):
     n = lambda t: t.float().numpy()
     _, _, want = oracle.na_qk_rpb_backward(n(q), n(k), n(rpb), n(gl), kernel_size=K, dilation=dil)
     check("drpb", got, want, dtype, scale_rel=True)
+
+
+# every score far below -1e30 (a query against keys that a program pushed away); ties are exact, so the weights are 1 / n or 0
+def test_scores_of_any_size():
+    sp, H, D, K = (19, 23), 2, 32, (5, 7)
+    q, k = np.zeros((1, *sp, H, D)), np.zeros((1, *sp, H, D))
+    q[..., 0] = 1e17
+    k[..., 0] = -1e17 * (1 + np.arange(19 * 23 * H).reshape(1, *sp, H) % 3)
+    v = np.random.default_rng(23).standard_normal((1, *sp, H, D))
+    f = lambda t: torch.as_tensor(t).float().cuda()
+    for push in (1., -1.):
+        out, lse = F.na2d(f(push * q), f(k), f(v), K, return_lse=True)
+        want, want_lse = oracle.na_forward(push * q, k, v, K)
+        check("out", out, want, torch.float32)
+        check("lse", lse, want_lse, torch.float32)
+    with np.errstate(all="ignore"):              # beyond float32: no key is left, 0 / 0 like torch.softmax over -inf
+        assert torch.isnan(F.na2d(f(1e8 * q), f(1e8 * k), f(v), K)).all()
