@@ -52,10 +52,12 @@ template <typename A> __device__ __forceinline__ A neg_inf();
 template <> __device__ __forceinline__ float neg_inf<float>() { return -CUDART_INF_F; }
 template <> __device__ __forceinline__ double neg_inf<double>() { return -CUDART_INF; }
 
+// NaN if either is: every lane of warp_max has to end up with the same value, or the warp would part ways on it.
+template <typename A> __device__ __forceinline__ A max_or_nan(A a, A b) { return a > b || a != a ? a : b; }
 template <typename A> __device__ __forceinline__ A warp_max(A v)
 {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) { A t = __shfl_xor_sync(kFull, v, o); v = t > v ? t : v; }
+    for (int o = 16; o > 0; o >>= 1) v = max_or_nan(__shfl_xor_sync(kFull, v, o), v);
     return v;
 }
 template <typename A> __device__ __forceinline__ A warp_sum(A v)
@@ -270,7 +272,7 @@ fused_fwd_kernel(const __grid_constant__ Geo g, const T* __restrict__ q, const T
         A s = neg_inf<A>();
         if (valid) s = dot_row<T, A>(qsh, krow, g.D, g.vec_ok) * scale;
         const A mx = warp_max(s);
-        const A m_new = mx > m ? mx : m;
+        const A m_new = max_or_nan(mx, m);
         if (m_new == neg_inf<A>()) continue;          // nothing valid yet
         const A alpha = (m == neg_inf<A>()) ? A(0) : exp_acc(m - m_new);
         const A p = valid ? exp_acc(s - m_new) : A(0);

@@ -45,6 +45,19 @@ def check(name, got, want, dtype, scale_rel=False):
     return err
 
 
+def same_finite_values(name, got, want, dtype):
+    """`check` for results that hold NaN or Inf: the same elements finite, and those within its bounds."""
+    finite = np.isfinite(want)
+    assert finite.any()
+    assert np.array_equal(torch.isfinite(got).cpu().numpy(), finite), f"{name}: finite pattern differs"
+    check(name, torch.where(torch.isfinite(got), got, 0), np.where(finite, want, 0.), dtype, scale_rel=True)
+
+
+def poison(t, head, value, at):
+    """`value` in one token's head, `at` a fraction of every spatial extent (first sample)."""
+    t[(0, *[int(at * n) for n in t.shape[1:-2]], head)] = value
+
+
 def run_fused(rank, dtype, q, k, v, gout, kwargs, ek=None, ev=None, glse=None, sizes=None):
     """Run the CUDA path (forward + autograd backward) and the float64 oracle on the
     same rounded inputs; returns two dicts of results."""

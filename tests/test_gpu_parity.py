@@ -8,7 +8,7 @@ import oracle
 from natten_mps_b200 import _cabi, functional as F
 from tests import _golden as G
 from natten_mps_b200.utils import normalize_tuple_param as _ntp
-from tests._gpu_util import AV, FUSED, QK, check, compare_fused, dev, rounded, run_fused
+from tests._gpu_util import AV, FUSED, QK, check, compare_fused, dev, poison, rounded, run_fused, same_finite_values
 
 pytestmark = pytest.mark.gpu
 
@@ -204,3 +204,18 @@ def test_gradcheck_float64():
     assert torch.autograd.gradcheck(lambda a, b: F.na2d_qk(a, b, 3, scale=0.7), (q2, k2), atol=1e-6)
     attn = torch.randn(1, 4, 5, 2, 9, device="cuda", dtype=torch.float64, requires_grad=True)
     assert torch.autograd.gradcheck(lambda a, b: F.na2d_av(a, b, 3), (attn, v2), atol=1e-6)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")], ids=["nan", "inf"])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32, torch.bfloat16], ids=lambda d: str(d).split(".")[-1])
+@pytest.mark.parametrize("K,dil", [((3, 5), (2, 1)), ((6, 8), (1, 2))], ids=["one_slot_per_lane", "two_slots_per_lane"])
+def test_general_kernels_keep_a_bad_key_to_its_window(K, dil, dtype, value):
+    """A NaN score makes its row NaN, whichever lane holds it, and no other row."""
+    sp, H, D = (13, 19), 2, 24
+    rng = np.random.default_rng(29)
+    q, k, v, go = (rng.standard_normal((1, *sp, H, D)) for _ in range(4))
+    poison(k, 0, value, 0.4)
+    _cabi.set_force("simt")
+    got, want = run_fused(2, dtype, q, k, v, go, dict(kernel_size=K, dilation=dil, return_lse=True))
+    for name in ("out", "lse", "dq", "dk", "dv"):
+        same_finite_values(name, got[name], want[name], dtype)

@@ -8,7 +8,7 @@ import torch
 import oracle
 from natten_mps_b200 import _cabi
 from natten_mps_b200 import functional as F
-from tests._gpu_util import TOL, check, run_fused, rounded
+from tests._gpu_util import TOL, check, poison, run_fused, rounded, same_finite_values
 
 pytestmark = pytest.mark.gpu
 
@@ -33,19 +33,6 @@ def test_fused_float32(case):
                           dict(kernel_size=K, dilation=dil, is_causal=causal, return_lse=True))
     for name in ("out", "lse", "dq", "dk", "dv"):
         check(name, got[name], want[name], torch.float32)
-
-
-def same_finite_values(name, got, want, dtype):
-    """`check` for results that hold NaN or Inf: the same elements finite, and those within its bounds."""
-    finite = np.isfinite(want)
-    assert finite.any()
-    assert np.array_equal(torch.isfinite(got).cpu().numpy(), finite), f"{name}: finite pattern differs"
-    check(name, torch.where(torch.isfinite(got), got, 0), np.where(finite, want, 0.), dtype, scale_rel=True)
-
-
-def poison(t, head, value, at):
-    """`value` in one token's head, `at` a fraction of every spatial extent (first sample)."""
-    t[(0, *[int(at * n) for n in t.shape[1:-2]], head)] = value
 
 
 POISON_CASES = [c for c in FUSED_CASES if c[0] in ("1d_remainders", "2d_tiles_plus_one", "2d_box_past_a_chunk", "3d_ragged")]
