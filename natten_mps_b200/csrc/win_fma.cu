@@ -1045,9 +1045,11 @@ int fma_scores(int dtype, const Geo& g, const void* x, const long long xs[3], co
     if (dtype > 2 || !enough_pairs(g, dtype, 400000) || !vec_rows(x, xs, elt_of(dtype)) || !vec_rows(y, ys, elt_of(dtype)) ||
         !make_split(dtype, g, p, false, scale, (size_t)rows * g.ktot * elt_of(dtype), grid, smem))
         return -2;
-    if (rpb)
+    if (rpb) {
+        if (g.Hq != g.Hkv) return -2;
         for (int a = 0; a < g.rank; ++a)
             if (g.causal[a] || (g.K[a] & 1) == 0) return -2;
+    }
     p.row1 = tensor_of(x, xs);
     p.col1 = tensor_of(y, ys);
     cudaError_t err = cudaSuccess;

@@ -86,6 +86,15 @@ def test_rpb_rejects_even_kernels():
         F.na1d_qk_rpb(q, q, torch.randn(2, 7, device="cuda"), 4)
 
 
+@pytest.mark.parametrize("D,dtype", [(32, torch.float32), (32, torch.bfloat16), (64, torch.bfloat16), (20, torch.float32)],
+                         ids=["d32_f32", "d32_bf16", "d64_bf16", "d20_f32"])
+def test_rpb_rejects_grouped_heads(D, dtype):
+    """Whatever kernel the size would go to (the front end asks for equal shapes; this is the operator below it)."""
+    q, k = (torch.randn(2, 40, 44, h, D, device="cuda", dtype=dtype) for h in (4, 2))
+    with pytest.raises(NotImplementedError, match="unsupported"):
+        torch.ops.natten_b200.na_qk_rpb(q, k, torch.randn(4, 13, 13, device="cuda", dtype=dtype), [7, 7], [1, 1], None)
+
+
 def test_compat_wrappers_are_heads_first():
     torch.manual_seed(0)
     B, H, L, D, K = 2, 3, 21, 16, 5
