@@ -968,7 +968,7 @@ int tc_fused_bwd(int dtype, const Geo& g_in, const void* q, const void* k, const
         ex.dout_full = base + 2 * align256(rows_full * 4);
     }
     Plan plan;
-    if (!make_plan(g, plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return -2;
+    if (const int rc = make_plan(g, plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return rc;
     if (g.B == 0) return 0;
     if (g.Hq > 65535 || g.B > 65535) return -2;
     float* delta = reinterpret_cast<float*>(workspace);

@@ -673,7 +673,7 @@ int tc_fused_fwd_small(int dtype, const Geo& g, const void* q, const void* k, co
     if (!tc_eligible(dtype, g, q, k, v, /*allow_stride=*/true)) return -2;
     if (g.n_extra > 0 && ((reinterpret_cast<uintptr_t>(ek) | reinterpret_cast<uintptr_t>(ev)) & 15u)) return -2;
     Plan plan;
-    if (!make_plan(g, plan, kKeys, /*with_stride=*/true, /*interleave=*/true)) return -2;
+    if (const int rc = make_plan(g, plan, kKeys, /*with_stride=*/true, /*interleave=*/true)) return rc;
     const bool bf16 = dtype == 2;
     CUtensorMap mq, mk, mv, mek, mev;
     if (!encode_map(&mq, q, bf16, plan.p, g.Hq, g.D, g.qs, plan.box_q, /*query_lattice=*/true) ||

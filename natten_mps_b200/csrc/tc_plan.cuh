@@ -64,8 +64,9 @@ struct TcParams {
     long long otot;
 };
 
-int* status_host_ptr();   // the current device's word in mapped host memory
-int* status_ptr();   // device address of the library's status word on the current device (tc_status.cu)
+// The library's status word on the current device, and the device's word in mapped host memory (tc_status.cu)
+cudaError_t status_ptr(int*& p);
+cudaError_t status_host_ptr(int*& p);
 long long debug_wait_budget();   // barrier-wait budget in cycles (test hook; default kWaitBudgetCycles)
 int debug_inject();              // test hook, see TcParams::inject
 
@@ -376,7 +377,9 @@ struct Plan {
 };
 
 // Pick the row-tile shape (128 rows) whose column box needs the fewest chunks of `chunk` columns.
-inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_stride = false, bool interleave = false, bool backward = false)
+// 0, -2 where the tensor-core kernels do not cover the geometry (another kernel serves the call), or the CUDA error that
+// kept a plan they do cover from being made (the call has to report it).
+inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_stride = false, bool interleave = false, bool backward = false)
 {
     TcParams& p = plan.p;
     const int pad = 3 - g.rank;
@@ -388,7 +391,7 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
         p.causal[a] = s >= 0 ? g.causal[s] : 0;
         p.st[a] = (with_stride && s >= 0) ? g.st[s] : 1;
         p.O[a] = (p.L[a] + p.st[a] - 1) / p.st[a];
-        if (p.dil[a] > 8) return false;                          // tensor-map element strides, qx0 table
+        if (p.dil[a] > 8) return -2;                             // tensor-map element strides, qx0 table
         int gcd = p.dil[a], r = p.st[a];
         while (r) { const int t = gcd % r; gcd = r; r = t; }
         p.qstep[a] = p.st[a] / gcd;
@@ -443,7 +446,7 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
                 p.nchunk[0] = (E0 + cb0 - 1) / cb0; p.nchunk[1] = (E1 + cb1 - 1) / cb1; p.nchunk[2] = (E2 + cb2 - 1) / cb2;
             }
         }
-    if (best < 0) return false;
+    if (best < 0) return -2;
     p.cb0_log = ilog2(p.cb[0]); p.cb1_log = ilog2(p.cb[1]); p.cb2_log = ilog2(p.cb[2]);
     p.tile1_log = ilog2(p.tile[1]); p.tile2_log = ilog2(p.tile[2]);
     p.nchunks = (int)best;
@@ -457,13 +460,13 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
         p.dil_mul[a] = p.dil[a] >= 2 ? (unsigned)((0x100000000ull + p.dil[a] - 1) / p.dil[a]) : 0u;
         plan.box_q[a] = p.tile[a] * p.dil[a] * p.qstep[a];
         plan.box_kv[a] = p.cb[a] * p.dil[a];
-        if (plan.box_q[a] > 256) return false;
+        if (plan.box_q[a] > 256) return -2;
     }
     {
         long long blocks = p.ntiles;
         int dmax = 1;
         for (int a = 0; a < 3; ++a) { blocks *= p.grp_n[a]; dmax = p.dil[a] > dmax ? p.dil[a] : dmax; dmax = p.ntile[a] > dmax ? p.ntile[a] : dmax; }
-        if (blocks * dmax >= (1ll << 32) || (long long)(p.L[0] + p.L[1] + p.L[2] + dmax) * dmax >= (1ll << 32)) return false;
+        if (blocks * dmax >= (1ll << 32) || (long long)(p.L[0] + p.L[1] + p.L[2] + dmax) * dmax >= (1ll << 32)) return -2;
     }
     for (int a = 0; a < 3; ++a) { p.il[a] = 1; p.il_mul[a] = 0u; }
     if (interleave) {
@@ -490,7 +493,7 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
     p.ngroups = 1;
     for (int a = 0; a < 3; ++a) p.ngroups *= p.grp_n[a];
     p.per_head = (unsigned)p.ntiles * (unsigned)p.ngroups;
-    if ((long long)p.per_head * g.B * g.Hq >= (1ll << 31)) return false;
+    if ((long long)p.per_head * g.B * g.Hq >= (1ll << 31)) return -2;
     p.work_q = p.per_head * (unsigned)g.B * (unsigned)g.Hq;
     p.work_kv = p.per_head * (unsigned)g.B * (unsigned)g.Hkv;
     p.scale_log2 = (float)(g.scale * 1.4426950408889634);
@@ -499,9 +502,11 @@ inline bool make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_st
     p.ltot = g.ltot;
     p.wait_budget = debug_wait_budget();
     p.inject = debug_inject();
-    p.status = status_ptr();
-    p.status_host = status_host_ptr();
-    return p.status && p.status_host;
+    if (!get_encode()) return (int)cudaErrorNotSupported;       // a driver without tensor maps
+    cudaError_t err = status_ptr(p.status);
+    if (err == cudaSuccess) err = status_host_ptr(p.status_host);
+    if (err != cudaSuccess) cudaGetLastError();                 // reported here, not by the next launch
+    return (int)err;
 }
 
 // Column count of an interleaved axis for key tiles.  A key next to a clamped edge is read by every query of the edge, so a
@@ -537,8 +542,7 @@ inline void fit_key_boxes(Plan& plan)
 inline bool encode_map(CUtensorMap* map, const void* base, bool bf16, const TcParams& p, int heads, int dh,
                 const long long strides[3], const int box[3], bool query_lattice = false, bool interleaved = false)
 {
-    EncodeFn enc = get_encode();
-    if (!enc) return false;
+    const EncodeFn enc = get_encode();
     const cuuint64_t tok = (cuuint64_t)strides[1] * 2;
     cuuint64_t dims[5] = {(cuuint64_t)heads * dh, (cuuint64_t)p.L[2], (cuuint64_t)p.L[1], (cuuint64_t)p.L[0], (cuuint64_t)p.B};
     cuuint64_t gstr[4] = {tok, tok * p.L[2], tok * p.L[2] * p.L[1], (cuuint64_t)strides[0] * 2};
@@ -570,8 +574,8 @@ inline bool encode_map(CUtensorMap* map, const void* base, bool bf16, const TcPa
 inline bool encode_extra_map(CUtensorMap* map, const void* base, bool bf16, int B, int n_extra, int heads,
                              int dh, int box_cols, bool split_heads = false)
 {
-    EncodeFn enc = get_encode();
-    if (!enc || n_extra <= 0) return false;
+    const EncodeFn enc = get_encode();
+    if (n_extra <= 0) return false;
     const cuuint64_t tok = (cuuint64_t)heads * dh * 2;
     cuuint64_t dims[5] = {(cuuint64_t)heads * dh, (cuuint64_t)n_extra, 1, 1, (cuuint64_t)B};
     cuuint64_t gstr[4] = {tok, tok * n_extra, tok * n_extra, tok * n_extra};

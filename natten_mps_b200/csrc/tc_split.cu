@@ -391,9 +391,10 @@ int launch_scores_inner(const Plan& plan, const CUtensorMap& mx, const CUtensorM
     using SM = SmemS<DH>;
     const size_t smem = (size_t)SM::kOut + (((size_t)kTileRows * g.ktot * 2 + 15) & ~(size_t)15) + (rpb ? 4 * (kTileRows + (size_t)g.ktot) : 0);
     if (smem > kMaxDynamicSmem) return -2;
-    if (ensure_dynamic_smem((const void*)tc_scores_kernel<DH, BF16, kInner>, kMaxDynamicSmem) != cudaSuccess) {
+    cudaError_t err = ensure_dynamic_smem((const void*)tc_scores_kernel<DH, BF16, kInner>, kMaxDynamicSmem);
+    if (err != cudaSuccess) {
         cudaGetLastError();
-        return -2;
+        return (int)err;
     }
     int ngroups = 1;
     for (int a = 0; a < 3; ++a) ngroups *= plan.p.grp_n[a];
@@ -402,7 +403,7 @@ int launch_scores_inner(const Plan& plan, const CUtensorMap& mx, const CUtensorM
     tc_scores_kernel<DH, BF16, kInner><<<grid, kThreads, smem, s>>>(mx, my, plan.p, (uint16_t*)out, scale, fill, g.ktot,
                                                                    (const uint16_t*)rpb, rpb_table);
     tc_count_launch();
-    const cudaError_t err = cudaGetLastError();
+    err = cudaGetLastError();
     return err == cudaSuccess ? 0 : (int)err;
 }
 
@@ -651,9 +652,10 @@ int launch_apply_inner(const Plan& plan, const CUtensorMap& my, const Geo& g, co
     using SM = SmemA<DH>;
     const size_t smem = (size_t)SM::kW + (size_t)kTileRows * g.ktot * 2;
     if (smem > kMaxDynamicSmem) return -2;
-    if (ensure_dynamic_smem((const void*)tc_apply_kernel<DH, BF16, kInner>, kMaxDynamicSmem) != cudaSuccess) {
+    cudaError_t err = ensure_dynamic_smem((const void*)tc_apply_kernel<DH, BF16, kInner>, kMaxDynamicSmem);
+    if (err != cudaSuccess) {
         cudaGetLastError();
-        return -2;
+        return (int)err;
     }
     int ngroups = 1;
     for (int a = 0; a < 3; ++a) ngroups *= plan.p.grp_n[a];
@@ -661,7 +663,7 @@ int launch_apply_inner(const Plan& plan, const CUtensorMap& my, const Geo& g, co
     tc_apply_kernel<DH, BF16, kInner><<<grid, kThreads, smem, s>>>(my, plan.p, (const uint16_t*)w, (uint16_t*)out, scale, g.ktot,
                                                          out_by_position ? 1 : 0);
     tc_count_launch();
-    const cudaError_t err = cudaGetLastError();
+    err = cudaGetLastError();
     return err == cudaSuccess ? 0 : (int)err;
 }
 
@@ -903,16 +905,17 @@ int launch_gather(const Plan& plan, const CUtensorMap& mx, const Geo& g, const v
                   cudaStream_t s)
 {
     using SM = SmemG<DH>;
-    if (ensure_dynamic_smem((const void*)tc_gather_kernel<DH, BF16>, SM::kTotal) != cudaSuccess) {
+    cudaError_t err = ensure_dynamic_smem((const void*)tc_gather_kernel<DH, BF16>, SM::kTotal);
+    if (err != cudaSuccess) {
         cudaGetLastError();
-        return -2;
+        return (int)err;
     }
     int ngroups = 1;
     for (int a = 0; a < 3; ++a) ngroups *= plan.p.grp_n[a];
     const dim3 grid((unsigned)(plan.p.ntiles * ngroups), (unsigned)g.Hkv, (unsigned)g.B);
     tc_gather_kernel<DH, BF16><<<grid, kThreads, SM::kTotal, s>>>(mx, plan.p, (const uint16_t*)w, (uint16_t*)dst, scale, g.ktot);
     tc_count_launch();
-    const cudaError_t err = cudaGetLastError();
+    err = cudaGetLastError();
     return err == cudaSuccess ? 0 : (int)err;
 }
 
@@ -947,7 +950,7 @@ int tc_scores(int dtype, const Geo& g, const void* x, const long long xs[3], con
     const size_t base = g.D == 64 ? (size_t)SmemS<64>::kOut : (size_t)SmemS<128>::kOut;
     if (base + (size_t)kTileRows * g.ktot * 2 + 16 + (rpb ? 4 * (kTileRows + (size_t)g.ktot) : 0) > budget) return -2;
     Plan plan;
-    if (!make_plan(g, plan, kChunk, /*with_stride=*/true)) return -2;
+    if (const int rc = make_plan(g, plan, kChunk, /*with_stride=*/true)) return rc;
     const bool bf16 = dtype == 2;
     CUtensorMap mx, my;
     if (!encode_map(&mx, x, bf16, plan.p, g.Hq, g.D, xs, plan.box_q, /*query_lattice=*/true) ||
@@ -980,7 +983,7 @@ int tc_apply(int dtype, const Geo& g, const void* w, const void* y, const long l
     const size_t base = g.D == 64 ? (size_t)SmemA<64>::kW : (size_t)SmemA<128>::kW;
     if (base + (size_t)kTileRows * g.ktot * 2 > budget) return -2;
     Plan plan;
-    if (!make_plan(g, plan, kChunk, /*with_stride=*/true)) return -2;
+    if (const int rc = make_plan(g, plan, kChunk, /*with_stride=*/true)) return rc;
     const bool bf16 = dtype == 2;
     CUtensorMap my;
     if (!encode_map(&my, y, bf16, plan.p, g.Hkv, g.D, ys, plan.box_kv)) return -2;
@@ -1006,7 +1009,7 @@ int tc_gather(int dtype, const Geo& g, const void* w, const void* x, const long 
     if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dst)) & 15u) return -2;
     if (g.Hkv > 65535 || g.B > 65535) return -2;
     Plan plan;
-    if (!make_plan(g, plan, kChunk)) return -2;
+    if (const int rc = make_plan(g, plan, kChunk)) return rc;
     const bool bf16 = dtype == 2;
     CUtensorMap mx;
     if (!encode_map(&mx, x, bf16, plan.p, g.Hq, g.D, xs, plan.box_kv)) return -2;

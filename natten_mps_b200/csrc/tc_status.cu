@@ -24,34 +24,46 @@ std::atomic<int> g_inject{0};
 
 namespace tcplan {
 
-int* status_ptr()
+static cudaError_t current_device(int& dev)
 {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    std::lock_guard<std::mutex> lock(g_status_mutex);
-    if (!g_status_addr[dev]) {
-        int* p = nullptr;
-        if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_tc_status) != cudaSuccess) return nullptr;
-        g_status_addr[dev] = p;
-    }
-    return g_status_addr[dev];
+    const cudaError_t err = cudaGetDevice(&dev);
+    return err == cudaSuccess && (dev < 0 || dev >= 64) ? cudaErrorInvalidDevice : err;
 }
 
-int* status_host_ptr()
+cudaError_t status_ptr(int*& p)
 {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    if (int* w = g_status_host[dev].load(std::memory_order_acquire)) return w;
+    cudaError_t err = current_device(dev);
+    if (err != cudaSuccess) return err;
     std::lock_guard<std::mutex> lock(g_status_mutex);
-    int* w = g_status_host[dev].load(std::memory_order_acquire);
-    if (!w) {
-        void* p = nullptr;
-        if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return nullptr;
-        w = static_cast<int*>(p);
-        *w = 0;
-        g_status_host[dev].store(w, std::memory_order_release);
+    if (!g_status_addr[dev]) {
+        void* word = nullptr;
+        err = cudaGetSymbolAddress(&word, g_tc_status);
+        if (err != cudaSuccess) return err;
+        g_status_addr[dev] = static_cast<int*>(word);
     }
-    return w;
+    p = g_status_addr[dev];
+    return cudaSuccess;
+}
+
+cudaError_t status_host_ptr(int*& p)
+{
+    int dev = 0;
+    cudaError_t err = current_device(dev);
+    if (err != cudaSuccess) return err;
+    p = g_status_host[dev].load(std::memory_order_acquire);
+    if (p) return cudaSuccess;
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    p = g_status_host[dev].load(std::memory_order_acquire);
+    if (!p) {
+        void* word = nullptr;
+        err = cudaHostAlloc(&word, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+        if (err != cudaSuccess) return err;
+        p = static_cast<int*>(word);
+        *p = 0;
+        g_status_host[dev].store(p, std::memory_order_release);
+    }
+    return cudaSuccess;
 }
 
 long long debug_wait_budget() { return g_wait_budget.load(); }
@@ -77,8 +89,10 @@ int tc_clear_status()
 
 int tc_status_async(int* host_word, cudaStream_t s)
 {
-    int* p = tcplan::status_ptr();
-    if (!p || !host_word) return (int)cudaErrorInvalidValue;
+    if (!host_word) return (int)cudaErrorInvalidValue;
+    int* p = nullptr;
+    const cudaError_t err = tcplan::status_ptr(p);
+    if (err != cudaSuccess) return (int)err;
     return (int)cudaMemcpyAsync(host_word, p, sizeof(int), cudaMemcpyDeviceToHost, s);
 }
 

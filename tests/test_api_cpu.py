@@ -48,6 +48,22 @@ def test_params_are_checked_without_a_gpu():
         _cabi.check(-1, "x")
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="a CUDA call has to fail: there is no device here")
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_cuda_error_of_a_plan_is_not_taken_for_an_unsupported_shape(D):
+    """-2 would send the call to another kernel family without a word."""
+    L, buf = _cabi.lib(), ctypes.create_string_buffer(64)
+    at = (ctypes.addressof(buf) + 15) // 16 * 16                    # never read: the batch is empty
+    p = _cabi.make_params(2, torch.bfloat16, 0, 2, 2, D, D, (16, 16), (3, 3), (1, 1), (1, 1), (False, False), 0.125,
+                          0, *[(512 * D, 2 * D, D)] * 3)
+    for flags in (0, _cabi.FLAG_FORCE_TC):
+        p.flags = flags
+        assert L.natten_fused_fwd(p, at, at, at, None, None, at, at, None) > 0
+    p.dilation[0] = p.dilation[1] = 9                               # not a plan's shape, device or none
+    p.extent[0] = p.extent[1] = 32
+    assert L.natten_fused_fwd(p, at, at, at, None, None, at, at, None) == -2
+
+
 def test_workspace_size():
     p = _cabi.make_params(2, torch.bfloat16, 2, 4, 2, 64, 64, (16, 16), (3, 3), (1, 1), (1, 1),
                           (False, False), 0.125)
