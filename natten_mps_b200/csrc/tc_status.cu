@@ -57,7 +57,12 @@ cudaError_t status_host_ptr(int*& p)
     p = g_status_host[dev].load(std::memory_order_acquire);
     if (!p) {
         void* word = nullptr;
+        // the process's first call may be made while its stream is captured; allocating is no part of the graph
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        err = cudaThreadExchangeStreamCaptureMode(&mode);
+        if (err != cudaSuccess) return err;
         err = cudaHostAlloc(&word, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+        cudaThreadExchangeStreamCaptureMode(&mode);
         if (err != cudaSuccess) return err;
         p = static_cast<int*>(word);
         *p = 0;

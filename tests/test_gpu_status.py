@@ -5,10 +5,15 @@
   loads deliver and shortens the wait budget to a fraction of a millisecond, so the wait gives up
   (it never hangs), the kernel returns with the device's status word set, the next call raises,
   and after ``clear_status()`` the same call computes correctly again.
+* A process whose first call is made under stream capture.
 * One process using two GPUs in turn (skipped with a single GPU).
 * Per-sample extents: whatever sits in the padding rows (NaN here) must not reach the results,
   which the reference guarantees by slicing each sample (``src/natten_mps/_core/pure.py:586-599``).
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -17,6 +22,7 @@ import oracle
 from natten_mps_b200 import _backend, _cabi, functional as F
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _case(seed=0, B=2, H=24, W=40, heads=2, D=64, dtype=torch.bfloat16, device="cuda"):
@@ -52,6 +58,29 @@ def test_wait_that_runs_out_is_reported_and_recoverable():
     assert _cabi.device_status() == 0
     err = np.abs(out.float().cpu().numpy() - _oracle_out(q, k, v, 7)).max()
     assert err <= 2e-2, err
+
+
+FIRST_CALL = """
+import torch
+from natten_mps_b200 import _cabi, functional as F
+q, k, v, go = (torch.randn(1, 24, 24, 2, 64, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+q.requires_grad_(True)
+step = lambda: torch.autograd.grad(F.na2d(q, k, v, 7), [q], go)[0]
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    got = step()
+graph.replay()
+torch.cuda.synchronize()
+assert _cabi.last_path() == "tcgen05"
+assert torch.equal(got, step())
+"""
+
+
+def test_first_call_of_a_process_may_be_captured():
+    """The library sets itself up on first use; nothing of that may break the capture (a process of its own)."""
+    done = subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
 
 
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
