@@ -5,8 +5,10 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <map>
 #include <mutex>
 #include <set>
+#include <tuple>
 #include <utility>
 
 namespace natten {
@@ -17,6 +19,7 @@ struct DeviceCache {
     std::mutex mutex;
     int sms[64] = {0};
     std::set<std::pair<int, const void*>> smem_attr_done;
+    std::map<std::tuple<int, const void*, unsigned, size_t>, int> clusters;
 };
 inline DeviceCache& device_cache()
 {
@@ -52,6 +55,25 @@ inline cudaError_t ensure_dynamic_smem(const void* kernel, int bytes)
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (err == cudaSuccess) c.smem_attr_done.insert(key);
     return err;
+}
+
+// Clusters of cfg's size that the current device can hold at a time: 0 on a device that is partitioned or whose SMs are spread
+// too thinly over its GPCs, where such a launch would fail.
+inline int cluster_room(const void* kernel, const cudaLaunchConfig_t& cfg)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    DeviceCache& c = device_cache();
+    std::lock_guard<std::mutex> lock(c.mutex);
+    const auto key = std::make_tuple(dev, kernel, cfg.attrs[0].val.clusterDim.x, cfg.dynamicSmemBytes);
+    const auto known = c.clusters.find(key);
+    if (known != c.clusters.end()) return known->second;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return c.clusters[key] = n;
 }
 
 } // namespace natten

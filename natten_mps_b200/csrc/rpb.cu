@@ -12,6 +12,7 @@
 #include "rpb.cuh"
 
 #include "device_cache.cuh"
+#include "tc_kernels.cuh"
 
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -203,36 +204,41 @@ rpb_grad_pass_kernel(const __grid_constant__ Geo g, const T* __restrict__ dlogit
     cluster.sync();                                         // nobody leaves while its table is being read
 }
 
-// false: does not apply (table too large for shared memory, too many positions for 32-bit indices, or so few values that
-// the other kernel's many blocks are done sooner: 10 us against 13 at 39 K values)
+// false: does not apply (no room for a cluster of eight, table too large for shared memory, too many positions for 32-bit
+// indices, or so few values that the other kernel's many blocks are done sooner: 10 us against 13 at 39 K values)
 template <typename T>
 bool rpb_grad_pass(const Geo& g, const void* dlogits, void* drpb, long long table, cudaStream_t s, cudaError_t& err)
 {
     const size_t smem = (size_t)kGradWarps * table * 4 + (size_t)g.ktot * 4;
     const long long positions = (long long)g.B * g.ltot;
     if (table > 8192 || smem > 200 * 1024 || positions > 0x7fff0000ll || g.Hq > 65535 || positions * g.Hq * g.ktot < 100000) return false;
+    const int inject = tc_debug_inject();
+    const unsigned limit = inject == 2 ? 8 : inject == 3 ? 0 : 16;
+    // one cluster per head: 16 CTAs while two fit on an SM (so that a GPC can hold the cluster) and the clusters of all
+    // heads find room side by side (8 heads, 9 x 9 on 61 x 67: 14 us slower than with 8 CTAs), else 8
     auto launch = [&](auto* kernel) {
         err = ensure_dynamic_smem((const void*)kernel, kMaxDynamicSmem);
-        // one cluster per head: 16 CTAs while two fit on an SM (so that a GPC can hold the cluster) and the clusters of all
-        // heads find room side by side (8 heads, 9 x 9 on 61 x 67: 14 us slower than with 8 CTAs), else 8
         if (err == cudaSuccess) err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (err != cudaSuccess) return;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = smem <= 100 * 1024 && g.Hq <= 4 ? 16 : 8;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(attr[0].val.clusterDim.x, (unsigned)g.Hq);
-        cfg.blockDim = dim3(kGradWarps * 32);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        err = cudaLaunchKernelEx(&cfg, kernel, g, (const T*)dlogits, (T*)drpb, (int)table);
+        if (err != cudaSuccess) return true;
+        for (unsigned ctas = smem <= 100 * 1024 && g.Hq <= 4 ? 16 : 8; ctas >= 8; ctas /= 2) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = ctas;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(ctas, (unsigned)g.Hq);
+            cfg.blockDim = dim3(kGradWarps * 32);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (ctas > limit || cluster_room((const void*)kernel, cfg) == 0) continue;
+            err = cudaLaunchKernelEx(&cfg, kernel, g, (const T*)dlogits, (T*)drpb, (int)table);
+            return true;
+        }
+        return false;
     };
-    if (g.ktot <= 64) launch(rpb_grad_pass_kernel<T, 2>);
-    else launch(rpb_grad_pass_kernel<T, 6>);
-    return true;
+    return g.ktot <= 64 ? launch(rpb_grad_pass_kernel<T, 2>) : launch(rpb_grad_pass_kernel<T, 6>);
 }
 
 long long table_size(const Geo& g)

@@ -40,7 +40,9 @@ int tc_host_status(int device);
 int tc_status_async(int* host_word, cudaStream_t s);
 // Test hooks: cycle budget of the barrier waits (<= 0 restores the default) and a fault to inject
 // on the host side of the next launches (0 = none, 1 = the fused forward's first barrier expects
-// more bytes than its loads deliver, so that its wait runs out).
+// more bytes than its loads deliver, so that its wait runs out; 2, 3 = the device has no room for
+// a cluster of 16 CTAs, for any cluster).
 void tc_debug_wait(long long budget_cycles, int inject);
+int tc_debug_inject();
 
 } // namespace natten

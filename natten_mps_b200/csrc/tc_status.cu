@@ -114,4 +114,6 @@ void tc_debug_wait(long long budget_cycles, int inject)
     g_inject.store(inject);
 }
 
+int tc_debug_inject() { return tcplan::debug_inject(); }
+
 } // namespace natten

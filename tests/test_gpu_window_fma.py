@@ -127,6 +127,15 @@ def test_bias_gradient_in_one_pass(case, dtype):
     check("drpb", got, want, dtype, scale_rel=True)
 
 
+@pytest.mark.parametrize("inject", [2, 3], ids=["no_cluster_of_16", "no_cluster"])
+def test_bias_gradient_where_the_cluster_finds_no_room(inject):
+    try:
+        _cabi.lib().natten_debug_wait(0, inject)
+        test_bias_gradient_in_one_pass(BIAS_CASES[1], torch.float32)
+    finally:
+        _cabi.lib().natten_debug_wait(0, 0)
+
+
 # every score far below -1e30 (a query against keys that a program pushed away); ties are exact, so the weights are 1 / n or 0
 def test_scores_of_any_size():
     sp, H, D, K = (19, 23), 2, 32, (5, 7)
