@@ -214,13 +214,15 @@ bool rpb_grad_pass(const Geo& g, const void* dlogits, void* drpb, long long tabl
     if (table > 8192 || smem > 200 * 1024 || positions > 0x7fff0000ll || g.Hq > 65535 || positions * g.Hq * g.ktot < 100000) return false;
     const int inject = tc_debug_inject();
     const unsigned limit = inject == 2 ? 8 : inject == 3 ? 0 : 16;
-    // one cluster per head: 16 CTAs while two fit on an SM (so that a GPC can hold the cluster) and the clusters of all
-    // heads find room side by side (8 heads, 9 x 9 on 61 x 67: 14 us slower than with 8 CTAs), else 8
+    // One cluster per head: 16 CTAs while the clusters of all heads find room side by side, else 8.  With two CTAs on an SM
+    // (up to 64 slots) 12 heads of 7 x 7 on 56 x 56, batch 4, take 28 us with 16 and 33 with 8, 16 heads 43.5 and 43.9.  With
+    // one, seven clusters of 16 fit: 7 and 8 heads of 13 x 13 on 40 x 40, batch 2, take 15.4 and 28.9 with 16, 24.4 with 8;
+    // 23 x 23, 47.8 and 92.6 with 16, 86.4 with 8.
     auto launch = [&](auto* kernel) {
         err = ensure_dynamic_smem((const void*)kernel, kMaxDynamicSmem);
         if (err == cudaSuccess) err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (err != cudaSuccess) return true;
-        for (unsigned ctas = smem <= 100 * 1024 && g.Hq <= 4 ? 16 : 8; ctas >= 8; ctas /= 2) {
+        for (unsigned ctas = 16; ctas >= 8; ctas /= 2) {
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = ctas;
@@ -232,7 +234,7 @@ bool rpb_grad_pass(const Geo& g, const void* dlogits, void* drpb, long long tabl
             cfg.stream = s;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (ctas > limit || cluster_room((const void*)kernel, cfg) == 0) continue;
+            if (ctas > limit || cluster_room((const void*)kernel, cfg) < (ctas > 8 ? g.Hq : 1)) continue;
             err = cudaLaunchKernelEx(&cfg, kernel, g, (const T*)dlogits, (T*)drpb, (int)table);
             return true;
         }
