@@ -1028,10 +1028,19 @@ bool make_split(int dtype, const Geo& g, FmaParams& p, bool key_side, float scal
 }
 } // namespace
 
-long long pairs_per_sample(const Geo& g) { return g.ltot * g.Hq * g.ktot; }
-// The general kernels of the split operators spread a small problem over more blocks: they took 6 us + pairs / 25 per ns
-// for 16-bit types, about five times that for float32, where a block of these kernels alone lives for 10 to 50 us.
-bool enough_pairs(const Geo& g, int dtype, long long least) { return g.B * pairs_per_sample(g) * (dtype == 0 ? 5 : 1) >= least; }
+// Enough (query, head) rows for these kernels?  The general kernels spread a small problem over more blocks; theirs is a time
+// per pair, and a block of these kernels lives as long as its window is large, however few blocks there are, so the two meet
+// at a number of rows that hardly depends on the window.  Microseconds here | general, head dim 32:
+//   scores, 16 bits   7 x 7: 3136 rows 13.0 | 10.2, 6400 14.4 | 15.6, 12544 13.3 | 28.2;  13 x 13: 3136 27 | 25, 6400 33 | 42;
+//                     3 x 5 x 5: 4704 19.6 | 17.5, 6400 19.8 | 22.5;  33: 2000 11.6 | 6.6, 8000 11.8 | 15.2
+//   scores, float32   7 x 7: 1600 10.9 | 7.6, 3136 11.1 | 10.5;  13 x 13: 1600 22.4 | 16.2, 3136 23.8 | 25.9 (larger head dims:
+//                     the general kernel's time grows faster, so the line is on the safe side)
+//   apply, 16 bits    7 x 7: 6400 15.3 | 15.5, 12544 15.3 | 28.7;  13 x 13: 6400 43 | 41, 12544 35 | 83;
+//                     3 x 5 x 5: 6400 25 | 22, 12800 27 | 42;  33: 8000 11.6 | 15.3
+//   gather, 16 bits   7 x 7: 6400 25.7 | 22.1, 12544 25.6 | 36.9;  13 x 13: 6400 73 | 56, 12544 87 | 101;
+//                     3 x 5 x 5: 6400 53 | 39, 12800 57 | 60;  3 x 3: 3136 8.4 | 7.3, 12544 8.8 | 18.8
+//   apply and gather, float32   784 rows 13.2 | 33 and 22.4 | 30;  3 x 3: 3136 6.2 | 10.7 and 6.7 | 9.3
+bool enough_rows(const Geo& g, long long least) { return g.B * g.ltot * g.Hq >= least; }
 
 // The same three products as tc_scores / tc_apply / tc_gather (tc_kernels.cuh), in fp32; unit stride.
 int fma_scores(int dtype, const Geo& g, const void* x, const long long xs[3], const void* y, const long long ys[3], float scale,
@@ -1041,8 +1050,7 @@ int fma_scores(int dtype, const Geo& g, const void* x, const long long xs[3], co
     FmaParams p;
     dim3 grid;
     size_t smem;
-    // 25 us against 6 + 98 at 2.5 M pairs, 23 against 33 at 0.76 M, 10.7 against 6.8 at 39 K
-    if (dtype > 2 || !enough_pairs(g, dtype, 400000) || !vec_rows(x, xs, elt_of(dtype)) || !vec_rows(y, ys, elt_of(dtype)) ||
+    if (dtype > 2 || !enough_rows(g, dtype == 0 ? 3000 : 8000) || !vec_rows(x, xs, elt_of(dtype)) || !vec_rows(y, ys, elt_of(dtype)) ||
         !make_split(dtype, g, p, false, scale, (size_t)rows * g.ktot * elt_of(dtype), grid, smem))
         return -2;
     if (rpb) {
@@ -1074,7 +1082,7 @@ int fma_apply(int dtype, const Geo& g, const void* w, const void* y, const long 
     FmaParams p;
     dim3 grid;
     size_t smem;
-    if (dtype > 2 || !enough_pairs(g, dtype, 400000) || !vec_rows(y, ys, elt_of(dtype)) || (reinterpret_cast<uintptr_t>(out) & 15u) ||
+    if (dtype > 2 || !enough_rows(g, dtype == 0 ? 800 : 8000) || !vec_rows(y, ys, elt_of(dtype)) || (reinterpret_cast<uintptr_t>(out) & 15u) ||
         !make_split(dtype, g, p, false, scale, 0, grid, smem))
         return -2;
     p.col1 = tensor_of(y, ys);
@@ -1099,7 +1107,8 @@ int fma_gather(int dtype, const Geo& g, const void* w, const void* x, const long
     FmaParams p;
     dim3 grid;
     size_t smem;
-    if (dtype > 2 || !enough_pairs(g, dtype, 1500000) || !vec_rows(x, xs, elt_of(dtype)) || (reinterpret_cast<uintptr_t>(dst) & 15u) || pairs_per_sample(g) >= (1ll << 31) ||
+    if (dtype > 2 || !enough_rows(g, dtype == 0 ? 800 : 12000) || !vec_rows(x, xs, elt_of(dtype)) ||
+        (reinterpret_cast<uintptr_t>(dst) & 15u) || g.ltot * g.Hq * g.ktot >= (1ll << 31) ||                // 32-bit offsets
         !make_split(dtype, g, p, true, scale, 0, grid, smem))
         return -2;
     p.col1 = tensor_of(x, xs);
