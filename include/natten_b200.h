@@ -50,8 +50,9 @@ enum {
 
 enum { NATTEN_OP_FUSED_FWD = 0, NATTEN_OP_FUSED_BWD = 1 };
 
-/* Which kernel family served the last call on this thread. */
-enum { NATTEN_PATH_NONE = 0, NATTEN_PATH_SIMT = 1, NATTEN_PATH_TCGEN05 = 2 };
+/* Which kernel family served the last call on this thread: the tensor-core kernels (some part of it),
+ * else the fp32 window kernels (all of it), else the general kernels. */
+enum { NATTEN_PATH_NONE = 0, NATTEN_PATH_SIMT = 1, NATTEN_PATH_TCGEN05 = 2, NATTEN_PATH_WINDOW = 3 };
 
 typedef struct natten_params {
     int32_t rank;          /* 1, 2 or 3                                           */

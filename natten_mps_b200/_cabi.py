@@ -17,7 +17,7 @@ LIB_PATH = os.path.join(_PKG, "libnatten_b200.so")
 F32, F16, BF16, F64 = 0, 1, 2, 3
 FLAG_FORCE_SIMT, FLAG_FORCE_TC = 1, 2
 OP_FUSED_FWD, OP_FUSED_BWD = 0, 1
-PATH_NAMES = {0: "none", 1: "simt", 2: "tcgen05"}
+PATH_NAMES = {0: "none", 1: "simt", 2: "tcgen05", 3: "window"}
 
 EXPORTS = (
     "natten_fused_fwd", "natten_fused_bwd", "natten_workspace_bytes", "natten_qk_fwd",

@@ -1,5 +1,5 @@
 // C-ABI entry points (include/natten_b200.h): argument checks, geometry set-up
-// and dispatch between the tcgen05 kernels and the SIMT kernels.
+// and dispatch between the tcgen05, the fp32 window and the general SIMT kernels.
 #include "../../include/natten_b200.h"
 
 #include "rpb.cuh"
@@ -105,7 +105,7 @@ int natten_fused_fwd(const natten_params_t* p, const void* q, const void* k, con
     t_last_path = NATTEN_PATH_SIMT;
     if (!(p->flags & NATTEN_FLAG_FORCE_SIMT)) {
         rc = fma_fused_fwd(p->dtype, g, q, k, v, out, lse, s);
-        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+        if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_WINDOW; return rc; }
     }
     return from_cuda(simt_fused_fwd(p->dtype, g, q, k, v, extra_k, extra_v, out, lse, s));
 }
@@ -149,7 +149,7 @@ int natten_fused_bwd(const natten_params_t* p, const void* q, const void* k, con
     t_last_path = NATTEN_PATH_SIMT;
     if (!(p->flags & NATTEN_FLAG_FORCE_SIMT)) {
         rc = fma_fused_bwd(p->dtype, g, q, k, v, out, lse, dout, dlse, dq, dk, dv, workspace, s);
-        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+        if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_WINDOW; return rc; }
     }
     return from_cuda(simt_fused_bwd(p->dtype, g, q, k, v, extra_k, extra_v, out, lse, dout, dlse, dq, dk,
                                     dv, dextra_k, dextra_v, workspace, s));
@@ -173,7 +173,7 @@ int natten_qk_fwd(const natten_params_t* p, const void* q, const void* k, void* 
     t_last_path = NATTEN_PATH_SIMT;
     if (!(p->flags & NATTEN_FLAG_FORCE_SIMT)) {
         rc = fma_scores(p->dtype, g, q, g.qs, k, g.ks, g.has_scale ? (float)g.scale : 1.f, true, logits, (cudaStream_t)stream);
-        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+        if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_WINDOW; return rc; }
     }
     return from_cuda(simt_qk_fwd(p->dtype, g, q, k, logits, (cudaStream_t)stream));
 }
@@ -198,7 +198,8 @@ int natten_qk_bwd(const natten_params_t* p, const void* q, const void* k, const 
         rc = tc_gather(p->dtype, g, dlogits, q, g.qs, sc, dk, (cudaStream_t)stream);
         if (rc > 0) return rc;
         dk_done = rc == 0;
-        if (dq_done || dk_done) t_last_path = NATTEN_PATH_TCGEN05;
+        const bool tensor_cores = dq_done || dk_done;
+        if (tensor_cores) t_last_path = NATTEN_PATH_TCGEN05;
         if ((p->flags & NATTEN_FLAG_FORCE_TC) && !(dq_done && dk_done)) return NATTEN_E_UNSUPPORTED;
         if (!dq_done) {
             rc = fma_apply(p->dtype, g, dlogits, k, g.ks, sc, dq, (cudaStream_t)stream);
@@ -210,7 +211,10 @@ int natten_qk_bwd(const natten_params_t* p, const void* q, const void* k, const 
             if (rc > 0) return rc;
             dk_done = rc == 0;
         }
-        if (dq_done && dk_done) return NATTEN_OK;
+        if (dq_done && dk_done) {
+            if (!tensor_cores) t_last_path = NATTEN_PATH_WINDOW;
+            return NATTEN_OK;
+        }
     }
     return from_cuda(simt_qk_bwd(p->dtype, g, q, k, dlogits, dq_done ? nullptr : dq, dk_done ? nullptr : dk,
                                  (cudaStream_t)stream));
@@ -231,7 +235,7 @@ int natten_qk_rpb_fwd(const natten_params_t* p, const void* q, const void* k, co
         if (rc == 0) { t_last_path = NATTEN_PATH_TCGEN05; return NATTEN_OK; }
         if (rc > 0) return rc;
         rc = fma_scores(p->dtype, g, q, g.qs, k, g.ks, g.has_scale ? (float)g.scale : 1.f, true, logits, (cudaStream_t)stream, rpb);
-        if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_SIMT; return rc; }
+        if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_WINDOW; return rc; }
     }
     // otherwise the logits first, then the bias in a second pass
     rc = natten_qk_fwd(p, q, k, logits, stream);
@@ -273,7 +277,7 @@ int natten_av_fwd(const natten_params_t* p, const void* attn, const void* v, voi
         Geo gv = g;
         gv.D = g.Dv;
         rc = fma_apply(p->dtype, gv, attn, v, g.vs, 1.f, out, (cudaStream_t)stream);
-        if (rc != NATTEN_E_UNSUPPORTED) return rc;
+        if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_WINDOW; return rc; }
     }
     return from_cuda(simt_av_fwd(p->dtype, g, attn, v, out, (cudaStream_t)stream));
 }
@@ -303,7 +307,8 @@ int natten_av_bwd(const natten_params_t* p, const void* attn, const void* v, con
         rc = tc_gather(p->dtype, gv, attn, dout, dos, 1.f, dv, (cudaStream_t)stream);
         if (rc > 0) return rc;
         dv_done = rc == 0;
-        if (da_done || dv_done) t_last_path = NATTEN_PATH_TCGEN05;
+        const bool tensor_cores = da_done || dv_done;
+        if (tensor_cores) t_last_path = NATTEN_PATH_TCGEN05;
         if (da_done && dv_done) return NATTEN_OK;
         if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
         if (!da_done) {
@@ -316,7 +321,10 @@ int natten_av_bwd(const natten_params_t* p, const void* attn, const void* v, con
             if (rc > 0) return rc;
             dv_done = rc == 0;
         }
-        if (da_done && dv_done) return NATTEN_OK;
+        if (da_done && dv_done) {
+            if (!tensor_cores) t_last_path = NATTEN_PATH_WINDOW;
+            return NATTEN_OK;
+        }
     }
     if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
     return from_cuda(simt_av_bwd(p->dtype, g, attn, v, dout, da_done ? nullptr : dattn, dv_done ? nullptr : dv,
