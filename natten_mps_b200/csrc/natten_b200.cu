@@ -234,6 +234,7 @@ int natten_qk_rpb_fwd(const natten_params_t* p, const void* q, const void* k, co
                        (cudaStream_t)stream, rpb);
         if (rc == 0) { t_last_path = NATTEN_PATH_TCGEN05; return NATTEN_OK; }
         if (rc > 0) return rc;
+        if (p->flags & NATTEN_FLAG_FORCE_TC) return NATTEN_E_UNSUPPORTED;
         rc = fma_scores(p->dtype, g, q, g.qs, k, g.ks, g.has_scale ? (float)g.scale : 1.f, true, logits, (cudaStream_t)stream, rpb);
         if (rc != NATTEN_E_UNSUPPORTED) { t_last_path = NATTEN_PATH_WINDOW; return rc; }
     }

@@ -95,6 +95,16 @@ def test_rpb_rejects_grouped_heads(D, dtype):
         torch.ops.natten_b200.na_qk_rpb(q, k, torch.randn(4, 13, 13, device="cuda", dtype=dtype), [7, 7], [1, 1], None)
 
 
+def test_forced_tensor_cores_do_not_fall_back():
+    q = torch.randn(2, 40, 44, 4, 32, device="cuda", dtype=torch.bfloat16)
+    _cabi.set_force("tc")
+    try:
+        with pytest.raises(NotImplementedError, match="unsupported"):
+            F.na2d_qk_rpb(q, q, torch.randn(4, 13, 13, device="cuda", dtype=torch.bfloat16), 7)
+    finally:
+        _cabi.set_force(None)
+
+
 def test_compat_wrappers_are_heads_first():
     torch.manual_seed(0)
     B, H, L, D, K = 2, 3, 21, 16, 5
