@@ -294,20 +294,6 @@ template <bool BF16> __device__ __forceinline__ uint32_t cvt_pack(float lo, floa
     else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
     return d;
 }
-template <bool BF16> __device__ __forceinline__ uint32_t ex2_x2(uint32_t x)
-{
-    uint32_t d;
-    if (BF16) asm("ex2.approx.ftz.bf16x2 %0, %1;" : "=r"(d) : "r"(x));
-    else asm("ex2.approx.f16x2 %0, %1;" : "=r"(d) : "r"(x));
-    return d;
-}
-template <bool BF16> __device__ __forceinline__ uint32_t mul_x2(uint32_t a, uint32_t b)
-{
-    uint32_t d;
-    if (BF16) asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
 
 // Two fp32 values in one 64-bit register pair, and the packed fp32 arithmetic of sm_100 on them (one
 // instruction for two lanes of an fma / mul).

@@ -17,7 +17,7 @@ of the autograd backward (autograd/_factory.py:63-102).
 """
 from __future__ import annotations
 
-from typing import Optional, Sequence
+from typing import Optional
 
 import torch
 
