@@ -13,9 +13,14 @@
 //     alone does the scalar work of that row (mask, exponential), and four shuffles hand the results back.
 // A pass over the columns of K = 7 x 7 costs 23 shared-memory cycles for 32 pairs of which 70 % are needed.
 //
-// Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, float32, against the general SIMT kernels: forward 34 us (185), dQ 43 (236),
-// dK and dV 70 (304); split operators (any type; bf16 before): scores 25 (95), apply 26 (95, float32 471), gather 37 (116).
-// What is left is instruction issue: every pair of columns costs a warp about 100 instructions for 64 pairs.
+// Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, against the general SIMT kernels: float32 forward 36 us (185), dQ 43 (236),
+// dK and dV 72 (304); split operators in bf16: scores 25 (93), apply 24 (93), gather 36 (115); in float32: 25 (96), 24 (469),
+// 32 (152).
+// What bounds them there: too few warps.  448 CTAs have 444 (forward, dQ), 296 (dK and dV, 245 to 255 registers) or 592 (split)
+// places, 7 to 12 warps on an SM.  Schedulers issue in 44, 41, 33 % of the active cycles (forward, dQ, dK and dV) and in 49, 38,
+// 36 % (scores, apply, gather); the largest stalls are the barriers around a chunk, whose loads nothing overlaps, then the
+// latency of dependent instructions, in apply and gather also that of the weights.  DRAM is at 2 to 8 %.  Apply and gather spill
+// 16 to 52 bytes at the 128 registers that four CTAs on an SM leave them.
 //
 // Rows are queries and columns keys, or the other way round (key side: dK, dV; columns = the queries that attend to a key,
 // a contiguous range per axis).  Fixed order of summation everywhere, no atomics.
@@ -341,15 +346,19 @@ template <int D, bool LINE, bool kKeySide> struct RowsF {
         a = ok_a ? a : 0.f;
         b = ok_b ? b : 0.f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint64_t a2 = twice(row_value(a, lane, c, j)), b2 = twice(row_value(b, lane, c, j));
-            if constexpr (kExact) {
-                add_if(in_a & (1u << j), acc[j], a2, xa);
-                add_if(in_b & (1u << j), acc[j], b2, xb);
-            } else {
+        for (int j = 0; j < 4; ++j) add_row<kExact>(j, acc[j], in_a, a, xa, in_b, b, xb);
+    }
+    template <bool kExact>
+    __device__ __forceinline__ void add_row(int j, uint64_t (&acc)[4], uint32_t in_a, float a, const uint64_t (&xa)[4], uint32_t in_b,
+                                            float b, const uint64_t (&xb)[4]) const
+    {
+        const uint64_t a2 = twice(row_value(a, lane, c, j)), b2 = twice(row_value(b, lane, c, j));
+        if constexpr (kExact) {
+            add_if(in_a & (1u << j), acc, a2, xa);
+            add_if(in_b & (1u << j), acc, b2, xb);
+        } else {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[j][i] = fma2(b2, xb[i], fma2(a2, xa[i], acc[j][i]));
-            }
+            for (int i = 0; i < 4; ++i) acc[i] = fma2(b2, xb[i], fma2(a2, xa[i], acc[i]));
         }
     }
     // Walk the staged chunk [y0, y1) x [s0, s1) two columns at a time (independent chains for the scheduler): neighbours along
@@ -432,7 +441,7 @@ __device__ __forceinline__ int tainted(const uint64_t (&acc)[4][4])
 // Runs pass(false), and pass(true) over it if that left a NaN or Inf in the CTA's sums (taint()).  Four rows share every column,
 // and the plain pass gives a row that does not attend to it a weight of zero, which a NaN or Inf turns into NaN; the exact pass
 // leaves it out.  Exact arithmetic throughout (a vote, and a predicate per row and column) took a float32 training step of
-// 56 x 56, 7 x 7, 4 heads of 32, batch 4 from 155 to 199 us; the test at the end takes it to 160.
+// 56 x 56, 7 x 7, 4 heads of 32, batch 4 from 155 to 199 us; the test at the end takes it to 158.
 template <typename Pass, typename Taint> __device__ __forceinline__ void exact_if_tainted(Pass&& pass, Taint&& taint)
 {
     pass(std::false_type{});
@@ -610,7 +619,7 @@ fma_bwd_k_kernel(const __grid_constant__ FmaParams P, const float* __restrict__ 
                 },
                 [&](int, int y0, int y1, int s0, int s1) {
                     R.walk(P, y0, y1, s0, s1, [&](int xa, int xb, bool ok_a, bool ok_b, int, int) {
-                        auto one = [&](int x, uint64_t (&q)[4], uint64_t (&go)[4], float& p, float& ds) {
+                        auto one = [&](int x, bool ok, uint64_t (&q)[4], uint64_t (&go)[4], float& p, float& ds) {
                             read_col<D, LINE>(sm, x, R.c, q);
                             read_col<D, LINE>(gs, x, R.c, go);
                             const float2 st = stats[x];
@@ -618,13 +627,19 @@ fma_bwd_k_kernel(const __grid_constant__ FmaParams P, const float* __restrict__ 
                             const float dp = reduce4<LF::LPQ>(dot8(v[0], go), dot8(v[1], go), dot8(v[2], go), dot8(v[3], go), R.c);
                             p = fast_exp2(fmaf(s, P.scale_log2, -st.x));
                             ds = p * (dp - st.y) * P.scale;
+                            p = ok ? p : 0.f;
+                            ds = ok ? ds : 0.f;
                         };
                         uint64_t qa[4], qb[4], ga[4], gb[4];
                         float pa, pb, da, db;
-                        one(xa, qa, ga, pa, da);
-                        one(xb, qb, gb, pb, db);
-                        R.template add_pair<kExact>(av, ok_a, pa, ga, ok_b, pb, gb);
-                        R.template add_pair<kExact>(ak, ok_a, da, qa, ok_b, db, qb);
+                        one(xa, ok_a, qa, ga, pa, da);
+                        one(xb, ok_b, qb, gb, pb, db);
+                        const uint32_t in_a = kExact ? rows_with(ok_a, R.lane, R.c) : 0u, in_b = kExact ? rows_with(ok_b, R.lane, R.c) : 0u;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            R.template add_row<kExact>(j, av[j], in_a, pa, ga, in_b, pb, gb);
+                            R.template add_row<kExact>(j, ak[j], in_a, da, qa, in_b, db, qb);
+                        }
                     });
                 });
     }, [&] { return tainted(ak) | tainted(av); });
@@ -862,7 +877,10 @@ fma_gather_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ w, 
 // ---------------------------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int kFusedChunk = 64 * 1024;   // three CTAs share an SM's 227 KB
+// Three CTAs of the forward and of dQ share an SM's 227 KB.  The key side, two CTAs by its registers, uses the same.  Measured,
+// 56 x 56, 7 x 7, head dim 32 | 64, with 48, 64, 100 KB: forward 34.7, 35.4, 34.0 us | 30.5, 30.9, 39.6 (two CTAs); dK and dV
+// 75.0, 74.3, 66.7 | 79.3, 69.0, 64.3.
+constexpr int kFusedChunk = 64 * 1024;
 
 // Rows of a warp are 4 x (256 / D) (rank 1: one row of 1024 / D).  `tensors`: column tensors staged side by side,
 // `extra`: further shared-memory bytes per staged column, `budget`: bytes of a chunk.
