@@ -2,9 +2,11 @@
  * natten_b200 -- C ABI of the B200 neighbourhood-attention library.
  *
  * Plain C: device pointers, sizes and a CUDA stream handle.  No PyTorch types.
- * Every entry point is asynchronous on the given stream, allocates nothing,
- * never synchronises, and returns 0 on success, a negative NATTEN_E_* code for
- * a rejected argument, or a positive cudaError_t value.
+ * Every entry point is asynchronous on the given stream, allocates no device
+ * memory, never synchronises, and returns 0 on success, a negative NATTEN_E_*
+ * code for a rejected argument, or a positive cudaError_t value.  The first
+ * call on a device also allocates one word of pinned host memory (the status
+ * word below); it may be made while its stream is captured.
  *
  * The reference (natten-mps) has no foreign-function interface: its backends
  * are Python modules that implement the nine-function protocol of

@@ -60,6 +60,27 @@ def test_wait_that_runs_out_is_reported_and_recoverable():
     assert err <= 2e-2, err
 
 
+def test_status_words_on_the_host_and_on_the_stream():
+    """The word that the kernel itself writes into host memory, and the copy that a caller queues behind it."""
+    q, k, v = _case(seed=1)
+    L = _cabi.lib()
+    word = torch.full((1,), 7, dtype=torch.int32).pin_memory()
+    stream = torch.cuda.current_stream()
+    try:
+        assert L.natten_status_async(word.data_ptr(), stream.cuda_stream) == 0
+        stream.synchronize()
+        assert int(word) == 0 and L.natten_host_status(0) == 0
+        L.natten_debug_wait(400_000, 1)
+        F.na2d(q, k, v, 7)
+        assert L.natten_status_async(word.data_ptr(), stream.cuda_stream) == 0
+        stream.synchronize()
+        assert int(word) != 0 and L.natten_host_status(0) != 0
+    finally:
+        L.natten_debug_wait(0, 0)
+        _cabi.clear_status()
+    assert L.natten_host_status(0) == 0
+
+
 FIRST_CALL = """
 import torch
 from natten_mps_b200 import _cabi, functional as F
