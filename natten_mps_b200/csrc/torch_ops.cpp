@@ -16,6 +16,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/autocast_mode.h>
@@ -609,7 +610,44 @@ struct ModuleFn : public torch::autograd::Function<ModuleFn> {
         ctx->saved_data["s"] = scale;
         ctx->saved_data["m"] = (int64_t)((b1 ? 4 : 0) | (w2 ? 8 : 0) | (b2 ? 16 : 0) | (bp ? 64 : 0) | 35);     // arguments that are there
         ctx->save_for_backward({x, w1, w2.value_or(Tensor()), wp, r.q, r.k, r.v, out, lse});
+        ctx->saved_data["h"] = std::vector<int64_t>{heads, kv, version_of(b1), version_of(b2)};
+        ctx->saved_data["b1"] = b1;              // for differentiable() alone: a plain backward does not look at them, and
+        ctx->saved_data["b2"] = b2;              // does not mind if they have been written to since
         return at::linear(joined_heads(out), wp, bp);
+    }
+    static int64_t version_of(const OptTensor& t) { return t && !t->is_inference() ? t->_version() : 0; }
+    // The gradients with a graph of their own (create_graph): from the separate operators, run again.  `stand_in` keeps the
+    // arguments apart where one was computed from another (a weight shared between layers).
+    static variable_list differentiable(AutogradContext* ctx, const variable_list& s, const Tensor& grad, const bool (&needs)[7])
+    {
+        auto stand_in = [](const Tensor& t) { return t.defined() ? t.view_as(t) : t; };
+        auto bias = [&](const char* name, int64_t version) {
+            const OptTensor b = ctx->saved_data.at(name).toOptional<Tensor>();
+            TORCH_CHECK(version_of(b) == version, "natten_b200: a projection's bias was modified in place since the forward pass; "
+                        "its gradients can't be given a graph");
+            return b ? OptTensor(stand_in(*b)) : b;
+        };
+        const c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);     // as in the forward pass
+        const auto h = ctx->saved_data.at("h").toIntVector();
+        const Unpacked u(ctx, 3);
+        const Tensor x = stand_in(s[0]), w1 = stand_in(s[1]), w2 = stand_in(s[2]), wp = stand_in(s[3]);
+        const OptTensor b1 = bias("b1", h[2]), b2 = bias("b2", h[3]);
+        const Projected r = project(x, w1, b1, w2, b2, h[0], h[1]);
+        const Tensor out = std::get<0>(call_fused(r.q, r.k, r.v, std::nullopt, std::nullopt, std::nullopt, u.list(0), u.list(1),
+                                                  u.list(2), u.flags(3), *saved_scale(ctx)));
+        const Tensor y = at::linear(joined_heads(out), wp);
+        const Tensor args[6] = {x, w1, b1.value_or(Tensor()), w2, b2.value_or(Tensor()), wp};
+        variable_list wanted, result(14);
+        for (int i = 0; i < 6; ++i)
+            if (needs[i]) wanted.push_back(args[i]);
+        if (!wanted.empty()) {
+            const variable_list got = torch::autograd::grad({y}, wanted, {grad}, /*retain_graph=*/true, /*create_graph=*/true,
+                                                            /*allow_unused=*/true);
+            for (int i = 0, n = 0; i < 6; ++i)
+                if (needs[i]) result[i] = got[n++];
+        }
+        if (needs[6]) result[6] = rows_of(grad).sum(0);
+        return result;
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads)
     {
@@ -621,6 +659,7 @@ struct ModuleFn : public torch::autograd::Function<ModuleFn> {
         const int64_t there = ctx->saved_data.at("m").toInt();
         bool needs[7];
         for (int i = 0, edge = 0; i < 7; ++i) needs[i] = ((there >> i) & 1) && ctx->needs_input_grad(edge++);
+        if (at::GradMode::is_enabled()) return differentiable(ctx, s, grads[0], needs);
         const Tensor g = rows_of(grads[0]), x2 = rows_of(x);
         if (needs[6]) r[6] = g.sum(0);           // (a kernel first: it makes the device's context current on the engine's thread)
         if (needs[5]) r[5] = g.t().mm(rows_of(joined_heads(s[7])));

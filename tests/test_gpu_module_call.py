@@ -42,3 +42,43 @@ def test_one_call_matches_the_separate_operators(case, dtype):
         for a, b in zip(*got):
             tol = 1e-5 if dtype == torch.float32 else 1e-2
             assert a.shape == b.shape and (a.float() - b.float()).norm() <= tol * b.float().norm().clamp_min(1e-3)
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: c[0])
+def test_gradients_with_a_graph_of_their_own(case):
+    """create_graph: what the separate operators allow (the attention itself is differentiable once), with the module applied
+    twice so that its weights are shared and its second input depends on them."""
+    _, cls, size, kw = case
+    if kw.get("stride", 1) != 1:
+        size = (83,)                                             # the second application needs its kernel, too
+    torch.manual_seed(2)
+    m = cls(64, 2, **{**kw, **({"num_kv_heads": 1} if "num_kv_heads" in kw else {})}).to("cuda", torch.float32)
+    x = torch.randn(2, *size, 64, device="cuda", requires_grad=True)
+    results = []
+    for hook in (False, True):
+        h = m.proj.register_forward_hook(lambda *a: None) if hook else None
+        y = m(m(x))
+        leaves = [x, *m.parameters()]
+        first = torch.autograd.grad(y.square().sum(), leaves, create_graph=True)
+        penalty = m(x).mul(0.5).tanh().sum()
+        by_weight = torch.autograd.grad(penalty, [m.proj.weight, m.proj.bias], create_graph=True)
+        second = torch.autograd.grad(sum(g.square().sum() for g in by_weight), leaves, allow_unused=True)
+        results.append([*first, *second])
+        if h is not None:
+            h.remove()
+    names = [n for n, _ in m.named_parameters()]
+    for name, a, b in zip(2 * ["x", *names], *results):
+        assert (a is None) == (b is None), name
+        if a is not None:
+            assert (a - b).norm() <= 1e-4 * b.norm().clamp_min(1e-3), name
+
+
+def test_gradients_with_a_graph_refuse_a_changed_bias():
+    m = nb.NeighborhoodAttention1D(64, 2, 7).to("cuda", torch.float32)
+    x = torch.randn(1, 40, 64, device="cuda", requires_grad=True)
+    y = m(x).sum()
+    with torch.no_grad():
+        m.qkv.bias.add_(1)
+    torch.autograd.grad(y, x, retain_graph=True)                 # no bias is needed for this one
+    with pytest.raises(RuntimeError, match="modified in place"):
+        torch.autograd.grad(y, x, create_graph=True)
