@@ -110,10 +110,12 @@ __device__ __forceinline__ bool tile_of(const FmaParams& P, unsigned bx, TileF& 
     if (!active) return false;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+        // along a0 there is one row, and nothing but this box says which columns are its own (a key that no query attends to,
+        // the last one of an even kernel, has none); along a1 and a2 each row has its own range in RowsF
         const int last = min(T.o[a] + tile[a], T.Lp[a]) - 1;
         int t, hi;
-        range_of<kKeySide>(P, a, T.o[a], T.Lp[a], T.lo[a], t, false);
-        range_of<kKeySide>(P, a, last, T.Lp[a], t, hi, false);
+        range_of<kKeySide>(P, a, T.o[a], T.Lp[a], T.lo[a], t, a == 0);
+        range_of<kKeySide>(P, a, last, T.Lp[a], t, hi, a == 0);
         T.n[a] = hi - T.lo[a];
     }
     return true;

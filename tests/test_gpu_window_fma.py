@@ -24,6 +24,8 @@ FUSED_CASES = [
     ("1d_d128", (261,), 2, 4, 2, (31,), (1,), (False,), 128),
     ("2d_d64_gqa", (21, 26), 1, 4, 2, (5, 9), (2, 1), (False, True), 64),
     ("2d_even", (23, 30), 1, 4, 2, (4, 6), (1, 1), (True, False), 32),
+    ("3d_even", (5, 6, 13), 2, 4, 2, (4, 3, 2), (1, 2, 1), (False, False, False), 32),
+    ("3d_even_causal", (9, 7, 10), 1, 2, 2, (2, 4, 3), (1, 1, 1), (False, True, False), 128),
     ("3d_d64", (4, 7, 11), 1, 2, 2, (3, 3, 5), (1, 2, 1), (False, True, False), 64),
 ]
 
@@ -75,6 +77,7 @@ SPLIT_CASES = [
     ("3d_d32", (6, 23, 25), 2, 4, 4, (3, 5, 5), (1, 1, 2), (True, False, False), 32),
     ("2d_d32_gqa", (45, 47), 2, 4, 2, (5, 3), (1, 2), (False, False), 32),
     ("2d_d32_even", (66, 45), 2, 4, 4, (6, 12), (1, 1), (False, True), 32),
+    ("3d_d32_even", (7, 21, 23), 2, 4, 4, (4, 3, 4), (1, 2, 1), (False, False, True), 32),
 ]
 # with these head dims the 16-bit types go to the tensor cores
 SPLIT_FLOAT32_CASES = [
