@@ -97,6 +97,11 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
         : "memory");
 }
+// The first load through a map otherwise waits for the map itself.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map)
+{
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 // Tile store, shared memory -> global (bulk group of the issuing thread).  Rows of the box that fall outside
 // the tensor are not written.  The first coordinate times the element size must be a multiple of 16 bytes and
 // no coordinate may be negative.

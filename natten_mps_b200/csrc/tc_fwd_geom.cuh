@@ -15,6 +15,7 @@ struct FwdTile {
     int rg[3], origin[3], Lp[3], lo[3], nc[3], x0[3], sx[3], nq[3], nqf[3];
     int nnb, nch;          // nch == 0 in a published header: no more tiles
     int active;
+    int mapped;            // the row maps of the tables are valid
 };
 
 // Walks the work items of a lane (w0, w0 + step, ...) without divisions: tile index inside the
@@ -113,6 +114,90 @@ __device__ __forceinline__ long long row_geometry(const TcParams& P, const FwdTi
     }
     if (!valid_q) { e[0] = f[0]; e[1] = f[1]; e[2] = f[2]; }
     return ((long long)T.b * P.otot + oflat) * P.Hq + T.h;
+}
+
+// What a softmax thread needs to know about its row is separable: along every axis the query's coordinate alone decides its
+// position, whether it exists and its window.  The loader writes one entry per (axis, coordinate of the tile) a tile ahead,
+// tile[0] + tile[1] + tile[2] of them instead of 128 rows x 3 axes.  A slot: FwdTile, row maps, axis entries.
+constexpr int kMapOff = 160, kEntOff = kMapOff + 8 * kTileRows, kTabBytes = kEntOff + 16 * (kTileRows + 2);
+static_assert(sizeof(FwdTile) <= kMapOff, "no room for the tile in front of its tables");
+
+// Query coordinate i of the tile along axis a: window [f, e) in the box, output position, flags (bit 0 query of the sample, bit 1
+// position of the tensor).
+__device__ __forceinline__ int4 axis_entry(const TcParams& P, const FwdTile& T, int a, int i)
+{
+    const int qa = T.origin[a] + i, xq = T.x0[a] + T.sx[a] * qa, pa = T.rg[a] + P.dil[a] * xq;
+    const int first = P.causal[a] ? xq - (P.K[a] - 1) : window_start(xq, T.Lp[a], P.K[a], 1);
+    return make_int4((first > 0 ? first : 0) - T.lo[a], (first + P.K[a] < T.Lp[a] ? first + P.K[a] : T.Lp[a]) - T.lo[a],
+                     P.st[a] == 1 ? pa : pa / P.st[a], (qa < T.nq[a] ? 1 : 0) | (qa < T.nqf[a] ? 2 : 0));
+}
+
+// One warp.  `mapped`: chunks of 16-column rows, one chunk along the innermost axis and at most 16 chunks in all.  Then which of
+// a chunk's four rows lie in a query's window depends on its two outer coordinates: a map per pair of them, four bits a chunk
+// (every row of the window lands in one row of one chunk), and the window's columns as bits beside the flags.
+__device__ __forceinline__ void write_tables(const TcParams& P, const FwdTile& T, int lane, uint8_t* slot)
+{
+    int4* ent = reinterpret_cast<int4*>(slot + kEntOff);
+    int base = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        for (int i = lane; i < P.tile[a]; i += 32) {
+            int4 en = axis_entry(P, T, a, i);
+            if (a == 2 && T.mapped) {
+                int lo, hi;
+                chunk_range(P, 2, 0, en.x, en.y, lo, hi);
+                if (hi > lo) en.w |= (low_bits(hi) & ~low_bits(lo)) << 16;
+            }
+            ent[base + i] = en;
+        }
+        base += P.tile[a];
+    }
+    if (!T.mapped) return;
+    unsigned long long* map = reinterpret_cast<unsigned long long*>(slot + kMapOff);
+    for (int r = lane; r < P.tile[0] * P.tile[1]; r += 32) {
+        const int4 e0 = axis_entry(P, T, 0, r >> P.tile1_log), e1 = axis_entry(P, T, 1, r & (P.tile[1] - 1));
+        unsigned long long bits = 0ull;
+        if (e0.w & e1.w & 1)
+            for (int x0 = e0.x; x0 < e0.y; ++x0) {
+                const int j0 = P.il[0] == 1 ? x0 & (P.cb[0] - 1) : (int)fast_div((unsigned)x0, P.il_mul[0]);
+                const int c0 = P.il[0] == 1 ? x0 >> P.cb0_log : x0 - j0 * P.il[0];
+                int j1 = P.il[1] == 1 ? e1.x & (P.cb[1] - 1) : (int)fast_div((unsigned)e1.x, P.il_mul[1]);
+                int at = 4 * (c0 * T.nc[1] + (P.il[1] == 1 ? e1.x >> P.cb1_log : e1.x - j1 * P.il[1])) + (j0 << P.cb1_log);
+                int c1 = P.il[1] == 1 ? 0 : e1.x - j1 * P.il[1];
+                for (int x1 = e1.x; x1 < e1.y; ++x1) {
+                    bits |= 1ull << (at + j1);
+                    if (P.il[1] == 1) {                      // along the chunk, then on to the next
+                        if (++j1 == P.cb[1]) { j1 = 0; at += 4; }
+                    } else {                                 // through the chunks, then one row further
+                        at += 4;
+                        if (++c1 == P.il[1]) { c1 = 0; ++j1; at -= 4 * P.il[1]; }
+                    }
+                }
+            }
+        map[r] = bits;
+    }
+}
+
+// A thread's row from the tables (what row_geometry gives, and the maps).
+__device__ __forceinline__ long long row_from_tables(const TcParams& P, const uint8_t* slot, int row, int (&f)[3], int (&e)[3],
+                                                     bool& valid_q, bool& in_tensor, unsigned long long& rowmap, uint32_t& colbits)
+{
+    const FwdTile* T = reinterpret_cast<const FwdTile*>(slot);
+    const int4* ent = reinterpret_cast<const int4*>(slot + kEntOff);
+    const int r01 = row >> P.tile2_log;
+    const int4 e0 = ent[r01 >> P.tile1_log], e1 = ent[P.tile[0] + (r01 & (P.tile[1] - 1))],
+               e2 = ent[P.tile[0] + P.tile[1] + (row & (P.tile[2] - 1))];
+    const int flags = e0.w & e1.w & e2.w;
+    valid_q = flags & 1;
+    in_tensor = flags & 2;
+    f[0] = e0.x; f[1] = e1.x; f[2] = e2.x;
+    e[0] = valid_q ? e0.y : e0.x;
+    e[1] = valid_q ? e1.y : e1.x;
+    e[2] = valid_q ? e2.y : e2.x;
+    rowmap = T->mapped ? reinterpret_cast<const unsigned long long*>(slot + kMapOff)[r01] : 0ull;
+    colbits = T->mapped && valid_q ? (uint32_t)e2.w >> 16 : 0u;
+    const long long oflat = ((long long)e0.z * P.O[1] + e1.z) * P.O[2] + e2.z;
+    return ((long long)T->b * P.otot + oflat) * P.Hq + T->h;
 }
 
 } // namespace fwdgeom

@@ -18,6 +18,15 @@
 // (128 TMEM columns and 49 KB of shared memory per CTA).  Above it only two CTAs fit (256 columns, 97 KB),
 // so the scores get two buffers there: S(c + 1) is computed while the threads work on S(c).
 //
+// Eight warps: four of softmax (a warpgroup), one that issues the products, one that loads, one for the geometry, one idle (a
+// register split goes by warpgroups).  What bounds it is the chain of a chunk, not an issue rate: S -> softmax -> P -> the
+// issuing warp -> P V and the next S, about 2800 cycles of which the softmax is 1500; four tiles in flight per SM share the
+// gaps.  So whatever is not the chain is kept off the issuing warp and the softmax warps.  Measured on one B200 (us), one warp that
+// loaded, issued and did the geometry | loads and geometry apart (kernel alone): 64 x 64, 7 x 7, 8 heads of 64, batch 8,
+// bf16 61.7 | 53.5; 128 x 128, 13 x 13, dilation 2, batch 4 196 | 177; 16 x 32 x 32, 3 x 7 x 7, causal frames, batch 2 137 | 120;
+// 135 x 241, 7 x 9, 6 heads of 32, batch 2, fp16 80 | 70; 8191 causal, window 255, 16 heads of 128 on 4, batch 2 98 | 82;
+// 28 x 28, 8 heads of 32 12.6 | 12.2.
+//
 // TMEM columns: head dim 64: S [0,64) (P over [0,32)), O [64,128);
 //               head dim 128: S of even chunks [0,64), of odd chunks [64,128), O [128,256).
 #include "tc_kernels.cuh"
@@ -38,10 +47,7 @@ namespace {
 constexpr int kKeys = 64;                   // keys per chunk
 constexpr int kKeysLog = 6;
 constexpr int kStages = 2;
-constexpr int kThreads = 160;               // 4 softmax warps + 1 warp that loads and issues
-constexpr int kHdrSlots = 3;                // tile headers published by the issuing warp
-constexpr int kHdrBytes = 144;
-static_assert(sizeof(FwdTile) <= kHdrBytes, "header slot too small");
+constexpr int kThreads = 256;               // 4 softmax warps; one that issues the products, one that loads, one for the geometry
 constexpr uint32_t kColS = 0;
 
 // Shared memory and TMEM of one CTA for head dim DH (64: four CTAs per SM, 128 TMEM columns; 128: two CTAs per
@@ -55,13 +61,18 @@ struct FwdSmall {
     static constexpr int kKVBytes = kKVHalf * kHalves;
     static constexpr int kOffQ = 0, kOffK = kQBytes, kOffV = kQBytes + kStages * kKVBytes;
     static constexpr int kBar = kQBytes + 2 * kStages * kKVBytes;
-    static constexpr int kHdr = kBar + 160;
-    static constexpr int kSmemTotal = kHdr + kHdrSlots * kHdrBytes;
+    static constexpr int kTab = kBar + 208;
+    static constexpr int kSmemTotal = kTab + 2 * kTabBytes;
     static constexpr uint32_t kTmemCols = DH == 64 ? 128 : 256;     // S 64 + O DH, rounded up to a power of two
     static constexpr int kPerSm = DH == 64 ? 4 : 2;
+    // 65536 / kPerSm / kThreads registers a thread at launch, 64 or 128; the helpers hand what they do not need to the softmax
+    // warps, which spill with less than 88 (32 | 96, where the helpers spill: 59.5 us instead of 53.5; 48 | 80: 54.0)
+    static constexpr int kHelperRegs = DH == 64 ? 40 : 104, kSoftmaxRegs = DH == 64 ? 88 : 152;
     // At head dim 128 the 256 TMEM columns hold two score buffers: S(c + 1) is computed while the threads turn
     // S(c) into probabilities (at 64 the four CTAs of an SM fill each other's gaps instead).
     static constexpr bool kTwoS = DH == 128;
+    // There K has to be a chunk ahead of V, so the two are loaded and freed apart; with one score buffer they come and go together.
+    static constexpr bool kSplitKV = kTwoS;
     static constexpr uint32_t kColO = kTwoS ? 128 : 64;
 };
 
@@ -75,33 +86,34 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 {
     using FS = FwdSmall<DH>;
     constexpr int kHalves = FS::kHalves, kQHalf = FS::kQHalf, kKVHalf = FS::kKVHalf, kQBytes = FS::kQBytes, kKVBytes = FS::kKVBytes;
-    constexpr int kOffQ = FS::kOffQ, kOffK = FS::kOffK, kOffV = FS::kOffV, kBar = FS::kBar, kHdr = FS::kHdr;
+    constexpr int kOffQ = FS::kOffQ, kOffK = FS::kOffK, kOffV = FS::kOffV, kBar = FS::kBar, kTab = FS::kTab;
     constexpr uint32_t kTmemCols = FS::kTmemCols, kColO = FS::kColO;
-    constexpr bool kTwoS = FS::kTwoS;
+    constexpr bool kTwoS = FS::kTwoS, kSplitKV = FS::kSplitKV;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int prior_abort = *reinterpret_cast<volatile int*>(P.status);
 
     const uint32_t sbase = smem_u32(smem);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kBar + 112);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kBar + 120);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kBar + 192);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kBar + 200);
     const uint32_t bar_q = sbase + kBar + 0;            // Q tile landed
     const uint32_t bar_qfree = sbase + kBar + 8;        // last Q K^T of the tile finished: Q may be overwritten
-    const uint32_t bar_kv = sbase + kBar + 16;          // [2] K, V chunk landed
-    const uint32_t bar_kvfree = sbase + kBar + 32;      // [2] P V of the chunk finished: stage may be overwritten
-    const uint32_t bar_s = sbase + kBar + 48;           // S of the chunk is in TMEM (and every earlier product is done)
-    const uint32_t bar_p = sbase + kBar + 56;           // every thread stored its P
-    const uint32_t bar_o = sbase + kBar + 64;           // last P V of the tile finished
-    const uint32_t bar_hdr = sbase + kBar + 72;         // [3] geometry of the CTA's t-th tile published
-    const uint32_t bar_s1 = sbase + kBar + 96;          // two score buffers: bar_s / bar_p of the odd chunks
-    const uint32_t bar_p1 = sbase + kBar + 104;
-    const uint32_t bar_pv = sbase + kBar + 128;         // [2] two score buffers: P V of the chunk finished (by chunk parity)
+    const uint32_t bar_k = sbase + kBar + 16;           // [2] K chunk landed
+    const uint32_t bar_v = sbase + kBar + 32;           // [2] V chunk landed
+    const uint32_t bar_kfree = sbase + kBar + 48;       // [2] Q K^T of the chunk finished: its K may be overwritten
+    const uint32_t bar_vfree = sbase + kBar + 64;       // [2] P V of the chunk finished: its V may be overwritten
+    const uint32_t bar_s = sbase + kBar + 80;           // [2] S of the chunk is in TMEM (one score buffer: and every earlier product is done)
+    const uint32_t bar_p = sbase + kBar + 96;           // [2] every thread stored its P
+    const uint32_t bar_o = sbase + kBar + 112;          // last P V of the tile finished
+    const uint32_t bar_head = sbase + kBar + 120;       // [2] geometry of the CTA's t-th tile published
+    const uint32_t bar_tab_full = sbase + kBar + 136;   // [2] ... and its tables
+    const uint32_t bar_tab_empty = sbase + kBar + 152;  // [2] ... read by the softmax threads and the other helpers
     // chunk n (counted over the CTA's whole run) -> its score columns, barriers and wait parity
     auto s_cols = [&](unsigned n) -> uint32_t { return kTwoS ? 64u * (n & 1u) : 0u; };
-    auto bar_s_of = [&](unsigned n) -> uint32_t { return (kTwoS && (n & 1u)) ? bar_s1 : bar_s; };
-    auto bar_p_of = [&](unsigned n) -> uint32_t { return (kTwoS && (n & 1u)) ? bar_p1 : bar_p; };
+    auto bar_s_of = [&](unsigned n) -> uint32_t { return bar_s + (kTwoS ? 8u * (n & 1u) : 0u); };
+    auto bar_p_of = [&](unsigned n) -> uint32_t { return bar_p + (kTwoS ? 8u * (n & 1u) : 0u); };
     auto par_of = [&](unsigned n) -> uint32_t { return kTwoS ? ((n >> 1) & 1u) : (n & 1u); };
-    auto hdr_slot = [&](unsigned t) { return reinterpret_cast<FwdTile*>(smem + kHdr + (t % kHdrSlots) * kHdrBytes); };
+    auto tab_slot = [&](unsigned t) { return reinterpret_cast<FwdTile*>(smem + kTab + (t & 1) * kTabBytes); };
 
     if (warp == 4) {
         if (lane == 0) {
@@ -109,198 +121,227 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             *abort_flag = ((sbase & 1023u) || prior_abort) ? 1 : 0;
             mbar_init(bar_q, 1);
             mbar_init(bar_qfree, 1);
-            for (int s = 0; s < kStages; ++s) { mbar_init(bar_kv + 8 * s, 1); mbar_init(bar_kvfree + 8 * s, 1); }
-            mbar_init(bar_s, 1);
-            mbar_init(bar_p, 128);
-            mbar_init(bar_s1, 1);
-            mbar_init(bar_p1, 128);
-            mbar_init(bar_pv, 1);
-            mbar_init(bar_pv + 8, 1);
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(bar_k + 8 * i, 1);
+                mbar_init(bar_v + 8 * i, 1);
+                mbar_init(bar_kfree + 8 * i, 1);
+                mbar_init(bar_vfree + 8 * i, 1);
+                mbar_init(bar_s + 8 * i, 1);
+                mbar_init(bar_p + 8 * i, 128);
+                mbar_init(bar_head + 8 * i, 1);
+                mbar_init(bar_tab_full + 8 * i, 32);
+                mbar_init(bar_tab_empty + 8 * i, 130);
+            }
             mbar_init(bar_o, 1);
-            for (int i = 0; i < kHdrSlots; ++i) mbar_init(bar_hdr + 8 * i, 1);
             mbar_init_fence();
             fence_async_smem();
         }
         __syncwarp();
         tmem_alloc(smem_u32(tmem_slot), kTmemCols);
+    } else if (warp == 5 && lane == 0) {
+        prefetch_map(&tmQ);
+        prefetch_map(&tmK);
+        prefetch_map(&tmV);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const unsigned nwork = P.work_q;
-
-    if (warp == 4) {
-        // =====================================================================
-        // Geometry, TMA loads and MMA issue.  The whole warp walks the CTA's work items (blockIdx.x,
-        // + gridDim.x, ...): it works out each tile's geometry and publishes it for the softmax warps,
-        // writes the zero rows of tiles that have nothing to attend to, and lane 0 issues the loads (Q of
-        // the next tile and the K/V ring run ahead across tile boundaries) and the matrix products.
-        // =====================================================================
-        if (!*abort_flag) {
-            constexpr uint32_t idesc_qk = instr_desc(BF16 ? 1 : 0, kKeys, 0, 0);
-            constexpr uint32_t idesc_pv = instr_desc(BF16 ? 1 : 0, DH, 0, 1);
-            const uint64_t dq0 = smem_desc(sbase + kOffQ, 16, 1024);
-            const uint32_t leader = elect_one();
-            bool ok = true;
-            Cursor cur;
-            cur.init(P, blockIdx.x, gridDim.x);
-            unsigned pub = 0;                    // headers published (the last one may be the end marker)
-            bool exhausted = false;
-            auto discover = [&]() {              // next tile with work -> header ring
-                if (exhausted) return;
-                FwdTile Tn;
-                bool found = false;
-                while (cur.w < nwork) {
-                    fwd_tile(P, cur, kKeysLog, Tn);
-                    cur.advance(P, gridDim.x);
-                    if (Tn.active) { found = true; break; }
-#pragma unroll 1
-                    for (int r = lane; r < kTileRows; r += 32) {         // rows that exist in the output are zero
-                        int f[3], e[3];
-                        bool valid_q, in_tensor;
-                        const long long out_row = row_geometry(P, Tn, r, f, e, valid_q, in_tensor);
-                        if (in_tensor) {
-                            uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
+    if (warp >= 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FS::kHelperRegs));
+        if (warp == 4) {
+            // =====================================================================
+            // MMA issue.  The whole warp walks the CTA's tiles; the tensor-core instructions execute on one elected lane.  What it
+            // does between a chunk's last probability and the next chunk's scores is on the chain of every chunk, so the loads
+            // and the geometry are the loader's, descriptors are ready and the next chunk's operands have been waited for.
+            // =====================================================================
+            if (!*abort_flag) {
+                constexpr uint32_t idesc_qk = instr_desc(BF16 ? 1 : 0, kKeys, 0, 0);
+                constexpr uint32_t idesc_pv = instr_desc(BF16 ? 1 : 0, DH, 0, 1);
+                const uint64_t dq0 = smem_desc(sbase + kOffQ, 16, 1024);
+                const uint64_t dk_even = smem_desc(sbase + kOffK, 16, 1024), dk_odd = smem_desc(sbase + kOffK + kKVBytes, 16, 1024);
+                const uint64_t dv_even = smem_desc(sbase + kOffV, kKVHalf, 1024), dv_odd = smem_desc(sbase + kOffV + kKVBytes, kKVHalf, 1024);
+                const uint32_t leader = elect_one();
+                bool ok = true;
+                unsigned n_qk = 0, n_pv = 0;
+                for (unsigned t = 0;; ++t) {
+                    ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
+                    if (!ok) break;
+                    const FwdTile* H = tab_slot(t);
+                    const int nch = H->nch;
+                    int nnb = 0, lo[3] = {0, 0, 0}, Lp[3] = {0, 0, 0}, nc[3] = {1, 1, 1};
+                    bool padded = false;             // some chunk reaches past the sample's extent: those rows are zeroed
+                    if (P.extents) {
+                        nnb = H->nnb;
 #pragma unroll
-                            for (int i = 0; i < DH / 8; ++i)
-                                if (8 * i < P.dreal) o4[i] = make_uint4(0, 0, 0, 0);
-                            lse[out_row] = 0.f;
+                        for (int a = 0; a < 3; ++a) {
+                            lo[a] = H->lo[a]; Lp[a] = H->Lp[a]; nc[a] = H->nc[a];
+                            padded = padded || lo[a] + chunk_coord(P, a, nc[a] - 1, P.cb[a] - 1) >= Lp[a];
                         }
                     }
+                    __syncwarp();                    // every lane has read the header
+                    if (leader) mbar_arrive(bar_tab_empty + 8 * (t & 1));
+                    if (nch == 0) break;
+                    auto zero_padding = [&](int c, uint8_t* tile) {
+                        if (c >= nnb) return;
+                        const int c2 = c % nc[2], c1 = c / nc[2] % nc[1], c0 = c / nc[2] / nc[1];
+                        const int box0[3] = {lo[0] + chunk_coord(P, 0, c0, 0), lo[1] + chunk_coord(P, 1, c1, 0), lo[2] + chunk_coord(P, 2, c2, 0)};
+                        if (leader) zero_rows_past_extent(P, box0, Lp, kKeys, kHalves, kKVHalf, tile, tile);
+                        __syncwarp();
+                    };
+                    auto wait_k = [&](int c) {       // chunk c's K has landed (and ends where the sample ends)
+                        const unsigned s = n_qk & 1u;
+                        ok = ok && mbar_wait(bar_k + 8 * s, (n_qk >> 1) & 1, abort_flag, P.wait_budget);
+                        if (ok && padded) zero_padding(c, smem + kOffK + s * kKVBytes);
+                    };
+                    auto issue_qk = [&](bool last) {
+                        const uint64_t dk0 = (n_qk & 1u) ? dk_odd : dk_even;
+#pragma unroll
+                        for (int ks = 0; ks < (kShort ? DH / 16 - 2 : DH / 16); ++ks) {     // 32 bytes per k-step inside a 64-channel block
+                            mma_ss_e(tmem + kColS + s_cols(n_qk), dq0 + ((((ks / 4) * kQHalf) + (ks % 4) * 32) >> 4),
+                                     dk0 + ((((ks / 4) * kKVHalf) + (ks % 4) * 32) >> 4), idesc_qk, ks > 0, leader);
+                        }
+                        mma_commit_e(bar_s_of(n_qk), leader);
+                        if (kSplitKV) mma_commit_e(bar_kfree + 8 * (n_qk & 1u), leader);
+                        if (last) mma_commit_e(bar_qfree, leader);        // last scores of the tile: Q may go once they are done
+                        ++n_qk;
+                    };
+                    ok = mbar_wait(bar_q, t & 1, abort_flag, P.wait_budget);
+                    wait_k(0);
+                    if (!ok) break;
+                    tc_fence_after();
+                    issue_qk(nch == 1);
+                    for (int c = 0; c < nch; ++c) {
+                        const bool more = c + 1 < nch;
+                        if (more) wait_k(c + 1);
+                        // two score buffers: S(c + 1) goes into the other buffer while the threads work on S(c); that
+                        // buffer's P(c - 1) is read by a product issued earlier from this warp, so the order holds
+                        if (kTwoS && more && ok) { tc_fence_after(); issue_qk(c + 2 == nch); }
+                        const unsigned sv = n_pv & 1u;
+                        if (kSplitKV) ok = ok && mbar_wait(bar_v + 8 * sv, (n_pv >> 1) & 1, abort_flag, P.wait_budget);
+                        if (ok && padded) zero_padding(c, smem + kOffV + sv * kKVBytes);
+                        ok = ok && mbar_wait(bar_p_of(n_pv), par_of(n_pv), abort_flag, P.wait_budget);      // P(c) stored over S(c)
+                        if (!ok) break;
+                        tc_fence_after();
+                        // V read MN-major: 16 key rows per k-step; P sits as 16-bit pairs in the first 32 S columns
+                        const uint64_t dv0 = sv ? dv_odd : dv_even;
+#pragma unroll
+                        for (int ks = 0; ks < kKeys / 16; ++ks)
+                            mma_ts_e(tmem + kColO, tmem + kColS + s_cols(n_pv) + 8 * ks, dv0 + 128 * ks, idesc_pv, (c > 0 || ks > 0) ? 1u : 0u, leader);
+                        mma_commit_e(bar_vfree + 8 * sv, leader);
+                        if (!kTwoS && more) issue_qk(c + 2 == nch);      // after P(c) has been read (issue order): over it
+                        if (!more) mma_commit_e(bar_o, leader);
+                        ++n_pv;
+                    }
+                    if (!ok) break;
                 }
-                if (!found) { exhausted = true; Tn.nch = 0; }
-                if (lane == 0) {
-                    *hdr_slot(pub) = Tn;
-                    mbar_arrive(bar_hdr + 8 * (pub % kHdrSlots));
-                }
-                __syncwarp();
-                ++pub;
-            };
-
-            // ---- loads: tile tl, its Q, then its chunks; never waits for work that has not been issued ----
-            unsigned tl = 0, n_load = 0, n_pv = 0, n_qk = 0, qk_done_tiles = 0;
-            int cl = 0, ldc[3] = {0, 0, 0};
-            bool q_loaded = false;
-            auto refill = [&]() -> bool {
-                if (!ok || tl >= pub) return false;
-                const FwdTile* H = hdr_slot(tl);
-                if (H->nch == 0) return false;
-                if (!q_loaded) {
-                    if (tl > qk_done_tiles) return false;                // the previous tile still needs its Q
-                    if (tl > 0) ok = mbar_wait(bar_qfree, (tl - 1) & 1, abort_flag, P.wait_budget);
-                    if (!ok) return false;
+            }
+        } else if (warp == 5) {
+            // =====================================================================
+            // Loads: Q of a tile, then its chunks; both run ahead across tile boundaries as far as the buffers allow.
+            // =====================================================================
+            if (!*abort_flag) {
+                bool ok = true;
+                unsigned n = 0;                                  // chunks loaded
+                for (unsigned t = 0;; ++t) {
+                    ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
+                    if (!ok) break;
+                    const FwdTile* H = tab_slot(t);
+                    const int b = H->b, h = H->h, hk = H->hk, nnb = H->nnb, nch = H->nch, nc1 = H->nc[1], nc2 = H->nc[2];
+                    const int X0 = H->rg[0] + P.dil[0] * H->lo[0], X1 = H->rg[1] + P.dil[1] * H->lo[1], X2 = H->rg[2] + P.dil[2] * H->lo[2];
+                    const int Q0 = H->rg[0] + P.dil[0] * (H->x0[0] + H->sx[0] * H->origin[0]),
+                              Q1 = H->rg[1] + P.dil[1] * (H->x0[1] + H->sx[1] * H->origin[1]),
+                              Q2 = H->rg[2] + P.dil[2] * (H->x0[2] + H->sx[2] * H->origin[2]);
+                    __syncwarp();                                // every lane has read the header
+                    if (lane == 0) mbar_arrive(bar_tab_empty + 8 * (t & 1));
+                    if (nch == 0) break;
+                    if (t > 0) ok = mbar_wait(bar_qfree, (t - 1) & 1, abort_flag, P.wait_budget);
+                    if (!ok) break;
                     if (lane == 0) {
-                        mbar_expect_tx(bar_q, kQBytes + ((P.inject == 1 && tl == 0) ? 16u : 0u));
+                        mbar_expect_tx(bar_q, kQBytes + ((P.inject == 1 && t == 0) ? 16u : 0u));
 #pragma unroll
                         for (int hf = 0; hf < kHalves; ++hf)
-                            tma_load_heads(sbase + kOffQ + hf * kQHalf, &tmQ, bar_q, P, H->h, 64 * hf,
-                                        H->rg[2] + P.dil[2] * (H->x0[2] + H->sx[2] * H->origin[2]),
-                                        H->rg[1] + P.dil[1] * (H->x0[1] + H->sx[1] * H->origin[1]),
-                                        H->rg[0] + P.dil[0] * (H->x0[0] + H->sx[0] * H->origin[0]), H->b);
+                            tma_load_heads(sbase + kOffQ + hf * kQHalf, &tmQ, bar_q, P, h, 64 * hf, Q2, Q1, Q0, b);
                     }
-                    q_loaded = true;
-                    return true;
-                }
-                if (n_load >= n_pv + kStages) return false;              // both stages wait for products not issued yet
-                const int s = n_load % kStages;
-                if (n_load >= (unsigned)kStages)
-                    ok = mbar_wait(bar_kvfree + 8 * s, ((n_load / kStages) - 1) & 1, abort_flag, P.wait_budget);
-                if (!ok) return false;
-                if (lane == 0) {
-                    const uint32_t bar = bar_kv + 8 * s;
-                    mbar_expect_tx(bar, 2 * kKVBytes);
-                    if (cl < H->nnb) {
-                        const int X0 = H->rg[0] + P.dil[0] * (H->lo[0] + chunk_coord(P, 0, ldc[0], 0));
-                        const int X1 = H->rg[1] + P.dil[1] * (H->lo[1] + chunk_coord(P, 1, ldc[1], 0));
-                        const int X2 = H->rg[2] + P.dil[2] * (H->lo[2] + chunk_coord(P, 2, ldc[2], 0));
+                    int c0 = 0, c1 = 0, c2 = 0;
+                    for (int c = 0; c < nch; ++c, ++n) {
+                        const unsigned s = n & 1u, parity = ((n >> 1) - 1) & 1;
+                        const bool box = c < nnb;                // else additional tokens (rows past n_extra are zero-filled)
+                        const int x0 = box ? X0 + P.dil[0] * chunk_coord(P, 0, c0, 0) : 0, x1 = box ? X1 + P.dil[1] * chunk_coord(P, 1, c1, 0) : 0,
+                                  x2 = box ? X2 + P.dil[2] * chunk_coord(P, 2, c2, 0) : (c - nnb) * kKeys;
+                        if (++c2 == nc2) { c2 = 0; if (++c1 == nc1) { c1 = 0; ++c0; } }
+                        if (n >= (unsigned)kStages) ok = mbar_wait((kSplitKV ? bar_kfree : bar_vfree) + 8 * s, parity, abort_flag, P.wait_budget);
+                        if (!ok) break;
+                        const uint32_t full_k = bar_k + 8 * s, full_v = (kSplitKV ? bar_v : bar_k) + 8 * s;
+                        if (lane == 0) {
+                            mbar_expect_tx(full_k, kSplitKV ? kKVBytes : 2 * kKVBytes);
 #pragma unroll
-                        for (int hf = 0; hf < kHalves; ++hf) {
-                            tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, &tmK, bar, P, H->hk, 64 * hf, X2, X1, X0, H->b);
-                            tma_load_heads(sbase + kOffV + s * kKVBytes + hf * kKVHalf, &tmV, bar, P, H->hk, 64 * hf, X2, X1, X0, H->b);
+                            for (int hf = 0; hf < kHalves; ++hf)
+                                tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, box ? &tmK : &tmEK, full_k, P, hk, 64 * hf, x2, x1, x0, b);
                         }
-                    } else {                     // additional tokens (rows past n_extra are zero-filled)
-                        const int e0 = (cl - H->nnb) * kKeys;
+                        __syncwarp();
+                        if (kSplitKV && n >= (unsigned)kStages) ok = mbar_wait(bar_vfree + 8 * s, parity, abort_flag, P.wait_budget);
+                        if (!ok) break;
+                        if (lane == 0) {
+                            if (kSplitKV) mbar_expect_tx(full_v, kKVBytes);
 #pragma unroll
-                        for (int hf = 0; hf < kHalves; ++hf) {
-                            tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, &tmEK, bar, P, H->hk, 64 * hf, e0, 0, 0, H->b);
-                            tma_load_heads(sbase + kOffV + s * kKVBytes + hf * kKVHalf, &tmEV, bar, P, H->hk, 64 * hf, e0, 0, 0, H->b);
+                            for (int hf = 0; hf < kHalves; ++hf)
+                                tma_load_heads(sbase + kOffV + s * kKVBytes + hf * kKVHalf, box ? &tmV : &tmEV, full_v, P, hk, 64 * hf, x2, x1, x0, b);
+                        }
+                        __syncwarp();
+                    }
+                    if (!ok) break;
+                }
+            }
+        } else if (warp == 6) {
+            // =====================================================================
+            // Geometry: the CTA's tiles (blockIdx.x, + gridDim.x, ...), each one's tables as soon as its slot is free.  Rows of padding
+            // tiles (per-sample extents) are zeroed here.
+            // =====================================================================
+            if (!*abort_flag) {
+                bool ok = true, found = true;
+                Cursor cur;
+                cur.init(P, blockIdx.x, gridDim.x);
+                for (unsigned t = 0; ok && found; ++t) {
+                    FwdTile T;
+                    found = false;
+                    while (cur.w < nwork && !found) {
+                        fwd_tile(P, cur, kKeysLog, T);
+                        cur.advance(P, gridDim.x);
+                        found = T.active != 0;
+                        if (found || !P.extents) continue;
+#pragma unroll 1
+                        for (int r = lane; r < kTileRows; r += 32) {
+                            int f[3], e[3];
+                            bool valid_q, in_tensor;
+                            const long long out_row = row_geometry(P, T, r, f, e, valid_q, in_tensor);
+                            if (in_tensor) {
+                                uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
+#pragma unroll
+                                for (int i = 0; i < DH / 8; ++i)
+                                    if (8 * i < P.dreal) o4[i] = make_uint4(0, 0, 0, 0);
+                                lse[out_row] = 0.f;
+                            }
                         }
                     }
-                }
-                if (cl < H->nnb) { if (++ldc[2] == H->nc[2]) { ldc[2] = 0; if (++ldc[1] == H->nc[1]) { ldc[1] = 0; ++ldc[0]; } } }
-                ++n_load;
-                if (++cl == H->nch) { ++tl; cl = 0; ldc[0] = ldc[1] = ldc[2] = 0; q_loaded = false; }
-                return true;
-            };
-
-            int qc[3] = {0, 0, 0};
-            auto issue_qk = [&](const FwdTile* H, int c) {
-                const int s = n_qk % kStages;
-                ok = ok && mbar_wait(bar_kv + 8 * s, (n_qk / kStages) & 1, abort_flag, P.wait_budget);
-                if (!ok) return;
-                if (P.extents && c < H->nnb) {
-                    const int box0[3] = {H->lo[0] + chunk_coord(P, 0, qc[0], 0), H->lo[1] + chunk_coord(P, 1, qc[1], 0),
-                                         H->lo[2] + chunk_coord(P, 2, qc[2], 0)};
-                    if (lane == 0)
-                        zero_rows_past_extent(P, box0, H->Lp, kKeys, kHalves, kKVHalf, smem + kOffK + s * kKVBytes, smem + kOffV + s * kKVBytes);
+                    if (!found) T.nch = 0;
+                    if (t >= 2) ok = mbar_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
+                    if (!ok) break;
+                    FwdTile* H = tab_slot(t);
+                    T.mapped = kInner == 16 && T.nc[2] == 1 && T.nnb <= 16;
+                    if (lane == 0) {
+                        *H = T;
+                        mbar_arrive(bar_head + 8 * (t & 1));
+                    }
                     __syncwarp();
-                }
-                {   // warp-uniform code; the tensor-core instructions execute on the elected lane
-                    const uint64_t dk0 = smem_desc(sbase + kOffK + s * kKVBytes, 16, 1024);
-                    tc_fence_after();
-#pragma unroll
-                    for (int ks = 0; ks < (kShort ? DH / 16 - 2 : DH / 16); ++ks) {     // 32 bytes per k-step inside a 64-channel block
-                        mma_ss_e(tmem + kColS + s_cols(n_qk), dq0 + ((((ks / 4) * kQHalf) + (ks % 4) * 32) >> 4),
-                                 dk0 + ((((ks / 4) * kKVHalf) + (ks % 4) * 32) >> 4), idesc_qk, ks > 0, leader);
-                    }
-                    mma_commit_e(bar_s_of(n_qk), leader);
-                    if (c + 1 == H->nch) mma_commit_e(bar_qfree, leader);     // last scores of the tile: Q may go once they are done
-                }
-                if (c < H->nnb) { if (++qc[2] == H->nc[2]) { qc[2] = 0; if (++qc[1] == H->nc[1]) { qc[1] = 0; ++qc[0]; } } }
-                ++n_qk;
-                if (c + 1 == H->nch) { ++qk_done_tiles; qc[0] = qc[1] = qc[2] = 0; }
-            };
-            auto issue_pv = [&](int c, bool last) {
-                // V read MN-major: 16 key rows per k-step; P sits as 16-bit pairs in the first 32 S columns
-                const int s = n_pv % kStages;
-                {
-                    const uint64_t dv0 = smem_desc(sbase + kOffV + s * kKVBytes, kKVHalf, 1024);
-                    tc_fence_after();
-#pragma unroll
-                    for (int ks = 0; ks < kKeys / 16; ++ks)
-                        mma_ts_e(tmem + kColO, tmem + kColS + s_cols(n_pv) + 8 * ks, dv0 + 128 * ks, idesc_pv, (c > 0 || ks > 0) ? 1u : 0u, leader);
-                    mma_commit_e(bar_kvfree + 8 * s, leader);
-                    if (kTwoS) mma_commit_e(bar_pv + 8 * (n_pv & 1u), leader);
-                    if (last) mma_commit_e(bar_o, leader);
-                }
-                ++n_pv;
-            };
-
-            discover();
-            while (refill()) {}
-            for (unsigned ti = 0; ok; ++ti) {
-                const FwdTile* H = hdr_slot(ti);
-                const int nch = H->nch;
-                if (nch == 0) break;
-                ok = mbar_wait(bar_q, ti & 1, abort_flag, P.wait_budget);
-                issue_qk(H, 0);
-                discover();                      // the next tile's geometry, while the threads work on this chunk
-                while (refill()) {}
-                for (int c = 0; c < nch && ok; ++c) {
-                    // two score buffers: S(c + 1) goes into the other buffer while the threads work on S(c); that
-                    // buffer's P(c - 1) is read by a product issued earlier from this warp, so the order holds
-                    if (kTwoS && c + 1 < nch) issue_qk(H, c + 1);
-                    if (!ok) break;
-                    ok = mbar_wait(bar_p_of(n_pv), par_of(n_pv), abort_flag, P.wait_budget);      // P(c) stored over S(c)
-                    if (!ok) break;
-                    issue_pv(c, c + 1 == nch);       // reads P(c) ...
-                    if (!kTwoS && c + 1 < nch) issue_qk(H, c + 1);   // ... before the next scores overwrite it (issue order)
-                    while (refill()) {}
+                    if (found) write_tables(P, T, lane, reinterpret_cast<uint8_t*>(H));
+                    mbar_arrive(bar_tab_full + 8 * (t & 1));
                 }
             }
         }
     } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FS::kSoftmaxRegs));
         // =====================================================================
         // softmax warps: thread = one query row, the chunk's 64 columns in 16-column pieces
         // =====================================================================
@@ -333,7 +374,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             if (c > 0) {
                 // with two score buffers S(c) was issued before P V of chunk c - 1: wait for that product itself
                 if (kTwoS) {
-                    ok = mbar_wait(bar_pv + 8 * ((n - 1) & 1u), par_of(n - 1), abort_flag, P.wait_budget) && ok;
+                    ok = mbar_wait(bar_vfree + 8 * ((n - 1) & 1u), par_of(n - 1), abort_flag, P.wait_budget) && ok;
                     tc_fence_after();
                 }
 #pragma unroll 1
@@ -375,55 +416,37 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         };
 
         for (unsigned t = 0;; ++t) {
-        ok = mbar_wait(bar_hdr + 8 * (t % kHdrSlots), (t / kHdrSlots) & 1, abort_flag, P.wait_budget) && ok;
+        ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
         if (!ok) break;
-        const FwdTile T = *hdr_slot(t);
-        if (T.nch == 0) break;
-        // ---- this thread's query row ----
+        const FwdTile* H = tab_slot(t);
+        const int nch = H->nch;
+        if (nch == 0) break;
+        // ---- this thread's query row, from the loader's tables ----
+        const int nnb = H->nnb, nc1 = H->nc[1], nc2 = H->nc[2];
+        const bool mapped = kRows16 && H->mapped;
         int f[3], e[3];
         bool valid_q, in_tensor;
-        const long long out_row = row_geometry(P, T, warp * 32 + lane, f, e, valid_q, in_tensor);
+        unsigned long long rowmap;
+        uint32_t colbits;                    // 16-column rows: one bit per column
+        const long long out_row = row_from_tables(P, reinterpret_cast<const uint8_t*>(H), warp * 32 + lane, f, e, valid_q, in_tensor, rowmap, colbits);
+        mbar_arrive(bar_tab_empty + 8 * (t & 1));
         m = -INFINITY;
         l = 0.f;
         add_cols = 0xffffffffu;              // the addends belong to the previous tile's stabiliser
         int ci[3] = {0, 0, 0};
         const bool line = line_chunks(P);    // chunks are runs of the innermost axis (1-D windows): cheap validity words
         int jl[3] = {0, 0, 0}, jh[3] = {0, 0, 0};
-        uint32_t rowbits = 0u, colbits = 0u, dirty = 7u;     // 16-column rows: one bit per piece, one per column
-        // 16-column rows with a single chunk along the innermost axis and at most 16 chunks: which pieces of
-        // which chunk lie inside the row's window is worked out once per tile from the row's side (a loop over
-        // the window's rows, each of which lands in one piece of one chunk), four bits per chunk.
-        bool mapped = false;
-        unsigned long long rowmap = 0ull;
-        if constexpr (kRows16) {
-            if (T.nc[2] == 1 && T.nnb <= 16) {
-                mapped = true;
-                for (int x0 = f[0]; x0 < e[0]; ++x0) {
-                    int c0, j0;
-                    if (P.il[0] == 1) { c0 = x0 >> P.cb0_log; j0 = x0 & (P.cb[0] - 1); }
-                    else { j0 = (int)fast_div((unsigned)x0, P.il_mul[0]); c0 = x0 - j0 * P.il[0]; }
-                    for (int x1 = f[1]; x1 < e[1]; ++x1) {
-                        int c1, j1;
-                        if (P.il[1] == 1) { c1 = x1 >> P.cb1_log; j1 = x1 & (P.cb[1] - 1); }
-                        else { j1 = (int)fast_div((unsigned)x1, P.il_mul[1]); c1 = x1 - j1 * P.il[1]; }
-                        rowmap |= 1ull << (4 * (c0 * T.nc[1] + c1) + (j0 << P.cb1_log) + j1);
-                    }
-                }
-                int l2, h2;
-                chunk_range(P, 2, 0, f[2], e[2], l2, h2);
-                colbits = h2 > l2 ? (low_bits(h2) & ~low_bits(l2)) : 0u;
-            }
-        }
-        for (int c = 0; c < T.nch; ++c, ++n) {
+        uint32_t rowbits = 0u, dirty = 7u;   // 16-column rows: one bit per piece
+        for (int c = 0; c < nch; ++c, ++n) {
             // ---- validity of this row's columns in this chunk ----
             // jl/jh (columns of the chunk inside the row's window, per axis) only change along the axes whose
             // chunk index moved since the last chunk: `dirty` has a bit per axis.
-            const bool extra = c >= T.nnb;   // additional tokens: every live row sees the first n_extra columns
+            const bool extra = c >= nnb;   // additional tokens: every live row sees the first n_extra columns
             uint32_t words[2] = {0u, 0u};    // generic form: one bit per column
             if (extra) {
 #pragma unroll
                 for (int pc = 0; pc < 2; ++pc)
-                    words[pc] = valid_q ? low_bits(P.n_extra - ((c - T.nnb) * kKeys + 32 * pc)) : 0u;
+                    words[pc] = valid_q ? low_bits(P.n_extra - ((c - nnb) * kKeys + 32 * pc)) : 0u;
             } else if (mapped) {
                 rowbits = (uint32_t)(rowmap >> (4 * c)) & 15u;
             } else {
@@ -455,11 +478,16 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
             const bool fast = kRows16 && !extra;
             if (fast && colbits != add_cols) refresh_add(colbits);
+            uint32_t mine = 0u, act = 0u;    // pieces inside this row's window, inside that of any row of the warp
+            if (fast) {
+                mine = colbits != 0u ? rowbits & 15u : 0u;
+                act = __reduce_or_sync(0xffffffffu, mine);
+            }
 
             scol = trow + kColS + s_cols(n);
             ok = ok && mbar_wait(bar_s_of(n), par_of(n), abort_flag, P.wait_budget);     // one score buffer: every earlier product has finished, too
             tc_fence_after();
-            if (!ok) { words[0] = 0u; words[1] = 0u; rowbits = 0u; dirty = 7u; }
+            if (!__all_sync(0xffffffffu, ok)) { words[0] = 0u; words[1] = 0u; act = 0u; dirty = 7u; }
 
             uint32_t stored = 0u;            // pieces of this chunk that hold probabilities (bit per piece)
             // one 16-column piece on the general path: scores s, validity bits wd -> probabilities pk
@@ -526,67 +554,77 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 stored |= 1u << pc;
                 }
             };
-#pragma unroll 1
-            for (int pc = 0; pc < 4; ++pc) {
-                uint32_t pk[8];
-                if (fast) {
-                    const bool rowok = ((rowbits >> pc) & 1u) && colbits != 0u;
-                    if (__any_sync(0xffffffffu, rowok)) {
-                        uint32_t s[16];
-                        tmem_ld16(scol + 16 * pc, s);
-                        tmem_ld_wait();
-                        if (m == -INFINITY && rowok) {           // first valid columns of this row: fix the stabiliser
-                            float mm = -INFINITY;
+            if (fast) {
+                // one 16-column row: scores s -> probabilities over the scores they came from (piece pc lands in columns this
+                // thread has already read)
+                auto row_piece = [&](int pc, uint32_t (&s)[16], uint32_t (&pk)[8]) {
+                    const bool rowok = (mine >> pc) & 1u;
+                    if (m == -INFINITY && rowok) {           // first valid columns of this row: fix the stabiliser
+                        float mm = -INFINITY;
 #pragma unroll
-                            for (int i = 0; i < 16; ++i)
-                                if ((colbits >> i) & 1u) mm = fmaxf(mm, __uint_as_float(s[i]));
-                            m = mm;
-                            refresh_add(colbits);
+                        for (int i = 0; i < 16; ++i)
+                            if ((colbits >> i) & 1u) mm = fmaxf(mm, __uint_as_float(s[i]));
+                        m = mm;
+                        refresh_add(colbits);
+                    }
+                    // No running maximum in the common case: the probabilities are formed at once and their
+                    // row sum tells whether one of them may have outgrown the stabiliser; only then are the
+                    // exponents looked at one by one (and, if it is so, everything rescaled and redone).
+                    const uint64_t sc2 = pack2(P.scale_log2, P.scale_log2);
+                    const uint32_t keep = rowok ? 0xffffffffu : 0u;     // rows outside their window store zeros
+                    uint64_t rr = 0ull;                                 // two partial row sums
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {                       // two columns per packed fp32 fma
+                        const uint64_t xx = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, pack2(add[2 * i], add[2 * i + 1]));
+                        const float p0 = fast_exp2(lo_of(xx)), p1 = fast_exp2(hi_of(xx));
+                        rr = add2(rr, pack2(p0, p1));
+                        pk[i] = cvt_pack<BF16>(p0, p1) & keep;
+                    }
+                    if (__any_sync(0xffffffffu, rowok && !(lo_of(rr) + hi_of(rr) <= kGrowSum))) {
+                        float x[16], xmax = -INFINITY;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            x[i] = fmaf(__uint_as_float(s[i]), P.scale_log2, add[i]);
+                            xmax = fmaxf(xmax, x[i]);
                         }
-                        // No running maximum in the common case: the probabilities are formed at once and their
-                        // row sum tells whether one of them may have outgrown the stabiliser; only then are the
-                        // exponents looked at one by one (and, if it is so, everything rescaled and redone).
-                        const uint64_t sc2 = pack2(P.scale_log2, P.scale_log2);
-                        const uint32_t keep = rowok ? 0xffffffffu : 0u;     // rows outside their window store zeros
-                        uint64_t rr = 0ull;                                 // two partial row sums
+                        const bool grow = rowok && xmax > kGrow;
+                        if (__any_sync(0xffffffffu, grow)) {
+                            rescale(grow, xmax, c, pc, stored);
+                            if (grow) {
+                                refresh_add(colbits);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {                       // two columns per packed fp32 fma
-                            const uint64_t xx = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, pack2(add[2 * i], add[2 * i + 1]));
-                            const float p0 = fast_exp2(lo_of(xx)), p1 = fast_exp2(hi_of(xx));
+                                for (int i = 0; i < 16; ++i) x[i] -= xmax;
+                            }
+                        }
+                        rr = 0ull;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const float p0 = fast_exp2(x[2 * i]), p1 = fast_exp2(x[2 * i + 1]);
                             rr = add2(rr, pack2(p0, p1));
                             pk[i] = cvt_pack<BF16>(p0, p1) & keep;
                         }
-                        if (__any_sync(0xffffffffu, rowok && !(lo_of(rr) + hi_of(rr) <= kGrowSum))) {
-                            float x[16], xmax = -INFINITY;
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                x[i] = fmaf(__uint_as_float(s[i]), P.scale_log2, add[i]);
-                                xmax = fmaxf(xmax, x[i]);
-                            }
-                            const bool grow = rowok && xmax > kGrow;
-                            if (__any_sync(0xffffffffu, grow)) {
-                                rescale(grow, xmax, c, pc, stored);
-                                if (grow) {
-                                    refresh_add(colbits);
-#pragma unroll
-                                    for (int i = 0; i < 16; ++i) x[i] -= xmax;
-                                }
-                            }
-                            rr = 0ull;
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                const float p0 = fast_exp2(x[2 * i]), p1 = fast_exp2(x[2 * i + 1]);
-                                rr = add2(rr, pack2(p0, p1));
-                                pk[i] = cvt_pack<BF16>(p0, p1) & keep;
-                            }
-                        }
-                        if (rowok) l += lo_of(rr) + hi_of(rr);
-                        stored |= 1u << pc;
+                    }
+                    if (rowok) l += lo_of(rr) + hi_of(rr);
+                    stored |= 1u << pc;
+                };
+#pragma unroll 1
+                for (int pc = 0; pc < 4; ++pc) {
+                    uint32_t pk[8];
+                    if ((act >> pc) & 1u) {
+                        uint32_t s[16];
+                        tmem_ld16(scol + 16 * pc, s);
+                        tmem_ld_wait();
+                        row_piece(pc, s, pk);
                     } else {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) pk[i] = 0u;
                     }
-                } else {
+                    tmem_st8(scol + 8 * pc, pk);
+                }
+            } else {
+#pragma unroll 1
+                for (int pc = 0; pc < 4; ++pc) {
+                    uint32_t pk[8];
                     const uint32_t wd = ((pc & 2) ? words[1] : words[0]) >> (16 * (pc & 1)) & 0xFFFFu;
                     if (__any_sync(0xffffffffu, wd != 0u)) {
                         uint32_t s[16];
@@ -597,9 +635,9 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
                         for (int i = 0; i < 8; ++i) pk[i] = 0u;
                     }
+                    // P over the scores it came from: piece pc lands in columns this thread has already read
+                    tmem_st8(scol + 8 * pc, pk);
                 }
-                // P over the scores it came from: piece pc lands in columns this thread has already read
-                tmem_st8(scol + 8 * pc, pk);
             }
             tmem_st_wait();
             tc_fence_before();
@@ -607,9 +645,9 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             if (!mapped) {
                 ++ci[2];
                 dirty = 4u;
-                if (ci[2] == T.nc[2]) {
-                    ci[2] = 0; ++ci[1]; dirty = T.nc[2] > 1 ? 6u : 2u;
-                    if (ci[1] == T.nc[1]) { ci[1] = 0; ++ci[0]; dirty = 1u | (T.nc[1] > 1 ? 2u : 0u) | (T.nc[2] > 1 ? 4u : 0u); }
+                if (ci[2] == nc2) {
+                    ci[2] = 0; ++ci[1]; dirty = nc2 > 1 ? 6u : 2u;
+                    if (ci[1] == nc1) { ci[1] = 0; ++ci[0]; dirty = 1u | (nc1 > 1 ? 2u : 0u) | (nc2 > 1 ? 4u : 0u); }
                 }
             }
         }
