@@ -12,14 +12,19 @@
 // The row accumulators live in TMEM for the whole tile, so dK/dV are reduced in a
 // fixed order: results are bit-reproducible, no atomics.
 //
-// Chunks are 64 columns wide so that, up to head dim 64, a CTA needs only 256 TMEM columns and 102 KB of
+// Chunks are 64 columns wide so that, up to head dim 64, a CTA needs only 256 TMEM columns and 105 KB of
 // shared memory: two CTAs share an SM and one computes while the other waits for its MMAs or loads.  At head
 // dim 128 one CTA owns the SM's 512 columns; the 128 spare ones hold a second S / dP buffer, so that the
 // products of chunk g + 1 run while the threads work on chunk g.  The grid is persistent (CTAs walk the
 // tiles), so barriers, TMEM and the column-stage ring are set up once and the next tile's loads run ahead.
 // Warps: 8 compute warps (two per TMEM lane quadrant, each owns half of the chunk's columns), two MMA-issuing
-// warps (independent streams: dP / acc1 and S / acc2), one helper warp (per-axis tables one tile ahead, the
-// TMA loads, column statistics on the key side).
+// warps (independent streams: dP / acc1 and S / acc2), one that loads, one for the geometry (per-axis tables and row maps one
+// tile ahead; column statistics on the key side).
+// What bounds it: the round trip of a chunk (threads 700 to 1000 cycles, then the issuing warps and the products, 1300 to 1800)
+// with two tiles in flight, the tensor pipe busy for 45 % of it.  With one helper that loaded and did the geometry, tables held up
+// the row tiles and the loads.  Measured before | now (us, kernel alone, query side and key side): 64 x 64, 7 x 7, 8 heads of 64,
+// batch 8: 68.6, 87.5 | 64.6, 83.8; 128 x 128, 13 x 13, dilation 2, batch 4: 219, 278 | 199, 264; 16 x 32 x 32, 3 x 7 x 7 causal,
+// batch 2: 146, 187 | 135, 175; 8 lengths up to 16384, window 255, 16 heads of 128 on 4: 722, 712 | 578, 606.
 // TMEM: S [0,64)  dP [64,128)  acc1 [128,128+D)  acc2 [128+D,128+2D); head dim 128: second S [384,448) and
 // dP [448,512).  The 16-bit P and dS that feed the accumulating MMAs overwrite the first half of the S / dP
 // columns of the piece they were computed from (same warp, after it has read them).
@@ -41,10 +46,19 @@ namespace {
 
 constexpr int kStages = 3;
 constexpr int kComputeWarps = 8;
-constexpr int kThreads = (kComputeWarps + 3) * 32;    // + MMA issue, helper (tables, statistics), loader
+constexpr int kThreads = (kComputeWarps + 4) * 32;    // + two that issue products, one that loads, one for tables and statistics
 constexpr uint32_t kColS = 0, kColDP = 64, kColA1 = 128;   // acc2 follows acc1 (64 or 128 columns each)
 constexpr int kRowHalf = kTileRows * 128;   // bytes of one [128 x 64] 16-bit block of a row tile
 constexpr int kColHalf = kCols * 128;       // bytes of one [64 x 64] 16-bit block of a column tile
+
+// Barrier 2 of the compute warps: does any of their threads say yes?
+__device__ __forceinline__ bool any_of_compute(bool yes)
+{
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 2, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)yes), "n"(32 * kComputeWarps) : "memory");
+    return r != 0u;
+}
 
 template <int DH>
 struct SmemB {
@@ -57,8 +71,10 @@ struct SmemB {
     static constexpr int kC2 = kC1 + kStages * kColTile;        // [kStages]
     static constexpr int kStats = kC2 + kStages * kColTile;     // [kStages][2][64] float
     static constexpr int kTab = kStats + kStages * 512;         // [2] tables: axis entries, then a TileHead
-    static constexpr int kTabBytes = kAxisEntries * 16 + 96;
     static constexpr int kBar = kTab + 2 * kTabBytes;
+    // Up to head dim 64 two CTAs leave a thread 80 registers at launch.  On the query side the helpers hand some of theirs to the
+    // compute warps; on the key side they need them for the statistics (64 x 64, 7 x 7: 84 us as it is, 101 with 64 | 88).
+    static constexpr int kHelperRegs = 64, kComputeRegs = 88;
     static constexpr int kStage = (kBar + 256 + 1023) & ~1023;   // output staging: a row tile [128 x DH] 16-bit, swizzled like the loads
     static constexpr int kTotal = kStage + kTile;
     static constexpr uint32_t kTmemCols = DH == 64 ? 256 : 512;
@@ -100,8 +116,9 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
     const uint32_t bar_s = sbase + Smem::kBar + 72;           // S and dP of the chunk are in TMEM
     const uint32_t bar_sp = sbase + Smem::kBar + 80;          // threads consumed S/dP, wrote P/dS
     const uint32_t bar_free = sbase + Smem::kBar + 96;        // [kStages] accumulating MMAs of the stage's chunk finished
+    const uint32_t bar_head = sbase + Smem::kBar + 208;       // [2] tile head written
     const uint32_t bar_tab_full = sbase + Smem::kBar + 128;   // [2] row table written
-    const uint32_t bar_tab_empty = sbase + Smem::kBar + 144;  // [2] row table read by every compute thread and the MMA warp
+    const uint32_t bar_tab_empty = sbase + Smem::kBar + 144;  // [2] both read by every compute thread, the issuing warps and the loader
     const uint32_t bar_rowfree = sbase + Smem::kBar + 176;    // every S / dP product of the tile finished: the row tiles are free
     // At head dim 128 one CTA owns all 512 TMEM columns and 128 of them are spare: S and dP get a second buffer
     // ([384,448) and [448,512), used by the odd chunks), so the products of chunk g + 1 run while the threads work
@@ -127,7 +144,11 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             mbar_init(bar_sp, kComputeWarps * 32);
             mbar_init(bar_s1, 2);
             mbar_init(bar_sp1, kComputeWarps * 32);
-            for (int i = 0; i < 2; ++i) { mbar_init(bar_tab_full + 8 * i, 32); mbar_init(bar_tab_empty + 8 * i, kComputeWarps * 32 + 2); }
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(bar_head + 8 * i, 1);
+                mbar_init(bar_tab_full + 8 * i, 32);
+                mbar_init(bar_tab_empty + 8 * i, kComputeWarps * 32 + 3);
+            }
             mbar_init(bar_rowfree, 2);
             mbar_init_fence();
             fence_async_smem();
@@ -140,323 +161,356 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // next work item of this CTA with anything to do for the tensor cores
-    auto next_active = [&](unsigned w, BwdTile& X) {
-        for (; w < nwork; w += gridDim.x) {
-            bwd_tile_setup<kKeySide>(P, w, X);
-            if (X.active) break;
-        }
-        return w;
-    };
+    auto tab_slot = [&](unsigned t) { return smem + Smem::kTab + (t & 1) * kTabBytes; };
 
-    if (warp == kComputeWarps || warp == kComputeWarps + 2) {
-        // =====================================================================
-        // MMA issue: one thread in each of two warps.  A single thread gets a tcgen05.mma out every ~65
-        // cycles whatever its N, so the chunk's products are split into two independent streams:
-        //   first  (warp 8):  acc1 += dS x C1   then   dP(next) = R2 x C2^T     (both touch the dP columns)
-        //   second (warp 10): acc2 += P x C2    then   S(next)  = R1 x C1^T     (both touch the S columns; acc2 on
-        //                                                                        the key side only)
-        // Each stream is ordered by its own issue order; the streams share no TMEM columns.  Every barrier that
-        // tracks the products takes one commit from each stream.
-        // =====================================================================
-        // The whole warp runs the loop (warp-uniform code); the tensor-core instructions execute on one elected lane.
-        const uint32_t leader = elect_one();
-        if (!*abort_flag) {
-            const bool second = warp != kComputeWarps;
-            constexpr uint32_t idesc_kk = instr_desc(BF16 ? 1 : 0, kCols, 0, 0);    // both operands K-major
-            constexpr uint32_t idesc_acc = instr_desc(BF16 ? 1 : 0, DH, 0, 1);      // A from TMEM, B MN-major
-            const uint64_t dR = smem_desc(sbase + (second ? Smem::kR1 : Smem::kR2), 16, 1024);
-            const uint32_t col_tiles = second ? Smem::kC1 : Smem::kC2;             // column tiles of this stream's S / dP
-            const uint32_t acc_tiles = second ? Smem::kC2 : Smem::kC1;             // ... and of its accumulating product
-            const uint32_t col_out = second ? kColS : kColDP;                      // TMEM columns of S | dP (and of P | dS)
-            const bool has_acc = !second || kKeySide;
-            auto issue_s_dp = [&](unsigned g, int cc, const TileHead& X) {
-                const int s = g % kStages;
-                if (P.extents && cc < X.nbox) {      // rows of the column tile past the sample's extent -> zeros
-                    int r = cc % X.nchunks;
-                    const int c2 = r % X.nc[2]; r /= X.nc[2];
-                    const int c1 = r % X.nc[1], c0 = r / X.nc[1];
-                    const int box0[3] = {X.boxlo[0] + chunk_coord(P, 0, c0, 0), X.boxlo[1] + chunk_coord(P, 1, c1, 0),
-                                         X.boxlo[2] + chunk_coord(P, 2, c2, 0)};
-                    uint8_t* tile = smem + col_tiles + s * kColTile;     // the other stream zeroes the other tile
-                    if (leader) zero_rows_past_extent(P, box0, X.Lp, kCols, Smem::kHalves, kColHalf, tile, tile);
-                    __syncwarp();
-                }
-                const uint64_t dC = smem_desc(sbase + col_tiles + s * kColTile, 16, 1024);
-                tc_fence_after();
-                // 32 bytes per k-step inside a 64-channel block; blocks are kRowHalf / kColHalf apart
-#pragma unroll
-                for (int ks = 0; ks < (kShort ? DH / 16 - 2 : DH / 16); ++ks) {
-                    mma_ss_e(tmem + col_out + buf_cols(g), dR + (((ks / 4) * kRowHalf + (ks % 4) * 32) >> 4),
-                             dC + (((ks / 4) * kColHalf + (ks % 4) * 32) >> 4), idesc_kk, ks > 0, leader);
-                }
-                mma_commit_e(bar_s_of(g), leader);
-                if (cc + 1 == X.total) mma_commit_e(bar_rowfree, leader);      // the tile's last read of this stream's row tile
-            };
-            // k-step ks covers columns 16*ks..16*ks+15 of the chunk; their 16-bit pairs sit in the first 8 of
-            // those columns (16-column inner rows) or in the first 16 TMEM columns of the 32-column piece
-            // they came from.  The column tile is read MN-major: 16 rows (2048 bytes) per k-step, the second
-            // 64-channel block kColHalf further.
-            auto pair_col = [](int ks) { return kInner == 16 ? 16 * ks : 32 * (ks / 2) + 8 * (ks % 2); };
-            auto issue_acc = [&](unsigned g, bool accumulate) {
-                const int s = g % kStages;
-                if (has_acc) {
-                    const uint64_t dC = smem_desc(sbase + acc_tiles + s * kColTile, kColHalf, 1024);
-                    tc_fence_after();
-#pragma unroll
-                    for (int ks = 0; ks < kCols / 16; ++ks)
-                        mma_ts_e(tmem + (second ? kColA2 : kColA1), tmem + col_out + buf_cols(g) + pair_col(ks), dC + 128 * ks, idesc_acc,
-                                 (accumulate || ks > 0) ? 1u : 0u, leader);
-                }
-                if (has_acc) mma_commit_e(bar_free + 8 * s, leader);     // the stage's column tiles (and statistics) may be replaced
-            };
-
-            unsigned g = 0, tileno = 0, item = 0;
-            bool ok = true;
-            for (unsigned work = blockIdx.x; work < nwork && ok; work += gridDim.x, ++item) {
-                const unsigned slot = item & 1;
-                ok = mbar_wait(bar_tab_full + 8 * slot, (item >> 1) & 1, abort_flag, P.wait_budget);
-                if (!ok) break;
-                const TileHead T = *reinterpret_cast<const TileHead*>(smem + Smem::kTab + slot * Smem::kTabBytes + kAxisEntries * 16);
-                __syncwarp();                    // every lane has read the head
-                if (leader) mbar_arrive(bar_tab_empty + 8 * slot);
-                if (!T.active) continue;
-                ok = mbar_wait(bar_row, tileno & 1, abort_flag, P.wait_budget);
-                ok = ok && mbar_wait(bar_col + 8 * (g % kStages), (g / kStages) & 1, abort_flag, P.wait_budget);
-                if (!ok) break;
-                issue_s_dp(g, 0, T);
-                for (int cc = 0; cc < T.total && ok; ++cc, ++g) {
-                    if (kTwoBuf && cc + 1 < T.total) {
-                        // two buffers: the next chunk's products go into the other buffer, whose P / dS were read
-                        // by products this warp issued earlier, so they need not wait for the threads
-                        ok = mbar_wait(bar_col + 8 * ((g + 1) % kStages), ((g + 1) / kStages) & 1, abort_flag, P.wait_budget);
-                        if (!ok) break;
-                        issue_s_dp(g + 1, cc + 1, T);
-                    }
-                    ok = mbar_wait(bar_sp_of(g), par_of(g), abort_flag, P.wait_budget);               // S/dP consumed, P/dS stored
+    if (warp >= kComputeWarps) {
+        if (DH == 64 && !kKeySide) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Smem::kHelperRegs));
+        if (warp == kComputeWarps || warp == kComputeWarps + 2) {
+            // =====================================================================
+            // MMA issue: one thread in each of two warps.  A single thread gets a tcgen05.mma out every ~65
+            // cycles whatever its N, so the chunk's products are split into two independent streams:
+            //   first  (warp 8):  acc1 += dS x C1   then   dP(next) = R2 x C2^T     (both touch the dP columns)
+            //   second (warp 10): acc2 += P x C2    then   S(next)  = R1 x C1^T     (both touch the S columns; acc2 on
+            //                                                                        the key side only)
+            // Each stream is ordered by its own issue order; the streams share no TMEM columns.  Every barrier that
+            // tracks the products takes one commit from each stream.  From the threads' last P / dS to the next scores is on
+            // the chain of every chunk: the next column tile has been waited for by then.
+            // =====================================================================
+            // The whole warp runs the loop (warp-uniform code); the tensor-core instructions execute on one elected lane.
+            const uint32_t leader = elect_one();
+            if (!*abort_flag) {
+                const bool second = warp != kComputeWarps;
+                constexpr uint32_t idesc_kk = instr_desc(BF16 ? 1 : 0, kCols, 0, 0);    // both operands K-major
+                constexpr uint32_t idesc_acc = instr_desc(BF16 ? 1 : 0, DH, 0, 1);      // A from TMEM, B MN-major
+                const uint64_t dR = smem_desc(sbase + (second ? Smem::kR1 : Smem::kR2), 16, 1024);
+                const uint32_t col_tiles = second ? Smem::kC1 : Smem::kC2;             // column tiles of this stream's S / dP
+                const uint64_t dCol0 = smem_desc(sbase + col_tiles, 16, 1024);
+                const uint64_t dAcc0 = smem_desc(sbase + (second ? Smem::kC2 : Smem::kC1), kColHalf, 1024);   // ... of its accumulating product
+                const uint32_t col_out = tmem + (second ? kColS : kColDP);             // TMEM columns of S | dP (and of P | dS)
+                const uint32_t acc_out = tmem + (second ? kColA2 : kColA1);
+                const bool has_acc = !second || kKeySide;
+                // k-step ks of an accumulating product covers columns 16*ks..16*ks+15 of the chunk; their 16-bit pairs sit in the
+                // first 8 of those columns (16-column inner rows) or in the first 16 TMEM columns of the 32-column piece
+                // they came from.  The column tile is read MN-major: 16 rows (2048 bytes) per k-step, the second
+                // 64-channel block kColHalf further.
+                auto pair_col = [](int ks) { return kInner == 16 ? 16 * ks : 32 * (ks / 2) + 8 * (ks % 2); };
+                unsigned g = 0;
+                unsigned stage = 0, phase = 0;       // of chunk g + 1 once a tile runs (its column tile is the next one waited for)
+                unsigned acc_stage = 0;
+                bool ok = true;
+                for (unsigned t = 0; ok; ++t) {
+                    ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
-                    issue_acc(g, cc > 0);                                    // reads P/dS ...
-                    if (!kTwoBuf && cc + 1 < T.total) {
-                        ok = mbar_wait(bar_col + 8 * ((g + 1) % kStages), ((g + 1) / kStages) & 1, abort_flag, P.wait_budget);
+                    const TileHead* H = reinterpret_cast<const TileHead*>(tab_slot(t));
+                    const int total = H->total;
+                    int nbox = 0, nchunks = 1, boxlo[3] = {0, 0, 0}, Lp[3] = {0, 0, 0}, nc[3] = {1, 1, 1};
+                    bool padded = false;             // some chunk reaches past the sample's extent
+                    if (P.extents) {
+                        nbox = H->nbox;
+                        nchunks = H->nchunks;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            boxlo[a] = H->boxlo[a]; Lp[a] = H->Lp[a]; nc[a] = H->nc[a];
+                            padded = padded || boxlo[a] + chunk_coord(P, a, nc[a] - 1, P.cb[a] - 1) >= Lp[a];
+                        }
+                    }
+                    __syncwarp();                    // every lane has read the head
+                    if (leader) mbar_arrive(bar_tab_empty + 8 * (t & 1));
+                    if (total == 0) break;
+                    auto wait_columns = [&](int cc) {
+                        ok = ok && mbar_wait(bar_col + 8 * stage, phase, abort_flag, P.wait_budget);
+                        if (!ok || !padded || cc >= nbox) return;
+                        // rows of the column tile past the sample's extent -> zeros; the other stream zeroes the other tile
+                        int r = cc % nchunks;
+                        const int c2 = r % nc[2]; r /= nc[2];
+                        const int c1 = r % nc[1], c0 = r / nc[1];
+                        const int box0[3] = {boxlo[0] + chunk_coord(P, 0, c0, 0), boxlo[1] + chunk_coord(P, 1, c1, 0),
+                                             boxlo[2] + chunk_coord(P, 2, c2, 0)};
+                        uint8_t* tile = smem + col_tiles + stage * kColTile;
+                        if (leader) zero_rows_past_extent(P, box0, Lp, kCols, Smem::kHalves, kColHalf, tile, tile);
+                        __syncwarp();
+                    };
+                    auto issue_s_dp = [&](unsigned gg, bool last) {
+                        const uint64_t dC = dCol0 + stage * (kColTile >> 4);
+                        // 32 bytes per k-step inside a 64-channel block; blocks are kRowHalf / kColHalf apart
+#pragma unroll
+                        for (int ks = 0; ks < (kShort ? DH / 16 - 2 : DH / 16); ++ks) {
+                            mma_ss_e(col_out + buf_cols(gg), dR + (((ks / 4) * kRowHalf + (ks % 4) * 32) >> 4),
+                                     dC + (((ks / 4) * kColHalf + (ks % 4) * 32) >> 4), idesc_kk, ks > 0, leader);
+                        }
+                        mma_commit_e(bar_s_of(gg), leader);
+                        if (last) mma_commit_e(bar_rowfree, leader);      // the tile's last read of this stream's row tile
+                        if (++stage == kStages) { stage = 0; phase ^= 1; }
+                    };
+                    ok = mbar_wait(bar_row, t & 1, abort_flag, P.wait_budget);
+                    wait_columns(0);
+                    if (!ok) break;
+                    tc_fence_after();
+                    issue_s_dp(g, total == 1);
+                    for (int cc = 0; cc < total; ++cc, ++g) {
+                        const bool more = cc + 1 < total;
+                        if (more) wait_columns(cc + 1);
+                        if (kTwoBuf && more && ok) {
+                            // two buffers: the next chunk's products go into the other buffer, whose P / dS were read
+                            // by products this warp issued earlier, so they need not wait for the threads
+                            tc_fence_after();
+                            issue_s_dp(g + 1, cc + 2 == total);
+                        }
+                        ok = ok && mbar_wait(bar_sp_of(g), par_of(g), abort_flag, P.wait_budget);         // S/dP consumed, P/dS stored
                         if (!ok) break;
-                        issue_s_dp(g + 1, cc + 1, T);                                // ... before the next S/dP overwrite them
+                        tc_fence_after();
+                        if (has_acc) {                                           // reads P/dS ...
+                            const uint64_t dC = dAcc0 + acc_stage * (kColTile >> 4);
+#pragma unroll
+                            for (int ks = 0; ks < kCols / 16; ++ks)
+                                mma_ts_e(acc_out, col_out + buf_cols(g) + pair_col(ks), dC + 128 * ks, idesc_acc,
+                                         (cc > 0 || ks > 0) ? 1u : 0u, leader);
+                            mma_commit_e(bar_free + 8 * acc_stage, leader);     // the stage's column tiles (and statistics) may be replaced
+                        }
+                        if (++acc_stage == kStages) acc_stage = 0;
+                        if (!kTwoBuf && more) issue_s_dp(g + 1, cc + 2 == total);       // ... before the next S/dP overwrite them
                     }
                 }
-                ++tileno;
             }
-        }
-    } else if (warp == kComputeWarps + 1) {
-        // =====================================================================
-        // helper warp: row tables one tile ahead; the loads (lane 0: row tiles, then the ring of column tiles,
-        // as far ahead of the tensor cores as the stages allow); on the key side also the column statistics
-        // (lse*log2e and delta of the chunk's queries) that go with each column tile
-        // =====================================================================
-        bool ok = !*abort_flag;
-        unsigned g = 0;
-        // table of work item `work` (the item-th of this CTA) into slot item & 1
-        auto write_table = [&](unsigned work, unsigned item, const BwdTile& X) {
-            const unsigned slot = item & 1;
-            if (item >= 2) ok = ok && mbar_wait(bar_tab_empty + 8 * slot, ((item >> 1) - 1) & 1, abort_flag, P.wait_budget);
-            uint8_t* tab = smem + Smem::kTab + slot * Smem::kTabBytes;
-            AxisEntry* ent = reinterpret_cast<AxisEntry*>(tab);
-            int base = 0;
+        } else if (warp == kComputeWarps + 1) {
+            // =====================================================================
+            // loads: row tiles as soon as the previous tile's last S / dP product has finished, then the ring of column tiles,
+            // as far ahead of the tensor cores as the stages allow.  Rows of padding tiles (per-sample extents) are zeroed in between.
+            // =====================================================================
+            bool ok = !*abort_flag;
+            unsigned stage = 0, parity = 1, g = 0;       // parity: of the stage's last release
+            unsigned zw = blockIdx.x;                    // next work item to look at for padding
+            auto zero_one = [&]() {
+                BwdTile Z;
+                bwd_tile_setup<kKeySide>(P, zw, Z);
+                zw += gridDim.x;
+                if (Z.active) return;
+#pragma unroll 1
+                for (int r = lane; r < kTileRows; r += 32) {
+                    int ri[3];
+                    row_offsets(P, r, ri);
+                    bool in_tensor = true;
+                    long long pflat = 0;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                for (int i = lane; i < P.tile[a]; i += 32) {
-                    const int xa = X.origin[a] + i;
-                    AxisEntry en;
-                    en.pa = X.rg[a] + P.dil[a] * xa;
-                    en.flags = (xa < X.Lp[a] ? 1 : 0) | (en.pa < P.L[a] ? 2 : 0);
-                    int fa = 0, ea = 0;
-                    if (X.active) {
-                        if (kKeySide) {
-                            int qlo, qhi;
-                            inverse_range(xa, X.Lp[a], P.K[a], P.causal[a], qlo, qhi);
-                            fa = qlo - X.boxlo[a];
-                            ea = qhi + 1 - X.boxlo[a];
-                        } else {
-                            const int first = P.causal[a] ? xa - (P.K[a] - 1) : ws1(xa, X.Lp[a], P.K[a]);
-                            fa = (first > 0 ? first : 0) - X.boxlo[a];
-                            ea = (first + P.K[a] < X.Lp[a] ? first + P.K[a] : X.Lp[a]) - X.boxlo[a];
-                        }
+                    for (int a = 0; a < 3; ++a) {
+                        const int pa = Z.rg[a] + P.dil[a] * (Z.origin[a] + ri[a]);
+                        in_tensor = in_tensor && pa < P.L[a];
+                        pflat = pflat * P.L[a] + pa;
                     }
-                    en.f = (short)fa;
-                    en.e = (short)ea;
-                    en.pad = 0;
-                    ent[base + i] = en;
+                    if (!in_tensor) continue;
+                    const long long row = ((long long)Z.b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + Z.hy;
+#pragma unroll
+                    for (int which = 0; which < (kKeySide ? 2 : 1); ++which) {
+                        uint4* o = reinterpret_cast<uint4*>((which == 0 ? out1 : out2) + row * P.dreal);
+#pragma unroll
+                        for (int i = 0; i < DH / 8; ++i)
+                            if (8 * i < P.dreal) o[i] = make_uint4(0, 0, 0, 0);
+                    }
                 }
-                base += P.tile[a];
-            }
-            if (lane == 0) {
-                TileHead* hd = reinterpret_cast<TileHead*>(tab + kAxisEntries * 16);
-                hd->active = X.active ? 1 : 0;
-                hd->total = X.total;
-                hd->nbox = X.nbox;
-                hd->nchunks = X.nchunks;
-                hd->b = X.b;
-                hd->hy = X.hy;
-                hd->rg0 = (short)X.rg[0]; hd->rg1 = (short)X.rg[1]; hd->rg2 = (short)X.rg[2];
-                hd->origin0 = (short)X.origin[0]; hd->origin1 = (short)X.origin[1]; hd->origin2 = (short)X.origin[2];
+            };
+            for (unsigned t = 0; ok; ++t) {
+                ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
+                if (!ok) break;
+                const TileHead* H = reinterpret_cast<const TileHead*>(tab_slot(t));
+                const int total = H->total, nbox = H->nbox, b = H->b, hy = H->hy, nc0 = H->nc[0], nc1 = H->nc[1], nc2 = H->nc[2];
+                int Y[3], R[3];
 #pragma unroll
-                for (int a = 0; a < 3; ++a) { hd->nc[a] = X.nc[a]; hd->boxlo[a] = X.boxlo[a]; hd->Lp[a] = X.Lp[a]; }
-            }
-            mbar_arrive(bar_tab_full + 8 * slot);
-        };
-        auto issue_rows = [&](const BwdTile& X) {
-            const int hx = X.hy;
-            mbar_expect_tx(bar_row, 2 * kTile);
+                for (int a = 0; a < 3; ++a) {
+                    Y[a] = H->rg[a] + P.dil[a] * H->boxlo[a];
+                    R[a] = H->rg[a] + P.dil[a] * H->origin[a];
+                }
+                __syncwarp();                            // every lane has read the head
+                if (lane == 0) mbar_arrive(bar_tab_empty + 8 * (t & 1));
+                if (total == 0) break;
+                if (t > 0) ok = mbar_wait(bar_rowfree, (t - 1) & 1, abort_flag, P.wait_budget);
+                if (!ok) break;
+                if (lane == 0) {
+                    mbar_expect_tx(bar_row, 2 * kTile);
 #pragma unroll
-            for (int hf = 0; hf < Smem::kHalves; ++hf) {
-                tma_load_heads(sbase + Smem::kR1 + hf * kRowHalf, &tmR1, bar_row, P, hx, 64 * hf, X.rg[2] + P.dil[2] * X.origin[2],
-                            X.rg[1] + P.dil[1] * X.origin[1], X.rg[0] + P.dil[0] * X.origin[0], X.b);
-                tma_load_heads(sbase + Smem::kR2 + hf * kRowHalf, &tmR2, bar_row, P, hx, 64 * hf, X.rg[2] + P.dil[2] * X.origin[2],
-                            X.rg[1] + P.dil[1] * X.origin[1], X.rg[0] + P.dil[0] * X.origin[0], X.b);
-            }
-        };
-        BwdTile T, Tn;
-        unsigned item = 0, tiles = 0;
-        if (blockIdx.x < nwork) {
-            bwd_tile_setup<kKeySide>(P, blockIdx.x, T);
-            write_table(blockIdx.x, 0, T);
-        }
-        for (unsigned work = blockIdx.x; work < nwork; work += gridDim.x, ++item) {
-            const unsigned wn = work + gridDim.x;
-            if (wn < nwork) {                    // the next item's table first: it is needed before this tile ends
-                bwd_tile_setup<kKeySide>(P, wn, Tn);
-                write_table(wn, item + 1, Tn);
-            }
-            if (T.active) {
-                // the row tiles are free once the previous tile's last S / dP products have finished
-                if (tiles > 0) ok = ok && mbar_wait(bar_rowfree, (tiles - 1) & 1, abort_flag, P.wait_budget);
-                if (lane == 0 && ok) issue_rows(T);
-                ++tiles;
-                int ci[3] = {0, 0, 0}, hc = T.hy * P.group;
-                const int head_kv = kKeySide ? T.hy : T.hy / P.group;
-                for (int cc = 0; cc < T.total; ++cc, ++g) {
-                    const int s = g % kStages;
-                    // key side: the chunk's column statistics are fetched before the wait for the stage, so that
-                    // their latency is not part of what follows it
-                    float raw_lse[kCols / 32], raw_delta[kCols / 32];
-                    if (kKeySide) {
-#pragma unroll
-                        for (int k = 0; k < kCols / 32; ++k) {
-                            const int j = lane + 32 * k;
-                            const int j2 = j & (P.cb[2] - 1);
-                            const int j1 = (j >> P.cb2_log) & (P.cb[1] - 1);
-                            const int j0 = j >> (P.cb2_log + P.cb1_log);
-                            const int q0 = T.boxlo[0] + chunk_coord(P, 0, ci[0], j0);
-                            const int q1 = T.boxlo[1] + chunk_coord(P, 1, ci[1], j1);
-                            const int q2 = T.boxlo[2] + chunk_coord(P, 2, ci[2], j2);
-                            const bool inside = ok && q0 >= 0 && q0 < T.Lp[0] && q1 >= 0 && q1 < T.Lp[1] && q2 >= 0 && q2 < T.Lp[2];
-                            raw_lse[k] = 0.f;
-                            raw_delta[k] = 0.f;
-                            if (inside) {
-                                const long long pflat = ((long long)(T.rg[0] + P.dil[0] * q0) * P.L[1] + (T.rg[1] + P.dil[1] * q1)) * P.L[2]
-                                                        + (T.rg[2] + P.dil[2] * q2);
-                                const long long row = ((long long)T.b * P.ltot + pflat) * P.Hq + hc;
-                                raw_lse[k] = lse[row];
-                                raw_delta[k] = delta[row];
-                            }
-                        }
+                    for (int hf = 0; hf < Smem::kHalves; ++hf) {
+                        tma_load_heads(sbase + Smem::kR1 + hf * kRowHalf, &tmR1, bar_row, P, hy, 64 * hf, R[2], R[1], R[0], b);
+                        tma_load_heads(sbase + Smem::kR2 + hf * kRowHalf, &tmR2, bar_row, P, hy, 64 * hf, R[2], R[1], R[0], b);
                     }
-                    if (g >= (unsigned)kStages) ok = ok && mbar_wait(bar_free + 8 * s, ((g / kStages) - 1) & 1, abort_flag, P.wait_budget);
-                    if (lane == 0 && ok) {
-                        const uint32_t bar = bar_col + 8 * s;
+                }
+                __syncwarp();
+                int c0 = 0, c1 = 0, c2 = 0;
+                // query side: columns are keys (kv head); key side: columns are queries (query heads of the group)
+                int hx = kKeySide ? hy * P.group : (int)fast_div((unsigned)hy, P.group_mul);
+                for (int cc = 0; cc < total; ++cc, ++g) {
+                    const bool box = cc < nbox;          // else additional tokens (rows past n_extra are zero-filled)
+                    const int x0 = box ? Y[0] + P.dil[0] * chunk_coord(P, 0, c0, 0) : 0, x1 = box ? Y[1] + P.dil[1] * chunk_coord(P, 1, c1, 0) : 0,
+                              x2 = box ? Y[2] + P.dil[2] * chunk_coord(P, 2, c2, 0) : (cc - nbox) * kCols;
+                    if (g >= (unsigned)kStages) ok = mbar_wait(bar_free + 8 * stage, parity, abort_flag, P.wait_budget);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        const uint32_t bar = bar_col + 8 * stage;
                         mbar_expect_tx(bar, 2 * kColTile);
-                        if (cc < T.nbox) {
-                            int X[3];
 #pragma unroll
-                            for (int a = 0; a < 3; ++a) X[a] = T.rg[a] + P.dil[a] * (T.boxlo[a] + chunk_coord(P, a, ci[a], 0));
-                            // query side: columns are keys (kv head); key side: columns are queries (query head)
-                            const int hx = kKeySide ? hc : head_kv;
-#pragma unroll
-                            for (int hf = 0; hf < Smem::kHalves; ++hf) {
-                                tma_load_heads(sbase + Smem::kC1 + s * kColTile + hf * kColHalf, &tmC1, bar, P, hx, 64 * hf, X[2], X[1], X[0], T.b);
-                                tma_load_heads(sbase + Smem::kC2 + s * kColTile + hf * kColHalf, &tmC2, bar, P, hx, 64 * hf, X[2], X[1], X[0], T.b);
-                            }
-                        } else {                             // additional tokens (rows past n_extra are zero-filled)
-                            const int e0 = (cc - T.nbox) * kCols;
-#pragma unroll
-                            for (int hf = 0; hf < Smem::kHalves; ++hf) {
-                                tma_load_heads(sbase + Smem::kC1 + s * kColTile + hf * kColHalf, &tmE1, bar, P, head_kv, 64 * hf, e0, 0, 0, T.b);
-                                tma_load_heads(sbase + Smem::kC2 + s * kColTile + hf * kColHalf, &tmE2, bar, P, head_kv, 64 * hf, e0, 0, 0, T.b);
-                            }
+                        for (int hf = 0; hf < Smem::kHalves; ++hf) {
+                            tma_load_heads(sbase + Smem::kC1 + stage * kColTile + hf * kColHalf, box ? &tmC1 : &tmE1, bar, P, hx, 64 * hf, x2, x1, x0, b);
+                            tma_load_heads(sbase + Smem::kC2 + stage * kColTile + hf * kColHalf, box ? &tmC2 : &tmE2, bar, P, hx, 64 * hf, x2, x1, x0, b);
                         }
                     }
                     __syncwarp();
-                    if (!kKeySide) {
-                        if (cc < T.nbox && ++ci[2] == T.nc[2]) { ci[2] = 0; if (++ci[1] == T.nc[1]) { ci[1] = 0; ++ci[0]; } }
-                        continue;
+                    if (++stage == kStages) { stage = 0; parity ^= 1; }
+                    if (box && ++c2 == nc2) { c2 = 0; if (++c1 == nc1) { c1 = 0; if (++c0 == nc0) { c0 = 0; if (kKeySide) ++hx; } } }
+                    if (P.extents && zw < nwork) zero_one();
+                }
+            }
+            while (ok && P.extents && zw < nwork) zero_one();
+        } else {
+            // =====================================================================
+            // geometry: tables one tile ahead; on the key side also the column statistics (lse*log2e and delta of the chunk's
+            // queries) that go with each column tile, fetched a chunk ahead
+            // =====================================================================
+            bool ok = !*abort_flag;
+            unsigned w = blockIdx.x, stage = 0, parity = 1, g = 0;
+            auto publish = [&](unsigned t) -> bool {     // the next work item with rows of a sample -> slot t & 1; false: none is left
+                BwdTile X;
+                bool found = false;
+                for (; w < nwork && !found; w += gridDim.x) {
+                    bwd_tile_setup<kKeySide>(P, w, X);
+                    found = X.active;
+                }
+                if (t >= 2) ok = ok && mbar_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
+                if (!ok) return false;
+                uint8_t* slot = tab_slot(t);
+                const bool mapped = kInner == 16 && found && X.nc[2] == 1 && X.nchunks <= 16;
+                if (lane == 0) {
+                    TileHead* hd = reinterpret_cast<TileHead*>(slot);
+                    hd->total = found ? X.total : 0;
+                    if (found) {
+                        hd->nbox = X.nbox;
+                        hd->nchunks = X.nchunks;
+                        hd->b = X.b;
+                        hd->hy = X.hy;
+                        hd->mapped = mapped;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            hd->nc[a] = X.nc[a]; hd->boxlo[a] = X.boxlo[a]; hd->Lp[a] = X.Lp[a];
+                            hd->rg[a] = X.rg[a]; hd->origin[a] = X.origin[a];
+                        }
                     }
-                    float* st = stats + s * 128;
+                    mbar_arrive(bar_head + 8 * (t & 1));
+                }
+                __syncwarp();
+                if (found) write_tables<kKeySide>(P, X, mapped, lane, slot);
+                mbar_arrive(bar_tab_full + 8 * (t & 1));
+                return found;
+            };
+            bool have = ok && publish(0);
+            for (unsigned t = 0; have && ok; ++t) {
+                if (!kKeySide) {
+                    have = publish(t + 1);
+                    continue;
+                }
+                const TileHead* H = reinterpret_cast<const TileHead*>(tab_slot(t));   // stays until the table of tile t + 2
+                const int total = H->total, nc0 = H->nc[0], nc1 = H->nc[1], nc2 = H->nc[2];
+                // this lane's columns j = lane and lane + 32 of chunk (0, 0, 0): position along the axes, relative to the sub-grid
+                int at[kCols / 32][3], Lp[3], c0 = 0, c1 = 0, c2 = 0;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) Lp[a] = H->Lp[a];
+#pragma unroll
+                for (int k = 0; k < kCols / 32; ++k) {
+                    const int j = lane + 32 * k;
+                    at[k][0] = H->boxlo[0] + chunk_coord(P, 0, 0, j >> (P.cb2_log + P.cb1_log));
+                    at[k][1] = H->boxlo[1] + chunk_coord(P, 1, 0, (j >> P.cb2_log) & (P.cb[1] - 1));
+                    at[k][2] = H->boxlo[2] + chunk_coord(P, 2, 0, j & (P.cb[2] - 1));
+                }
+                // statistics of the sub-grid's origin for the first query head
+                const long long origin = ((long long)H->b * P.ltot + ((long long)H->rg[0] * P.L[1] + H->rg[1]) * P.L[2] + H->rg[2]) * P.Hq + H->hy * P.group;
+                const float *lse_h = lse + origin, *delta_h = delta + origin;
+                float nl[kCols / 32], nd[kCols / 32];
+                auto fetch = [&]() {
+                    const int s0 = chunk_coord(P, 0, c0, 0), s1 = chunk_coord(P, 1, c1, 0), s2 = chunk_coord(P, 2, c2, 0);
+#pragma unroll
+                    for (int k = 0; k < kCols / 32; ++k) {
+                        const int q0 = at[k][0] + s0, q1 = at[k][1] + s1, q2 = at[k][2] + s2;
+                        nl[k] = 0.f;
+                        nd[k] = 0.f;
+                        if (q0 >= 0 && q0 < Lp[0] && q1 >= 0 && q1 < Lp[1] && q2 >= 0 && q2 < Lp[2]) {
+                            const long long row = (((long long)(P.dil[0] * q0) * P.L[1] + P.dil[1] * q1) * P.L[2] + P.dil[2] * q2) * P.Hq;
+                            nl[k] = lse_h[row];
+                            nd[k] = delta_h[row];
+                        }
+                    }
+                    if (++c2 == nc2) { c2 = 0; if (++c1 == nc1) { c1 = 0; if (++c0 == nc0) { c0 = 0; ++lse_h; ++delta_h; } } }
+                };
+                fetch();
+                bool next = false;
+                for (int cc = 0; cc < total; ++cc, ++g) {
+                    float l0[kCols / 32], d0[kCols / 32];
+#pragma unroll
+                    for (int k = 0; k < kCols / 32; ++k) { l0[k] = nl[k]; d0[k] = nd[k]; }
+                    if (cc + 1 < total) fetch();
+                    if (g >= (unsigned)kStages) ok = ok && mbar_wait(bar_free + 8 * stage, parity, abort_flag, P.wait_budget);
+                    if (!ok) break;
+                    float* st = stats + stage * 128;
 #pragma unroll
                     for (int k = 0; k < kCols / 32; ++k) {               // negated, pre-scaled addends
-                        st[lane + 32 * k] = -raw_lse[k] * 1.4426950408889634f;
-                        st[kCols + lane + 32 * k] = -raw_delta[k] * P.scale;
+                        st[lane + 32 * k] = -l0[k] * 1.4426950408889634f;
+                        st[kCols + lane + 32 * k] = -d0[k] * P.scale;
                     }
-                    mbar_arrive(bar_stats + 8 * s);
-                    if (++ci[2] == T.nc[2]) { ci[2] = 0; if (++ci[1] == T.nc[1]) { ci[1] = 0; if (++ci[0] == T.nc[0]) { ci[0] = 0; ++hc; } } }
+                    mbar_arrive(bar_stats + 8 * stage);
+                    if (++stage == kStages) { stage = 0; parity ^= 1; }
+                    // the next tile's tables once the stages are full: they are not needed before this tile ends
+                    if (cc == (total < kStages ? total : kStages) - 1) next = publish(t + 1);
                 }
+                have = next;
             }
-            T = Tn;
         }
     } else {
         // =====================================================================
         // compute warps: thread = (row, 32-column piece)
         // =====================================================================
+        if (DH == 64 && !kKeySide) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Smem::kComputeRegs));
         const uint32_t trow = tmem + (static_cast<uint32_t>(quad * 32) << 16);
         bool ok = true;
         unsigned g = 0;                          // chunks processed so far (all tiles)
         constexpr int kPairs = kInner > 0 ? kInner / 2 : 1;
-        unsigned item = 0;
-        for (unsigned work = blockIdx.x; work < nwork; work += gridDim.x, ++item) {
-            // ---- this thread's row, from the helper warp's table ----
-            const unsigned slot = item & 1;
-            ok = mbar_wait(bar_tab_full + 8 * slot, (item >> 1) & 1, abort_flag, P.wait_budget) && ok;
-            const uint8_t* tab = smem + Smem::kTab + slot * Smem::kTabBytes;
-            const TileHead T = *reinterpret_cast<const TileHead*>(tab + kAxisEntries * 16);
+        for (unsigned t = 0;; ++t) {
+            // ---- this thread's row, from the geometry warp's tables ----
+            ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
+            if (any_of_compute(!ok)) break;      // all of them or none: the stores below are behind a barrier of theirs
+            const uint8_t* tab = tab_slot(t);
+            const TileHead* H = reinterpret_cast<const TileHead*>(tab);
+            const int total = H->total;
+            if (total == 0) break;
+            const int nbox = H->nbox, nchunks = H->nchunks, nc[3] = {H->nc[0], H->nc[1], H->nc[2]}, b = H->b, hy = H->hy;
+            const bool mapped = kInner == 16 && H->mapped;
+            int R[3];                            // first row of the tile (for its store)
             int f[3], e[3];
             bool valid_row = true, in_tensor = true;
             long long pflat = 0;
+            unsigned long long rowmap = 0ull;    // mapped: which of a chunk's four rows are in this thread's range, four bits a chunk
             {
                 int ri[3];
                 row_offsets(P, quad * 32 + lane, ri);
-                const AxisEntry* ent = reinterpret_cast<const AxisEntry*>(tab);
+                const AxisEntry* ent = reinterpret_cast<const AxisEntry*>(tab + kHeadBytes + kMapBytes);
                 int base = 0;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
+                    R[a] = H->rg[a] + P.dil[a] * H->origin[a];
                     const AxisEntry en = ent[base + ri[a]];
                     base += P.tile[a];
-                    f[a] = en.f;
-                    e[a] = en.e;
-                    valid_row = valid_row && (en.flags & 1);
-                    in_tensor = in_tensor && (en.flags & 2);
-                    pflat = pflat * P.L[a] + en.pa;
+                    f[a] = en.x;
+                    e[a] = en.y;
+                    valid_row = valid_row && (en.w & 1);
+                    in_tensor = in_tensor && (en.w & 2);
+                    pflat = pflat * P.L[a] + en.z;
                 }
+                if (mapped) rowmap = reinterpret_cast<const unsigned long long*>(tab + kHeadBytes)[(quad * 32 + lane) >> P.tile2_log];
             }
-            mbar_arrive(bar_tab_empty + 8 * slot);
+            mbar_arrive(bar_tab_empty + 8 * (t & 1));
             if (!valid_row) { e[0] = f[0]; e[1] = f[1]; e[2] = f[2]; }
-            const long long out_row = ((long long)T.b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + T.hy;
+            const long long out_row = ((long long)b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + hy;
             // query side: the row's lse and delta; scaled where they are first used, so that the loads' latency
             // runs under the set-up of the first chunk and the wait for its scores
             float raw_lse = 0.f, raw_delta = 0.f;
-            if (!kKeySide && valid_row && in_tensor && T.active && ok) {
+            if (!kKeySide && valid_row && in_tensor && ok) {
                 raw_lse = lse[out_row];
                 raw_delta = delta[out_row];
             }
-            if (!T.active) {                     // padding rows get zero gradients
-                if (in_tensor) {
-#pragma unroll
-                    for (int which = 0; which < (kKeySide ? 2 : 1); ++which) {
-                        uint4* o = reinterpret_cast<uint4*>((which == 0 ? out1 : out2) + out_row * P.dreal + piece * CH);
-#pragma unroll
-                        for (int i = 0; i < CH / 8; ++i)
-                            if (piece * CH + 8 * i < P.dreal) o[i] = make_uint4(0, 0, 0, 0);
-                    }
-                }
-                continue;
-            }
-            const int nbox = T.nbox;
             // Chunk columns of this warp's half h, and where its 16-bit pairs go.  With 16-column inner rows a
             // chunk is four rows: the warp takes rows piece and piece + 2, so that the two warps of a lane
             // quadrant share a row's window evenly when the chunk rows are interleaved; the pairs of a row
@@ -469,27 +523,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             uint32_t colmask[kPairs];            // separable geometry: 16-bit lane masks per column pair
             bool cols_any = false;
             int cached_c2 = -1;
-            // 16-column inner rows, one chunk along the innermost axis, at most 16 chunks in the box: which of a
-            // chunk's four rows lie inside this thread's range is worked out once per tile from the row's side
-            // (every row of the range lands in one row of one chunk), four bits per chunk.
-            bool mapped = false;
-            unsigned long long rowmap = 0ull;
             int cl = 0;                          // chunk of the box (wraps with every query head on the key side)
-            if (kInner == 16 && T.nc[2] == 1 && T.nchunks <= 16) {
-                mapped = true;
-                for (int x0 = f[0]; x0 < e[0]; ++x0) {
-                    int c0, j0;
-                    if (P.il[0] == 1) { c0 = x0 >> P.cb0_log; j0 = x0 & (P.cb[0] - 1); }
-                    else { j0 = (int)fast_div((unsigned)x0, P.il_mul[0]); c0 = x0 - j0 * P.il[0]; }
-                    for (int x1 = f[1]; x1 < e[1]; ++x1) {
-                        int c1, j1;
-                        if (P.il[1] == 1) { c1 = x1 >> P.cb1_log; j1 = x1 & (P.cb[1] - 1); }
-                        else { j1 = (int)fast_div((unsigned)x1, P.il_mul[1]); c1 = x1 - j1 * P.il[1]; }
-                        rowmap |= 1ull << (4 * (c0 * T.nc[1] + c1) + (j0 << P.cb1_log) + j1);
-                    }
-                }
-            }
-            for (int cc = 0; cc < T.total; ++cc, ++g) {
+            for (int cc = 0; cc < total; ++cc, ++g) {
                 // ---- validity of this warp's two 16-column halves for this thread's row ----
                 // half h covers chunk columns col0(h) .. col0(h)+15; bits [16h, 16h+16) of `word` belong to it
                 uint32_t word = 0u;                  // generic geometry / additional tokens: one bit per column
@@ -632,12 +667,12 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 mbar_arrive(bar_sp_of(g));
                 // next chunk (innermost axis fastest; wraps to the next query head on the key side)
                 if (mapped) {
-                    if (++cl == T.nchunks) cl = 0;
-                } else if (++ci[2] == T.nc[2]) {
+                    if (++cl == nchunks) cl = 0;
+                } else if (++ci[2] == nc[2]) {
                     ci[2] = 0;
-                    if (++ci[1] == T.nc[1]) {
+                    if (++ci[1] == nc[1]) {
                         ci[1] = 0;
-                        if (++ci[0] == T.nc[0]) ci[0] = 0;
+                        if (++ci[0] == nc[0]) ci[0] = 0;
                     }
                 }
             }
@@ -704,8 +739,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     const CUtensorMap* map = which == 0 ? &tmO1 : &tmO2;
 #pragma unroll
                     for (int hf = 0; hf < Smem::kHalves; ++hf)
-                        tma_store_heads(map, sbase + Smem::kStage + hf * kRowHalf, P, DH, T.hy * DH + 64 * hf,
-                                        T.rg2 + P.dil[2] * T.origin2, T.rg1 + P.dil[1] * T.origin1, T.rg0 + P.dil[0] * T.origin0, T.b);
+                        tma_store_heads(map, sbase + Smem::kStage + hf * kRowHalf, P, DH, hy * DH + 64 * hf, R[2], R[1], R[0], b);
                     tma_store_commit();
                 }
             }

@@ -156,25 +156,7 @@ __device__ __forceinline__ void write_tables(const TcParams& P, const FwdTile& T
     unsigned long long* map = reinterpret_cast<unsigned long long*>(slot + kMapOff);
     for (int r = lane; r < P.tile[0] * P.tile[1]; r += 32) {
         const int4 e0 = axis_entry(P, T, 0, r >> P.tile1_log), e1 = axis_entry(P, T, 1, r & (P.tile[1] - 1));
-        unsigned long long bits = 0ull;
-        if (e0.w & e1.w & 1)
-            for (int x0 = e0.x; x0 < e0.y; ++x0) {
-                const int j0 = P.il[0] == 1 ? x0 & (P.cb[0] - 1) : (int)fast_div((unsigned)x0, P.il_mul[0]);
-                const int c0 = P.il[0] == 1 ? x0 >> P.cb0_log : x0 - j0 * P.il[0];
-                int j1 = P.il[1] == 1 ? e1.x & (P.cb[1] - 1) : (int)fast_div((unsigned)e1.x, P.il_mul[1]);
-                int at = 4 * (c0 * T.nc[1] + (P.il[1] == 1 ? e1.x >> P.cb1_log : e1.x - j1 * P.il[1])) + (j0 << P.cb1_log);
-                int c1 = P.il[1] == 1 ? 0 : e1.x - j1 * P.il[1];
-                for (int x1 = e1.x; x1 < e1.y; ++x1) {
-                    bits |= 1ull << (at + j1);
-                    if (P.il[1] == 1) {                      // along the chunk, then on to the next
-                        if (++j1 == P.cb[1]) { j1 = 0; at += 4; }
-                    } else {                                 // through the chunks, then one row further
-                        at += 4;
-                        if (++c1 == P.il[1]) { c1 = 0; ++j1; at -= 4 * P.il[1]; }
-                    }
-                }
-            }
-        map[r] = bits;
+        map[r] = (e0.w & e1.w & 1) ? row_map(P, T.nc[1], e0.x, e0.y, e1.x, e1.y) : 0ull;
     }
 }
 

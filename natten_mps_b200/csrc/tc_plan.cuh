@@ -245,6 +245,30 @@ __device__ __forceinline__ int chunk_coord(const TcParams& P, int a, int ci, int
     return P.il[a] == 1 ? ci * P.cb[a] + j : ci + P.il[a] * j;
 }
 
+// Chunks of four 16-column rows, one chunk along the innermost axis, at most 16 in all: which rows of which chunk the box rows
+// [f0, e0) x [f1, e1) are, four bits a chunk (every box row is one row of one chunk).  n1: chunks along axis 1.
+__device__ __forceinline__ unsigned long long row_map(const TcParams& P, int n1, int f0, int e0, int f1, int e1)
+{
+    unsigned long long bits = 0ull;
+    for (int x0 = f0; x0 < e0; ++x0) {
+        const int j0 = P.il[0] == 1 ? x0 & (P.cb[0] - 1) : (int)fast_div((unsigned)x0, P.il_mul[0]);
+        const int c0 = P.il[0] == 1 ? x0 >> P.cb0_log : x0 - j0 * P.il[0];
+        int j1 = P.il[1] == 1 ? f1 & (P.cb[1] - 1) : (int)fast_div((unsigned)f1, P.il_mul[1]);
+        int c1 = P.il[1] == 1 ? f1 >> P.cb1_log : f1 - j1 * P.il[1];
+        int at = 4 * (c0 * n1 + c1) + (j0 << P.cb1_log);
+        for (int x1 = f1; x1 < e1; ++x1) {
+            bits |= 1ull << (at + j1);
+            if (P.il[1] == 1) {                              // along the chunk, then on to the next
+                if (++j1 == P.cb[1]) { j1 = 0; at += 4; }
+            } else {                                         // through the chunks, then one row further
+                at += 4;
+                if (++c1 == P.il[1]) { c1 = 0; ++j1; at -= 4 * P.il[1]; }
+            }
+        }
+    }
+    return bits;
+}
+
 // Validity bits of one 32-column piece from per-axis column ranges [jl, jh) (see chunk_range).
 __device__ __forceinline__ uint32_t piece_word_ranges(const TcParams& P, int pc, const int (&jl)[3], const int (&jh)[3])
 {

@@ -26,22 +26,21 @@ struct BwdTile {
 
 // What a compute thread needs to know about its row of a tile is separable: along every axis the row's
 // coordinate alone decides its position in the tensor, whether it exists, and its valid column range.  The
-// helper warp writes one entry per (axis, coordinate of the tile) one tile ahead, tile[0] + tile[1] + tile[2]
+// geometry warp writes one entry per (axis, coordinate of the tile) one tile ahead, tile[0] + tile[1] + tile[2]
 // entries instead of 128 rows x 3 axes; a compute thread combines the three entries of its row.
-struct __align__(16) AxisEntry {
-    short f, e;                // valid column range along the axis, relative to the column box
-    int pa;                    // position along the axis in the tensor
-    int flags;                 // bit 0: inside the (sub-grid of the) sample, bit 1: inside the tensor
-    int pad;
-};
-static_assert(sizeof(AxisEntry) == 16, "axis table entries are 16 bytes");
+// x, y: valid column range [f, e) along the axis, relative to the column box; z: position along the axis in the tensor;
+// w: bit 0 inside the (sub-grid of the) sample, bit 1 inside the tensor.
+using AxisEntry = int4;
 struct TileHead {
-    int active, total, nbox, nc[3];
-    int nchunks, boxlo[3], Lp[3];      // for the MMA warps: chunks of the column box, its origin, sub-grid extents
+    int total, nbox, nc[3];            // total == 0: no more tiles
+    int nchunks, boxlo[3], Lp[3];      // chunks of the column box, its origin, sub-grid extents
     int b, hy;                         // batch and head of the rows
-    short rg0, rg1, rg2, origin0, origin1, origin2;   // dilation residues and origin of the row tile (for its store)
+    int rg[3], origin[3];              // dilation residues and origin of the row tile
+    int mapped;                        // the row maps are valid
 };
-static_assert(sizeof(TileHead) <= 96, "the tile head has 96 bytes behind the axis table");
+// A slot: head, row maps, axis entries.
+constexpr int kHeadBytes = 96, kMapBytes = 8 * kTileRows, kTabBytes = kHeadBytes + kMapBytes + 16 * kAxisEntries;
+static_assert(sizeof(TileHead) <= kHeadBytes, "the tile head has 96 bytes in front of the tables");
 
 template <bool kKeySide>
 __device__ __forceinline__ void bwd_tile_setup(const TcParams& P, unsigned work, BwdTile& T)
@@ -72,6 +71,47 @@ __device__ __forceinline__ void bwd_tile_setup(const TcParams& P, unsigned work,
     }
     T.nbox = T.nchunks * (kKeySide ? P.group : 1);
     T.total = T.nbox + (kKeySide ? 0 : ((P.n_extra + kCols - 1) >> 6));
+}
+
+// Entry of the tile's row coordinate i along axis a.
+template <bool kKeySide>
+__device__ __forceinline__ AxisEntry axis_entry(const TcParams& P, const BwdTile& X, int a, int i)
+{
+    const int xa = X.origin[a] + i, pa = X.rg[a] + P.dil[a] * xa;
+    AxisEntry en;
+    en.z = pa;
+    en.w = (xa < X.Lp[a] ? 1 : 0) | (pa < P.L[a] ? 2 : 0);
+    if (kKeySide) {
+        int qlo, qhi;
+        inverse_range(xa, X.Lp[a], P.K[a], P.causal[a], qlo, qhi);
+        en.x = qlo - X.boxlo[a];
+        en.y = qhi + 1 - X.boxlo[a];
+    } else {
+        const int first = P.causal[a] ? xa - (P.K[a] - 1) : ws1(xa, X.Lp[a], P.K[a]);
+        en.x = (first > 0 ? first : 0) - X.boxlo[a];
+        en.y = (first + P.K[a] < X.Lp[a] ? first + P.K[a] : X.Lp[a]) - X.boxlo[a];
+    }
+    return en;
+}
+
+// One warp writes a tile's tables.  mapped: chunks of 16-column rows, one along the innermost axis, at most 16 in the box.  Then
+// which of a chunk's four rows lie in a row's range depends on its two outer coordinates: a map per pair of them, four bits a chunk.
+template <bool kKeySide>
+__device__ __forceinline__ void write_tables(const TcParams& P, const BwdTile& X, bool mapped, int lane, uint8_t* slot)
+{
+    AxisEntry* ent = reinterpret_cast<AxisEntry*>(slot + kHeadBytes + kMapBytes);
+    int base = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        for (int i = lane; i < P.tile[a]; i += 32) ent[base + i] = axis_entry<kKeySide>(P, X, a, i);
+        base += P.tile[a];
+    }
+    if (!mapped) return;
+    unsigned long long* map = reinterpret_cast<unsigned long long*>(slot + kHeadBytes);
+    for (int r = lane; r < P.tile[0] * P.tile[1]; r += 32) {
+        const AxisEntry e0 = axis_entry<kKeySide>(P, X, 0, r >> P.tile1_log), e1 = axis_entry<kKeySide>(P, X, 1, r & (P.tile[1] - 1));
+        map[r] = (e0.w & e1.w & 1) ? row_map(P, X.nc[1], e0.x, e0.y, e1.x, e1.y) : 0ull;
+    }
 }
 
 } // namespace rowtile
