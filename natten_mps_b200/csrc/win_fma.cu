@@ -13,8 +13,8 @@
 //     alone does the scalar work of that row (mask, exponential), and four shuffles hand the results back.
 // A pass over the columns of K = 7 x 7 costs 23 shared-memory cycles for 32 pairs of which 70 % are needed.
 //
-// Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, against the general SIMT kernels: float32 forward 36 us (185), dQ 43 (236),
-// dK and dV 72 (304); split operators in bf16: scores 25 (93), apply 24 (93), gather 36 (115); in float32: 25 (96), 24 (469),
+// Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, against the general SIMT kernels: float32 forward 30 us (185), dQ 38 (236),
+// dK and dV 67 (304); split operators in bf16: scores 25 (93), apply 24 (93), gather 36 (115); in float32: 25 (96), 24 (469),
 // 32 (152).
 // What bounds them there: too few warps.  448 CTAs have 444 (forward, dQ), 296 (dK and dV, 245 to 255 registers) or 592 (split)
 // places, 7 to 12 warps on an SM.  Schedulers issue in 44, 41, 33 % of the active cycles (forward, dQ, dK and dV) and in 49, 38,
@@ -879,10 +879,11 @@ fma_gather_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ w, 
 // ---------------------------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------------------------
-// Three CTAs of the forward and of dQ share an SM's 227 KB.  The key side, two CTAs by its registers, uses the same.  Measured,
-// 56 x 56, 7 x 7, head dim 32 | 64, with 48, 64, 100 KB: forward 34.7, 35.4, 34.0 us | 30.5, 30.9, 39.6 (two CTAs); dK and dV
-// 75.0, 74.3, 66.7 | 79.3, 69.0, 64.3.
-constexpr int kFusedChunk = 64 * 1024;
+// As much of the column box at a time as the CTAs that registers allow on an SM can have of its 227 KB: three of the forward and of
+// dQ, two of the key side.  Every chunk is a barrier that nothing overlaps.  Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, with
+// 32, 48, 64, 72, 100 KB: forward 35.6, 34.3, 35.3, 30.2, 33.7 us (the last with two CTAs); dQ 42.9, 42.5, 43.5, 37.5, 42.1;
+// dK and dV 80.6, 75.7, 75.5, 72.5, 67.0.
+constexpr int kQueryChunk = 72 * 1024, kKeyChunk = 100 * 1024;
 
 // Rows of a warp are 4 x (256 / D) (rank 1: one row of 1024 / D).  `tensors`: column tensors staged side by side,
 // `extra`: further shared-memory bytes per staged column, `budget`: bytes of a chunk.
@@ -977,7 +978,7 @@ int fma_fused_fwd(int dtype, const Geo& g, const void* q, const void* k, const v
     FmaParams p;
     dim3 grid;
     size_t smem;
-    if (!make_fma(g, p, false, 2, 0, 0, kFusedChunk, grid, smem)) return -2;
+    if (!make_fma(g, p, false, 2, 0, 0, kQueryChunk, grid, smem)) return -2;
     p.row1 = tensor_of(q, g.qs);
     p.col1 = tensor_of(k, g.ks);
     p.col2 = tensor_of(v, g.vs);
@@ -1003,7 +1004,7 @@ int fma_fused_bwd(int dtype, const Geo& g, const void* q, const void* k, const v
     FmaParams pq, pk;
     dim3 gq, gk;
     size_t sq, sk;
-    if (!make_fma(g, pq, false, 2, 0, 0, kFusedChunk, gq, sq) || !make_fma(g, pk, true, 2, 8, 0, kFusedChunk, gk, sk)) return -2;
+    if (!make_fma(g, pq, false, 2, 0, 0, kQueryChunk, gq, sq) || !make_fma(g, pk, true, 2, 8, 0, kKeyChunk, gk, sk)) return -2;
     float* delta = static_cast<float*>(workspace);
     pq.row1 = tensor_of(q, g.qs);
     pq.row2 = dense(dout, g, g.Hq, g.D);
