@@ -23,6 +23,9 @@ namespace {
 
 constexpr int kThreads = 288;            // 8 scatter warps + TMA/MMA warp
 constexpr int kStages = 3;
+// Loads of weights that a thread has in flight.  One at a time the staging was most of the apply kernel: 61 x 67, 9 x 9, 8 heads of 64,
+// batch 2: 42 us, now 30 (16 in flight: the same).
+constexpr int kAhead = 8;
 
 template <int DH>
 struct SmemS {
@@ -247,7 +250,9 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             const int j0 = tid >> (P.cb2_log + P.cb1_log);
             colslot[tid] = (j0 * P.K[1] + j1) * P.K[2] + j2;
         }
-        for (int j = team; j < ktot; j += 2) tile[row * ktot + j] = static_cast<uint16_t>(fill16);
+        // without a causal axis every slot of a row that is written out gets a score
+        if (P.causal[0] | P.causal[1] | P.causal[2])
+            for (int j = team; j < ktot; j += 2) tile[row * ktot + j] = static_cast<uint16_t>(fill16);
     }
     tc_fence_before();
     __syncthreads();
@@ -343,6 +348,7 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             int r = tid / ktot, j = tid - r * ktot;
             const int dr = 256 / ktot, dj = 256 - dr * ktot;
             const int total = kTileRows * ktot;
+#pragma unroll 4
             for (int idx = tid; idx < total; idx += 256) {
                 const long long off = rowout[r];
                 if (off >= 0) {
@@ -424,13 +430,14 @@ struct SmemA {
     static constexpr int kColSlot = kBar + 128;
     static constexpr int kRowOut = kColSlot + 512;        // [128] long long: row of w / out, or -1
     static constexpr int kW = kRowOut + 1024;             // [128][slots] 16-bit
-    static constexpr uint32_t kColP = 0;                  // two buffers of 64 columns
-    static constexpr uint32_t kColO = 128;
-    static constexpr uint32_t kTmemCols = 256;
+    // One P buffer at head dim 64, so that three CTAs share an SM: what bounds these kernels is the chain of a tile (geometry, weights,
+    // gathering, product), not an issue rate.
+    static constexpr int kPBufs = DH == 64 ? 1 : 2, kPerSm = DH == 64 ? 3 : 1;
+    static constexpr uint32_t kColP = 0, kColO = 64 * kPBufs, kTmemCols = kColO + DH;
 };
 
 template <int DH, bool BF16, int kInner>
-__global__ void __launch_bounds__(kThreads, (DH == 64 ? 2 : 1))
+__global__ void __launch_bounds__(kThreads, SmemA<DH>::kPerSm)
 tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ TcParams P,
                 const uint16_t* __restrict__ w, uint16_t* __restrict__ out, float scale, int ktot,
                 int out_by_position)
@@ -470,6 +477,9 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
         if (++ld[2] == G.nc[2]) { ld[2] = 0; if (++ld[1] == G.nc[1]) { ld[1] = 0; ++ld[0]; } }
         ++loaded;
     };
+    // P buffer of chunk c, and the parity of its barriers
+    auto buf_of = [](int c) { return SM::kPBufs == 2 ? c & 1 : 0; };
+    auto par_of = [](int c) { return (uint32_t)(SM::kPBufs == 2 ? (c >> 1) & 1 : c & 1); };
     if (warp == 8) {
         if (lane == 0) {
             *abort_flag = ((sbase & 1023u) || prior_abort) ? 1 : 0;
@@ -516,16 +526,17 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
             bool ok = true;
             for (int c = 0; c < nch && ok; ++c) {
                 ok = mbar_wait(bar_y + 8 * (c % kStages), (c / kStages) & 1, abort_flag, P.wait_budget) &&
-                     mbar_wait(bar_p + 8 * (c & 1), (c >> 1) & 1, abort_flag, P.wait_budget);
+                     mbar_wait(bar_p + 8 * buf_of(c), par_of(c), abort_flag, P.wait_budget);
                 if (!ok) break;
                 const uint64_t dy0 = smem_desc(sbase + SM::kY + (c % kStages) * SM::kTile, SM::kHalf, 1024);
                 tc_fence_after();
 #pragma unroll
                 for (int ks = 0; ks < kChunk / 16; ++ks)
-                    mma_ts_e(tmem + SM::kColO, tmem + SM::kColP + 64 * (c & 1) + 8 * ks, dy0 + 128 * ks, idesc, c > 0 || ks > 0, leader);
-                mma_commit_e(bar_o + 8 * (c & 1), leader);
-                if (c >= 1 && c + 2 < nch) {             // the product before this one is done: its Y stage is free
-                    ok = mbar_wait(bar_o + 8 * ((c - 1) & 1), ((c - 1) >> 1) & 1, abort_flag, P.wait_budget);
+                    mma_ts_e(tmem + SM::kColO, tmem + SM::kColP + 64 * buf_of(c) + 8 * ks, dy0 + 128 * ks, idesc, c > 0 || ks > 0, leader);
+                mma_commit_e(bar_o + 8 * buf_of(c), leader);
+                if (c >= 1 && c + 2 < nch) {             // the product before this one is done: its stage is free
+                    // (one P buffer: the threads waited for it before they stored P(c))
+                    if (SM::kPBufs == 2) ok = mbar_wait(bar_o + 8 * buf_of(c - 1), par_of(c - 1), abort_flag, P.wait_budget);
                     if (!ok) break;
                     if (leader) issue_y();
                     __syncwarp();
@@ -534,17 +545,24 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
         }
     } else {
         const uint32_t trow = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-        // ---- stage this tile's weights: rows are contiguous runs of `ktot` values ----
+        // ---- stage this tile's weights: rows are contiguous runs of `ktot` values; kAhead loads in flight a thread ----
         {
             int r = tid / ktot, j = tid - r * ktot;
             const int dr = 256 / ktot, dj = 256 - dr * ktot;
             const int total = kTileRows * ktot;
-            for (int idx = tid; idx < total; idx += 256) {
-                const long long off = rowout[r];
-                wt[idx] = off >= 0 ? w[off + j] : static_cast<uint16_t>(0);
-                r += dr;
-                j += dj;
-                if (j >= ktot) { j -= ktot; ++r; }
+            for (int idx = tid; idx < total; idx += 256 * kAhead) {
+                uint16_t v[kAhead];
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) {
+                    const long long off = idx + 256 * u < total ? rowout[r] : -1;
+                    v[u] = off >= 0 ? w[off + j] : static_cast<uint16_t>(0);
+                    r += dr;
+                    j += dj;
+                    if (j >= ktot) { j -= ktot; ++r; }
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u)
+                    if (idx + 256 * u < total) wt[idx + 256 * u] = v[u];
             }
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -557,9 +575,9 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
             for (int pc = 0; pc < 2; ++pc) words[pc] = piece_word(P, ci, 2 * team + pc, f, e);
             const int base = ((ci[0] * P.cb[0] - fs[0]) * P.K[1] + (ci[1] * P.cb[1] - fs[1])) * P.K[2] + (ci[2] * P.cb[2] - fs[2]);
             const uint16_t* srcp = myrow + base;  // slot 0 of this chunk's first column, for this row
-            // P buffer c & 1 was last read by the product of chunk c - 2
-            if (c >= 2) {
-                ok = ok && mbar_wait(bar_o + 8 * (c & 1), ((c - 2) >> 1) & 1, abort_flag, P.wait_budget);
+            // the buffer was last read by the product of chunk c - kPBufs
+            if (c >= SM::kPBufs) {
+                ok = ok && mbar_wait(bar_o + 8 * buf_of(c), par_of(c - SM::kPBufs), abort_flag, P.wait_budget);
                 tc_fence_after();
             }
 #pragma unroll
@@ -594,15 +612,15 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
 #pragma unroll
                     for (int i = 0; i < 16; ++i) packed[i] = 0u;
                 }
-                tmem_st16(trow + SM::kColP + 64 * (c & 1) + 32 * team + 16 * pc, packed);
+                tmem_st16(trow + SM::kColP + 64 * buf_of(c) + 32 * team + 16 * pc, packed);
             }
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(bar_p + 8 * (c & 1));
+            mbar_arrive(bar_p + 8 * buf_of(c));
             if (++ci[2] == G.nc[2]) { ci[2] = 0; if (++ci[1] == G.nc[1]) { ci[1] = 0; ++ci[0]; } }
         }
         // ---- every product is in O: scale, write out this thread's channels ----
-        ok = ok && mbar_wait(bar_o + 8 * ((nch - 1) & 1), ((nch - 1) >> 1) & 1, abort_flag, P.wait_budget);
+        ok = ok && mbar_wait(bar_o + 8 * buf_of(nch - 1), par_of(nch - 1), abort_flag, P.wait_budget);
         tc_fence_after();
 #pragma unroll
         for (int part = 0; part < CH / 32; ++part) {
@@ -687,11 +705,12 @@ struct SmemG {
     static constexpr int kColRow = kBar + 128;            // [2][128] long long: element offset of the column's row of w, -1 = no query
     static constexpr int kColFirst = kColRow + 2048;      // [2][3][128] int: first key of the column's window, per axis
     static constexpr int kTotal = kColFirst + 3072;
-    static constexpr uint32_t kColP = 0, kColO = 128, kTmemCols = 256;
+    static constexpr int kPBufs = DH == 64 ? 1 : 2, kPerSm = DH == 64 ? 3 : 1;
+    static constexpr uint32_t kColP = 0, kColO = 64 * kPBufs, kTmemCols = kColO + DH;
 };
 
 template <int DH, bool BF16>
-__global__ void __launch_bounds__(kThreads, (DH == 64 ? 2 : 1))
+__global__ void __launch_bounds__(kThreads, SmemG<DH>::kPerSm)
 tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ TcParams P,
                  const uint16_t* __restrict__ w, uint16_t* __restrict__ dst, float scale, int ktot)
 {
@@ -740,6 +759,9 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (++ld[2] == nc[2]) { ld[2] = 0; if (++ld[1] == nc[1]) { ld[1] = 0; if (++ld[0] == nc[0]) { ld[0] = 0; ++ld_head; } } }
         ++loaded;
     };
+    // P buffer of chunk c, and the parity of its barriers
+    auto buf_of = [](int c) { return SM::kPBufs == 2 ? c & 1 : 0; };
+    auto par_of = [](int c) { return (uint32_t)(SM::kPBufs == 2 ? (c >> 1) & 1 : c & 1); };
     if (warp == 8) {
         if (lane == 0) {
             *abort_flag = ((sbase & 1023u) || prior_abort) ? 1 : 0;
@@ -793,16 +815,17 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             bool ok = true;
             for (int c = 0; c < total && ok; ++c) {
                 ok = mbar_wait(bar_x + 8 * (c % kStages), (c / kStages) & 1, abort_flag, P.wait_budget) &&
-                     mbar_wait(bar_p + 8 * (c & 1), (c >> 1) & 1, abort_flag, P.wait_budget);
+                     mbar_wait(bar_p + 8 * buf_of(c), par_of(c), abort_flag, P.wait_budget);
                 if (!ok) break;
                 const uint64_t dx0 = smem_desc(sbase + SM::kX + (c % kStages) * SM::kTile, SM::kHalf, 1024);
                 tc_fence_after();
 #pragma unroll
                 for (int ks = 0; ks < kChunk / 16; ++ks)
-                    mma_ts_e(tmem + SM::kColO, tmem + SM::kColP + 64 * (c & 1) + 8 * ks, dx0 + 128 * ks, idesc, c > 0 || ks > 0, leader);
-                mma_commit_e(bar_o + 8 * (c & 1), leader);
-                if (c >= 1 && c + 2 < total) {           // the product before this one is done: its X stage is free
-                    ok = mbar_wait(bar_o + 8 * ((c - 1) & 1), ((c - 1) >> 1) & 1, abort_flag, P.wait_budget);
+                    mma_ts_e(tmem + SM::kColO, tmem + SM::kColP + 64 * buf_of(c) + 8 * ks, dx0 + 128 * ks, idesc, c > 0 || ks > 0, leader);
+                mma_commit_e(bar_o + 8 * buf_of(c), leader);
+                if (c >= 1 && c + 2 < total) {             // the product before this one is done: its stage is free
+                    // (one P buffer: the threads waited for it before they stored P(c))
+                    if (SM::kPBufs == 2) ok = mbar_wait(bar_o + 8 * buf_of(c - 1), par_of(c - 1), abort_flag, P.wait_budget);
                     if (!ok) break;
                     if (leader) issue_x();
                     __syncwarp();
@@ -839,8 +862,8 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             uint32_t words[2];
 #pragma unroll
             for (int pc = 0; pc < 2; ++pc) words[pc] = piece_word(P, ci, 2 * team + pc, f, e);
-            if (c >= 2) {                         // P buffer c & 1 was last read by the product of chunk c - 2
-                ok = ok && mbar_wait(bar_o + 8 * (c & 1), ((c - 2) >> 1) & 1, abort_flag, P.wait_budget);
+            if (c >= SM::kPBufs) {                         // the buffer was last read by the product of chunk c - kPBufs
+                ok = ok && mbar_wait(bar_o + 8 * buf_of(c), par_of(c - SM::kPBufs), abort_flag, P.wait_budget);
                 tc_fence_after();
             }
 #pragma unroll
@@ -861,15 +884,15 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 #pragma unroll
                     for (int i = 0; i < 16; ++i) packed[i] = 0u;
                 }
-                tmem_st16(trow + SM::kColP + 64 * (c & 1) + 32 * team + 16 * pc, packed);
+                tmem_st16(trow + SM::kColP + 64 * buf_of(c) + 32 * team + 16 * pc, packed);
             }
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(bar_p + 8 * (c & 1));
+            mbar_arrive(bar_p + 8 * buf_of(c));
             if (++ci[2] == nc[2]) { ci[2] = 0; if (++ci[1] == nc[1]) { ci[1] = 0; if (++ci[0] == nc[0]) { ci[0] = 0; ++hc; } } }
         }
         // ---- every product is in the accumulator: scale, write out this thread's channels ----
-        ok = ok && mbar_wait(bar_o + 8 * ((total - 1) & 1), ((total - 1) >> 1) & 1, abort_flag, P.wait_budget);
+        ok = ok && mbar_wait(bar_o + 8 * buf_of(total - 1), par_of(total - 1), abort_flag, P.wait_budget);
         tc_fence_after();
 #pragma unroll
         for (int part = 0; part < CH / 32; ++part) {
