@@ -1,5 +1,5 @@
 // Fused neighbourhood-attention forward for head dims up to 128 on tcgen05 tensor cores (sm_100a),
-// built from small persistent CTAs: four of them share an SM up to head dim 64, two above it, each working
+// built from small persistent CTAs: four of them share an SM up to head dim 64 (two where there are few tiles), two above it, each working
 // on one tile of 128 queries at a time (tiles blockIdx.x, + gridDim.x, ...).
 //
 // Per tile the union of the queries' neighbourhoods is a box of keys walked in chunks of 64 keys
@@ -49,10 +49,14 @@ constexpr int kKeysLog = 6;
 constexpr int kStages = 2;
 constexpr int kThreads = 256;               // 4 softmax warps; one that issues the products, one that loads, one for the geometry
 constexpr uint32_t kColS = 0;
+// Up to this many tiles an SM, head dims up to 64 run with two score buffers and two CTAs an SM, too: there is nothing else to fill a
+// chunk's gaps.  7 x 7, one buffer | two: 28 x 28, 8 heads of 32 (56 tiles) 12.2 | 10.6 us, 16 heads of 64 (112) 13.8 | 11.9; batch 2,
+// 16 heads of 32 (224) 14.0 | 12.8; 48 x 60, 6 heads of 64 (270) 15.2 | 13.6.  Above it the second buffer costs a second wave.
+constexpr unsigned kFewTiles = 2;
 
 // Shared memory and TMEM of one CTA for head dim DH (64: four CTAs per SM, 128 TMEM columns; 128: two CTAs per
 // SM, 256 TMEM columns).  Tiles are stored as blocks of 64 channels (128-byte rows, 128-byte swizzle).
-template <int DH>
+template <int DH, bool TWO_S>
 struct FwdSmall {
     static constexpr int kHalves = DH / 64;
     static constexpr int kQHalf = kTileRows * 128;          // [128 x 64] 16-bit
@@ -63,28 +67,28 @@ struct FwdSmall {
     static constexpr int kBar = kQBytes + 2 * kStages * kKVBytes;
     static constexpr int kTab = kBar + 208;
     static constexpr int kSmemTotal = kTab + 2 * kTabBytes;
-    static constexpr uint32_t kTmemCols = DH == 64 ? 128 : 256;     // S 64 + O DH, rounded up to a power of two
-    static constexpr int kPerSm = DH == 64 ? 4 : 2;
+    // Two score buffers where TMEM has the room: S(c + 1) is computed while the threads turn S(c) into probabilities.  With four CTAs
+    // an SM (one buffer, 128 columns each) the CTAs fill each other's gaps instead.
+    static constexpr bool kTwoS = TWO_S;
+    static constexpr uint32_t kTmemCols = kTwoS ? 256 : 128;        // S, O, rounded up to a power of two
+    static constexpr int kPerSm = kTwoS ? 2 : 4;
     // 65536 / kPerSm / kThreads registers a thread at launch, 64 or 128; the helpers hand what they do not need to the softmax
     // warps, which spill with less than 88 (32 | 96, where the helpers spill: 59.5 us instead of 53.5; 48 | 80: 54.0)
-    static constexpr int kHelperRegs = DH == 64 ? 40 : 104, kSoftmaxRegs = DH == 64 ? 88 : 152;
-    // At head dim 128 the 256 TMEM columns hold two score buffers: S(c + 1) is computed while the threads turn
-    // S(c) into probabilities (at 64 the four CTAs of an SM fill each other's gaps instead).
-    static constexpr bool kTwoS = DH == 128;
+    static constexpr int kHelperRegs = kTwoS ? 104 : 40, kSoftmaxRegs = kTwoS ? 152 : 88;
     // There K has to be a chunk ahead of V, so the two are loaded and freed apart; with one score buffer they come and go together.
     static constexpr bool kSplitKV = kTwoS;
     static constexpr uint32_t kColO = kTwoS ? 128 : 64;
 };
 
 // kShort: the last 32 of the DH channels are padding.
-template <int DH, bool BF16, int kInner, bool kShort>
-__global__ void __launch_bounds__(kThreads, FwdSmall<DH>::kPerSm)
+template <int DH, bool BF16, int kInner, bool kShort, bool TWO_S>
+__global__ void __launch_bounds__(kThreads, FwdSmall<DH, TWO_S>::kPerSm)
 tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmEK,
                     const __grid_constant__ CUtensorMap tmEV, const __grid_constant__ TcParams P,
                     uint16_t* __restrict__ out, float* __restrict__ lse)
 {
-    using FS = FwdSmall<DH>;
+    using FS = FwdSmall<DH, TWO_S>;
     constexpr int kHalves = FS::kHalves, kQHalf = FS::kQHalf, kKVHalf = FS::kKVHalf, kQBytes = FS::kQBytes, kKVBytes = FS::kKVBytes;
     constexpr int kOffQ = FS::kOffQ, kOffK = FS::kOffK, kOffV = FS::kOffV, kBar = FS::kBar, kTab = FS::kTab;
     constexpr uint32_t kTmemCols = FS::kTmemCols, kColO = FS::kColO;
@@ -724,15 +728,20 @@ int tc_fused_fwd_small(int dtype, const Geo& g, const void* q, const void* k, co
         return -2;
     if (plan.p.work_q == 0 || g.B == 0) return 0;
     cudaError_t err = cudaSuccess;
-    auto launch = [&](auto dh, auto bf, auto inner, auto shorter) {
+    auto launch_as = [&](auto dh, auto bf, auto inner, auto shorter, auto two_s) {
         constexpr int kDh = decltype(dh)::value;
-        constexpr bool kBf = decltype(bf)::value;
-        constexpr int kInner = decltype(inner)::value;
-        using FS = FwdSmall<kDh>;
+        using FS = FwdSmall<kDh, decltype(two_s)::value>;
+        auto* kernel = tc_fwd_small_kernel<kDh, decltype(bf)::value, decltype(inner)::value, decltype(shorter)::value, decltype(two_s)::value>;
         const unsigned grid = persistent_grid(plan.p.work_q, FS::kPerSm);
-        err = ensure_dynamic_smem((const void*)tc_fwd_small_kernel<kDh, kBf, kInner, decltype(shorter)::value>, FS::kSmemTotal);
+        err = ensure_dynamic_smem((const void*)kernel, FS::kSmemTotal);
         if (err != cudaSuccess) return;
-        tc_fwd_small_kernel<kDh, kBf, kInner, decltype(shorter)::value><<<grid, kThreads, FS::kSmemTotal, s>>>(mq, mk, mv, mek, mev, plan.p, (uint16_t*)out, (float*)lse);
+        kernel<<<grid, kThreads, FS::kSmemTotal, s>>>(mq, mk, mv, mek, mev, plan.p, (uint16_t*)out, (float*)lse);
+    };
+    auto launch = [&](auto dh, auto bf, auto inner, auto shorter) {
+        if constexpr (decltype(dh)::value == 64) {
+            if (plan.p.work_q > kFewTiles * (unsigned)sm_count()) return launch_as(dh, bf, inner, shorter, std::false_type{});
+        }
+        launch_as(dh, bf, inner, shorter, std::true_type{});
     };
     auto by_short = [&](auto dh, auto bf, auto inner) {
         if (g.D <= decltype(dh)::value - 32) launch(dh, bf, inner, std::true_type{});
