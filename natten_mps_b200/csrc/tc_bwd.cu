@@ -366,35 +366,15 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             bool ok = !*abort_flag;
             unsigned w = blockIdx.x, stage = 0, parity = 1, g = 0;
             auto publish = [&](unsigned t) -> bool {     // the next work item with rows of a sample -> slot t & 1; false: none is left
-                BwdTile X;
-                bool found = false;
-                for (; w < nwork && !found; w += gridDim.x) {
-                    bwd_tile_setup<kKeySide>(P, w, X);
-                    found = X.active;
-                }
                 if (t >= 2) ok = ok && mbar_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
                 if (!ok) return false;
-                uint8_t* slot = tab_slot(t);
-                const bool mapped = kInner == 16 && found && X.nc[2] == 1 && X.nchunks <= 16;
-                if (lane == 0) {
-                    TileHead* hd = reinterpret_cast<TileHead*>(slot);
-                    hd->total = found ? X.total : 0;
-                    if (found) {
-                        hd->nbox = X.nbox;
-                        hd->nchunks = X.nchunks;
-                        hd->b = X.b;
-                        hd->hy = X.hy;
-                        hd->mapped = mapped;
-#pragma unroll
-                        for (int a = 0; a < 3; ++a) {
-                            hd->nc[a] = X.nc[a]; hd->boxlo[a] = X.boxlo[a]; hd->Lp[a] = X.Lp[a];
-                            hd->rg[a] = X.rg[a]; hd->origin[a] = X.origin[a];
-                        }
-                    }
-                    mbar_arrive(bar_head + 8 * (t & 1));
-                }
+                TileHead* H = reinterpret_cast<TileHead*>(tab_slot(t));
+                bool found = false;
+                for (; w < nwork && !found; w += gridDim.x) found = publish_tile<kKeySide>(P, w, kInner == 16, lane, H);
+                if (!found && lane == 0) H->total = 0;
                 __syncwarp();
-                if (found) write_tables<kKeySide>(P, X, mapped, lane, slot);
+                if (lane == 0) mbar_arrive(bar_head + 8 * (t & 1));
+                if (found) write_tables<kKeySide>(P, lane, tab_slot(t));
                 mbar_arrive(bar_tab_full + 8 * (t & 1));
                 return found;
             };

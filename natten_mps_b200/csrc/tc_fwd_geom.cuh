@@ -122,41 +122,83 @@ __device__ __forceinline__ long long row_geometry(const TcParams& P, const FwdTi
 constexpr int kMapOff = 160, kEntOff = kMapOff + 8 * kTileRows, kTabBytes = kEntOff + 16 * (kTileRows + 2);
 static_assert(sizeof(FwdTile) <= kMapOff, "no room for the tile in front of its tables");
 
-// Query coordinate i of the tile along axis a: window [f, e) in the box, output position, flags (bit 0 query of the sample, bit 1
-// position of the tensor).
-__device__ __forceinline__ int4 axis_entry(const TcParams& P, const FwdTile& T, int a, int i)
+// The cursor's work item into the head of a slot, by one warp (the same as fwd_tile, an axis per lane); returns whether it is
+// active.  rows16: chunks of 16-column rows.
+__device__ __forceinline__ bool publish_tile(const TcParams& P, const Cursor& cur, int chunk_log, bool rows16, int lane, FwdTile* H)
 {
-    const int qa = T.origin[a] + i, xq = T.x0[a] + T.sx[a] * qa, pa = T.rg[a] + P.dil[a] * xq;
-    const int first = P.causal[a] ? xq - (P.K[a] - 1) : window_start(xq, T.Lp[a], P.K[a], 1);
-    return make_int4((first > 0 ? first : 0) - T.lo[a], (first + P.K[a] < T.Lp[a] ? first + P.K[a] : T.Lp[a]) - T.lo[a],
-                     P.st[a] == 1 ? pa : pa / P.st[a], (qa < T.nq[a] ? 1 : 0) | (qa < T.nqf[a] ? 2 : 0));
+    const int a = lane < 2 ? lane : 2;
+    int rg, origin, Lp, nq, nqf, lo = 0, nc = 1;
+    bool active = lane_geometry(P, cur.bx, cur.b, a, rg, origin, Lp);
+    const int sx = P.qstep[a];
+    int x0 = P.qx0[a][rg];
+    const int lpf = (int)fast_div((unsigned)(P.L[a] - rg + P.dil[a] - 1), P.dil_mul[a]);
+    if (x0 < 0) {
+        nq = 0; nqf = 0; x0 = 0;
+    } else if (sx == 1) {
+        nq = Lp;
+        nqf = rg < P.L[a] ? lpf : 0;
+    } else {
+        nq = x0 < Lp ? (Lp - x0 + sx - 1) / sx : 0;
+        nqf = x0 < lpf ? (lpf - x0 + sx - 1) / sx : 0;
+    }
+    active = __all_sync(0xffffffffu, active && origin < nq);
+    if (!active) return false;
+    {
+        const int lastq = origin + P.tile[a] - 1 < nq - 1 ? origin + P.tile[a] - 1 : nq - 1;
+        const int xf = x0 + sx * origin, xl = x0 + sx * lastq;
+        lo = P.causal[a] ? xf - (P.K[a] - 1) : window_start(xf, Lp, P.K[a], 1);
+        const int hi = P.causal[a] ? xl : window_start(xl, Lp, P.K[a], 1) + P.K[a] - 1;
+        nc = chunks_along(P, a, hi - lo + 1);
+    }
+    const int nnb = __shfl_sync(0xffffffffu, nc, 0) * __shfl_sync(0xffffffffu, nc, 1) * __shfl_sync(0xffffffffu, nc, 2);
+    if (lane < 3) {
+        H->rg[lane] = rg; H->origin[lane] = origin; H->Lp[lane] = Lp; H->lo[lane] = lo; H->nc[lane] = nc;
+        H->x0[lane] = x0; H->sx[lane] = sx; H->nq[lane] = nq; H->nqf[lane] = nqf;
+    }
+    if (lane == 2) {
+        H->b = cur.b;
+        H->h = cur.h;
+        H->hk = (int)fast_div((unsigned)cur.h, P.group_mul);
+        H->nnb = nnb;
+        H->nch = nnb + ((P.n_extra + (1 << chunk_log) - 1) >> chunk_log);    // then the additional tokens, one chunk at a time
+        H->active = 1;
+        H->mapped = rows16 && nc == 1 && nnb <= 16;
+    }
+    return true;
 }
 
-// One warp.  `mapped`: chunks of 16-column rows, one chunk along the innermost axis and at most 16 chunks in all.  Then which of
+// The slot's tables, by one warp.  An entry is for a query coordinate of the tile along an axis: window [f, e) in the box, output
+// position, flags (bit 0 query of the sample, bit 1 position of the tensor).
+// `mapped`: chunks of 16-column rows, one chunk along the innermost axis and at most 16 chunks in all.  Then which of
 // a chunk's four rows lie in a query's window depends on its two outer coordinates: a map per pair of them, four bits a chunk
 // (every row of the window lands in one row of one chunk), and the window's columns as bits beside the flags.
-__device__ __forceinline__ void write_tables(const TcParams& P, const FwdTile& T, int lane, uint8_t* slot)
+__device__ __forceinline__ void write_tables(const TcParams& P, int lane, uint8_t* slot)
 {
+    const FwdTile* T = reinterpret_cast<const FwdTile*>(slot);
     int4* ent = reinterpret_cast<int4*>(slot + kEntOff);
-    int base = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        for (int i = lane; i < P.tile[a]; i += 32) {
-            int4 en = axis_entry(P, T, a, i);
-            if (a == 2 && T.mapped) {
-                int lo, hi;
-                chunk_range(P, 2, 0, en.x, en.y, lo, hi);
-                if (hi > lo) en.w |= (low_bits(hi) & ~low_bits(lo)) << 16;
-            }
-            ent[base + i] = en;
+    const int t0 = P.tile[0], t01 = t0 + P.tile[1], all = t01 + P.tile[2];
+    const bool mapped = T->mapped;
+#pragma unroll 1
+    for (int i = lane; i < all; i += 32) {
+        const int a = i < t0 ? 0 : i < t01 ? 1 : 2;
+        const int qa = T->origin[a] + i - (a == 0 ? 0 : a == 1 ? t0 : t01), xq = T->x0[a] + T->sx[a] * qa, pa = T->rg[a] + P.dil[a] * xq;
+        const int lo = T->lo[a], Lp = T->Lp[a], K = P.K[a], st = P.st[a];
+        const int first = P.causal[a] ? xq - (K - 1) : window_start(xq, Lp, K, 1);
+        int4 en = make_int4((first > 0 ? first : 0) - lo, (first + K < Lp ? first + K : Lp) - lo, st == 1 ? pa : pa / st,
+                            (qa < T->nq[a] ? 1 : 0) | (qa < T->nqf[a] ? 2 : 0));
+        if (a == 2 && mapped) {
+            int jl, jh;
+            chunk_range(P, 2, 0, en.x, en.y, jl, jh);
+            if (jh > jl) en.w |= (low_bits(jh) & ~low_bits(jl)) << 16;
         }
-        base += P.tile[a];
+        ent[i] = en;
     }
-    if (!T.mapped) return;
+    __syncwarp();
+    if (!mapped) return;
     unsigned long long* map = reinterpret_cast<unsigned long long*>(slot + kMapOff);
-    for (int r = lane; r < P.tile[0] * P.tile[1]; r += 32) {
-        const int4 e0 = axis_entry(P, T, 0, r >> P.tile1_log), e1 = axis_entry(P, T, 1, r & (P.tile[1] - 1));
-        map[r] = (e0.w & e1.w & 1) ? row_map(P, T.nc[1], e0.x, e0.y, e1.x, e1.y) : 0ull;
+    for (int r = lane; r < t0 * P.tile[1]; r += 32) {
+        const int4 e0 = ent[r >> P.tile1_log], e1 = ent[t0 + (r & (P.tile[1] - 1))];
+        map[r] = (e0.w & e1.w & 1) ? row_map(P, T->nc[1], e0.x, e0.y, e1.x, e1.y) : 0ull;
     }
 }
 

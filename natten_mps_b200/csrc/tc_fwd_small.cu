@@ -304,42 +304,40 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             // tiles (per-sample extents) are zeroed here.
             // =====================================================================
             if (!*abort_flag) {
+                auto zero_rows = [&](const Cursor& at) {     // rows of a padding tile that exist in the output are zero
+                    FwdTile T;
+                    fwd_tile(P, at, kKeysLog, T);
+#pragma unroll 1
+                    for (int r = lane; r < kTileRows; r += 32) {
+                        int f[3], e[3];
+                        bool valid_q, in_tensor;
+                        const long long out_row = row_geometry(P, T, r, f, e, valid_q, in_tensor);
+                        if (in_tensor) {
+                            uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
+#pragma unroll
+                            for (int i = 0; i < DH / 8; ++i)
+                                if (8 * i < P.dreal) o4[i] = make_uint4(0, 0, 0, 0);
+                            lse[out_row] = 0.f;
+                        }
+                    }
+                };
                 bool ok = true, found = true;
                 Cursor cur;
                 cur.init(P, blockIdx.x, gridDim.x);
                 for (unsigned t = 0; ok && found; ++t) {
-                    FwdTile T;
-                    found = false;
-                    while (cur.w < nwork && !found) {
-                        fwd_tile(P, cur, kKeysLog, T);
-                        cur.advance(P, gridDim.x);
-                        found = T.active != 0;
-                        if (found || !P.extents) continue;
-#pragma unroll 1
-                        for (int r = lane; r < kTileRows; r += 32) {
-                            int f[3], e[3];
-                            bool valid_q, in_tensor;
-                            const long long out_row = row_geometry(P, T, r, f, e, valid_q, in_tensor);
-                            if (in_tensor) {
-                                uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
-#pragma unroll
-                                for (int i = 0; i < DH / 8; ++i)
-                                    if (8 * i < P.dreal) o4[i] = make_uint4(0, 0, 0, 0);
-                                lse[out_row] = 0.f;
-                            }
-                        }
-                    }
-                    if (!found) T.nch = 0;
                     if (t >= 2) ok = mbar_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
                     FwdTile* H = tab_slot(t);
-                    T.mapped = kInner == 16 && T.nc[2] == 1 && T.nnb <= 16;
-                    if (lane == 0) {
-                        *H = T;
-                        mbar_arrive(bar_head + 8 * (t & 1));
+                    found = false;
+                    while (cur.w < nwork && !found) {
+                        found = publish_tile(P, cur, kKeysLog, kInner == 16, lane, H);
+                        if (!found && P.extents) zero_rows(cur);
+                        cur.advance(P, gridDim.x);
                     }
+                    if (!found && lane == 0) H->nch = 0;
                     __syncwarp();
-                    if (found) write_tables(P, T, lane, reinterpret_cast<uint8_t*>(H));
+                    if (lane == 0) mbar_arrive(bar_head + 8 * (t & 1));
+                    if (found) write_tables(P, lane, reinterpret_cast<uint8_t*>(H));
                     mbar_arrive(bar_tab_full + 8 * (t & 1));
                 }
             }

@@ -109,6 +109,32 @@ __device__ __forceinline__ bool cta_geometry(const TcParams& P, unsigned bx, int
     return active;
 }
 
+// What cta_geometry works out, one axis per lane (lane 2 and up: the innermost one): a third of the instructions, which counts where
+// they run for the first time and come from memory.  Returns whether the tile holds a row of the sample along the lane's axis.
+__device__ __forceinline__ bool lane_geometry(const TcParams& P, unsigned bx, int b, int a, int& rg, int& origin, int& Lp)
+{
+    unsigned x = bx;
+    int o[3], r[3];
+#pragma unroll
+    for (int i = 2; i >= 0; --i) {
+        const unsigned q = fast_div(x, P.ntile_mul[i]);
+        o[i] = static_cast<int>(x - q * P.ntile[i]) * P.tile[i];
+        x = q;
+    }
+#pragma unroll
+    for (int i = 2; i >= 0; --i) {
+        const unsigned q = fast_div(x, P.grp_mul[i]);
+        r[i] = static_cast<int>(x - q * P.grp_n[i]) * P.grp_step[i];
+        x = q;
+    }
+    rg = a == 0 ? r[0] : a == 1 ? r[1] : r[2];
+    origin = a == 0 ? o[0] : a == 1 ? o[1] : o[2];
+    const int ea = a - (3 - P.rank);
+    const int Ls = (P.extents && ea >= 0) ? P.extents[b * P.rank + ea] : P.L[a];
+    Lp = rg < Ls ? static_cast<int>(fast_div(Ls - rg + P.dil[a] - 1, P.dil_mul[a])) : 0;
+    return origin < Lp;
+}
+
 // Tile load of channels ch .. ch + 63 of head h: one coordinate, or two where the map has a head axis of its own.
 __device__ __forceinline__ void tma_load_heads(uint32_t dst, const CUtensorMap* map, uint32_t bar, const TcParams& P,
                                                int h, int ch, int c1, int c2, int c3, int c4)

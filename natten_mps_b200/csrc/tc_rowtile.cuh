@@ -73,44 +73,74 @@ __device__ __forceinline__ void bwd_tile_setup(const TcParams& P, unsigned work,
     T.total = T.nbox + (kKeySide ? 0 : ((P.n_extra + kCols - 1) >> 6));
 }
 
-// Entry of the tile's row coordinate i along axis a.
+// The work item into the head of a slot, by one warp (what bwd_tile_setup gives, an axis per lane); returns whether it is active.
+// rows16: chunks of 16-column rows.
 template <bool kKeySide>
-__device__ __forceinline__ AxisEntry axis_entry(const TcParams& P, const BwdTile& X, int a, int i)
+__device__ __forceinline__ bool publish_tile(const TcParams& P, unsigned work, bool rows16, int lane, TileHead* H)
 {
-    const int xa = X.origin[a] + i, pa = X.rg[a] + P.dil[a] * xa;
-    AxisEntry en;
-    en.z = pa;
-    en.w = (xa < X.Lp[a] ? 1 : 0) | (pa < P.L[a] ? 2 : 0);
+    const unsigned hb = work / P.per_head, heads = (unsigned)(kKeySide ? P.Hkv : P.Hq);
+    const int b = (int)(hb / heads), hy = (int)(hb - (unsigned)b * heads), a = lane < 2 ? lane : 2;
+    int rg, origin, Lp;
+    if (!__all_sync(0xffffffffu, lane_geometry(P, work - hb * P.per_head, b, a, rg, origin, Lp))) return false;
+    const int last = origin + P.tile[a] - 1 < Lp - 1 ? origin + P.tile[a] - 1 : Lp - 1;
+    int boxlo, hi;
     if (kKeySide) {
-        int qlo, qhi;
-        inverse_range(xa, X.Lp[a], P.K[a], P.causal[a], qlo, qhi);
-        en.x = qlo - X.boxlo[a];
-        en.y = qhi + 1 - X.boxlo[a];
+        int t;
+        inverse_range(origin, Lp, P.K[a], P.causal[a], boxlo, t, /*exact=*/false);
+        inverse_range(last, Lp, P.K[a], P.causal[a], t, hi, /*exact=*/false);
     } else {
-        const int first = P.causal[a] ? xa - (P.K[a] - 1) : ws1(xa, X.Lp[a], P.K[a]);
-        en.x = (first > 0 ? first : 0) - X.boxlo[a];
-        en.y = (first + P.K[a] < X.Lp[a] ? first + P.K[a] : X.Lp[a]) - X.boxlo[a];
+        boxlo = P.causal[a] ? origin - (P.K[a] - 1) : ws1(origin, Lp, P.K[a]);
+        hi = P.causal[a] ? last : ws1(last, Lp, P.K[a]) + P.K[a] - 1;
     }
-    return en;
+    const int nc = chunks_along(P, a, hi - boxlo + 1);
+    const int nchunks = __shfl_sync(0xffffffffu, nc, 0) * __shfl_sync(0xffffffffu, nc, 1) * __shfl_sync(0xffffffffu, nc, 2);
+    if (lane < 3) {
+        H->nc[lane] = nc; H->boxlo[lane] = boxlo; H->Lp[lane] = Lp; H->rg[lane] = rg; H->origin[lane] = origin;
+    }
+    if (lane == 2) {
+        H->b = b;
+        H->hy = hy;
+        H->nchunks = nchunks;
+        H->nbox = nchunks * (kKeySide ? P.group : 1);
+        H->total = H->nbox + (kKeySide ? 0 : ((P.n_extra + kCols - 1) >> 6));
+        H->mapped = rows16 && nc == 1 && nchunks <= 16;
+    }
+    return true;
 }
 
-// One warp writes a tile's tables.  mapped: chunks of 16-column rows, one along the innermost axis, at most 16 in the box.  Then
+// The slot's tables, by one warp.  mapped: chunks of 16-column rows, one along the innermost axis, at most 16 in the box.  Then
 // which of a chunk's four rows lie in a row's range depends on its two outer coordinates: a map per pair of them, four bits a chunk.
 template <bool kKeySide>
-__device__ __forceinline__ void write_tables(const TcParams& P, const BwdTile& X, bool mapped, int lane, uint8_t* slot)
+__device__ __forceinline__ void write_tables(const TcParams& P, int lane, uint8_t* slot)
 {
+    const TileHead* H = reinterpret_cast<const TileHead*>(slot);
     AxisEntry* ent = reinterpret_cast<AxisEntry*>(slot + kHeadBytes + kMapBytes);
-    int base = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        for (int i = lane; i < P.tile[a]; i += 32) ent[base + i] = axis_entry<kKeySide>(P, X, a, i);
-        base += P.tile[a];
+    const int t0 = P.tile[0], t01 = t0 + P.tile[1], all = t01 + P.tile[2];
+#pragma unroll 1
+    for (int i = lane; i < all; i += 32) {
+        const int a = i < t0 ? 0 : i < t01 ? 1 : 2;
+        const int xa = H->origin[a] + i - (a == 0 ? 0 : a == 1 ? t0 : t01), Lp = H->Lp[a], lo = H->boxlo[a], K = P.K[a];
+        AxisEntry en;
+        en.z = H->rg[a] + P.dil[a] * xa;
+        en.w = (xa < Lp ? 1 : 0) | (en.z < P.L[a] ? 2 : 0);
+        if (kKeySide) {
+            int qlo, qhi;
+            inverse_range(xa, Lp, K, P.causal[a], qlo, qhi);
+            en.x = qlo - lo;
+            en.y = qhi + 1 - lo;
+        } else {
+            const int first = P.causal[a] ? xa - (K - 1) : ws1(xa, Lp, K);
+            en.x = (first > 0 ? first : 0) - lo;
+            en.y = (first + K < Lp ? first + K : Lp) - lo;
+        }
+        ent[i] = en;
     }
-    if (!mapped) return;
+    __syncwarp();
+    if (!H->mapped) return;
     unsigned long long* map = reinterpret_cast<unsigned long long*>(slot + kHeadBytes);
-    for (int r = lane; r < P.tile[0] * P.tile[1]; r += 32) {
-        const AxisEntry e0 = axis_entry<kKeySide>(P, X, 0, r >> P.tile1_log), e1 = axis_entry<kKeySide>(P, X, 1, r & (P.tile[1] - 1));
-        map[r] = (e0.w & e1.w & 1) ? row_map(P, X.nc[1], e0.x, e0.y, e1.x, e1.y) : 0ull;
+    for (int r = lane; r < t0 * P.tile[1]; r += 32) {
+        const AxisEntry e0 = ent[r >> P.tile1_log], e1 = ent[t0 + (r & (P.tile[1] - 1))];
+        map[r] = (e0.w & e1.w & 1) ? row_map(P, H->nc[1], e0.x, e0.y, e1.x, e1.y) : 0ull;
     }
 }
 
