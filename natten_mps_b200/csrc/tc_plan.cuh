@@ -574,11 +574,26 @@ inline void fit_key_boxes(Plan& plan)
     }
 }
 
+// Encodes a 16-bit map of five dimensions.  The driver wants a current context, which a thread that has not made a CUDA runtime call
+// yet (autograd's, on memory that was cached) does not have: the device's own is bound then.
+inline bool encode_16bit(CUtensorMap* map, const void* base, bool bf16, const cuuint64_t* dims, const cuuint64_t* gstr, const cuuint32_t* bx,
+                         const cuuint32_t* es)
+{
+    const EncodeFn enc = get_encode();
+    for (int attempt = 0;; ++attempt) {
+        const CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(base),
+                               dims, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_ERROR_INVALID_CONTEXT || attempt) return r == CUDA_SUCCESS;
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return false;
+    }
+}
+
 // 5-D map over [B, X0, X1, X2, heads*D] (innermost first in the arrays below).
 inline bool encode_map(CUtensorMap* map, const void* base, bool bf16, const TcParams& p, int heads, int dh,
                 const long long strides[3], const int box[3], bool query_lattice = false, bool interleaved = false)
 {
-    const EncodeFn enc = get_encode();
     const cuuint64_t tok = (cuuint64_t)strides[1] * 2;
     cuuint64_t dims[5] = {(cuuint64_t)heads * dh, (cuuint64_t)p.L[2], (cuuint64_t)p.L[1], (cuuint64_t)p.L[0], (cuuint64_t)p.B};
     cuuint64_t gstr[4] = {tok, tok * p.L[2], tok * p.L[2] * p.L[1], (cuuint64_t)strides[0] * 2};
@@ -599,18 +614,13 @@ inline bool encode_map(CUtensorMap* map, const void* base, bool bf16, const TcPa
     for (int i = 1; i < 4; ++i)
         if (es[i] > 8) return false;
     if (dims[4] == 0) return false;
-    const CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5,
-                           const_cast<void*>(base), dims, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
+    return encode_16bit(map, base, bf16, dims, gstr, bx, es);
 }
 
 // Map over the additional tokens [B, Ne, heads, dh]: same 5-D form, one spatial axis of extent Ne.
 inline bool encode_extra_map(CUtensorMap* map, const void* base, bool bf16, int B, int n_extra, int heads,
                              int dh, int box_cols, bool split_heads = false)
 {
-    const EncodeFn enc = get_encode();
     if (n_extra <= 0) return false;
     const cuuint64_t tok = (cuuint64_t)heads * dh * 2;
     cuuint64_t dims[5] = {(cuuint64_t)heads * dh, (cuuint64_t)n_extra, 1, 1, (cuuint64_t)B};
@@ -622,10 +632,7 @@ inline bool encode_extra_map(CUtensorMap* map, const void* base, bool bf16, int 
         gstr[0] = (cuuint64_t)dh * 2; gstr[1] = tok; gstr[2] = tok * n_extra;
         bx[1] = 1; bx[2] = (cuuint32_t)box_cols;
     }
-    return enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5,
-               const_cast<void*>(base), dims, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return encode_16bit(map, base, bf16, dims, gstr, bx, es);
 }
 
 // Bits [0, n) of a 32-bit word (n may be <= 0 or >= 32).
