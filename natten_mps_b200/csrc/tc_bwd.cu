@@ -72,8 +72,9 @@ struct SmemB {
     static constexpr int kStats = kC2 + kStages * kColTile;     // [kStages][2][64] float
     static constexpr int kTab = kStats + kStages * 512;         // [2] tables: axis entries, then a TileHead
     static constexpr int kBar = kTab + 2 * kTabBytes;
-    // Up to head dim 64 two CTAs leave a thread 80 registers at launch.  On the query side the helpers hand some of theirs to the
-    // compute warps; on the key side they need them for the statistics (64 x 64, 7 x 7: 84 us as it is, 101 with 64 | 88).
+    // Up to head dim 64 two CTAs leave a thread 80 registers at launch; the helpers hand to the compute warps what they do not need
+    // themselves (128 x 128, 13 x 13, dilation 2, query side and key side: all 80 209 and 256 us, 64 | 88 196 and 250; 48 | 96, where the
+    // statistics spill, 202 and 285).
     static constexpr int kHelperRegs = 64, kComputeRegs = 88;
     static constexpr int kStage = (kBar + 256 + 1023) & ~1023;   // output staging: a row tile [128 x DH] 16-bit, swizzled like the loads
     static constexpr int kTotal = kStage + kTile;
@@ -164,7 +165,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
     auto tab_slot = [&](unsigned t) { return smem + Smem::kTab + (t & 1) * kTabBytes; };
 
     if (warp >= kComputeWarps) {
-        if (DH == 64 && !kKeySide) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Smem::kHelperRegs));
+        if (DH == 64) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Smem::kHelperRegs));
         if (warp == kComputeWarps || warp == kComputeWarps + 2) {
             // =====================================================================
             // MMA issue: one thread in each of two warps.  A single thread gets a tcgen05.mma out every ~65
@@ -298,7 +299,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                         pflat = pflat * P.L[a] + pa;
                     }
                     if (!in_tensor) continue;
-                    const long long row = ((long long)Z.b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + Z.hy;
+                    const long long row = ((long long)Z.b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + Z.hy + (r & ((1 << P.pack_log) - 1));
 #pragma unroll
                     for (int which = 0; which < (kKeySide ? 2 : 1); ++which) {
                         uint4* o = reinterpret_cast<uint4*>((which == 0 ? out1 : out2) + row * P.dreal);
@@ -328,8 +329,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     mbar_expect_tx(bar_row, 2 * kTile);
 #pragma unroll
                     for (int hf = 0; hf < Smem::kHalves; ++hf) {
-                        tma_load_heads(sbase + Smem::kR1 + hf * kRowHalf, &tmR1, bar_row, P, hy, 64 * hf, R[2], R[1], R[0], b);
-                        tma_load_heads(sbase + Smem::kR2 + hf * kRowHalf, &tmR2, bar_row, P, hy, 64 * hf, R[2], R[1], R[0], b);
+                        tma_load_rows(sbase + Smem::kR1 + hf * kRowHalf, &tmR1, bar_row, P, hy, 64 * hf, R[2], R[1], R[0], b);
+                        tma_load_rows(sbase + Smem::kR2 + hf * kRowHalf, &tmR2, bar_row, P, hy, 64 * hf, R[2], R[1], R[0], b);
                     }
                 }
                 __syncwarp();
@@ -443,7 +444,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
         // =====================================================================
         // compute warps: thread = (row, 32-column piece)
         // =====================================================================
-        if (DH == 64 && !kKeySide) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Smem::kComputeRegs));
+        if (DH == 64) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Smem::kComputeRegs));
         const uint32_t trow = tmem + (static_cast<uint32_t>(quad * 32) << 16);
         bool ok = true;
         unsigned g = 0;                          // chunks processed so far (all tiles)
@@ -479,11 +480,11 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     in_tensor = in_tensor && (en.w & 2);
                     pflat = pflat * P.L[a] + en.z;
                 }
-                if (mapped) rowmap = reinterpret_cast<const unsigned long long*>(tab + kHeadBytes)[(quad * 32 + lane) >> P.tile2_log];
+                if (mapped) rowmap = reinterpret_cast<const unsigned long long*>(tab + kHeadBytes)[(quad * 32 + lane) >> (P.tile2_log + P.pack_log)];
             }
             mbar_arrive(bar_tab_empty + 8 * (t & 1));
             if (!valid_row) { e[0] = f[0]; e[1] = f[1]; e[2] = f[2]; }
-            const long long out_row = ((long long)b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + hy;
+            const long long out_row = ((long long)b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + hy + (lane & ((1 << P.pack_log) - 1));
             // query side: the row's lse and delta; scaled where they are first used, so that the loads' latency
             // runs under the set-up of the first chunk and the wait for its scores
             float raw_lse = 0.f, raw_delta = 0.f;
@@ -840,13 +841,11 @@ expand_strided_kernel(const __grid_constant__ Geo g, const uint4* __restrict__ d
 }
 
 template <int DH, bool BF16>
-int launch_bwd(int dtype, const Geo& g, const Plan& plan, const void* q, const void* k, const void* v,
+int launch_bwd(int dtype, const Geo& g, const Plan& plan, const Plan& key_plan, const void* q, const void* k, const void* v,
                const void* ek, const void* ev, void* dek, void* dev, const void* out, const void* lse, const void* dout, const void* dlse, void* dq, void* dk,
                void* dv, float* delta, cudaStream_t s, const Expanded* ex = nullptr)
 {
-    const TcParams& p = plan.p;
-    Plan key_plan = plan;
-    fit_key_boxes(key_plan);
+    const TcParams &p = plan.p, &pk = key_plan.p;    // rows are queries | keys
     // With an output stride the kernels run on the unit-stride geometry `g` over full-resolution copies of
     // dout / lse / delta (see expand_strided_kernel); the caller's arrays are only read to build them.
     const void* dout_k = ex ? ex->dout_full : dout;
@@ -856,22 +855,22 @@ int launch_bwd(int dtype, const Geo& g, const Plan& plan, const void* q, const v
     CUtensorMap q_tile, do_tile, k_chunk, v_chunk, k_tile, v_tile, q_chunk, do_chunk, ek_chunk, ev_chunk;
     const bool bf = BF16;
     using Smem = SmemB<DH>;
-    if (!encode_map(&q_tile, q, bf, p, g.Hq, g.D, g.qs, plan.box_q) ||
-        !encode_map(&do_tile, dout_k, bf, p, g.Hq, g.D, dos, plan.box_q) ||
+    if (!encode_map(&q_tile, q, bf, p, g.Hq, g.D, g.qs, plan.box_q, false, false, /*rows=*/true) ||
+        !encode_map(&do_tile, dout_k, bf, p, g.Hq, g.D, dos, plan.box_q, false, false, true) ||
         !encode_map(&k_chunk, k, bf, p, g.Hkv, g.D, g.ks, plan.box_kv, false, /*interleaved=*/true) ||
         !encode_map(&v_chunk, v, bf, p, g.Hkv, g.D, g.vs, plan.box_kv, false, true) ||
-        !encode_map(&k_tile, k, bf, p, g.Hkv, g.D, g.ks, plan.box_q) ||
-        !encode_map(&v_tile, v, bf, p, g.Hkv, g.D, g.vs, plan.box_q) ||
-        !encode_map(&q_chunk, q, bf, key_plan.p, g.Hq, g.D, g.qs, key_plan.box_kv, false, true) ||
-        !encode_map(&do_chunk, dout_k, bf, key_plan.p, g.Hq, g.D, dos, key_plan.box_kv, false, true))
+        !encode_map(&k_tile, k, bf, pk, g.Hkv, g.D, g.ks, key_plan.box_q, false, false, true) ||
+        !encode_map(&v_tile, v, bf, pk, g.Hkv, g.D, g.vs, key_plan.box_q, false, false, true) ||
+        !encode_map(&q_chunk, q, bf, pk, g.Hq, g.D, g.qs, key_plan.box_kv, false, true) ||
+        !encode_map(&do_chunk, dout_k, bf, pk, g.Hq, g.D, dos, key_plan.box_kv, false, true))
         return -2;
     // outputs: contiguous [B, *L, H, D]; stored as row tiles
     CUtensorMap dq_tile, dk_tile, dv_tile;
     const long long dqs[3] = {g.ltot * g.Hq * g.D, (long long)g.Hq * g.D, g.D};
     const long long dks[3] = {g.ltot * g.Hkv * g.D, (long long)g.Hkv * g.D, g.D};
-    if (!encode_map(&dq_tile, dq, bf, p, g.Hq, g.D, dqs, plan.box_q) ||
-        !encode_map(&dk_tile, dk, bf, p, g.Hkv, g.D, dks, plan.box_q) ||
-        !encode_map(&dv_tile, dv, bf, p, g.Hkv, g.D, dks, plan.box_q))
+    if (!encode_map(&dq_tile, dq, bf, p, g.Hq, g.D, dqs, plan.box_q, false, false, true) ||
+        !encode_map(&dk_tile, dk, bf, pk, g.Hkv, g.D, dks, key_plan.box_q, false, false, true) ||
+        !encode_map(&dv_tile, dv, bf, pk, g.Hkv, g.D, dks, key_plan.box_q, false, false, true))
         return -2;
     ek_chunk = k_chunk; ev_chunk = v_chunk;      // placeholders when there are no additional tokens
     if (g.n_extra > 0 && (!encode_extra_map(&ek_chunk, ek, bf, g.B, g.n_extra, g.Hkv, g.D, kCols, p.split_heads) ||
@@ -915,29 +914,33 @@ int launch_bwd(int dtype, const Geo& g, const Plan& plan, const void* q, const v
         tc_count_launch();
     }
 
-    int ngroups = 1;
-    for (int a = 0; a < 3; ++a) ngroups *= p.dil[a];
     const dim3 grid_q(persistent_grid(p.work_q, DH == 64 ? 2 : 1));
-    const dim3 grid_k(persistent_grid(p.work_kv, DH == 64 ? 2 : 1));
-    auto launch = [&](auto inner, auto shorter) {
+    const dim3 grid_k(persistent_grid(pk.work_kv, DH == 64 ? 2 : 1));
+    auto launch = [&](auto key_side, auto inner, auto shorter) {
         constexpr int kInner = decltype(inner)::value;
         constexpr bool kShort = decltype(shorter)::value;
-        ensure_dynamic_smem((const void*)tc_bwd_kernel<DH, BF16, false, kInner, kShort>, Smem::kTotal);
-        ensure_dynamic_smem((const void*)tc_bwd_kernel<DH, BF16, true, kInner, kShort>, Smem::kTotal);
-        tc_bwd_kernel<DH, BF16, false, kInner, kShort><<<grid_q, kThreads, Smem::kTotal, s>>>(
-            q_tile, do_tile, k_chunk, v_chunk, ek_chunk, ev_chunk, dq_tile, dq_tile, p, lse_k, delta_k, (uint16_t*)dq, nullptr);
-        tc_count_launch();
-        tc_bwd_kernel<DH, BF16, true, kInner, kShort><<<grid_k, kThreads, Smem::kTotal, s>>>(
-            k_tile, v_tile, q_chunk, do_chunk, ek_chunk, ev_chunk, dk_tile, dv_tile, key_plan.p, lse_k, delta_k, (uint16_t*)dk, (uint16_t*)dv);
+        constexpr bool kKey = decltype(key_side)::value;
+        auto* kernel = tc_bwd_kernel<DH, BF16, kKey, kInner, kShort>;
+        ensure_dynamic_smem((const void*)kernel, Smem::kTotal);
+        if constexpr (kKey)
+            kernel<<<grid_k, kThreads, Smem::kTotal, s>>>(k_tile, v_tile, q_chunk, do_chunk, ek_chunk, ev_chunk, dk_tile, dv_tile, pk, lse_k,
+                                                          delta_k, (uint16_t*)dk, (uint16_t*)dv);
+        else
+            kernel<<<grid_q, kThreads, Smem::kTotal, s>>>(q_tile, do_tile, k_chunk, v_chunk, ek_chunk, ev_chunk, dq_tile, dq_tile, p, lse_k,
+                                                          delta_k, (uint16_t*)dq, nullptr);
         tc_count_launch();
     };
-    auto by_short = [&](auto inner) {
-        if (g.D <= DH - 32) launch(inner, std::true_type{});
-        else launch(inner, std::false_type{});
+    auto by_short = [&](auto key_side, auto inner) {
+        if (g.D <= DH - 32) launch(key_side, inner, std::true_type{});
+        else launch(key_side, inner, std::false_type{});
     };
-    if (p.cb[2] == 16) by_short(std::integral_constant<int, 16>{});
-    else if (p.cb[2] == 32) by_short(std::integral_constant<int, 32>{});
-    else by_short(std::integral_constant<int, 0>{});
+    auto by_inner = [&](auto key_side, const TcParams& of) {
+        if (of.cb[2] == 16) by_short(key_side, std::integral_constant<int, 16>{});
+        else if (of.cb[2] == 32) by_short(key_side, std::integral_constant<int, 32>{});
+        else by_short(key_side, std::integral_constant<int, 0>{});
+    };
+    by_inner(std::false_type{}, p);
+    by_inner(std::true_type{}, pk);
     cudaError_t err = cudaGetLastError();
     // The additional tokens' own gradients sum over every query of the sample: SIMT kernel.
     if (err == cudaSuccess && g.n_extra > 0)
@@ -981,17 +984,19 @@ int tc_fused_bwd(int dtype, const Geo& g_in, const void* q, const void* k, const
         ex.lse_full = reinterpret_cast<float*>(base + align256(rows_full * 4));
         ex.dout_full = base + 2 * align256(rows_full * 4);
     }
-    Plan plan;
-    if (const int rc = make_plan(g, plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return rc;
+    Plan plan, key_plan;
+    if (const int rc = make_packed_plan(g, plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return rc;
+    if (const int rc = make_plan(g, key_plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return rc;
+    fit_key_boxes(key_plan);
     if (g.B == 0) return 0;
     if (g.Hq > 65535 || g.B > 65535) return -2;
     float* delta = reinterpret_cast<float*>(workspace);
     const Expanded* exp = strided ? &ex : nullptr;
     if (g.D <= 64)
-        return dtype == 2 ? launch_bwd<64, true>(dtype, g, plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp)
-                          : launch_bwd<64, false>(dtype, g, plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp);
-    return dtype == 2 ? launch_bwd<128, true>(dtype, g, plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp)
-                      : launch_bwd<128, false>(dtype, g, plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp);
+        return dtype == 2 ? launch_bwd<64, true>(dtype, g, plan, key_plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp)
+                          : launch_bwd<64, false>(dtype, g, plan, key_plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp);
+    return dtype == 2 ? launch_bwd<128, true>(dtype, g, plan, key_plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp)
+                      : launch_bwd<128, false>(dtype, g, plan, key_plan, q, k, v, ek, ev, dek, dev, out, lse, dout, dlse, dq, dk, dv, delta, s, exp);
 }
 
 // Scratch of the strided backward (full-resolution delta, lse and dout); sized for every 16-bit strided

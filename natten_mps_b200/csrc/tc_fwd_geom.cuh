@@ -28,8 +28,9 @@ struct Cursor {
         w = w0;
         const unsigned hb = w0 / P.per_head;
         bx = w0 - hb * P.per_head;
-        b = (int)(hb / (unsigned)P.Hq);
-        h = (int)(hb - (unsigned)b * (unsigned)P.Hq);
+        const unsigned heads = (unsigned)P.Hq >> P.pack_log;     // h counts groups of 1 << pack_log heads
+        b = (int)(hb / heads);
+        h = (int)(hb - (unsigned)b * heads);
         dq = step / P.per_head;
         dr = step - dq * P.per_head;
     }
@@ -40,7 +41,7 @@ struct Cursor {
         int dh = (int)dq;
         if (bx >= P.per_head) { bx -= P.per_head; ++dh; }
         h += dh;
-        while (h >= P.Hq) { h -= P.Hq; ++b; }
+        while (h >= P.Hq >> P.pack_log) { h -= P.Hq >> P.pack_log; ++b; }
     }
 };
 
@@ -51,8 +52,8 @@ __device__ __forceinline__ void fwd_tile(const TcParams& P, const Cursor& cur, i
 {
     const unsigned bx = cur.bx;
     T.b = cur.b;
-    T.h = cur.h;
-    T.hk = (int)fast_div((unsigned)cur.h, P.group_mul);
+    T.h = cur.h << P.pack_log;
+    T.hk = (int)fast_div((unsigned)T.h, P.group_mul);
     bool active = cta_geometry(P, bx, T.b, T.rg, T.origin, T.Lp);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -113,7 +114,7 @@ __device__ __forceinline__ long long row_geometry(const TcParams& P, const FwdTi
         }
     }
     if (!valid_q) { e[0] = f[0]; e[1] = f[1]; e[2] = f[2]; }
-    return ((long long)T.b * P.otot + oflat) * P.Hq + T.h;
+    return ((long long)T.b * P.otot + oflat) * P.Hq + T.h + (row & ((1 << P.pack_log) - 1));
 }
 
 // What a softmax thread needs to know about its row is separable: along every axis the query's coordinate alone decides its
@@ -157,8 +158,9 @@ __device__ __forceinline__ bool publish_tile(const TcParams& P, const Cursor& cu
     }
     if (lane == 2) {
         H->b = cur.b;
-        H->h = cur.h;
-        H->hk = (int)fast_div((unsigned)cur.h, P.group_mul);
+        const int h = cur.h << P.pack_log;
+        H->h = h;
+        H->hk = (int)fast_div((unsigned)h, P.group_mul);
         H->nnb = nnb;
         H->nch = nnb + ((P.n_extra + (1 << chunk_log) - 1) >> chunk_log);    // then the additional tokens, one chunk at a time
         H->active = 1;
@@ -208,9 +210,9 @@ __device__ __forceinline__ long long row_from_tables(const TcParams& P, const ui
 {
     const FwdTile* T = reinterpret_cast<const FwdTile*>(slot);
     const int4* ent = reinterpret_cast<const int4*>(slot + kEntOff);
-    const int r01 = row >> P.tile2_log;
+    const int head = row & ((1 << P.pack_log) - 1), pos = row >> P.pack_log, r01 = pos >> P.tile2_log;
     const int4 e0 = ent[r01 >> P.tile1_log], e1 = ent[P.tile[0] + (r01 & (P.tile[1] - 1))],
-               e2 = ent[P.tile[0] + P.tile[1] + (row & (P.tile[2] - 1))];
+               e2 = ent[P.tile[0] + P.tile[1] + (pos & (P.tile[2] - 1))];
     const int flags = e0.w & e1.w & e2.w;
     valid_q = flags & 1;
     in_tensor = flags & 2;
@@ -221,7 +223,7 @@ __device__ __forceinline__ long long row_from_tables(const TcParams& P, const ui
     rowmap = T->mapped ? reinterpret_cast<const unsigned long long*>(slot + kMapOff)[r01] : 0ull;
     colbits = T->mapped && valid_q ? (uint32_t)e2.w >> 16 : 0u;
     const long long oflat = ((long long)e0.z * P.O[1] + e1.z) * P.O[2] + e2.z;
-    return ((long long)T->b * P.otot + oflat) * P.Hq + T->h;
+    return ((long long)T->b * P.otot + oflat) * P.Hq + T->h + head;
 }
 
 } // namespace fwdgeom

@@ -266,7 +266,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         mbar_expect_tx(bar_q, kQBytes + ((P.inject == 1 && t == 0) ? 16u : 0u));
 #pragma unroll
                         for (int hf = 0; hf < kHalves; ++hf)
-                            tma_load_heads(sbase + kOffQ + hf * kQHalf, &tmQ, bar_q, P, h, 64 * hf, Q2, Q1, Q0, b);
+                            tma_load_rows(sbase + kOffQ + hf * kQHalf, &tmQ, bar_q, P, h, 64 * hf, Q2, Q1, Q0, b);
                     }
                     int c0 = 0, c1 = 0, c2 = 0;
                     for (int c = 0; c < nch; ++c, ++n) {
@@ -713,10 +713,10 @@ int tc_fused_fwd_small(int dtype, const Geo& g, const void* q, const void* k, co
     if (!tc_eligible(dtype, g, q, k, v, /*allow_stride=*/true)) return -2;
     if (g.n_extra > 0 && ((reinterpret_cast<uintptr_t>(ek) | reinterpret_cast<uintptr_t>(ev)) & 15u)) return -2;
     Plan plan;
-    if (const int rc = make_plan(g, plan, kKeys, /*with_stride=*/true, /*interleave=*/true)) return rc;
+    if (const int rc = make_packed_plan(g, plan, kKeys, /*with_stride=*/true, /*interleave=*/true, /*backward=*/false)) return rc;
     const bool bf16 = dtype == 2;
     CUtensorMap mq, mk, mv, mek, mev;
-    if (!encode_map(&mq, q, bf16, plan.p, g.Hq, g.D, g.qs, plan.box_q, /*query_lattice=*/true) ||
+    if (!encode_map(&mq, q, bf16, plan.p, g.Hq, g.D, g.qs, plan.box_q, /*query_lattice=*/true, /*interleaved=*/false, /*rows=*/true) ||
         !encode_map(&mk, k, bf16, plan.p, g.Hkv, g.D, g.ks, plan.box_kv, false, /*interleaved=*/true) ||
         !encode_map(&mv, v, bf16, plan.p, g.Hkv, g.Dv, g.vs, plan.box_kv, false, /*interleaved=*/true))
         return -2;

@@ -51,6 +51,10 @@ struct TcParams {
     // such maps are in use.  hpitch: channels from head to head.  (8 x 28 x 28, 3 x 5 x 5, 6 heads of 32, batch 2, bf16, against the
     // general kernels that took these before: forward 351 -> 33 us, backward 888 -> 140.)
     int shared_box, hpitch;
+    // Grouped heads on the query side: a row tile holds 1 << pack_log query heads of one KV head, 128 >> pack_log positions of each
+    // (row = position << pack_log | head).  They share their keys, so the column box is shorter by the positions left out.
+    // q_split: the maps of the rows have the head as an axis of their own.
+    int pack_log, q_split;
     long long wait_budget; // cycles a barrier wait may take before the CTA gives up
     int inject;            // test hook: 1 = the forward's first query barrier expects bytes that never arrive
     // Output stride (forward only).  Inside dilation group r of an axis the queries sit at the
@@ -142,11 +146,18 @@ __device__ __forceinline__ void tma_load_heads(uint32_t dst, const CUtensorMap* 
     if (P.split_heads) tma_load_5d(dst, map, bar, ch, h, c1, c2, c4);
     else tma_load_5d(dst, map, bar, h * P.hpitch + ch, c1, c2, c3, c4);
 }
+// Rows of a query tile, 64 channels of them: the head axis of its own covers the tile's heads.
+__device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* map, uint32_t bar, const TcParams& P,
+                                              int h, int ch, int c1, int c2, int c3, int c4)
+{
+    if (P.q_split) tma_load_5d(dst, map, bar, ch, h, c1, c2, c4);
+    else tma_load_5d(dst, map, bar, h * P.hpitch + ch, c1, c2, c3, c4);
+}
 // Tile store at head * dh + channel block, dh the kernel's (padded) head dim, a power of two.
 __device__ __forceinline__ void tma_store_heads(const CUtensorMap* map, uint32_t src, const TcParams& P, int dh, int c0,
                                                 int c1, int c2, int c3, int c4)
 {
-    if (P.split_heads) tma_store_5d(map, src, c0 & (dh - 1), c0 / dh, c1, c2, c4);
+    if (P.q_split) tma_store_5d(map, src, c0 & (dh - 1), c0 / dh, c1, c2, c4);
     else tma_store_5d(map, src, c0, c1, c2, c3, c4);
 }
 
@@ -177,9 +188,10 @@ __host__ __device__ __forceinline__ void inverse_range(int n, int L, int K, int 
     if (exact && n > last + K - 1) qhi = qlo - 1;
 }
 
-// Row r (0..127) of the tile -> offsets along the three axes.
+// Row r (0..127) of the tile -> offsets along the three axes (and head r & ((1 << pack_log) - 1) of the tile's).
 __device__ __forceinline__ void row_offsets(const TcParams& P, int r, int (&ri)[3])
 {
+    r >>= P.pack_log;
     ri[2] = r & (P.tile[2] - 1);
     ri[1] = (r >> P.tile2_log) & (P.tile[1] - 1);
     ri[0] = r >> (P.tile2_log + P.tile1_log);
@@ -409,13 +421,16 @@ inline int pow2ceil(int x) { return 1 << ilog2(x); }
 // Internal geometry always has three axes; lower ranks get leading axes of size 1.
 struct Plan {
     TcParams p;
+    long long cost;          // of the tile shape, see make_plan
     int box_q[3], box_kv[3];
 };
 
 // Pick the row-tile shape (128 rows) whose column box needs the fewest chunks of `chunk` columns.
 // 0, -2 where the tensor-core kernels do not cover the geometry (another kernel serves the call), or the CUDA error that
 // kept a plan they do cover from being made (the call has to report it).
-inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_stride = false, bool interleave = false, bool backward = false)
+// pack_log: see TcParams (ranks 1 and 2).
+inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_stride = false, bool interleave = false, bool backward = false,
+                     int pack_log = 0)
 {
     TcParams& p = plan.p;
     const int pad = 3 - g.rank;
@@ -443,9 +458,10 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
     }
     p.otot = (long long)p.O[0] * p.O[1] * p.O[2];
     long long best = -1, best_cost = 0;
-    for (int t2 = 1; t2 <= 128; t2 *= 2)
-        for (int t1 = 1; t1 * t2 <= 128; t1 *= 2) {
-            const int t0 = 128 / (t1 * t2);
+    const int positions = kTileRows >> pack_log;
+    for (int t2 = 1; t2 <= positions; t2 *= 2)
+        for (int t1 = 1; t1 * t2 <= positions; t1 *= 2) {
+            const int t0 = positions / (t1 * t2);
             const int t[3] = {t0, t1, t2};
             bool fits = true;
             for (int a = 0; a < 3; ++a) {
@@ -483,6 +499,7 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
             }
         }
     if (best < 0) return -2;
+    plan.cost = best_cost;
     p.cb0_log = ilog2(p.cb[0]); p.cb1_log = ilog2(p.cb[1]); p.cb2_log = ilog2(p.cb[2]);
     p.tile1_log = ilog2(p.tile[1]); p.tile2_log = ilog2(p.tile[2]);
     p.nchunks = (int)best;
@@ -509,7 +526,9 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
         // the first (slowest) axis that needs several chunks is the one along which the warps of a
         // tile differ; tensor maps take element strides up to 8
         for (int a = 0; a < 3; ++a) {
-            if (p.nchunk[a] <= 1) continue;
+            // (an axis with one row a chunk has nothing to interleave: the forward goes on to the next; 16 x 32 x 32, 3 x 7 x 7, causal
+            // frames, 8 heads of 64, batch 2: 117 -> 104 us.  The backward got slower that way, 129 -> 137 and 166 -> 175)
+            if (p.nchunk[a] <= 1 || (!backward && p.cb[a] == 1)) continue;
             const int il = p.nchunk[a];
             if (p.dil[a] * il <= 8 && p.cb[a] * p.dil[a] * il <= 256) {
                 p.il[a] = il;
@@ -521,6 +540,8 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
     }
     p.dreal = g.D;
     p.split_heads = (g.D != 64 && g.D != 128 && g.rank < 3) ? 1 : 0;
+    p.pack_log = pack_log;
+    p.q_split = p.split_heads || pack_log > 0;
     p.shared_box = g.D != 64 && g.D != 128 && !p.split_heads;
     p.hpitch = g.D;
     p.group_mul = g.group >= 2 ? (unsigned)((0x100000000ull + g.group - 1) / g.group) : 0u;
@@ -530,7 +551,7 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
     for (int a = 0; a < 3; ++a) p.ngroups *= p.grp_n[a];
     p.per_head = (unsigned)p.ntiles * (unsigned)p.ngroups;
     if ((long long)p.per_head * g.B * g.Hq >= (1ll << 31)) return -2;
-    p.work_q = p.per_head * (unsigned)g.B * (unsigned)g.Hq;
+    p.work_q = p.per_head * (unsigned)g.B * (unsigned)(g.Hq >> pack_log);
     p.work_kv = p.per_head * (unsigned)g.B * (unsigned)g.Hkv;
     p.scale_log2 = (float)(g.scale * 1.4426950408889634);
     p.scale = (float)g.scale;
@@ -543,6 +564,20 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
     if (err == cudaSuccess) err = status_host_ptr(p.status_host);
     if (err != cudaSuccess) cudaGetLastError();                 // reported here, not by the next launch
     return (int)err;
+}
+
+// The same with as many query heads of a KV head in a row tile as need the fewest chunks (ties: the fewest heads).  Measured, bf16,
+// one | packed heads a tile, window of 255 (6 chunks of 64 | 5), 16 heads of 128 on 4: 8191 causal, batch 2, forward 84.6 | 74.7 us;
+// 8 lengths up to 16384, forward 482 | 423, query side of the backward 580 | 515.
+inline int make_packed_plan(const Geo& g, Plan& plan, int chunk, bool with_stride, bool interleave, bool backward)
+{
+    const int rc = make_plan(g, plan, chunk, with_stride, interleave, backward);
+    if (rc || g.rank > 2) return rc;
+    for (int log = 1; log <= 3 && g.group % (1 << log) == 0; ++log) {
+        Plan other;
+        if (make_plan(g, other, chunk, with_stride, interleave, backward, log) == 0 && other.cost < plan.cost) plan = other;
+    }
+    return 0;
 }
 
 // Column count of an interleaved axis for key tiles.  A key next to a clamped edge is read by every query of the edge, so a
@@ -592,7 +627,7 @@ inline bool encode_16bit(CUtensorMap* map, const void* base, bool bf16, const cu
 
 // 5-D map over [B, X0, X1, X2, heads*D] (innermost first in the arrays below).
 inline bool encode_map(CUtensorMap* map, const void* base, bool bf16, const TcParams& p, int heads, int dh,
-                const long long strides[3], const int box[3], bool query_lattice = false, bool interleaved = false)
+                const long long strides[3], const int box[3], bool query_lattice = false, bool interleaved = false, bool rows = false)
 {
     const cuuint64_t tok = (cuuint64_t)strides[1] * 2;
     cuuint64_t dims[5] = {(cuuint64_t)heads * dh, (cuuint64_t)p.L[2], (cuuint64_t)p.L[1], (cuuint64_t)p.L[0], (cuuint64_t)p.B};
@@ -603,11 +638,11 @@ inline bool encode_map(CUtensorMap* map, const void* base, bool bf16, const TcPa
         for (int a = 0; a < 3; ++a) es[3 - a] *= (cuuint32_t)p.qstep[a];
     if (interleaved)                                             // chunk columns are il sub-grid positions apart
         for (int a = 0; a < 3; ++a) es[3 - a] *= (cuuint32_t)p.il[a];
-    if (p.split_heads) {                                         // [D, H, X2, X1, B]; the leading spatial axis has extent 1
+    if (p.split_heads || (rows && p.q_split)) {                  // [D, H, X2, X1, B]; the leading spatial axis has extent 1
         if (p.L[0] != 1) return false;
         dims[0] = (cuuint64_t)dh; dims[1] = (cuuint64_t)heads; dims[2] = (cuuint64_t)p.L[2]; dims[3] = (cuuint64_t)p.L[1];
         gstr[0] = (cuuint64_t)strides[2] * 2; gstr[1] = tok; gstr[2] = tok * p.L[2];
-        bx[1] = 1; bx[2] = (cuuint32_t)box[2]; bx[3] = (cuuint32_t)box[1];
+        bx[1] = rows ? 1u << p.pack_log : 1u; bx[2] = (cuuint32_t)box[2]; bx[3] = (cuuint32_t)box[1];
         const cuuint32_t e2 = es[1], e1 = es[2];
         es[1] = 1; es[2] = e2; es[3] = e1;
     }

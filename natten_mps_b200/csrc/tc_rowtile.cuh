@@ -47,9 +47,9 @@ __device__ __forceinline__ void bwd_tile_setup(const TcParams& P, unsigned work,
 {
     const unsigned hb = work / P.per_head;
     const unsigned bx = work - hb * P.per_head;
-    const unsigned H = (unsigned)(kKeySide ? P.Hkv : P.Hq);
+    const unsigned H = (unsigned)(kKeySide ? P.Hkv : P.Hq >> P.pack_log);
     T.b = (int)(hb / H);
-    T.hy = (int)(hb - (unsigned)T.b * H);
+    T.hy = (int)(hb - (unsigned)T.b * H) << (kKeySide ? 0 : P.pack_log);
     T.active = cta_geometry(P, bx, T.b, T.rg, T.origin, T.Lp);
     T.nchunks = 1;
     if (T.active) {
@@ -78,8 +78,8 @@ __device__ __forceinline__ void bwd_tile_setup(const TcParams& P, unsigned work,
 template <bool kKeySide>
 __device__ __forceinline__ bool publish_tile(const TcParams& P, unsigned work, bool rows16, int lane, TileHead* H)
 {
-    const unsigned hb = work / P.per_head, heads = (unsigned)(kKeySide ? P.Hkv : P.Hq);
-    const int b = (int)(hb / heads), hy = (int)(hb - (unsigned)b * heads), a = lane < 2 ? lane : 2;
+    const unsigned hb = work / P.per_head, heads = (unsigned)(kKeySide ? P.Hkv : P.Hq >> P.pack_log);
+    const int b = (int)(hb / heads), hy = (int)(hb - (unsigned)b * heads) << (kKeySide ? 0 : P.pack_log), a = lane < 2 ? lane : 2;
     int rg, origin, Lp;
     if (!__all_sync(0xffffffffu, lane_geometry(P, work - hb * P.per_head, b, a, rg, origin, Lp))) return false;
     const int last = origin + P.tile[a] - 1 < Lp - 1 ? origin + P.tile[a] - 1 : Lp - 1;

@@ -58,3 +58,46 @@ def test_forward_tables_varlen(lens, dim):
     assert float((got.float() - want.float()).abs().max()) <= 2e-2
     for b, n in enumerate(lens):
         assert not got[b, n:].any()
+
+
+# size, kernel, causal, (query heads, KV heads), dim: tiles of 2, 4 or 8 heads, ragged ends, one chunk and many
+PACKED = [((200,), (15,), (0,), (4, 2), 64), ((333,), (63,), (1,), (8, 1), 128), ((700,), (255,), (0,), (4, 1), 128),
+          ((129,), (33,), (1,), (6, 3), 64), ((97,), (17,), (0,), (16, 2), 32), ((23, 37), (5, 11), (0, 0), (8, 2), 64),
+          ((19, 30), (9, 9), (0, 1), (4, 2), 128), ((40, 33), (3, 21), (0, 0), (8, 1), 96)]
+
+
+@pytest.mark.parametrize("shape", PACKED, ids=lambda s: "x".join(map(str, s[0] + s[1] + s[3])) + f"d{s[-1]}")
+@pytest.mark.parametrize("extra", [0, 5])
+def test_grouped_heads_packed(shape, extra):
+    size, kernel, causal, (hq, hkv), dim = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(size))
+    t = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.float16).requires_grad_(True)
+    q, k, v, do = t(2, *size, hq, dim), t(2, *size, hkv, dim), t(2, *size, hkv, dim), t(2, *size, hq, dim).detach()
+    kw = {"additional_keys": t(2, extra, hkv, dim), "additional_values": t(2, extra, hkv, dim)} if extra else {}
+    op = {1: F.na1d, 2: F.na2d}[len(size)]
+
+    def run():
+        out = op(q, k, v, kernel_size=kernel, is_causal=tuple(bool(c) for c in causal), **kw)
+        return [out, *torch.autograd.grad(out, [q, k, v, *kw.values()], do)]
+
+    for got, want in zip(forced("tc", run), forced("simt", run)):
+        # sums of up to 16 heads x window rounded to fp16 on either side: 2e-2 of the tensor's scale
+        assert float((got.float() - want.float()).abs().max()) <= 2e-2 * max(1.0, float(want.float().abs().max()))
+
+
+@pytest.mark.parametrize("lens", [(300, 9, 128), (129, 300, 33)])
+def test_grouped_heads_packed_varlen(lens):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    t = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16).requires_grad_(True)
+    q, k, v = t(3, 300, 8, 64), t(3, 300, 2, 64), t(3, 300, 2, 64)
+    do = t(3, 300, 8, 64).detach()
+    sizes = torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+    def run():
+        out = F.na1d_varlen(q, k, v, sizes, kernel_size=9)
+        return [out, *torch.autograd.grad(out, [q, k, v], do)]
+
+    for got, want in zip(forced("tc", run), forced("simt", run)):
+        assert float((got.float() - want.float()).abs().max()) <= 2e-2 * max(1.0, float(want.float().abs().max()))
+        for b, n in enumerate(lens):
+            assert not got[b, n:].any()
