@@ -421,7 +421,6 @@ inline int pow2ceil(int x) { return 1 << ilog2(x); }
 // Internal geometry always has three axes; lower ranks get leading axes of size 1.
 struct Plan {
     TcParams p;
-    long long cost;          // of the tile shape, see make_plan
     int box_q[3], box_kv[3];
 };
 
@@ -499,7 +498,6 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
             }
         }
     if (best < 0) return -2;
-    plan.cost = best_cost;
     p.cb0_log = ilog2(p.cb[0]); p.cb1_log = ilog2(p.cb[1]); p.cb2_log = ilog2(p.cb[2]);
     p.tile1_log = ilog2(p.tile[1]); p.tile2_log = ilog2(p.tile[2]);
     p.nchunks = (int)best;
@@ -566,6 +564,18 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
     return (int)err;
 }
 
+// Chunks of a plan's largest box, which never outgrows the tensor, weighted like the tile shapes in make_plan.
+inline long long box_cost(const Plan& plan, bool interleave, bool backward)
+{
+    const TcParams& p = plan.p;
+    long long n = 1;
+    for (int a = 0; a < 3; ++a) {
+        const int lp = (p.L[a] + p.dil[a] - 1) / p.dil[a], box = (p.tile[a] - 1) * p.qstep[a] + p.K[a];
+        n *= ((box < lp ? box : lp) + p.cb[a] - 1) / p.cb[a];
+    }
+    return n * (interleave && p.rank == 2 && p.cb[2] == 16 && !(backward && p.tile[2] < p.K[2]) ? 10 : 12);
+}
+
 // The same with as many query heads of a KV head in a row tile as need the fewest chunks (ties: the fewest heads).  Measured, bf16,
 // one | packed heads a tile, window of 255 (6 chunks of 64 | 5), 16 heads of 128 on 4: 8191 causal, batch 2, forward 84.6 | 74.7 us;
 // 8 lengths up to 16384, forward 482 | 423, query side of the backward 580 | 515.
@@ -575,7 +585,9 @@ inline int make_packed_plan(const Geo& g, Plan& plan, int chunk, bool with_strid
     if (rc || g.rank > 2) return rc;
     for (int log = 1; log <= 3 && g.group % (1 << log) == 0; ++log) {
         Plan other;
-        if (make_plan(g, other, chunk, with_stride, interleave, backward, log) == 0 && other.cost < plan.cost) plan = other;
+        if (make_plan(g, other, chunk, with_stride, interleave, backward, log) == 0 &&
+            box_cost(other, interleave, backward) < box_cost(plan, interleave, backward))
+            plan = other;
     }
     return 0;
 }
