@@ -14,13 +14,13 @@
 // A pass over the columns of K = 7 x 7 costs 23 shared-memory cycles for 32 pairs of which 70 % are needed.
 //
 // Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, against the general SIMT kernels: float32 forward 30 us (185), dQ 38 (236),
-// dK and dV 67 (304); split operators in bf16: scores 25 (93), apply 24 (93), gather 36 (115); in float32: 25 (96), 24 (469),
+// dK and dV 67 (304); split operators in bf16: scores 25 (93), apply 24 (93), gather 31 (115); in float32: 25 (96), 24 (469),
 // 32 (152).
 // What bounds them there: too few warps.  448 CTAs have 444 (forward, dQ), 296 (dK and dV, 245 to 255 registers) or 592 (split)
 // places, 7 to 12 warps on an SM.  Schedulers issue in 44, 41, 33 % of the active cycles (forward, dQ, dK and dV) and in 49, 38,
 // 36 % (scores, apply, gather); the largest stalls are the barriers around a chunk, whose loads nothing overlaps, then the
-// latency of dependent instructions, in apply and gather also that of the weights.  DRAM is at 2 to 8 %.  Apply and gather spill
-// 16 to 52 bytes at the 128 registers that four CTAs on an SM leave them.
+// latency of dependent instructions, in apply and gather also that of the weights.  DRAM is at 2 to 8 %.  The weights are
+// half of the gather: 32 lanes read 32 sectors, which the few KB of L1 beside the staged columns do not keep.
 //
 // Rows are queries and columns keys, or the other way round (key side: dK, dV; columns = the queries that attend to a key,
 // a contiguous range per axis).  Fixed order of summation everywhere, no atomics.
@@ -48,7 +48,9 @@ using tcplan::pack2;
 
 constexpr int kWarpsF = 4;
 constexpr int kThreadsF = 32 * kWarpsF;
-constexpr int kAheadF = 4;               // pairs of weights a lane fetches ahead
+// Pairs of weights a lane fetches ahead.  With more the gather spills more at the 128 registers that four CTAs leave a thread: 56 x 56, 7 x 7,
+// head dim 32, bf16, two gathers 61.4 us with 2, 71.5 with 4, 84 with 8 (apply 49.1, 49.8, 53.1); three CTAs with 7: 94.7 and 59.6.
+constexpr int kAheadF = 2;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 
 // A tensor as the kernels see it: element strides of batch, token, head.
