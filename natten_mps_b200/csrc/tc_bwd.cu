@@ -23,8 +23,9 @@
 // What bounds it: the round trip of a chunk (threads 700 to 1000 cycles, then the issuing warps and the products, 1300 to 1800)
 // with two tiles in flight, the tensor pipe busy for 45 % of it.  With one helper that loaded and did the geometry, tables held up
 // the row tiles and the loads.  Measured before | now (us, kernel alone, query side and key side): 64 x 64, 7 x 7, 8 heads of 64,
-// batch 8: 68.6, 87.5 | 64.6, 83.8; 128 x 128, 13 x 13, dilation 2, batch 4: 219, 278 | 199, 264; 16 x 32 x 32, 3 x 7 x 7 causal,
-// batch 2: 146, 187 | 135, 175; 8 lengths up to 16384, window 255, 16 heads of 128 on 4: 722, 712 | 578, 606.
+// batch 8: 68.6, 87.5 | 61.3, 81.4; 128 x 128, 13 x 13, dilation 2, batch 4: 219, 278 | 199, 254; 16 x 32 x 32, 3 x 7 x 7 causal,
+// batch 2: 146, 187 | 131, 168; 8 lengths up to 16384, window 255, 16 heads of 128 on 4: 722, 712 | 580, 606 (query side 513 with
+// heads packed, see make_packed_plan).
 // TMEM: S [0,64)  dP [64,128)  acc1 [128,128+D)  acc2 [128+D,128+2D); head dim 128: second S [384,448) and
 // dP [448,512).  The 16-bit P and dS that feed the accumulating MMAs overwrite the first half of the S / dP
 // columns of the piece they were computed from (same warp, after it has read them).

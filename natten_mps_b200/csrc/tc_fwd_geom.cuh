@@ -118,7 +118,7 @@ __device__ __forceinline__ long long row_geometry(const TcParams& P, const FwdTi
 }
 
 // What a softmax thread needs to know about its row is separable: along every axis the query's coordinate alone decides its
-// position, whether it exists and its window.  The loader writes one entry per (axis, coordinate of the tile) a tile ahead,
+// position, whether it exists and its window.  The geometry warp writes one entry per (axis, coordinate of the tile) a tile ahead,
 // tile[0] + tile[1] + tile[2] of them instead of 128 rows x 3 axes.  A slot: FwdTile, row maps, axis entries.
 constexpr int kMapOff = 160, kEntOff = kMapOff + 8 * kTileRows, kTabBytes = kEntOff + 16 * (kTileRows + 2);
 static_assert(sizeof(FwdTile) <= kMapOff, "no room for the tile in front of its tables");

@@ -23,9 +23,9 @@
 // issuing warp -> P V and the next S, about 2800 cycles of which the softmax is 1500; four tiles in flight per SM share the
 // gaps.  So whatever is not the chain is kept off the issuing warp and the softmax warps.  Measured on one B200 (us), one warp that
 // loaded, issued and did the geometry | loads and geometry apart (kernel alone): 64 x 64, 7 x 7, 8 heads of 64, batch 8,
-// bf16 61.7 | 53.5; 128 x 128, 13 x 13, dilation 2, batch 4 196 | 177; 16 x 32 x 32, 3 x 7 x 7, causal frames, batch 2 137 | 120;
-// 135 x 241, 7 x 9, 6 heads of 32, batch 2, fp16 80 | 70; 8191 causal, window 255, 16 heads of 128 on 4, batch 2 98 | 82;
-// 28 x 28, 8 heads of 32 12.6 | 12.2.
+// bf16 61.7 | 50.3; 128 x 128, 13 x 13, dilation 2, batch 4 196 | 175; 16 x 32 x 32, 3 x 7 x 7, causal frames, batch 2 137 | 117 (104 with
+// its chunks interleaved, see make_plan); 135 x 241, 7 x 9, 6 heads of 32, batch 2, fp16 80 | 69; 8191 causal, window 255, 16 heads of
+// 128 on 4, batch 2 98 | 84.6 (74.5 with heads packed, see make_packed_plan).
 //
 // TMEM columns: head dim 64: S [0,64) (P over [0,32)), O [64,128);
 //               head dim 128: S of even chunks [0,64), of odd chunks [64,128), O [128,256).
@@ -73,7 +73,7 @@ struct FwdSmall {
     static constexpr uint32_t kTmemCols = kTwoS ? 256 : 128;        // S, O, rounded up to a power of two
     static constexpr int kPerSm = kTwoS ? 2 : 4;
     // 65536 / kPerSm / kThreads registers a thread at launch, 64 or 128; the helpers hand what they do not need to the softmax
-    // warps, which spill with less than 88 (32 | 96, where the helpers spill: 59.5 us instead of 53.5; 48 | 80: 54.0)
+    // warps, which spill with less than 88 (32 | 96, where the helpers spill: 64 x 64, 7 x 7 53.7 us instead of 49.8)
     static constexpr int kHelperRegs = kTwoS ? 104 : 40, kSoftmaxRegs = kTwoS ? 152 : 88;
     // There K has to be a chunk ahead of V, so the two are loaded and freed apart; with one score buffer they come and go together.
     static constexpr bool kSplitKV = kTwoS;
