@@ -987,7 +987,8 @@ int tc_fused_bwd(int dtype, const Geo& g_in, const void* q, const void* k, const
     }
     Plan plan, key_plan;
     if (const int rc = make_packed_plan(g, plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return rc;
-    if (const int rc = make_plan(g, key_plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return rc;
+    if (plan.p.pack_log == 0) key_plan = plan;   // (a plan is a microsecond or two of a small call's host time)
+    else if (const int rc = make_plan(g, key_plan, kCols, /*with_stride=*/false, /*interleave=*/true, /*backward=*/true)) return rc;
     fit_key_boxes(key_plan);
     if (g.B == 0) return 0;
     if (g.Hq > 65535 || g.B > 65535) return -2;

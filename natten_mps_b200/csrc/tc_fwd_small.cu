@@ -15,7 +15,7 @@
 // exceeds it by 2^60 (2^14 for fp16); O, the row sum and the probabilities already stored for the
 // chunk are then rescaled.  Up to head dim 64 four independent CTAs per SM give the schedulers sixteen
 // softmax warps in different phases of their tiles, which is what hides the TMEM / barrier / MMA latencies
-// (128 TMEM columns and 49 KB of shared memory per CTA).  Above it only two CTAs fit (256 columns, 97 KB),
+// (128 TMEM columns and 55 KB of shared memory per CTA).  Above it only two CTAs fit (256 columns, 103 KB),
 // so the scores get two buffers there: S(c + 1) is computed while the threads work on S(c).
 //
 // Eight warps: four of softmax (a warpgroup), one that issues the products, one that loads, one for the geometry, one idle (a
