@@ -390,6 +390,10 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 const int total = H->total, nc0 = H->nc[0], nc1 = H->nc[1], nc2 = H->nc[2];
                 // this lane's columns j = lane and lane + 32 of chunk (0, 0, 0): position along the axes, relative to the sub-grid
                 int at[kCols / 32][3], Lp[3], c0 = 0, c1 = 0, c2 = 0;
+                long long row_k[kCols / 32];     // their rows' distance from the sub-grid's origin
+                auto row_at = [&](int x0, int x1, int x2) {
+                    return (((long long)(P.dil[0] * x0) * P.L[1] + P.dil[1] * x1) * P.L[2] + P.dil[2] * x2) * P.Hq;
+                };
 #pragma unroll
                 for (int a = 0; a < 3; ++a) Lp[a] = H->Lp[a];
 #pragma unroll
@@ -398,6 +402,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     at[k][0] = H->boxlo[0] + chunk_coord(P, 0, 0, j >> (P.cb2_log + P.cb1_log));
                     at[k][1] = H->boxlo[1] + chunk_coord(P, 1, 0, (j >> P.cb2_log) & (P.cb[1] - 1));
                     at[k][2] = H->boxlo[2] + chunk_coord(P, 2, 0, j & (P.cb[2] - 1));
+                    row_k[k] = row_at(at[k][0], at[k][1], at[k][2]);
                 }
                 // statistics of the sub-grid's origin for the first query head
                 const long long origin = ((long long)H->b * P.ltot + ((long long)H->rg[0] * P.L[1] + H->rg[1]) * P.L[2] + H->rg[2]) * P.Hq + H->hy * P.group;
@@ -405,13 +410,14 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 float nl[kCols / 32], nd[kCols / 32];
                 auto fetch = [&]() {
                     const int s0 = chunk_coord(P, 0, c0, 0), s1 = chunk_coord(P, 1, c1, 0), s2 = chunk_coord(P, 2, c2, 0);
+                    const long long step = row_at(s0, s1, s2);           // linear in the coordinates: the same for every column
 #pragma unroll
                     for (int k = 0; k < kCols / 32; ++k) {
                         const int q0 = at[k][0] + s0, q1 = at[k][1] + s1, q2 = at[k][2] + s2;
                         nl[k] = 0.f;
                         nd[k] = 0.f;
                         if (q0 >= 0 && q0 < Lp[0] && q1 >= 0 && q1 < Lp[1] && q2 >= 0 && q2 < Lp[2]) {
-                            const long long row = (((long long)(P.dil[0] * q0) * P.L[1] + P.dil[1] * q1) * P.L[2] + P.dil[2] * q2) * P.Hq;
+                            const long long row = row_k[k] + step;
                             nl[k] = lse_h[row];
                             nd[k] = delta_h[row];
                         }
@@ -453,7 +459,9 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
         for (unsigned t = 0;; ++t) {
             // ---- this thread's row, from the geometry warp's tables ----
             ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
-            if (any_of_compute(!ok)) break;      // all of them or none: the stores below are behind a barrier of theirs
+// All of them or none where the stores are behind a barrier of theirs; without one a warp goes by itself.
+            const bool apart = kShort && P.shared_box;
+            if (apart ? !__all_sync(0xffffffffu, ok) : any_of_compute(!ok)) break;
             const uint8_t* tab = tab_slot(t);
             const TileHead* H = reinterpret_cast<const TileHead*>(tab);
             const int total = H->total;
