@@ -26,6 +26,13 @@
 // batch 8: 68.6, 87.5 | 61.3, 81.4; 128 x 128, 13 x 13, dilation 2, batch 4: 219, 278 | 199, 254; 16 x 32 x 32, 3 x 7 x 7 causal,
 // batch 2: 146, 187 | 131, 168; 8 lengths up to 16384, window 255, 16 heads of 128 on 4: 722, 712 | 580, 606 (query side 513 with
 // heads packed, see make_packed_plan).
+// Chunks of any shape (kInner = 0) are bound by how fast instructions arrive: the validity words and the unrolled halves are long code
+// that six roles share the instruction caches with.  When the geometry moved to a warp of its own, the key side of 3 x 3 x 3 windows
+// (9 short chunks a tile) went from 254 to 279 us (286 to 322 with padded heads; 12 x 40 x 40, 8 heads of 64 | 32, batch 2) with fewer
+// instructions executed, warps waiting for one four times as long (0.85 -> 3.3 of every issue).  One copy of the halves, of the two
+// outputs of the epilogue and of a segment of the validity words there: 238 and 264 (8 x 28 x 28 115 -> 98; 3 x 5 x 5 270 -> 263).  The
+// query side, one accumulator, keeps both halves: 188 and 189, with one copy 192 and 194; so does head dim 128, with half as many warps on
+// an SM (8 lengths up to 16384, window 255, key side 600, with one copy 620).
 // TMEM: S [0,64)  dP [64,128)  acc1 [128,128+D)  acc2 [128+D,128+2D); head dim 128: second S [384,448) and
 // dP [448,512).  The 16-bit P and dS that feed the accumulating MMAs overwrite the first half of the S / dP
 // columns of the piece they were computed from (same warp, after it has read them).
@@ -583,10 +590,11 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 tc_fence_after();
                 const float row_lse2 = -raw_lse * 1.4426950408889634f, row_delta = -raw_delta * P.scale;   // negated, pre-scaled addends
                 const uint64_t scale_log2_2 = pack2(P.scale_log2, P.scale_log2), scale_2 = pack2(P.scale, P.scale);
-#pragma unroll
+                // (one copy of the code on the key side of chunks of any shape: see the top of this file)
+#pragma unroll(kInner > 0 || !kKeySide || DH == 128 ? 2 : 1)
                 for (int half = 0; half < 2; ++half) {               // 16 columns at a time
                     uint32_t pk_p[8], pk_ds[8];
-                    if (any[half]) {
+                    if (half == 0 ? any[0] : any[1]) {
                         const float* stp = stats + (g % kStages) * 128 + col0(half);
                         const float4* st4 = reinterpret_cast<const float4*>(stp);
                         uint32_t s[16], dp[16];
@@ -677,7 +685,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             // threads go on.  The tile is reused only after that thread has seen the store finish reading it.
             const bool live = valid_row && ok;
             const int row = quad * 32 + lane;
-#pragma unroll
+#pragma unroll(DH == 128 ? 2 : 1)
             for (int which = 0; which < (kKeySide ? 2 : 1); ++which) {
                 if (kShort && P.shared_box) {               // a 64-channel box would write into the next head: 64-byte pieces of a row instead
                     const long long my_row = in_tensor ? out_row : -1;

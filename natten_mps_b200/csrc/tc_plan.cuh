@@ -313,6 +313,7 @@ __device__ __forceinline__ uint32_t piece_word_ranges(const TcParams& P, int pc,
     const int seg = P.cb[2] < 32 ? P.cb[2] : 32;
     const int nseg = 32 / seg;
     uint32_t w = 0;
+#pragma unroll 1                     // short code: what these chunks run at is how fast it arrives (see tc_bwd.cu)
     for (int sg = 0; sg < nseg; ++sg) {
         const int jj = 32 * pc + sg * seg;
         const int j2 = jj & (P.cb[2] - 1);
