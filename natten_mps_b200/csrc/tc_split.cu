@@ -26,6 +26,8 @@ constexpr int kStages = 3;
 // Loads of weights that a thread has in flight.  One at a time the staging was most of the apply kernel: 61 x 67, 9 x 9, 8 heads of 64,
 // batch 2: 42 us, now 30 (16 in flight: the same).
 constexpr int kAhead = 8;
+// Shared memory of a CTA when three share an SM's 228 KB, of which the system keeps 1 KB for each.
+constexpr size_t kThirdOfSm = 228 * 1024 / 3 - 1024;
 
 template <int DH>
 struct SmemS {
@@ -420,7 +422,12 @@ int launch_scores_inner(const Plan& plan, const CUtensorMap& mx, const CUtensorM
 // gather the weights of the columns inside each row's window into a dense 16-bit P tile in TMEM
 // (two buffers), and O += P Y runs on the tensor cores with Y read MN-major, as in the fused forward.
 // ---------------------------------------------------------------------------
-template <int DH>
+// kThree: three CTAs share an SM, which leaves each one P buffer and 72 registers.  What bounds these kernels is the chain of a tile
+// (geometry, weights, gathering, product), not an issue rate, so at head dim 64 that is the better form wherever the weights of three
+// tiles fit beside each other (101 slots); above it two CTAs with two buffers.  fp16, 8 heads of 64, batch 2, forward and dQ, three
+// CTAs | two with one buffer | two with two: 61 x 67, 49 slots 48.9 | 51.4 | 50.7 us, 81 slots 58.1 | 60.6 | 60.0, 99 slots
+// 81.5 | 89.0 | 85.9; 121 slots, where a third CTA has no room, 112.7 | 103.6 | 99.3, 147 133.5 | 122.4 | 119.0, 225 175.7 | 168.8 | 162.4.
+template <int DH, bool kThree>
 struct SmemA {
     static constexpr int kHalves = DH / 64;
     static constexpr int kHalf = kTileRows * 128;
@@ -430,19 +437,19 @@ struct SmemA {
     static constexpr int kColSlot = kBar + 128;
     static constexpr int kRowOut = kColSlot + 512;        // [128] long long: row of w / out, or -1
     static constexpr int kW = kRowOut + 1024;             // [128][slots] 16-bit
-    // One P buffer at head dim 64, so that three CTAs share an SM: what bounds these kernels is the chain of a tile (geometry, weights,
-    // gathering, product), not an issue rate.
-    static constexpr int kPBufs = DH == 64 ? 1 : 2, kPerSm = DH == 64 ? 3 : 1;
-    static constexpr uint32_t kColP = 0, kColO = 64 * kPBufs, kTmemCols = kColO + DH;
+    static constexpr int kPBufs = kThree ? 1 : 2, kPerSm = kThree ? 3 : DH == 64 ? 2 : 1;
+    static constexpr uint32_t kColP = 0, kColO = 64 * kPBufs;
+    static constexpr uint32_t kTmemCols = kColO + DH <= 128 ? 128 : 256;       // allocated in powers of two
+    static_assert(kTmemCols * kPerSm <= 512 && kColO + DH <= kTmemCols, "TMEM");
 };
 
-template <int DH, bool BF16, int kInner>
-__global__ void __launch_bounds__(kThreads, SmemA<DH>::kPerSm)
+template <int DH, bool BF16, int kInner, bool kThree>
+__global__ void __launch_bounds__(kThreads, SmemA<DH, kThree>::kPerSm)
 tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ TcParams P,
                 const uint16_t* __restrict__ w, uint16_t* __restrict__ out, float scale, int ktot,
                 int out_by_position)
 {
-    using SM = SmemA<DH>;
+    using SM = SmemA<DH, kThree>;
     constexpr int CH = DH / 2;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -651,26 +658,14 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
     }
 }
 
-template <int DH, bool BF16, int kInner>
-int launch_apply_inner(const Plan& plan, const CUtensorMap& my, const Geo& g, const void* w, void* out, float scale,
-                       bool out_by_position, cudaStream_t s);
-
-template <int DH, bool BF16>
-int launch_apply(const Plan& plan, const CUtensorMap& my, const Geo& g, const void* w, void* out, float scale,
-                 bool out_by_position, cudaStream_t s)
+template <int DH, bool BF16, int kInner, bool kThree>
+int launch_apply_as(const Plan& plan, const CUtensorMap& my, const Geo& g, const void* w, void* out, float scale,
+                    bool out_by_position, cudaStream_t s)
 {
-    return plan.p.cb[2] == 16 ? launch_apply_inner<DH, BF16, 16>(plan, my, g, w, out, scale, out_by_position, s)
-                              : launch_apply_inner<DH, BF16, 0>(plan, my, g, w, out, scale, out_by_position, s);
-}
-
-template <int DH, bool BF16, int kInner>
-int launch_apply_inner(const Plan& plan, const CUtensorMap& my, const Geo& g, const void* w, void* out, float scale,
-                       bool out_by_position, cudaStream_t s)
-{
-    using SM = SmemA<DH>;
-    const size_t smem = (size_t)SM::kW + (size_t)kTileRows * g.ktot * 2;
+    const size_t smem = (size_t)SmemA<DH, kThree>::kW + (size_t)kTileRows * g.ktot * 2;
     if (smem > kMaxDynamicSmem) return -2;
-    cudaError_t err = ensure_dynamic_smem((const void*)tc_apply_kernel<DH, BF16, kInner>, kMaxDynamicSmem);
+    auto* kernel = tc_apply_kernel<DH, BF16, kInner, kThree>;
+    cudaError_t err = ensure_dynamic_smem((const void*)kernel, kMaxDynamicSmem);
     if (err != cudaSuccess) {
         cudaGetLastError();
         return (int)err;
@@ -678,11 +673,29 @@ int launch_apply_inner(const Plan& plan, const CUtensorMap& my, const Geo& g, co
     int ngroups = 1;
     for (int a = 0; a < 3; ++a) ngroups *= plan.p.grp_n[a];
     const dim3 grid((unsigned)(plan.p.ntiles * ngroups), (unsigned)g.Hq, (unsigned)g.B);
-    tc_apply_kernel<DH, BF16, kInner><<<grid, kThreads, smem, s>>>(my, plan.p, (const uint16_t*)w, (uint16_t*)out, scale, g.ktot,
-                                                         out_by_position ? 1 : 0);
+    kernel<<<grid, kThreads, smem, s>>>(my, plan.p, (const uint16_t*)w, (uint16_t*)out, scale, g.ktot, out_by_position ? 1 : 0);
     tc_count_launch();
     err = cudaGetLastError();
     return err == cudaSuccess ? 0 : (int)err;
+}
+
+template <int DH, bool BF16, int kInner>
+int launch_apply_inner(const Plan& plan, const CUtensorMap& my, const Geo& g, const void* w, void* out, float scale,
+                       bool out_by_position, cudaStream_t s)
+{
+    if constexpr (DH == 64) {
+        if (SmemA<DH, true>::kW + (size_t)kTileRows * g.ktot * 2 <= kThirdOfSm)
+            return launch_apply_as<DH, BF16, kInner, true>(plan, my, g, w, out, scale, out_by_position, s);
+    }
+    return launch_apply_as<DH, BF16, kInner, false>(plan, my, g, w, out, scale, out_by_position, s);
+}
+
+template <int DH, bool BF16>
+int launch_apply(const Plan& plan, const CUtensorMap& my, const Geo& g, const void* w, void* out, float scale,
+                 bool out_by_position, cudaStream_t s)
+{
+    return plan.p.cb[2] == 16 ? launch_apply_inner<DH, BF16, 16>(plan, my, g, w, out, scale, out_by_position, s)
+                              : launch_apply_inner<DH, BF16, 0>(plan, my, g, w, out, scale, out_by_position, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1003,7 +1016,7 @@ int tc_apply(int dtype, const Geo& g, const void* w, const void* y, const long l
     if ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15u) return -2;
     if (g.Hq > 65535 || g.B > 65535) return -2;
     const size_t budget = g.D == 64 ? 113 * 1024 : 227 * 1024;
-    const size_t base = g.D == 64 ? (size_t)SmemA<64>::kW : (size_t)SmemA<128>::kW;
+    const size_t base = g.D == 64 ? (size_t)SmemA<64, true>::kW : (size_t)SmemA<128, false>::kW;
     if (base + (size_t)kTileRows * g.ktot * 2 > budget) return -2;
     Plan plan;
     if (const int rc = make_plan(g, plan, kChunk, /*with_stride=*/true)) return rc;
