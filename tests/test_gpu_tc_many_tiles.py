@@ -1,0 +1,130 @@
+"""The one-buffer form of the tcgen05 forward, which serves head dims up to 64 where there are more than two tiles an SM: edge
+shapes of the other tests with as many samples as that takes, against the general kernels."""
+import pytest
+import torch
+
+from natten_mps_b200 import _backend, _cabi
+from tests import test_gpu_tc as few, test_gpu_tc_tables as tables
+
+pytestmark = pytest.mark.gpu
+
+
+def samples(size, heads):
+    """Samples for which tiles of 128 rows number more than two an SM however they are cut."""
+    rows = heads
+    for n in size:
+        rows *= n
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return -(-(2 * sms + 1) * 128 // rows)
+
+
+def inputs(B, size, hq, hkv, dim, dtype, seed, extra=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    t = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)
+    q, k, v = t(B, *size, hq, dim), t(B, *size, hkv, dim), t(B, *size, hkv, dim)
+    return (q, k, v), (dict(extra_k=t(B, extra, hkv, dim), extra_v=t(B, extra, hkv, dim)) if extra else {})
+
+
+def compare(qkv, *geo, **kw):
+    try:
+        _cabi.set_force("simt")
+        want, want_lse = _backend.fused_forward(*qkv, *geo, **kw)
+        _cabi.set_force("tc")
+        got, lse = _backend.fused_forward(*qkv, *geo, **kw)
+        assert _cabi.last_path() == "tcgen05"
+    finally:
+        _cabi.set_force(None)
+    torch.cuda.synchronize()
+    assert _cabi.device_status() == 0
+    # the bounds of the same shapes with few tiles (test_gpu_tc.py)
+    assert float((got.float() - want.float()).abs().max()) <= 1.6e-2
+    assert float((lse - want_lse).abs().max()) <= 2e-3
+    return got, lse
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("case", [c for c in few.CASES if few._dim(c) <= 64], ids=few._id)
+def test_forward(case, dtype):
+    size, _, hq, hkv, kernel, dilation, causal, extents = case[:8]
+    dim = few._dim(case)
+    B = samples(size, hq)
+    qkv, _ = inputs(B, size, hq, hkv, dim, dtype, 7)
+    ext = None if extents is None else torch.tensor([extents[b % len(extents)] for b in range(B)], dtype=torch.int32).cuda()
+    compare(qkv, kernel, (1,) * len(size), dilation, causal, dim ** -0.5, extents=ext)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("case", [c for c in few.EXTRA_CASES if c[4] == 64], ids=lambda c: "x".join(map(str, c[0])) + f"_e{c[6]}")
+def test_additional_tokens(case, dtype):
+    size, _, hq, hkv, dim, kernel, extra, _ = case
+    qkv, kw = inputs(samples(size, hq), size, hq, hkv, dim, dtype, 23, extra)
+    compare(qkv, kernel, (1,) * len(size), (1,) * len(size), (False,) * len(size), dim ** -0.5, **kw)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("case", [c for c in few.STRIDE_CASES if c[9] == 64], ids=lambda c: "x".join(map(str, c[0])) + f"_s{c[6][-1]}")
+def test_output_stride(case, dtype):
+    size, _, hq, hkv, kernel, dilation, stride, causal, extents, dim = case
+    B = samples([-(-n // s) for n, s in zip(size, stride)], hq)
+    qkv, _ = inputs(B, size, hq, hkv, dim, dtype, 29)
+    ext = None if extents is None else torch.tensor([extents[b % len(extents)] for b in range(B)], dtype=torch.int32).cuda()
+    compare(qkv, kernel, stride, dilation, causal, dim ** -0.5, extents=ext)
+
+
+@pytest.mark.parametrize("shape", [s for s in tables.SHAPES if s[-1] <= 64], ids=lambda s: "x".join(map(str, s[1] + s[2])) + f"d{s[-1]}")
+@pytest.mark.parametrize("extra", [0, 5])
+def test_tables(shape, extra):
+    _, size, kernel, dilation, stride, causal, heads, dim = shape
+    B = samples([-(-n // s) for n, s in zip(size, stride)], heads)
+    qkv, kw = inputs(B, size, heads, heads, dim, torch.bfloat16, sum(size), extra)
+    compare(qkv, kernel, stride, dilation, tuple(bool(c) for c in causal), dim ** -0.5, **kw)
+
+
+@pytest.mark.parametrize("shape", [s for s in tables.PACKED if s[-1] <= 64], ids=lambda s: "x".join(map(str, s[0] + s[1] + s[3])))
+def test_grouped_heads_packed(shape):
+    size, kernel, causal, (hq, hkv), dim = shape
+    qkv, kw = inputs(samples(size, hq), size, hq, hkv, dim, torch.float16, sum(size), 5)
+    ones = (1,) * len(size)
+    compare(qkv, kernel, ones, ones, tuple(bool(c) for c in causal), dim ** -0.5, **kw)
+
+
+@pytest.mark.parametrize("lens", [(300, 7, 128), (129, 300, 15)])
+def test_lengths(lens):
+    B = samples((7,), 4) // 3 * 3 + 3            # (padding tiles are walked like the others)
+    (q, k, v), _ = inputs(B, (300,), 4, 2, 64, torch.float16, 5)
+    sizes = torch.tensor([lens[b % 3] for b in range(B)], dtype=torch.int32, device="cuda")
+    past = torch.arange(300, device="cuda")[None, :] >= sizes[:, None]
+    k[past], v[past] = float("nan"), float("nan")           # never read
+    got, lse = compare((q, k, v), (7,), (1,), (1,), (False,), 0.125, extents=sizes[:, None])
+    assert not got[past].any() and not lse[past].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("size,kernel,slope,axis", [((700,), (255,), 12.0 / 128.0, 0), ((40, 48), (13, 13), 1.0, 1),
+                                                    ((40, 48), (13, 13), 4.0, 1), ((48, 40), (7, 7), 12.0, 0)],
+                         ids=["1d", "2d", "2d_steep", "2d_k7_rows"])
+def test_rescale_when_later_chunks_dominate(size, kernel, slope, axis, dtype):
+    """Scores that grow along an axis by more than a stored probability may exceed its stabiliser: with one score buffer the
+    rescale of O, the row sum and the chunk's probabilities happens in place, without a wait for the product before."""
+    B, H, D = samples(size, 2), 2, 64
+    g = torch.Generator(device="cuda").manual_seed(23)
+    t = lambda: torch.randn(B, *size, H, D, device="cuda", generator=g)
+    shape = [1] * (len(size) + 3)
+    shape[1 + axis] = size[axis]
+    ramp = (torch.arange(size[axis], device="cuda", dtype=torch.float32) * slope).reshape(shape)
+    q, k, v = [x.to(dtype) for x in (t() * 0.1 + 1.0, t() * 0.1 + ramp / D ** 0.5, t())]
+    ones = (1,) * len(size)
+    args = (q, k, v, kernel, ones, ones, (False,) * len(size), D ** -0.5)
+    try:
+        _cabi.set_force("simt")
+        want, want_lse = _backend.fused_forward(*args)
+        _cabi.set_force("tc")
+        got, lse = _backend.fused_forward(*args)
+        assert _cabi.last_path() == "tcgen05"
+    finally:
+        _cabi.set_force(None)
+    torch.cuda.synchronize()
+    assert _cabi.device_status() == 0
+    assert float(want_lse.max() - want_lse.min()) > 20.0
+    assert float((got.float() - want.float()).abs().max()) <= 2e-2
+    assert float(((lse - want_lse).abs() / want_lse.abs().clamp(min=1.0)).max()) <= 2e-3
