@@ -290,10 +290,10 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             unsigned stage = 0, parity = 1, g = 0;       // parity: of the stage's last release
             unsigned zw = blockIdx.x;                    // next work item to look at for padding
             auto zero_one = [&]() {
-                BwdTile Z;
-                bwd_tile_setup<kKeySide>(P, zw, Z);
+                int zb, zh, rg[3], origin[3], Lp[3];
+                const unsigned bx = split_work<kKeySide>(P, zw, zb, zh);
                 zw += gridDim.x;
-                if (Z.active) return;
+                if (cta_geometry(P, bx, zb, rg, origin, Lp)) return;
 #pragma unroll 1
                 for (int r = lane; r < kTileRows; r += 32) {
                     int ri[3];
@@ -302,12 +302,12 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     long long pflat = 0;
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        const int pa = Z.rg[a] + P.dil[a] * (Z.origin[a] + ri[a]);
+                        const int pa = rg[a] + P.dil[a] * (origin[a] + ri[a]);
                         in_tensor = in_tensor && pa < P.L[a];
                         pflat = pflat * P.L[a] + pa;
                     }
                     if (!in_tensor) continue;
-                    const long long row = ((long long)Z.b * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + Z.hy + (r & ((1 << P.pack_log) - 1));
+                    const long long row = ((long long)zb * P.ltot + pflat) * (kKeySide ? P.Hkv : P.Hq) + zh + (r & ((1 << P.pack_log) - 1));
 #pragma unroll
                     for (int which = 0; which < (kKeySide ? 2 : 1); ++which) {
                         uint4* o = reinterpret_cast<uint4*>((which == 0 ? out1 : out2) + row * P.dreal);
@@ -466,7 +466,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
         for (unsigned t = 0;; ++t) {
             // ---- this thread's row, from the geometry warp's tables ----
             ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
-// All of them or none where the stores are behind a barrier of theirs; without one a warp goes by itself.
+            // All of them or none where the stores are behind a barrier of theirs; without one a warp goes by itself.
             const bool apart = kShort && P.shared_box;
             if (apart ? !__all_sync(0xffffffffu, ok) : any_of_compute(!ok)) break;
             const uint8_t* tab = tab_slot(t);

@@ -14,7 +14,6 @@ struct FwdTile {
     int b, h, hk;
     int rg[3], origin[3], Lp[3], lo[3], nc[3], x0[3], sx[3], nq[3], nqf[3];
     int nnb, nch;          // nch == 0 in a published header: no more tiles
-    int active;
     int mapped;            // the row maps of the tables are valid
 };
 
@@ -45,76 +44,27 @@ struct Cursor {
     }
 };
 
-// Geometry of the cursor's work item (tile bx of (batch, head)); the same for every role of a lane.
-// origin[] counts queries of the dilation group; query i of an axis sits at sub-grid index
-// x0 + sx * i (every index when the output stride is 1).
-__device__ __forceinline__ void fwd_tile(const TcParams& P, const Cursor& cur, int chunk_log, FwdTile& T)
+// Rows of the cursor's tile that exist in the output, by one warp: f(output row) for each.  (Position x0 + sx * i of the sub-grid is
+// query i of an axis; a dilation group without queries has x0 < 0.)
+template <typename F>
+__device__ __forceinline__ void for_each_row(const TcParams& P, const Cursor& cur, int lane, F&& f)
 {
-    const unsigned bx = cur.bx;
-    T.b = cur.b;
-    T.h = cur.h << P.pack_log;
-    T.hk = (int)fast_div((unsigned)T.h, P.group_mul);
-    bool active = cta_geometry(P, bx, T.b, T.rg, T.origin, T.Lp);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        T.sx[a] = P.qstep[a];
-        T.x0[a] = P.qx0[a][T.rg[a]];
-        const int lpf = (int)fast_div((unsigned)(P.L[a] - T.rg[a] + P.dil[a] - 1), P.dil_mul[a]);   // sub-grid length of the whole tensor
-        if (T.x0[a] < 0) {                       // no output position falls into this dilation group
-            T.nq[a] = 0; T.nqf[a] = 0; T.x0[a] = 0;
-        } else if (T.sx[a] == 1) {
-            T.nq[a] = T.Lp[a];
-            T.nqf[a] = T.rg[a] < P.L[a] ? lpf : 0;
-        } else {
-            T.nq[a] = T.x0[a] < T.Lp[a] ? (T.Lp[a] - T.x0[a] + T.sx[a] - 1) / T.sx[a] : 0;
-            T.nqf[a] = T.x0[a] < lpf ? (lpf - T.x0[a] + T.sx[a] - 1) / T.sx[a] : 0;
-        }
-        if (T.origin[a] >= T.nq[a]) active = false;
-    }
-    T.nnb = 1;
-    if (active) {
+    int rg[3], origin[3];
+    tile_of_block(P, cur.bx, rg, origin);
+#pragma unroll 1
+    for (int r = lane; r < kTileRows; r += 32) {
+        int qi[3];
+        row_offsets(P, r, qi);
+        bool in_tensor = true;
+        long long oflat = 0;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const int lastq = T.origin[a] + P.tile[a] - 1 < T.nq[a] - 1 ? T.origin[a] + P.tile[a] - 1 : T.nq[a] - 1;
-            const int xf = T.x0[a] + T.sx[a] * T.origin[a], xl = T.x0[a] + T.sx[a] * lastq;
-            T.lo[a] = P.causal[a] ? xf - (P.K[a] - 1) : window_start(xf, T.Lp[a], P.K[a], 1);
-            const int hi = P.causal[a] ? xl : window_start(xl, T.Lp[a], P.K[a], 1) + P.K[a] - 1;
-            T.nc[a] = chunks_along(P, a, hi - T.lo[a] + 1);       // chunks this tile really needs
-            T.nnb *= T.nc[a];
+            const int x0 = P.qx0[a][rg[a]], pa = rg[a] + P.dil[a] * (x0 + P.qstep[a] * (origin[a] + qi[a]));
+            in_tensor = in_tensor && x0 >= 0 && pa < P.L[a];
+            oflat = oflat * P.O[a] + (P.st[a] == 1 ? pa : pa / P.st[a]);
         }
+        if (in_tensor) f(((long long)cur.b * P.otot + oflat) * P.Hq + (cur.h << P.pack_log) + (r & ((1 << P.pack_log) - 1)));
     }
-    T.nch = T.nnb + ((P.n_extra + (1 << chunk_log) - 1) >> chunk_log);   // then the additional tokens, one chunk at a time
-    T.active = active ? 1 : 0;
-}
-
-// Output row of tile row `row`, whether it is a query of the sample / a row of the tensor, and (active
-// tiles) its window as a box-relative range [f, e) per axis.
-__device__ __forceinline__ long long row_geometry(const TcParams& P, const FwdTile& T, int row, int (&f)[3], int (&e)[3],
-                                                  bool& valid_q, bool& in_tensor)
-{
-    int qi[3];
-    row_offsets(P, row, qi);
-    valid_q = true;
-    in_tensor = true;
-    long long oflat = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int qa = T.origin[a] + qi[a];               // query count along the axis
-        const int xq = T.x0[a] + T.sx[a] * qa;            // its sub-grid index
-        const int pa = T.rg[a] + P.dil[a] * xq;           // its position in the tensor
-        if (qa >= T.nq[a]) valid_q = false;
-        if (qa >= T.nqf[a]) in_tensor = false;
-        oflat = oflat * P.O[a] + (P.st[a] == 1 ? pa : pa / P.st[a]);
-        f[a] = 0;
-        e[a] = 0;
-        if (T.active) {
-            const int first = P.causal[a] ? xq - (P.K[a] - 1) : window_start(xq, T.Lp[a], P.K[a], 1);
-            f[a] = (first > 0 ? first : 0) - T.lo[a];
-            e[a] = (first + P.K[a] < T.Lp[a] ? first + P.K[a] : T.Lp[a]) - T.lo[a];
-        }
-    }
-    if (!valid_q) { e[0] = f[0]; e[1] = f[1]; e[2] = f[2]; }
-    return ((long long)T.b * P.otot + oflat) * P.Hq + T.h + (row & ((1 << P.pack_log) - 1));
 }
 
 // What a softmax thread needs to know about its row is separable: along every axis the query's coordinate alone decides its
@@ -123,8 +73,9 @@ __device__ __forceinline__ long long row_geometry(const TcParams& P, const FwdTi
 constexpr int kMapOff = 160, kEntOff = kMapOff + 8 * kTileRows, kTabBytes = kEntOff + 16 * (kTileRows + 2);
 static_assert(sizeof(FwdTile) <= kMapOff, "no room for the tile in front of its tables");
 
-// The cursor's work item into the head of a slot, by one warp (the same as fwd_tile, an axis per lane); returns whether it is
-// active.  rows16: chunks of 16-column rows.
+// The cursor's work item (tile bx of (batch, head)) into the head of a slot, by one warp, an axis per lane; returns whether it holds a
+// query of the sample.  origin[] counts queries of the dilation group; query i of an axis sits at sub-grid index x0 + sx * i (every
+// index when the output stride is 1).  rows16: chunks of 16-column rows.
 __device__ __forceinline__ bool publish_tile(const TcParams& P, const Cursor& cur, int chunk_log, bool rows16, int lane, FwdTile* H)
 {
     const int a = lane < 2 ? lane : 2;
@@ -163,7 +114,6 @@ __device__ __forceinline__ bool publish_tile(const TcParams& P, const Cursor& cu
         H->hk = (int)fast_div((unsigned)h, P.group_mul);
         H->nnb = nnb;
         H->nch = nnb + ((P.n_extra + (1 << chunk_log) - 1) >> chunk_log);    // then the additional tokens, one chunk at a time
-        H->active = 1;
         H->mapped = rows16 && nc == 1 && nnb <= 16;
     }
     return true;
@@ -204,7 +154,8 @@ __device__ __forceinline__ void write_tables(const TcParams& P, int lane, uint8_
     }
 }
 
-// A thread's row from the tables (what row_geometry gives, and the maps).
+// A thread's row from the tables: its output row, whether it is a query of the sample / a row of the tensor, its window as a
+// box-relative range [f, e) per axis, and the maps.
 __device__ __forceinline__ long long row_from_tables(const TcParams& P, const uint8_t* slot, int row, int (&f)[3], int (&e)[3],
                                                      bool& valid_q, bool& in_tensor, unsigned long long& rowmap, uint32_t& colbits)
 {

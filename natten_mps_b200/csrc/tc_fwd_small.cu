@@ -54,8 +54,8 @@ constexpr uint32_t kColS = 0;
 // 16 heads of 32 (224) 14.0 | 12.8; 48 x 60, 6 heads of 64 (270) 15.2 | 13.6.  Above it the second buffer costs a second wave.
 constexpr unsigned kFewTiles = 2;
 
-// Shared memory and TMEM of one CTA for head dim DH (64: four CTAs per SM, 128 TMEM columns; 128: two CTAs per
-// SM, 256 TMEM columns).  Tiles are stored as blocks of 64 channels (128-byte rows, 128-byte swizzle).
+// Shared memory and TMEM of one CTA for head dim DH: four CTAs per SM with 128 TMEM columns each, or two with 256 and two score buffers
+// (head dim 128, and 64 where there are few tiles).  Tiles are stored as blocks of 64 channels (128-byte rows, 128-byte swizzle).
 template <int DH, bool TWO_S>
 struct FwdSmall {
     static constexpr int kHalves = DH / 64;
@@ -305,21 +305,13 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             // =====================================================================
             if (!*abort_flag) {
                 auto zero_rows = [&](const Cursor& at) {     // rows of a padding tile that exist in the output are zero
-                    FwdTile T;
-                    fwd_tile(P, at, kKeysLog, T);
-#pragma unroll 1
-                    for (int r = lane; r < kTileRows; r += 32) {
-                        int f[3], e[3];
-                        bool valid_q, in_tensor;
-                        const long long out_row = row_geometry(P, T, r, f, e, valid_q, in_tensor);
-                        if (in_tensor) {
-                            uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
+                    for_each_row(P, at, lane, [&](long long out_row) {
+                        uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
 #pragma unroll
-                            for (int i = 0; i < DH / 8; ++i)
-                                if (8 * i < P.dreal) o4[i] = make_uint4(0, 0, 0, 0);
-                            lse[out_row] = 0.f;
-                        }
-                    }
+                        for (int i = 0; i < DH / 8; ++i)
+                            if (8 * i < P.dreal) o4[i] = make_uint4(0, 0, 0, 0);
+                        lse[out_row] = 0.f;
+                    });
                 };
                 bool ok = true, found = true;
                 Cursor cur;
@@ -418,279 +410,279 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         };
 
         for (unsigned t = 0;; ++t) {
-        ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
-        if (!ok) break;
-        const FwdTile* H = tab_slot(t);
-        const int nch = H->nch;
-        if (nch == 0) break;
-        // ---- this thread's query row, from the loader's tables ----
-        const int nnb = H->nnb, nc1 = H->nc[1], nc2 = H->nc[2];
-        const bool mapped = kRows16 && H->mapped;
-        int f[3], e[3];
-        bool valid_q, in_tensor;
-        unsigned long long rowmap;
-        uint32_t colbits;                    // 16-column rows: one bit per column
-        const long long out_row = row_from_tables(P, reinterpret_cast<const uint8_t*>(H), warp * 32 + lane, f, e, valid_q, in_tensor, rowmap, colbits);
-        mbar_arrive(bar_tab_empty + 8 * (t & 1));
-        m = -INFINITY;
-        l = 0.f;
-        add_cols = 0xffffffffu;              // the addends belong to the previous tile's stabiliser
-        int ci[3] = {0, 0, 0};
-        const bool line = line_chunks(P);    // chunks are runs of the innermost axis (1-D windows): cheap validity words
-        int jl[3] = {0, 0, 0}, jh[3] = {0, 0, 0};
-        uint32_t rowbits = 0u, dirty = 7u;   // 16-column rows: one bit per piece
-        for (int c = 0; c < nch; ++c, ++n) {
-            // ---- validity of this row's columns in this chunk ----
-            // jl/jh (columns of the chunk inside the row's window, per axis) only change along the axes whose
-            // chunk index moved since the last chunk: `dirty` has a bit per axis.
-            const bool extra = c >= nnb;   // additional tokens: every live row sees the first n_extra columns
-            uint32_t words[2] = {0u, 0u};    // generic form: one bit per column
-            if (extra) {
+            ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
+            if (!ok) break;
+            const FwdTile* H = tab_slot(t);
+            const int nch = H->nch;
+            if (nch == 0) break;
+            // ---- this thread's query row, from the geometry warp's tables ----
+            const int nnb = H->nnb, nc1 = H->nc[1], nc2 = H->nc[2];
+            const bool mapped = kRows16 && H->mapped;
+            int f[3], e[3];
+            bool valid_q, in_tensor;
+            unsigned long long rowmap;
+            uint32_t colbits;                    // 16-column rows: one bit per column
+            const long long out_row = row_from_tables(P, reinterpret_cast<const uint8_t*>(H), warp * 32 + lane, f, e, valid_q, in_tensor, rowmap, colbits);
+            mbar_arrive(bar_tab_empty + 8 * (t & 1));
+            m = -INFINITY;
+            l = 0.f;
+            add_cols = 0xffffffffu;              // the addends belong to the previous tile's stabiliser
+            int ci[3] = {0, 0, 0};
+            const bool line = line_chunks(P);    // chunks are runs of the innermost axis (1-D windows): cheap validity words
+            int jl[3] = {0, 0, 0}, jh[3] = {0, 0, 0};
+            uint32_t rowbits = 0u, dirty = 7u;   // 16-column rows: one bit per piece
+            for (int c = 0; c < nch; ++c, ++n) {
+                // ---- validity of this row's columns in this chunk ----
+                // jl/jh (columns of the chunk inside the row's window, per axis) only change along the axes whose
+                // chunk index moved since the last chunk: `dirty` has a bit per axis.
+                const bool extra = c >= nnb;   // additional tokens: every live row sees the first n_extra columns
+                uint32_t words[2] = {0u, 0u};    // generic form: one bit per column
+                if (extra) {
 #pragma unroll
-                for (int pc = 0; pc < 2; ++pc)
-                    words[pc] = valid_q ? low_bits(P.n_extra - ((c - nnb) * kKeys + 32 * pc)) : 0u;
-            } else if (mapped) {
-                rowbits = (uint32_t)(rowmap >> (4 * c)) & 15u;
-            } else {
-                if (kInner == 0 && line) {
-#pragma unroll
-                    for (int pc = 0; pc < 2; ++pc) words[pc] = line_word(P, pc, ci, f, e);
+                    for (int pc = 0; pc < 2; ++pc)
+                        words[pc] = valid_q ? low_bits(P.n_extra - ((c - nnb) * kKeys + 32 * pc)) : 0u;
+                } else if (mapped) {
+                    rowbits = (uint32_t)(rowmap >> (4 * c)) & 15u;
                 } else {
+                    if (kInner == 0 && line) {
 #pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    if ((dirty >> a) & 1u) chunk_range(P, a, ci[a], f[a], e[a], jl[a], jh[a]);
-                if constexpr (kInner > 0) {
-                    // inner rows of the chunk (kInner columns each) are numbered r = j0 * cb1 + j1
-                    if (dirty & 3u) {
-                        const uint32_t m1 = jh[1] > jl[1] ? (low_bits(jh[1]) & ~low_bits(jl[1])) : 0u;
-                        rowbits = 0u;
-                        for (int j0 = jl[0]; j0 < jh[0]; ++j0) rowbits |= m1 << (j0 << P.cb1_log);
+                        for (int pc = 0; pc < 2; ++pc) words[pc] = line_word(P, pc, ci, f, e);
+                    } else {
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+                            if ((dirty >> a) & 1u) chunk_range(P, a, ci[a], f[a], e[a], jl[a], jh[a]);
+                        if constexpr (kInner > 0) {
+                            // inner rows of the chunk (kInner columns each) are numbered r = j0 * cb1 + j1
+                            if (dirty & 3u) {
+                                const uint32_t m1 = jh[1] > jl[1] ? (low_bits(jh[1]) & ~low_bits(jl[1])) : 0u;
+                                rowbits = 0u;
+                                for (int j0 = jl[0]; j0 < jh[0]; ++j0) rowbits |= m1 << (j0 << P.cb1_log);
+                            }
+                            if (dirty & 4u) colbits = jh[2] > jl[2] ? (low_bits(jh[2]) & ~low_bits(jl[2])) : 0u;
+                            if constexpr (!kRows16) {
+#pragma unroll
+                                for (int pc = 0; pc < 2; ++pc) words[pc] = ((rowbits >> pc) & 1u) ? colbits : 0u;
+                            }
+                        } else {
+#pragma unroll
+                            for (int pc = 0; pc < 2; ++pc) words[pc] = piece_word_ranges(P, pc, jl, jh);
+                        }
                     }
-                    if (dirty & 4u) colbits = jh[2] > jl[2] ? (low_bits(jh[2]) & ~low_bits(jl[2])) : 0u;
-                    if constexpr (!kRows16) {
-#pragma unroll
-                        for (int pc = 0; pc < 2; ++pc) words[pc] = ((rowbits >> pc) & 1u) ? colbits : 0u;
-                    }
-                } else {
-#pragma unroll
-                    for (int pc = 0; pc < 2; ++pc) words[pc] = piece_word_ranges(P, pc, jl, jh);
+                    dirty = 0u;
                 }
+                const bool fast = kRows16 && !extra;
+                if (fast && colbits != add_cols) refresh_add(colbits);
+                uint32_t mine = 0u, act = 0u;    // pieces inside this row's window, inside that of any row of the warp
+                if (fast) {
+                    mine = colbits != 0u ? rowbits & 15u : 0u;
+                    act = __reduce_or_sync(0xffffffffu, mine);
                 }
-                dirty = 0u;
-            }
-            const bool fast = kRows16 && !extra;
-            if (fast && colbits != add_cols) refresh_add(colbits);
-            uint32_t mine = 0u, act = 0u;    // pieces inside this row's window, inside that of any row of the warp
-            if (fast) {
-                mine = colbits != 0u ? rowbits & 15u : 0u;
-                act = __reduce_or_sync(0xffffffffu, mine);
-            }
 
-            scol = trow + kColS + s_cols(n);
-            ok = ok && mbar_wait(bar_s_of(n), par_of(n), abort_flag, P.wait_budget);     // one score buffer: every earlier product has finished, too
-            tc_fence_after();
-            if (!__all_sync(0xffffffffu, ok)) { words[0] = 0u; words[1] = 0u; act = 0u; dirty = 7u; }
+                scol = trow + kColS + s_cols(n);
+                ok = ok && mbar_wait(bar_s_of(n), par_of(n), abort_flag, P.wait_budget);     // one score buffer: every earlier product has finished, too
+                tc_fence_after();
+                if (!__all_sync(0xffffffffu, ok)) { words[0] = 0u; words[1] = 0u; act = 0u; dirty = 7u; }
 
-            uint32_t stored = 0u;            // pieces of this chunk that hold probabilities (bit per piece)
-            // one 16-column piece on the general path: scores s, validity bits wd -> probabilities pk
-            auto generic_piece = [&](int pc, uint32_t (&s)[16], uint32_t wd, uint32_t (&pk)[8]) {
-                if (m == -INFINITY && wd != 0u) {           // first valid columns of this row: fix the stabiliser
-                    float mm = -INFINITY;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if ((wd >> i) & 1u) mm = fmaxf(mm, __uint_as_float(s[i]));
-                    m = mm;
-                    add_cols = 0xffffffffu;                 // the addends of the fast path are stale now
-                }
-                const float mb = (m == -INFINITY) ? 0.f : m * P.scale_log2;
-                // A piece that lies inside every row's window (most pieces of a long 1-D window) needs no
-                // masks and no running maximum: two columns per packed instruction, and the row sum tells
-                // whether any probability may have outgrown its stabiliser (then the general form redoes it).
-                bool done = false;
-                if (__all_sync(0xffffffffu, wd == 0xFFFFu)) {
-                    const uint64_t sc2 = pack2(P.scale_log2, P.scale_log2), nb2 = pack2(-mb, -mb);
-                    uint64_t rr = 0ull;
-                    uint32_t pq[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const uint64_t xx = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, nb2);
-                        const float p0 = fast_exp2(lo_of(xx)), p1 = fast_exp2(hi_of(xx));
-                        rr = add2(rr, pack2(p0, p1));
-                        pq[i] = cvt_pack<BF16>(p0, p1);
-                    }
-                    const float rs = lo_of(rr) + hi_of(rr);
-                    if (!__any_sync(0xffffffffu, !(rs <= kGrowSum))) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) pk[i] = pq[i];
-                        l += rs;
-                        stored |= 1u << pc;
-                        done = true;
-                    }
-                }
-                if (!done) {
-                float x[16], xmax = -INFINITY;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    x[i] = fmaf(__uint_as_float(s[i]), P.scale_log2, -mb);
-                    if (!((wd >> i) & 1u)) x[i] = -INFINITY;
-                    xmax = fmaxf(xmax, x[i]);
-                }
-                const bool grow = xmax > kGrow;
-                if (__any_sync(0xffffffffu, grow)) {
-                    rescale(grow, xmax, c, pc, stored);
-                    if (grow) {
-                        add_cols = 0xffffffffu;
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) x[i] -= xmax;
-                    }
-                }
-                float r0 = 0.f, r1 = 0.f;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float p0 = fast_exp2(x[2 * i]), p1 = fast_exp2(x[2 * i + 1]);
-                    r0 += p0;
-                    r1 += p1;
-                    pk[i] = cvt_pack<BF16>(p0, p1);
-                }
-                l += r0 + r1;
-                stored |= 1u << pc;
-                }
-            };
-            if (fast) {
-                // one 16-column row: scores s -> probabilities over the scores they came from (piece pc lands in columns this
-                // thread has already read)
-                auto row_piece = [&](int pc, uint32_t (&s)[16], uint32_t (&pk)[8]) {
-                    const bool rowok = (mine >> pc) & 1u;
-                    if (m == -INFINITY && rowok) {           // first valid columns of this row: fix the stabiliser
+                uint32_t stored = 0u;            // pieces of this chunk that hold probabilities (bit per piece)
+                // one 16-column piece on the general path: scores s, validity bits wd -> probabilities pk
+                auto generic_piece = [&](int pc, uint32_t (&s)[16], uint32_t wd, uint32_t (&pk)[8]) {
+                    if (m == -INFINITY && wd != 0u) {           // first valid columns of this row: fix the stabiliser
                         float mm = -INFINITY;
 #pragma unroll
                         for (int i = 0; i < 16; ++i)
-                            if ((colbits >> i) & 1u) mm = fmaxf(mm, __uint_as_float(s[i]));
+                            if ((wd >> i) & 1u) mm = fmaxf(mm, __uint_as_float(s[i]));
                         m = mm;
-                        refresh_add(colbits);
+                        add_cols = 0xffffffffu;                 // the addends of the fast path are stale now
                     }
-                    // No running maximum in the common case: the probabilities are formed at once and their
-                    // row sum tells whether one of them may have outgrown the stabiliser; only then are the
-                    // exponents looked at one by one (and, if it is so, everything rescaled and redone).
-                    const uint64_t sc2 = pack2(P.scale_log2, P.scale_log2);
-                    const uint32_t keep = rowok ? 0xffffffffu : 0u;     // rows outside their window store zeros
-                    uint64_t rr = 0ull;                                 // two partial row sums
+                    const float mb = (m == -INFINITY) ? 0.f : m * P.scale_log2;
+                    // A piece that lies inside every row's window (most pieces of a long 1-D window) needs no
+                    // masks and no running maximum: two columns per packed instruction, and the row sum tells
+                    // whether any probability may have outgrown its stabiliser (then the general form redoes it).
+                    bool done = false;
+                    if (__all_sync(0xffffffffu, wd == 0xFFFFu)) {
+                        const uint64_t sc2 = pack2(P.scale_log2, P.scale_log2), nb2 = pack2(-mb, -mb);
+                        uint64_t rr = 0ull;
+                        uint32_t pq[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {                       // two columns per packed fp32 fma
-                        const uint64_t xx = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, pack2(add[2 * i], add[2 * i + 1]));
-                        const float p0 = fast_exp2(lo_of(xx)), p1 = fast_exp2(hi_of(xx));
-                        rr = add2(rr, pack2(p0, p1));
-                        pk[i] = cvt_pack<BF16>(p0, p1) & keep;
+                        for (int i = 0; i < 8; ++i) {
+                            const uint64_t xx = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, nb2);
+                            const float p0 = fast_exp2(lo_of(xx)), p1 = fast_exp2(hi_of(xx));
+                            rr = add2(rr, pack2(p0, p1));
+                            pq[i] = cvt_pack<BF16>(p0, p1);
+                        }
+                        const float rs = lo_of(rr) + hi_of(rr);
+                        if (!__any_sync(0xffffffffu, !(rs <= kGrowSum))) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) pk[i] = pq[i];
+                            l += rs;
+                            stored |= 1u << pc;
+                            done = true;
+                        }
                     }
-                    if (__any_sync(0xffffffffu, rowok && !(lo_of(rr) + hi_of(rr) <= kGrowSum))) {
+                    if (!done) {
                         float x[16], xmax = -INFINITY;
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
-                            x[i] = fmaf(__uint_as_float(s[i]), P.scale_log2, add[i]);
+                            x[i] = fmaf(__uint_as_float(s[i]), P.scale_log2, -mb);
+                            if (!((wd >> i) & 1u)) x[i] = -INFINITY;
                             xmax = fmaxf(xmax, x[i]);
                         }
-                        const bool grow = rowok && xmax > kGrow;
+                        const bool grow = xmax > kGrow;
                         if (__any_sync(0xffffffffu, grow)) {
                             rescale(grow, xmax, c, pc, stored);
                             if (grow) {
-                                refresh_add(colbits);
+                                add_cols = 0xffffffffu;
 #pragma unroll
                                 for (int i = 0; i < 16; ++i) x[i] -= xmax;
                             }
                         }
-                        rr = 0ull;
+                        float r0 = 0.f, r1 = 0.f;
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             const float p0 = fast_exp2(x[2 * i]), p1 = fast_exp2(x[2 * i + 1]);
+                            r0 += p0;
+                            r1 += p1;
+                            pk[i] = cvt_pack<BF16>(p0, p1);
+                        }
+                        l += r0 + r1;
+                        stored |= 1u << pc;
+                    }
+                };
+                if (fast) {
+                    // one 16-column row: scores s -> probabilities over the scores they came from (piece pc lands in columns this
+                    // thread has already read)
+                    auto row_piece = [&](int pc, uint32_t (&s)[16], uint32_t (&pk)[8]) {
+                        const bool rowok = (mine >> pc) & 1u;
+                        if (m == -INFINITY && rowok) {           // first valid columns of this row: fix the stabiliser
+                            float mm = -INFINITY;
+#pragma unroll
+                            for (int i = 0; i < 16; ++i)
+                                if ((colbits >> i) & 1u) mm = fmaxf(mm, __uint_as_float(s[i]));
+                            m = mm;
+                            refresh_add(colbits);
+                        }
+                        // No running maximum in the common case: the probabilities are formed at once and their
+                        // row sum tells whether one of them may have outgrown the stabiliser; only then are the
+                        // exponents looked at one by one (and, if it is so, everything rescaled and redone).
+                        const uint64_t sc2 = pack2(P.scale_log2, P.scale_log2);
+                        const uint32_t keep = rowok ? 0xffffffffu : 0u;     // rows outside their window store zeros
+                        uint64_t rr = 0ull;                                 // two partial row sums
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {                       // two columns per packed fp32 fma
+                            const uint64_t xx = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, pack2(add[2 * i], add[2 * i + 1]));
+                            const float p0 = fast_exp2(lo_of(xx)), p1 = fast_exp2(hi_of(xx));
                             rr = add2(rr, pack2(p0, p1));
                             pk[i] = cvt_pack<BF16>(p0, p1) & keep;
                         }
-                    }
-                    if (rowok) l += lo_of(rr) + hi_of(rr);
-                    stored |= 1u << pc;
-                };
-#pragma unroll 1
-                for (int pc = 0; pc < 4; ++pc) {
-                    uint32_t pk[8];
-                    if ((act >> pc) & 1u) {
-                        uint32_t s[16];
-                        tmem_ld16(scol + 16 * pc, s);
-                        tmem_ld_wait();
-                        row_piece(pc, s, pk);
-                    } else {
+                        if (__any_sync(0xffffffffu, rowok && !(lo_of(rr) + hi_of(rr) <= kGrowSum))) {
+                            float x[16], xmax = -INFINITY;
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) pk[i] = 0u;
+                            for (int i = 0; i < 16; ++i) {
+                                x[i] = fmaf(__uint_as_float(s[i]), P.scale_log2, add[i]);
+                                xmax = fmaxf(xmax, x[i]);
+                            }
+                            const bool grow = rowok && xmax > kGrow;
+                            if (__any_sync(0xffffffffu, grow)) {
+                                rescale(grow, xmax, c, pc, stored);
+                                if (grow) {
+                                    refresh_add(colbits);
+#pragma unroll
+                                    for (int i = 0; i < 16; ++i) x[i] -= xmax;
+                                }
+                            }
+                            rr = 0ull;
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                const float p0 = fast_exp2(x[2 * i]), p1 = fast_exp2(x[2 * i + 1]);
+                                rr = add2(rr, pack2(p0, p1));
+                                pk[i] = cvt_pack<BF16>(p0, p1) & keep;
+                            }
+                        }
+                        if (rowok) l += lo_of(rr) + hi_of(rr);
+                        stored |= 1u << pc;
+                    };
+#pragma unroll 1
+                    for (int pc = 0; pc < 4; ++pc) {
+                        uint32_t pk[8];
+                        if ((act >> pc) & 1u) {
+                            uint32_t s[16];
+                            tmem_ld16(scol + 16 * pc, s);
+                            tmem_ld_wait();
+                            row_piece(pc, s, pk);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) pk[i] = 0u;
+                        }
+                        tmem_st8(scol + 8 * pc, pk);
                     }
-                    tmem_st8(scol + 8 * pc, pk);
+                } else {
+#pragma unroll 1
+                    for (int pc = 0; pc < 4; ++pc) {
+                        uint32_t pk[8];
+                        const uint32_t wd = ((pc & 2) ? words[1] : words[0]) >> (16 * (pc & 1)) & 0xFFFFu;
+                        if (__any_sync(0xffffffffu, wd != 0u)) {
+                            uint32_t s[16];
+                            tmem_ld16(scol + 16 * pc, s);
+                            tmem_ld_wait();
+                            generic_piece(pc, s, wd, pk);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) pk[i] = 0u;
+                        }
+                        // P over the scores it came from: piece pc lands in columns this thread has already read
+                        tmem_st8(scol + 8 * pc, pk);
+                    }
                 }
-            } else {
-#pragma unroll 1
-                for (int pc = 0; pc < 4; ++pc) {
-                    uint32_t pk[8];
-                    const uint32_t wd = ((pc & 2) ? words[1] : words[0]) >> (16 * (pc & 1)) & 0xFFFFu;
-                    if (__any_sync(0xffffffffu, wd != 0u)) {
-                        uint32_t s[16];
-                        tmem_ld16(scol + 16 * pc, s);
-                        tmem_ld_wait();
-                        generic_piece(pc, s, wd, pk);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) pk[i] = 0u;
+                tmem_st_wait();
+                tc_fence_before();
+                mbar_arrive(bar_p_of(n));
+                if (!mapped) {
+                    ++ci[2];
+                    dirty = 4u;
+                    if (ci[2] == nc2) {
+                        ci[2] = 0; ++ci[1]; dirty = nc2 > 1 ? 6u : 2u;
+                        if (ci[1] == nc1) { ci[1] = 0; ++ci[0]; dirty = 1u | (nc1 > 1 ? 2u : 0u) | (nc2 > 1 ? 4u : 0u); }
                     }
-                    // P over the scores it came from: piece pc lands in columns this thread has already read
-                    tmem_st8(scol + 8 * pc, pk);
                 }
             }
-            tmem_st_wait();
-            tc_fence_before();
-            mbar_arrive(bar_p_of(n));
-            if (!mapped) {
-                ++ci[2];
-                dirty = 4u;
-                if (ci[2] == nc2) {
-                    ci[2] = 0; ++ci[1]; dirty = nc2 > 1 ? 6u : 2u;
-                    if (ci[1] == nc1) { ci[1] = 0; ++ci[0]; dirty = 1u | (nc1 > 1 ? 2u : 0u) | (nc2 > 1 ? 4u : 0u); }
-                }
-            }
-        }
 
-        // ---- normalise and write out ----
-        ok = mbar_wait(bar_o, t & 1, abort_flag, P.wait_budget) && ok;
-        tc_fence_after();
-        {
-            const bool live = valid_q && ok;
-            const float inv = (live && l > 0.f) ? 1.f / l : 0.f;
-            // A thread holds a row, but 32 rows written 16 bytes at a time are 32 lines per store instruction (the stores of
-            // the tile kept the load / store unit busy for 4200 cycles, 15 % of the kernel).  Four lanes exchange their
-            // 16-byte pieces of 32 channels, so that a store writes 64 bytes of each of eight rows.
-            const long long my_row = in_tensor ? out_row : -1;
-            long long rows4[4];
+            // ---- normalise and write out ----
+            ok = mbar_wait(bar_o, t & 1, abort_flag, P.wait_budget) && ok;
+            tc_fence_after();
+            {
+                const bool live = valid_q && ok;
+                const float inv = (live && l > 0.f) ? 1.f / l : 0.f;
+                // A thread holds a row, but 32 rows written 16 bytes at a time are 32 lines per store instruction (the stores of
+                // the tile kept the load / store unit busy for 4200 cycles, 15 % of the kernel).  Four lanes exchange their
+                // 16-byte pieces of 32 channels, so that a store writes 64 bytes of each of eight rows.
+                const long long my_row = in_tensor ? out_row : -1;
+                long long rows4[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) rows4[i] = __shfl_sync(0xffffffffu, my_row, (lane & ~3) | i);
-            const int piece = lane & 3;
+                for (int i = 0; i < 4; ++i) rows4[i] = __shfl_sync(0xffffffffu, my_row, (lane & ~3) | i);
+                const int piece = lane & 3;
 #pragma unroll
-            for (int part = 0; part < DH / 32; ++part) {
-                if (32 * part >= P.dreal) break;             // padded channels are not part of the output
-                uint32_t o[32], w[4][4];
-                tmem_ld32(trow + kColO + 32 * part, o);
-                tmem_ld_wait();
+                for (int part = 0; part < DH / 32; ++part) {
+                    if (32 * part >= P.dreal) break;             // padded channels are not part of the output
+                    uint32_t o[32], w[4][4];
+                    tmem_ld32(trow + kColO + 32 * part, o);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        w[i][j] = live ? cvt_pack<BF16>(__uint_as_float(o[8 * i + 2 * j]) * inv, __uint_as_float(o[8 * i + 2 * j + 1]) * inv) : 0u;
-                transpose4(w, piece);                        // w[i]: this lane's piece of row i of the four
+                        for (int j = 0; j < 4; ++j)
+                            w[i][j] = live ? cvt_pack<BF16>(__uint_as_float(o[8 * i + 2 * j]) * inv, __uint_as_float(o[8 * i + 2 * j + 1]) * inv) : 0u;
+                    transpose4(w, piece);                        // w[i]: this lane's piece of row i of the four
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (rows4[i] >= 0 && 32 * part + 8 * piece < P.dreal)
-                        reinterpret_cast<uint4*>(out + rows4[i] * P.dreal)[4 * part + piece] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+                    for (int i = 0; i < 4; ++i)
+                        if (rows4[i] >= 0 && 32 * part + 8 * piece < P.dreal)
+                            reinterpret_cast<uint4*>(out + rows4[i] * P.dreal)[4 * part + piece] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+                }
+                // natural-log lse of scale * logits
+                if (in_tensor)
+                    lse[out_row] = (live && l > 0.f) ? (m * P.scale_log2 + log2f(l)) * 0.6931471805599453f : 0.f;
             }
-            // natural-log lse of scale * logits
-            if (in_tensor)
-                lse[out_row] = (live && l > 0.f) ? (m * P.scale_log2 + log2f(l)) * 0.6931471805599453f : 0.f;
-        }
-        // the next tile's first P V is issued only after this thread has stored its next P
-        tc_fence_before();
+            // the next tile's first P V is issued only after this thread has stored its next P
+            tc_fence_before();
         }
     }
 

@@ -87,10 +87,8 @@ __device__ __forceinline__ void raise_status(const Params& P)
 // n / d with a precomputed multiplier; exact while n * d < 2^32 (checked on the host).
 __device__ __forceinline__ unsigned fast_div(unsigned n, unsigned mul) { return mul ? __umulhi(n, mul) : n; }
 
-// Block index -> dilation residues rg, tile origin, sub-grid extents Lp (innermost axis fastest,
-// dilation group slowest); returns whether the tile holds any row of this sample.
-__device__ __forceinline__ bool cta_geometry(const TcParams& P, unsigned bx, int b, int (&rg)[3],
-                                             int (&origin)[3], int (&Lp)[3])
+// Block index -> tile origin and dilation residues rg (innermost axis fastest, dilation group slowest).
+__device__ __forceinline__ void tile_of_block(const TcParams& P, unsigned bx, int (&rg)[3], int (&origin)[3])
 {
     unsigned x = bx;
 #pragma unroll
@@ -99,43 +97,45 @@ __device__ __forceinline__ bool cta_geometry(const TcParams& P, unsigned bx, int
         origin[a] = static_cast<int>(x - q * P.ntile[a]) * P.tile[a];
         x = q;
     }
-    bool active = true;
 #pragma unroll
     for (int a = 2; a >= 0; --a) {
         const unsigned q = fast_div(x, P.grp_mul[a]);
         rg[a] = static_cast<int>(x - q * P.grp_n[a]) * P.grp_step[a];
         x = q;
-        const int ea = a - (3 - P.rank);
-        const int Ls = (P.extents && ea >= 0) ? P.extents[b * P.rank + ea] : P.L[a];
-        Lp[a] = rg[a] < Ls ? static_cast<int>(fast_div(Ls - rg[a] + P.dil[a] - 1, P.dil_mul[a])) : 0;
+    }
+}
+
+// Extent along axis a of the sample's sub-grid of residue rg.
+__device__ __forceinline__ int sub_grid_extent(const TcParams& P, int a, int b, int rg)
+{
+    const int ea = a - (3 - P.rank);
+    const int Ls = (P.extents && ea >= 0) ? P.extents[b * P.rank + ea] : P.L[a];
+    return rg < Ls ? static_cast<int>(fast_div(Ls - rg + P.dil[a] - 1, P.dil_mul[a])) : 0;
+}
+
+// A block's tile and the sample's extents there; returns whether the tile holds any row of this sample.
+__device__ __forceinline__ bool cta_geometry(const TcParams& P, unsigned bx, int b, int (&rg)[3],
+                                             int (&origin)[3], int (&Lp)[3])
+{
+    tile_of_block(P, bx, rg, origin);
+    bool active = true;
+#pragma unroll
+    for (int a = 2; a >= 0; --a) {
+        Lp[a] = sub_grid_extent(P, a, b, rg[a]);
         if (origin[a] >= Lp[a]) active = false;
     }
     return active;
 }
 
-// What cta_geometry works out, one axis per lane (lane 2 and up: the innermost one): a third of the instructions, which counts where
-// they run for the first time and come from memory.  Returns whether the tile holds a row of the sample along the lane's axis.
+// The same, one axis per lane (lane 2 and up: the innermost one): a third of the instructions, which counts where they run for the
+// first time and come from memory.  Returns whether the tile holds a row of the sample along the lane's axis.
 __device__ __forceinline__ bool lane_geometry(const TcParams& P, unsigned bx, int b, int a, int& rg, int& origin, int& Lp)
 {
-    unsigned x = bx;
     int o[3], r[3];
-#pragma unroll
-    for (int i = 2; i >= 0; --i) {
-        const unsigned q = fast_div(x, P.ntile_mul[i]);
-        o[i] = static_cast<int>(x - q * P.ntile[i]) * P.tile[i];
-        x = q;
-    }
-#pragma unroll
-    for (int i = 2; i >= 0; --i) {
-        const unsigned q = fast_div(x, P.grp_mul[i]);
-        r[i] = static_cast<int>(x - q * P.grp_n[i]) * P.grp_step[i];
-        x = q;
-    }
+    tile_of_block(P, bx, r, o);
     rg = a == 0 ? r[0] : a == 1 ? r[1] : r[2];
     origin = a == 0 ? o[0] : a == 1 ? o[1] : o[2];
-    const int ea = a - (3 - P.rank);
-    const int Ls = (P.extents && ea >= 0) ? P.extents[b * P.rank + ea] : P.L[a];
-    Lp = rg < Ls ? static_cast<int>(fast_div(Ls - rg + P.dil[a] - 1, P.dil_mul[a])) : 0;
+    Lp = sub_grid_extent(P, a, b, rg);
     return origin < Lp;
 }
 

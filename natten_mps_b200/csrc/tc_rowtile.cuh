@@ -1,6 +1,6 @@
-// Row tiles of the persistent tensor-core kernels (fused backward, both sides; double-buffered fused forward):
-// geometry of one work item (128 rows of one (batch, head) and the box of columns their windows or inverse
-// windows cover) and the tables a helper warp publishes one tile ahead.
+// Row tiles of the fused backward on tensor cores, both sides: geometry of one work item (128 rows of one
+// (batch, head) and the box of columns their windows or inverse windows cover) and the tables that the geometry
+// warp publishes one tile ahead.
 #pragma once
 #include "tc_plan.cuh"
 
@@ -14,15 +14,6 @@ constexpr int kCols = 64;                   // columns per chunk
 constexpr int kAxisEntries = 130;           // entries of a tile's axis table: tile[0] + tile[1] + tile[2] <= 128 + 1 + 1
 
 __device__ __forceinline__ int ws1(int p, int L, int K) { return window_start(p, L, K, 1); }
-
-// Geometry of one work item: a tile of 128 rows (queries | keys) of one (batch, head).
-struct BwdTile {
-    int b, hy;                 // batch; head of the row tensors (query head | kv head)
-    int rg[3], origin[3], Lp[3], boxlo[3], nc[3];
-    int nchunks;               // chunks of the column box
-    int nbox, total;           // column passes: box chunks x query heads of the group, then additional tokens
-    bool active;
-};
 
 // What a compute thread needs to know about its row of a tile is separable: along every axis the row's
 // coordinate alone decides its position in the tensor, whether it exists, and its valid column range.  The
@@ -42,46 +33,25 @@ struct TileHead {
 constexpr int kHeadBytes = 96, kMapBytes = 8 * kTileRows, kTabBytes = kHeadBytes + kMapBytes + 16 * kAxisEntries;
 static_assert(sizeof(TileHead) <= kHeadBytes, "the tile head has 96 bytes in front of the tables");
 
+// Batch and (first) head of a work item's rows, and its block index among the tiles of that head.
 template <bool kKeySide>
-__device__ __forceinline__ void bwd_tile_setup(const TcParams& P, unsigned work, BwdTile& T)
+__device__ __forceinline__ unsigned split_work(const TcParams& P, unsigned work, int& b, int& hy)
 {
-    const unsigned hb = work / P.per_head;
-    const unsigned bx = work - hb * P.per_head;
-    const unsigned H = (unsigned)(kKeySide ? P.Hkv : P.Hq >> P.pack_log);
-    T.b = (int)(hb / H);
-    T.hy = (int)(hb - (unsigned)T.b * H) << (kKeySide ? 0 : P.pack_log);
-    T.active = cta_geometry(P, bx, T.b, T.rg, T.origin, T.Lp);
-    T.nchunks = 1;
-    if (T.active) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const int last = T.origin[a] + P.tile[a] - 1 < T.Lp[a] - 1 ? T.origin[a] + P.tile[a] - 1 : T.Lp[a] - 1;
-            int hi;
-            if (kKeySide) {
-                int t;
-                inverse_range(T.origin[a], T.Lp[a], P.K[a], P.causal[a], T.boxlo[a], t, /*exact=*/false);
-                inverse_range(last, T.Lp[a], P.K[a], P.causal[a], t, hi, /*exact=*/false);
-            } else {
-                T.boxlo[a] = P.causal[a] ? T.origin[a] - (P.K[a] - 1) : ws1(T.origin[a], T.Lp[a], P.K[a]);
-                hi = P.causal[a] ? last : ws1(last, T.Lp[a], P.K[a]) + P.K[a] - 1;
-            }
-            T.nc[a] = chunks_along(P, a, hi - T.boxlo[a] + 1);
-            T.nchunks *= T.nc[a];
-        }
-    }
-    T.nbox = T.nchunks * (kKeySide ? P.group : 1);
-    T.total = T.nbox + (kKeySide ? 0 : ((P.n_extra + kCols - 1) >> 6));
+    const unsigned hb = work / P.per_head, heads = (unsigned)(kKeySide ? P.Hkv : P.Hq >> P.pack_log);
+    b = (int)(hb / heads);
+    hy = (int)(hb - (unsigned)b * heads) << (kKeySide ? 0 : P.pack_log);
+    return work - hb * P.per_head;
 }
 
-// The work item into the head of a slot, by one warp (what bwd_tile_setup gives, an axis per lane); returns whether it is active.
+// The work item into the head of a slot, by one warp, an axis per lane; returns whether it holds a row of the sample.
 // rows16: chunks of 16-column rows.
 template <bool kKeySide>
 __device__ __forceinline__ bool publish_tile(const TcParams& P, unsigned work, bool rows16, int lane, TileHead* H)
 {
-    const unsigned hb = work / P.per_head, heads = (unsigned)(kKeySide ? P.Hkv : P.Hq >> P.pack_log);
-    const int b = (int)(hb / heads), hy = (int)(hb - (unsigned)b * heads) << (kKeySide ? 0 : P.pack_log), a = lane < 2 ? lane : 2;
-    int rg, origin, Lp;
-    if (!__all_sync(0xffffffffu, lane_geometry(P, work - hb * P.per_head, b, a, rg, origin, Lp))) return false;
+    int b, hy, rg, origin, Lp;
+    const unsigned bx = split_work<kKeySide>(P, work, b, hy);
+    const int a = lane < 2 ? lane : 2;
+    if (!__all_sync(0xffffffffu, lane_geometry(P, bx, b, a, rg, origin, Lp))) return false;
     const int last = origin + P.tile[a] - 1 < Lp - 1 ? origin + P.tile[a] - 1 : Lp - 1;
     int boxlo, hi;
     if (kKeySide) {

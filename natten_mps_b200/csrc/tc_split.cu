@@ -716,8 +716,7 @@ struct SmemG {
     static constexpr int kX = 0;                          // [kStages] query chunks
     static constexpr int kBar = kX + kStages * kTile;     // barriers, flags: 128 bytes
     static constexpr int kColRow = kBar + 128;            // [2][128] long long: element offset of the column's row of w, -1 = no query
-    static constexpr int kColFirst = kColRow + 2048;      // [2][3][128] int: first key of the column's window, per axis
-    static constexpr int kTotal = kColFirst + 3072;
+    static constexpr int kTotal = kColRow + 2048;
     static constexpr int kPBufs = DH == 64 ? 1 : 2, kPerSm = DH == 64 ? 3 : 1;
     static constexpr uint32_t kColP = 0, kColO = 64 * kPBufs, kTmemCols = kColO + DH;
 };

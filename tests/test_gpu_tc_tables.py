@@ -1,5 +1,6 @@
 """Tile tables of the tcgen05 forward: shapes at the edges of what the tables hold (one row per warp lane, tiles of one column,
-more chunks than a row map has room for, volumes, output stride, padding tiles), against the general kernels."""
+more chunks than a row map has room for, volumes, output stride, padding tiles), against the general kernels.  These calls have few
+tiles, so head dims up to 64 run the form with two score buffers; test_gpu_tc_many_tiles.py has the same shapes in the other form."""
 import pytest
 import torch
 
