@@ -345,8 +345,8 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         }
         // ---- the tile is complete: coalesced copy to the output ----
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (ok) {
-            // consecutive threads copy consecutive elements of a row: 256 elements ahead = dr rows and dj slots
+        // consecutive threads copy consecutive elements of a row: 256 elements ahead = dr rows and dj slots
+        auto copy_out = [&](auto biased) {
             int r = tid / ktot, j = tid - r * ktot;
             const int dr = 256 / ktot, dj = 256 - dr * ktot;
             const int total = kTileRows * ktot;
@@ -355,7 +355,7 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 const long long off = rowout[r];
                 if (off >= 0) {
                     uint16_t v = tile[idx];
-                    if (rpb) {                   // masked slots hold -inf and stay -inf
+                    if constexpr (decltype(biased)::value) {     // masked slots hold -inf and stay -inf
                         const uint32_t bv = rpb[(long long)h * rpb_table + rowpb[r] + slotpb[j]];
                         const float x = BF16 ? __uint_as_float(static_cast<uint32_t>(v) << 16) : __half2float(__ushort_as_half(v));
                         const float y = BF16 ? __uint_as_float(bv << 16) : __half2float(__ushort_as_half(static_cast<unsigned short>(bv)));
@@ -367,7 +367,10 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 j += dj;
                 if (j >= ktot) { j -= ktot; ++r; }
             }
-        }
+        };
+        // (a loop each: with the question inside it, 61 x 67, 9 x 9, 8 heads of 64, batch 2, 28 us or 22 as the compiler saw fit)
+        if (ok && rpb) copy_out(std::true_type{});
+        else if (ok) copy_out(std::false_type{});
     }
 
     if (*abort_flag) abort_grace_sleep();       // loads of a wait that gave up may still be landing
