@@ -167,9 +167,9 @@ int natten_host_status(int device);
 int natten_clear_status(void);
 int natten_status_async(int32_t* pinned_host_word, void* stream);
 /* Test hook: cycle budget of those waits (<= 0 restores the default of about two seconds) and a
- * host-side fault to inject into the following launches (0 = none; 1 = the fused forward's first
- * barrier expects more bytes than its loads deliver, so its wait runs out and the kernel
- * returns with the status word set; 2 = the device reports no room for a cluster of more than
+ * host-side fault to inject into the following launches (0 = none; 1 = the barrier of a CTA's
+ * first row tile (split operators: column tile) expects more bytes than its loads deliver, so its
+ * wait runs out and the kernel returns with the status word set; 2 = the device reports no room for a cluster of more than
  * eight CTAs, 3 = for none).  Process-wide.                                                    */
 void natten_debug_wait(long long budget_cycles, int inject);
 

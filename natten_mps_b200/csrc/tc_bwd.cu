@@ -187,7 +187,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             // =====================================================================
             // The whole warp runs the loop (warp-uniform code); the tensor-core instructions execute on one elected lane.
             const uint32_t leader = elect_one();
-            if (!*abort_flag) {
+            if (!gave_up(abort_flag)) {
                 const bool second = warp != kComputeWarps;
                 constexpr uint32_t idesc_kk = instr_desc(BF16 ? 1 : 0, kCols, 0, 0);    // both operands K-major
                 constexpr uint32_t idesc_acc = instr_desc(BF16 ? 1 : 0, DH, 0, 1);      // A from TMEM, B MN-major
@@ -286,7 +286,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             // loads: row tiles as soon as the previous tile's last S / dP product has finished, then the ring of column tiles,
             // as far ahead of the tensor cores as the stages allow.  Rows of padding tiles (per-sample extents) are zeroed in between.
             // =====================================================================
-            bool ok = !*abort_flag;
+            bool ok = !gave_up(abort_flag);
             unsigned stage = 0, parity = 1, g = 0;       // parity: of the stage's last release
             unsigned zw = blockIdx.x;                    // next work item to look at for padding
             auto zero_one = [&]() {
@@ -334,7 +334,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 if (t > 0) ok = mbar_wait(bar_rowfree, (t - 1) & 1, abort_flag, P.wait_budget);
                 if (!ok) break;
                 if (lane == 0) {
-                    mbar_expect_tx(bar_row, 2 * kTile);
+                    mbar_expect_tx(bar_row, 2 * kTile + ((P.inject == 1 && t == 0) ? 16u : 0u));
 #pragma unroll
                     for (int hf = 0; hf < Smem::kHalves; ++hf) {
                         tma_load_rows(sbase + Smem::kR1 + hf * kRowHalf, &tmR1, bar_row, P, hy, 64 * hf, R[2], R[1], R[0], b);
@@ -372,7 +372,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             // geometry: tables one tile ahead; on the key side also the column statistics (lse*log2e and delta of the chunk's
             // queries) that go with each column tile, fetched a chunk ahead
             // =====================================================================
-            bool ok = !*abort_flag;
+            bool ok = !gave_up(abort_flag);
             unsigned w = blockIdx.x, stage = 0, parity = 1, g = 0;
             auto publish = [&](unsigned t) -> bool {     // the next work item with rows of a sample -> slot t & 1; false: none is left
                 if (t >= 2) ok = ok && mbar_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
@@ -468,7 +468,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
             // All of them or none where the stores are behind a barrier of theirs; without one a warp goes by itself.
             const bool apart = kShort && P.shared_box;
-            if (apart ? !__all_sync(0xffffffffu, ok) : any_of_compute(!ok)) break;
+            if (apart ? !ok : any_of_compute(!ok)) break;
             const uint8_t* tab = tab_slot(t);
             const TileHead* H = reinterpret_cast<const TileHead*>(tab);
             const int total = H->total;

@@ -160,7 +160,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             // does between a chunk's last probability and the next chunk's scores is on the chain of every chunk, so the loads
             // and the geometry are the loader's, descriptors are ready and the next chunk's operands have been waited for.
             // =====================================================================
-            if (!*abort_flag) {
+            if (!gave_up(abort_flag)) {
                 constexpr uint32_t idesc_qk = instr_desc(BF16 ? 1 : 0, kKeys, 0, 0);
                 constexpr uint32_t idesc_pv = instr_desc(BF16 ? 1 : 0, DH, 0, 1);
                 const uint64_t dq0 = smem_desc(sbase + kOffQ, 16, 1024);
@@ -245,7 +245,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             // =====================================================================
             // Loads: Q of a tile, then its chunks; both run ahead across tile boundaries as far as the buffers allow.
             // =====================================================================
-            if (!*abort_flag) {
+            if (!gave_up(abort_flag)) {
                 bool ok = true;
                 unsigned n = 0;                                  // chunks loaded
                 for (unsigned t = 0;; ++t) {
@@ -303,7 +303,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             // Geometry: the CTA's tiles (blockIdx.x, + gridDim.x, ...), each one's tables as soon as its slot is free.  Rows of padding
             // tiles (per-sample extents) are zeroed here.
             // =====================================================================
-            if (!*abort_flag) {
+            if (!gave_up(abort_flag)) {
                 auto zero_rows = [&](const Cursor& at) {     // rows of a padding tile that exist in the output are zero
                     for_each_row(P, at, lane, [&](long long out_row) {
                         uint4* o4 = reinterpret_cast<uint4*>(out + out_row * P.dreal);
@@ -481,7 +481,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 scol = trow + kColS + s_cols(n);
                 ok = ok && mbar_wait(bar_s_of(n), par_of(n), abort_flag, P.wait_budget);     // one score buffer: every earlier product has finished, too
                 tc_fence_after();
-                if (!__all_sync(0xffffffffu, ok)) { words[0] = 0u; words[1] = 0u; act = 0u; dirty = 7u; }
+                if (!ok) { words[0] = 0u; words[1] = 0u; act = 0u; dirty = 7u; }
 
                 uint32_t stored = 0u;            // pieces of this chunk that hold probabilities (bit per piece)
                 // one 16-column piece on the general path: scores s, validity bits wd -> probabilities pk

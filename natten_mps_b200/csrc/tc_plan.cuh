@@ -56,7 +56,7 @@ struct TcParams {
     // q_split: the maps of the rows have the head as an axis of their own.
     int pack_log, q_split;
     long long wait_budget; // cycles a barrier wait may take before the CTA gives up
-    int inject;            // test hook: 1 = the forward's first query barrier expects bytes that never arrive
+    int inject;            // test hook: 1 = the barrier of a CTA's first row tile (split operators: column tile) expects bytes that never arrive
     // Output stride (forward only).  Inside dilation group r of an axis the queries sit at the
     // sub-grid indices x = qx0[axis][r] + qstep[axis] * i, i = 0, 1, ... (qx0 < 0: the group holds no
     // query); with stride 1 that is every index.  Output position = input position / st.

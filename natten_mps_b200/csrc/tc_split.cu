@@ -166,7 +166,7 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     auto issue_y = [&]() {
         const int s = loaded % kStages;
         const uint32_t bar = bar_y + 8 * s;
-        mbar_expect_tx(bar, SM::kTile);
+        mbar_expect_tx(bar, SM::kTile + ((P.inject == 1 && loaded == 0) ? 16u : 0u));
         int X[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) X[a] = rg[a] + P.dil[a] * (lo[a] + ld[a] * P.cb[a]);
@@ -264,7 +264,7 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     if (warp == 8) {
         // the warp runs the loop converged; the tensor-core instructions execute on an elected lane
         const uint32_t leader = elect_one();
-        if (!*abort_flag) {
+        if (!gave_up(abort_flag)) {
             constexpr uint32_t idesc = instr_desc(BF16 ? 1 : 0, kChunk, 0, 0);
             const uint64_t dx0 = smem_desc(sbase + SM::kX, 16, 1024);
             auto issue_s = [&](int c) {
@@ -477,7 +477,7 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
     auto issue_y = [&]() {
         const int s = loaded % kStages;
         const uint32_t bar = bar_y + 8 * s;
-        mbar_expect_tx(bar, SM::kTile);
+        mbar_expect_tx(bar, SM::kTile + ((P.inject == 1 && loaded == 0) ? 16u : 0u));
         int X[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) X[a] = G.rg[a] + P.dil[a] * (G.lo[a] + ld[a] * P.cb[a]);
@@ -531,7 +531,7 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
     if (warp == 8) {
         // the warp runs the loop converged; the tensor-core instructions execute on an elected lane
         const uint32_t leader = elect_one();
-        if (!*abort_flag) {
+        if (!gave_up(abort_flag)) {
             constexpr uint32_t idesc = instr_desc(BF16 ? 1 : 0, DH, 0, 1);      // A = P from TMEM, B = Y MN-major
             bool ok = true;
             for (int c = 0; c < nch && ok; ++c) {
@@ -763,7 +763,7 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     auto issue_x = [&]() {
         const int s = loaded % kStages;
         const uint32_t bar = bar_x + 8 * s;
-        mbar_expect_tx(bar, SM::kTile);
+        mbar_expect_tx(bar, SM::kTile + ((P.inject == 1 && loaded == 0) ? 16u : 0u));
         int X[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) X[a] = rg[a] + P.dil[a] * (boxlo[a] + ld[a] * P.cb[a]);
@@ -825,7 +825,7 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     if (warp == 8) {
         // the warp runs the loop converged; the tensor-core instructions execute on an elected lane
         const uint32_t leader = elect_one();
-        if (!*abort_flag) {
+        if (!gave_up(abort_flag)) {
             constexpr uint32_t idesc = instr_desc(BF16 ? 1 : 0, DH, 0, 1);      // A = P^T from TMEM, B = X MN-major
             bool ok = true;
             for (int c = 0; c < total && ok; ++c) {

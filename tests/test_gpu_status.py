@@ -60,6 +60,56 @@ def test_wait_that_runs_out_is_reported_and_recoverable():
     assert err <= 2e-2, err
 
 
+def same_after_giving_up(call):
+    """The call's kernels run out of their waits, say so and return; the call after that is as good as the one before."""
+    try:
+        _cabi.set_force("tc")
+        want = call()
+        _cabi.lib().natten_debug_wait(400_000, 1)
+        call()
+        assert _cabi.last_path() == "tcgen05"
+        torch.cuda.synchronize()
+        assert _cabi.device_status() == -4
+        _cabi.lib().natten_debug_wait(0, 0)
+        _cabi.clear_status()
+        got = call()
+        torch.cuda.synchronize()
+        assert _cabi.device_status() == 0
+    finally:
+        _cabi.lib().natten_debug_wait(0, 0)
+        _cabi.set_force(None)
+        _cabi.clear_status()
+    for a, b in zip(got, want):
+        assert (a is None and b is None) or torch.equal(a, b)
+
+
+# A wait that gives up raises a flag which the CTA's other warps, each at a wait of its own, find when they next look: every role
+# has to reach the end whichever of its lanes saw the flag first.
+@pytest.mark.parametrize("B", [1, 24], ids=["few", "many"])
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("K,sizes", [((7, 7), None), ((3, 40), None), ((7, 7), (9, 40))], ids=["rows16", "line", "lengths"])
+def test_every_role_ends_when_a_wait_runs_out(K, sizes, D, B):
+    q, k, v = _case(B=B, H=24, W=48, heads=4, D=D, dtype=torch.float16)
+    go = _case(seed=5, B=B, H=24, W=48, heads=4, D=D, dtype=torch.float16)[0]
+    ext = None if sizes is None else torch.tensor([sizes] * B, dtype=torch.int32, device="cuda")
+    args = (K, (1, 1), (1, 1), (False, False), D ** -0.5)
+    same_after_giving_up(lambda: _backend.fused_forward(q, k, v, *args, extents=ext))
+    out, lse = _backend.fused_forward(q, k, v, *args, extents=ext)
+    same_after_giving_up(lambda: _backend.fused_backward(q, k, v, out, lse, go, *args, extents=ext))
+
+
+@pytest.mark.parametrize("D,K", [(64, (7, 7)), (64, (11, 11)), (128, (7, 7))], ids=["d64", "d64_two_buffers", "d128"])
+def test_every_role_of_the_split_operators_ends(D, K):
+    q, k, v = _case(B=2, H=24, W=48, heads=4, D=D, dtype=torch.float16)
+    geo = (K, (1, 1), (1, 1), (False, False))
+    logits = _backend.qk_forward(q, k, *geo, None)
+    w = torch.softmax(logits.float(), -1).half()
+    same_after_giving_up(lambda: [_backend.qk_forward(q, k, *geo, None)])
+    same_after_giving_up(lambda: [_backend.av_forward(w, v, *geo)])
+    same_after_giving_up(lambda: _backend.qk_backward(logits, q, k, *geo, None))
+    same_after_giving_up(lambda: _backend.av_backward(q, w, v, *geo))
+
+
 def test_status_words_on_the_host_and_on_the_stream():
     """The word that the kernel itself writes into host memory, and the copy that a caller queues behind it."""
     q, k, v = _case(seed=1)
