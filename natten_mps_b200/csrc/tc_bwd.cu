@@ -208,7 +208,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 unsigned acc_stage = 0;
                 bool ok = true;
                 for (unsigned t = 0; ok; ++t) {
-                    ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
+                    ok = warp_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
                     const TileHead* H = reinterpret_cast<const TileHead*>(tab_slot(t));
                     const int total = H->total;
@@ -237,7 +237,6 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                                              boxlo[2] + chunk_coord(P, 2, c2, 0)};
                         uint8_t* tile = smem + col_tiles + stage * kColTile;
                         if (leader) zero_rows_past_extent(P, box0, Lp, kCols, Smem::kHalves, kColHalf, tile, tile);
-                        __syncwarp();
                     };
                     auto issue_s_dp = [&](unsigned gg, bool last) {
                         const uint64_t dC = dCol0 + stage * (kColTile >> 4);
@@ -253,9 +252,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     };
                     ok = mbar_wait(bar_row, t & 1, abort_flag, P.wait_budget);
                     wait_columns(0);
-                    if (!ok) break;
                     tc_fence_after();
-                    issue_s_dp(g, total == 1);
+                    if (ok) issue_s_dp(g, total == 1);
                     for (int cc = 0; cc < total; ++cc, ++g) {
                         const bool more = cc + 1 < total;
                         if (more) wait_columns(cc + 1);
@@ -279,6 +277,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                         if (++acc_stage == kStages) acc_stage = 0;
                         if (!kTwoBuf && more) issue_s_dp(g + 1, cc + 2 == total);       // ... before the next S/dP overwrite them
                     }
+                    // the lanes agree once a tile: nothing in between is for the whole warp, and a vote there is on every chunk's chain
+                    if (!__all_sync(0xffffffffu, ok)) break;
                 }
             }
         } else if (warp == kComputeWarps + 1) {
@@ -318,7 +318,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 }
             };
             for (unsigned t = 0; ok; ++t) {
-                ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
+                ok = warp_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
                 if (!ok) break;
                 const TileHead* H = reinterpret_cast<const TileHead*>(tab_slot(t));
                 const int total = H->total, nbox = H->nbox, b = H->b, hy = H->hy, nc0 = H->nc[0], nc1 = H->nc[1], nc2 = H->nc[2];
@@ -331,7 +331,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                 __syncwarp();                            // every lane has read the head
                 if (lane == 0) mbar_arrive(bar_tab_empty + 8 * (t & 1));
                 if (total == 0) break;
-                if (t > 0) ok = mbar_wait(bar_rowfree, (t - 1) & 1, abort_flag, P.wait_budget);
+                if (t > 0) ok = warp_wait(bar_rowfree, (t - 1) & 1, abort_flag, P.wait_budget);
                 if (!ok) break;
                 if (lane == 0) {
                     mbar_expect_tx(bar_row, 2 * kTile + ((P.inject == 1 && t == 0) ? 16u : 0u));
@@ -349,7 +349,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
                     const bool box = cc < nbox;          // else additional tokens (rows past n_extra are zero-filled)
                     const int x0 = box ? Y[0] + P.dil[0] * chunk_coord(P, 0, c0, 0) : 0, x1 = box ? Y[1] + P.dil[1] * chunk_coord(P, 1, c1, 0) : 0,
                               x2 = box ? Y[2] + P.dil[2] * chunk_coord(P, 2, c2, 0) : (cc - nbox) * kCols;
-                    if (g >= (unsigned)kStages) ok = mbar_wait(bar_free + 8 * stage, parity, abort_flag, P.wait_budget);
+                    if (g >= (unsigned)kStages) ok = warp_wait(bar_free + 8 * stage, parity, abort_flag, P.wait_budget);
                     if (!ok) break;
                     if (lane == 0) {
                         const uint32_t bar = bar_col + 8 * stage;
@@ -375,7 +375,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             bool ok = !gave_up(abort_flag);
             unsigned w = blockIdx.x, stage = 0, parity = 1, g = 0;
             auto publish = [&](unsigned t) -> bool {     // the next work item with rows of a sample -> slot t & 1; false: none is left
-                if (t >= 2) ok = ok && mbar_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
+                if (t >= 2) ok = ok && warp_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
                 if (!ok) return false;
                 TileHead* H = reinterpret_cast<TileHead*>(tab_slot(t));
                 bool found = false;
@@ -438,7 +438,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
 #pragma unroll
                     for (int k = 0; k < kCols / 32; ++k) { l0[k] = nl[k]; d0[k] = nd[k]; }
                     if (cc + 1 < total) fetch();
-                    if (g >= (unsigned)kStages) ok = ok && mbar_wait(bar_free + 8 * stage, parity, abort_flag, P.wait_budget);
+                    if (g >= (unsigned)kStages) ok = ok && warp_wait(bar_free + 8 * stage, parity, abort_flag, P.wait_budget);
                     if (!ok) break;
                     float* st = stats + stage * 128;
 #pragma unroll
@@ -468,7 +468,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ 
             ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
             // All of them or none where the stores are behind a barrier of theirs; without one a warp goes by itself.
             const bool apart = kShort && P.shared_box;
-            if (apart ? !ok : any_of_compute(!ok)) break;
+            if (apart ? !__all_sync(0xffffffffu, ok) : any_of_compute(!ok)) break;
             const uint8_t* tab = tab_slot(t);
             const TileHead* H = reinterpret_cast<const TileHead*>(tab);
             const int total = H->total;

@@ -54,27 +54,31 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
     return ok != 0;
 }
 
-// Wait with a cycle budget, by all lanes of a warp together.  On expiry (or when another warp already gave up)
+// Wait with a cycle budget.  On expiry (or when another thread already gave up)
 // the shared abort flag is raised and the wait returns false; callers keep going
 // without touching the data so that the CTA always reaches its final barrier,
-// frees its TMEM and exits.
-// The result is the same for every lane: what follows a wait is code for whole warps (votes, shuffles, aligned
-// TMEM accesses), and with a result per lane a flag raised while the phase completes could send some lanes to the
-// final barrier and leave the others waiting for them.  (A phase that one lane has seen complete stays so for the
-// lanes that ask again: the next one cannot complete before this warp has gone on.)
+// frees its TMEM and exits.  The result is the calling lane's: a flag that is raised while the phase
+// completes may be seen by some lanes of a warp only, so no code for whole warps (votes, shuffles,
+// __syncwarp, the next tile) may depend on it before the lanes have agreed (warp_wait, or a vote).
 constexpr long long kWaitBudgetCycles = 4000000000ll;   // default budget: about two seconds
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           long long budget = kWaitBudgetCycles)
 {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     // sleep at most 0.2 ms per try, and never longer than about a quarter of a short budget
     const uint32_t nap = budget < 1600000ll ? static_cast<uint32_t>(budget >> 3) + 1000u : 200000u;
     while (true) {
-        if (__all_sync(0xffffffffu, mbar_try_wait_hint(bar, parity, nap))) return true;
-        if (__any_sync(0xffffffffu, *abort_flag || clock64() - t0 > budget)) { *abort_flag = 1; return false; }
+        if (mbar_try_wait_hint(bar, parity, nap)) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > budget) { *abort_flag = 1; return false; }
     }
+}
+// The same for a whole warp, and the same answer for each of its lanes.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, long long budget)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, budget));
 }
 // Has any wait of the CTA given up?  The same answer for every lane of the warp.
 __device__ __forceinline__ bool gave_up(const volatile int* abort_flag) { return __any_sync(0xffffffffu, *abort_flag != 0); }

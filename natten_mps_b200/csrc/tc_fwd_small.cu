@@ -170,7 +170,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 bool ok = true;
                 unsigned n_qk = 0, n_pv = 0;
                 for (unsigned t = 0;; ++t) {
-                    ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
+                    ok = warp_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
                     const FwdTile* H = tab_slot(t);
                     const int nch = H->nch;
@@ -192,7 +192,6 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         const int c2 = c % nc[2], c1 = c / nc[2] % nc[1], c0 = c / nc[2] / nc[1];
                         const int box0[3] = {lo[0] + chunk_coord(P, 0, c0, 0), lo[1] + chunk_coord(P, 1, c1, 0), lo[2] + chunk_coord(P, 2, c2, 0)};
                         if (leader) zero_rows_past_extent(P, box0, Lp, kKeys, kHalves, kKVHalf, tile, tile);
-                        __syncwarp();
                     };
                     auto wait_k = [&](int c) {       // chunk c's K has landed (and ends where the sample ends)
                         const unsigned s = n_qk & 1u;
@@ -213,9 +212,8 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     };
                     ok = mbar_wait(bar_q, t & 1, abort_flag, P.wait_budget);
                     wait_k(0);
-                    if (!ok) break;
                     tc_fence_after();
-                    issue_qk(nch == 1);
+                    if (ok) issue_qk(nch == 1);
                     for (int c = 0; c < nch; ++c) {
                         const bool more = c + 1 < nch;
                         if (more) wait_k(c + 1);
@@ -238,7 +236,10 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         if (!more) mma_commit_e(bar_o, leader);
                         ++n_pv;
                     }
-                    if (!ok) break;
+                    // the lanes agree once a tile, not at every wait: nothing in between is for the whole warp, and a vote there is on
+                    // every chunk's chain (8 lengths up to 16384, window 255, 16 heads of 128 on 4: key side 601 us without any, 606
+                    // like this, 611 with a vote in every wait)
+                    if (!__all_sync(0xffffffffu, ok)) break;
                 }
             }
         } else if (warp == 5) {
@@ -249,7 +250,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 bool ok = true;
                 unsigned n = 0;                                  // chunks loaded
                 for (unsigned t = 0;; ++t) {
-                    ok = mbar_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
+                    ok = warp_wait(bar_head + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
                     const FwdTile* H = tab_slot(t);
                     const int b = H->b, h = H->h, hk = H->hk, nnb = H->nnb, nch = H->nch, nc1 = H->nc[1], nc2 = H->nc[2];
@@ -260,7 +261,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     __syncwarp();                                // every lane has read the header
                     if (lane == 0) mbar_arrive(bar_tab_empty + 8 * (t & 1));
                     if (nch == 0) break;
-                    if (t > 0) ok = mbar_wait(bar_qfree, (t - 1) & 1, abort_flag, P.wait_budget);
+                    if (t > 0) ok = warp_wait(bar_qfree, (t - 1) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
                     if (lane == 0) {
                         mbar_expect_tx(bar_q, kQBytes + ((P.inject == 1 && t == 0) ? 16u : 0u));
@@ -275,7 +276,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                         const int x0 = box ? X0 + P.dil[0] * chunk_coord(P, 0, c0, 0) : 0, x1 = box ? X1 + P.dil[1] * chunk_coord(P, 1, c1, 0) : 0,
                                   x2 = box ? X2 + P.dil[2] * chunk_coord(P, 2, c2, 0) : (c - nnb) * kKeys;
                         if (++c2 == nc2) { c2 = 0; if (++c1 == nc1) { c1 = 0; ++c0; } }
-                        if (n >= (unsigned)kStages) ok = mbar_wait((kSplitKV ? bar_kfree : bar_vfree) + 8 * s, parity, abort_flag, P.wait_budget);
+                        if (n >= (unsigned)kStages) ok = warp_wait((kSplitKV ? bar_kfree : bar_vfree) + 8 * s, parity, abort_flag, P.wait_budget);
                         if (!ok) break;
                         const uint32_t full_k = bar_k + 8 * s, full_v = (kSplitKV ? bar_v : bar_k) + 8 * s;
                         if (lane == 0) {
@@ -285,7 +286,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                                 tma_load_heads(sbase + kOffK + s * kKVBytes + hf * kKVHalf, box ? &tmK : &tmEK, full_k, P, hk, 64 * hf, x2, x1, x0, b);
                         }
                         __syncwarp();
-                        if (kSplitKV && n >= (unsigned)kStages) ok = mbar_wait(bar_vfree + 8 * s, parity, abort_flag, P.wait_budget);
+                        if (kSplitKV && n >= (unsigned)kStages) ok = warp_wait(bar_vfree + 8 * s, parity, abort_flag, P.wait_budget);
                         if (!ok) break;
                         if (lane == 0) {
                             if (kSplitKV) mbar_expect_tx(full_v, kKVBytes);
@@ -317,7 +318,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 Cursor cur;
                 cur.init(P, blockIdx.x, gridDim.x);
                 for (unsigned t = 0; ok && found; ++t) {
-                    if (t >= 2) ok = mbar_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
+                    if (t >= 2) ok = warp_wait(bar_tab_empty + 8 * (t & 1), ((t >> 1) - 1) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
                     FwdTile* H = tab_slot(t);
                     found = false;
@@ -411,7 +412,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
         for (unsigned t = 0;; ++t) {
             ok = mbar_wait(bar_tab_full + 8 * (t & 1), (t >> 1) & 1, abort_flag, P.wait_budget) && ok;
-            if (!ok) break;
+            if (!__all_sync(0xffffffffu, ok)) break;
             const FwdTile* H = tab_slot(t);
             const int nch = H->nch;
             if (nch == 0) break;
@@ -481,7 +482,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 scol = trow + kColS + s_cols(n);
                 ok = ok && mbar_wait(bar_s_of(n), par_of(n), abort_flag, P.wait_budget);     // one score buffer: every earlier product has finished, too
                 tc_fence_after();
-                if (!ok) { words[0] = 0u; words[1] = 0u; act = 0u; dirty = 7u; }
+                if (!__all_sync(0xffffffffu, ok)) { words[0] = 0u; words[1] = 0u; act = 0u; dirty = 7u; }
 
                 uint32_t stored = 0u;            // pieces of this chunk that hold probabilities (bit per piece)
                 // one 16-column piece on the general path: scores s, validity bits wd -> probabilities pk

@@ -277,17 +277,17 @@ tc_scores_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 }
                 mma_commit_e(bar_s, leader);
             };
-            bool ok = mbar_wait(bar_x, 0, abort_flag, P.wait_budget) && mbar_wait(bar_y, 0, abort_flag, P.wait_budget);
+            bool ok = warp_wait(bar_x, 0, abort_flag, P.wait_budget) && warp_wait(bar_y, 0, abort_flag, P.wait_budget);
             if (ok) issue_s(0);
             for (int c = 0; c < nch && ok; ++c) {
-                ok = mbar_wait(bar_s, c & 1, abort_flag, P.wait_budget);            // the product is done: its Y stage is free
+                ok = warp_wait(bar_s, c & 1, abort_flag, P.wait_budget);            // the product is done: its Y stage is free
                 if (!ok) break;
                 if (c + kStages < nch && leader) issue_y();
                 __syncwarp();
-                ok = mbar_wait(bar_sp, c & 1, abort_flag, P.wait_budget);           // S(c) read by every thread
+                ok = warp_wait(bar_sp, c & 1, abort_flag, P.wait_budget);           // S(c) read by every thread
                 if (!ok) break;
                 if (c + 1 < nch) {
-                    ok = mbar_wait(bar_y + 8 * ((c + 1) % kStages), ((c + 1) / kStages) & 1, abort_flag, P.wait_budget);
+                    ok = warp_wait(bar_y + 8 * ((c + 1) % kStages), ((c + 1) / kStages) & 1, abort_flag, P.wait_budget);
                     if (!ok) break;
                     issue_s(c + 1);
                 }
@@ -535,8 +535,8 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
             constexpr uint32_t idesc = instr_desc(BF16 ? 1 : 0, DH, 0, 1);      // A = P from TMEM, B = Y MN-major
             bool ok = true;
             for (int c = 0; c < nch && ok; ++c) {
-                ok = mbar_wait(bar_y + 8 * (c % kStages), (c / kStages) & 1, abort_flag, P.wait_budget) &&
-                     mbar_wait(bar_p + 8 * buf_of(c), par_of(c), abort_flag, P.wait_budget);
+                ok = warp_wait(bar_y + 8 * (c % kStages), (c / kStages) & 1, abort_flag, P.wait_budget) &&
+                     warp_wait(bar_p + 8 * buf_of(c), par_of(c), abort_flag, P.wait_budget);
                 if (!ok) break;
                 const uint64_t dy0 = smem_desc(sbase + SM::kY + (c % kStages) * SM::kTile, SM::kHalf, 1024);
                 tc_fence_after();
@@ -546,7 +546,7 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
                 mma_commit_e(bar_o + 8 * buf_of(c), leader);
                 if (c >= 1 && c + 2 < nch) {             // the product before this one is done: its stage is free
                     // (one P buffer: the threads waited for it before they stored P(c))
-                    if (SM::kPBufs == 2) ok = mbar_wait(bar_o + 8 * buf_of(c - 1), par_of(c - 1), abort_flag, P.wait_budget);
+                    if (SM::kPBufs == 2) ok = warp_wait(bar_o + 8 * buf_of(c - 1), par_of(c - 1), abort_flag, P.wait_budget);
                     if (!ok) break;
                     if (leader) issue_y();
                     __syncwarp();
@@ -829,8 +829,8 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             constexpr uint32_t idesc = instr_desc(BF16 ? 1 : 0, DH, 0, 1);      // A = P^T from TMEM, B = X MN-major
             bool ok = true;
             for (int c = 0; c < total && ok; ++c) {
-                ok = mbar_wait(bar_x + 8 * (c % kStages), (c / kStages) & 1, abort_flag, P.wait_budget) &&
-                     mbar_wait(bar_p + 8 * buf_of(c), par_of(c), abort_flag, P.wait_budget);
+                ok = warp_wait(bar_x + 8 * (c % kStages), (c / kStages) & 1, abort_flag, P.wait_budget) &&
+                     warp_wait(bar_p + 8 * buf_of(c), par_of(c), abort_flag, P.wait_budget);
                 if (!ok) break;
                 const uint64_t dx0 = smem_desc(sbase + SM::kX + (c % kStages) * SM::kTile, SM::kHalf, 1024);
                 tc_fence_after();
@@ -840,7 +840,7 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 mma_commit_e(bar_o + 8 * buf_of(c), leader);
                 if (c >= 1 && c + 2 < total) {             // the product before this one is done: its stage is free
                     // (one P buffer: the threads waited for it before they stored P(c))
-                    if (SM::kPBufs == 2) ok = mbar_wait(bar_o + 8 * buf_of(c - 1), par_of(c - 1), abort_flag, P.wait_budget);
+                    if (SM::kPBufs == 2) ok = warp_wait(bar_o + 8 * buf_of(c - 1), par_of(c - 1), abort_flag, P.wait_budget);
                     if (!ok) break;
                     if (leader) issue_x();
                     __syncwarp();
