@@ -21,16 +21,17 @@
 // warps (independent streams: dP / acc1 and S / acc2), one that loads, one for the geometry (per-axis tables and row maps one
 // tile ahead; column statistics on the key side).
 // What bounds it: the round trip of a chunk (threads 700 to 1000 cycles, then the issuing warps and the products, 1300 to 1800)
-// with two tiles in flight, the tensor pipe busy for 45 % of it.  With one helper that loaded and did the geometry, tables held up
-// the row tiles and the loads.  Measured before | now (us, kernel alone, query side and key side): 64 x 64, 7 x 7, 8 heads of 64,
-// batch 8: 68.6, 87.5 | 61.3, 81.4; 128 x 128, 13 x 13, dilation 2, batch 4: 219, 278 | 199, 254; 16 x 32 x 32, 3 x 7 x 7 causal,
-// batch 2: 146, 187 | 131, 168; 8 lengths up to 16384, window 255, 16 heads of 128 on 4: 722, 712 | 580, 606 (query side 513 with
+// with two tiles in flight.  Counters at 64 x 64, 7 x 7: tensor pipe active in 32 % of the cycles, issue slots 43 and 44 %, DRAM 29 and
+// 25 %; head dim 128, window 255, one tile an SM: 36 and 49 %, 35 and 39 %, 28 and 19 %.  With one helper that loaded and did the geometry,
+// tables held up the row tiles and the loads.  Measured before | now (us, kernel alone, query side and key side): 64 x 64, 7 x 7, 8 heads
+// of 64, batch 8: 68.6, 87.5 | 59.5, 80; 128 x 128, 13 x 13, dilation 2, batch 4: 219, 278 | 195, 256; 16 x 32 x 32, 3 x 7 x 7 causal,
+// batch 2: 146, 187 | 126, 165; 8 lengths up to 16384, window 255, 16 heads of 128 on 4: 722, 712 | 580, 606 (query side 517 with
 // heads packed, see make_packed_plan).
 // Chunks of any shape (kInner = 0) are bound by how fast instructions arrive: the validity words and the unrolled halves are long code
 // that six roles share the instruction caches with.  When the geometry moved to a warp of its own, the key side of 3 x 3 x 3 windows
 // (9 short chunks a tile) went from 254 to 279 us (286 to 322 with padded heads; 12 x 40 x 40, 8 heads of 64 | 32, batch 2) with fewer
 // instructions executed, warps waiting for one four times as long (0.85 -> 3.3 of every issue).  One copy of the halves, of the two
-// outputs of the epilogue and of a segment of the validity words there: 238 and 264 (8 x 28 x 28 115 -> 98; 3 x 5 x 5 270 -> 263).  The
+// outputs of the epilogue and of a segment of the validity words there: 234 and 257 (8 x 28 x 28 115 -> 98; 3 x 5 x 5 270 -> 263).  The
 // query side, one accumulator, keeps both halves: 188 and 189, with one copy 192 and 194; so does head dim 128, with half as many warps on
 // an SM (8 lengths up to 16384, window 255, key side 600, with one copy 620).
 // TMEM: S [0,64)  dP [64,128)  acc1 [128,128+D)  acc2 [128+D,128+2D); head dim 128: second S [384,448) and

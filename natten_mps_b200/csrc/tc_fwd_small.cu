@@ -21,11 +21,12 @@
 // Eight warps: four of softmax (a warpgroup), one that issues the products, one that loads, one for the geometry, one idle (a
 // register split goes by warpgroups).  What bounds it is the chain of a chunk, not an issue rate: S -> softmax -> P -> the
 // issuing warp -> P V and the next S, about 2800 cycles of which the softmax is 1500; four tiles in flight per SM share the
-// gaps.  So whatever is not the chain is kept off the issuing warp and the softmax warps.  Measured on one B200 (us), one warp that
+// gaps.  Counters at 64 x 64, 7 x 7: issue slots 49 %, tensor pipe active in 26 % of the cycles, DRAM 26 %; head dim 128, window 255:
+// 40, 29, 21 %.  So whatever is not the chain is kept off the issuing warp and the softmax warps.  Measured on one B200 (us), one warp that
 // loaded, issued and did the geometry | loads and geometry apart (kernel alone): 64 x 64, 7 x 7, 8 heads of 64, batch 8,
-// bf16 61.7 | 50.3; 128 x 128, 13 x 13, dilation 2, batch 4 196 | 175; 16 x 32 x 32, 3 x 7 x 7, causal frames, batch 2 137 | 117 (104 with
-// its chunks interleaved, see make_plan); 135 x 241, 7 x 9, 6 heads of 32, batch 2, fp16 80 | 69; 8191 causal, window 255, 16 heads of
-// 128 on 4, batch 2 98 | 84.6 (74.5 with heads packed, see make_packed_plan).
+// bf16 61.7 | 50.2; 128 x 128, 13 x 13, dilation 2, batch 4 196 | 174; 16 x 32 x 32, 3 x 7 x 7, causal frames, batch 2 137 | 117 (103 with
+// its chunks interleaved, see make_plan); 135 x 241, 7 x 9, 6 heads of 32, batch 2, fp16 80 | 68; 8191 causal, window 255, 16 heads of
+// 128 on 4, batch 2 98 | 84.6 (74 with heads packed, see make_packed_plan).
 //
 // TMEM columns: head dim 64: S [0,64) (P over [0,32)), O [64,128);
 //               head dim 128: S of even chunks [0,64), of odd chunks [64,128), O [128,256).
@@ -158,7 +159,7 @@ tc_fwd_small_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             // =====================================================================
             // MMA issue.  The whole warp walks the CTA's tiles; the tensor-core instructions execute on one elected lane.  What it
             // does between a chunk's last probability and the next chunk's scores is on the chain of every chunk, so the loads
-            // and the geometry are the loader's, descriptors are ready and the next chunk's operands have been waited for.
+            // and the geometry are other warps', descriptors are ready and the next chunk's operands have been waited for.
             // =====================================================================
             if (!gave_up(abort_flag)) {
                 constexpr uint32_t idesc_qk = instr_desc(BF16 ? 1 : 0, kKeys, 0, 0);

@@ -13,13 +13,13 @@
 //     alone does the scalar work of that row (mask, exponential), and four shuffles hand the results back.
 // A pass over the columns of K = 7 x 7 costs 23 shared-memory cycles for 32 pairs of which 70 % are needed.
 //
-// Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, against the general SIMT kernels: float32 forward 30 us (185), dQ 38 (236),
-// dK and dV 67 (304); split operators in bf16: scores 25 (93), apply 24 (93), gather 31 (115); in float32: 25 (96), 24 (469),
-// 32 (152).
+// Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, against the general SIMT kernels: float32 forward 31 us (185), dQ 37 (236),
+// dK and dV 65 (304); split operators in bf16: scores 24 (93), apply 24 (93), gather 30 (115); in float32: 25 (96), 23 (469),
+// 28 (152).
 // What bounds them there: too few warps.  448 CTAs have 444 (forward, dQ), 296 (dK and dV, 245 to 255 registers) or 592 (split)
-// places, 7 to 12 warps on an SM.  Schedulers issue in 44, 41, 33 % of the active cycles (forward, dQ, dK and dV) and in 49, 38,
-// 36 % (scores, apply, gather); the largest stalls are the barriers around a chunk, whose loads nothing overlaps, then the
-// latency of dependent instructions, in apply and gather also that of the weights.  DRAM is at 2 to 8 %.  The weights are
+// places, 7 to 12 warps on an SM.  Schedulers issue in 47, 43, 38 % of the active cycles (forward, dQ, dK and dV) and in 49, 38,
+// 39 % (scores, apply, gather); the largest stalls are the latency of dependent instructions and the barriers around a chunk, whose
+// loads nothing overlaps, in apply and gather that of the weights.  DRAM is at 3 to 9 %.  The weights are
 // half of the gather: 32 lanes read 32 sectors, which the few KB of L1 beside the staged columns do not keep.
 //
 // Rows are queries and columns keys, or the other way round (key side: dK, dV; columns = the queries that attend to a key,
@@ -50,6 +50,8 @@ constexpr int kWarpsF = 4;
 constexpr int kThreadsF = 32 * kWarpsF;
 // Pairs of weights a lane fetches ahead.  With more the gather spills more at the 128 registers that four CTAs leave a thread: 56 x 56, 7 x 7,
 // head dim 32, bf16, two gathers 61.4 us with 2, 71.5 with 4, 84 with 8 (apply 49.1, 49.8, 53.1); three CTAs with 7: 94.7 and 59.6.
+// With 4 in nine shapes of ranks 1 to 3 (windows of 27 to 255, head dims 32 to 128, float32 and bf16): gathers 4 to 28 % slower, applies
+// 1 to 9 % (two of 36 faster: head dim 32 in float32, 9 x 9 on 96 x 100 2 %, window 255 of 4097 4 %).
 constexpr int kAheadF = 2;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 
@@ -884,7 +886,10 @@ fma_gather_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ w, 
 // As much of the column box at a time as the CTAs that registers allow on an SM can have of its 227 KB: three of the forward and of
 // dQ, two of the key side.  Every chunk is a barrier that nothing overlaps.  Measured, 56 x 56, 7 x 7, 4 heads of 32, batch 4, with
 // 32, 48, 64, 72, 100 KB: forward 35.6, 34.3, 35.3, 30.2, 33.7 us (the last with two CTAs); dQ 42.9, 42.5, 43.5, 37.5, 42.1;
-// dK and dV 80.6, 75.7, 75.5, 72.5, 67.0.
+// dK and dV 80.6, 75.7, 75.5, 72.5, 67.0.  Against 64 KB for all, in nine shapes of ranks 1 to 3: forward and dQ equal or up to 15 %
+// faster at head dim 32, equal to 4 % at 64 and 128; dK and dV 2 to 18 % (head dims 32 | 64 | 128, 56 x 56: 72 -> 65, 114 -> 111,
+// 193 -> 179 us; 12 x 24 x 26, 3 x 3 x 3, 64: 169 -> 127; where the box then fits in one chunk 2 x: 48 x 60, 13 x 13, 128: 544 -> 286).
+// One was slower: 8 x 28 x 28, 3 x 5 x 5, 32: 123 -> 128.
 constexpr int kQueryChunk = 72 * 1024, kKeyChunk = 100 * 1024;
 
 // Rows of a warp are 4 x (256 / D) (rank 1: one row of 1024 / D).  `tensors`: column tensors staged side by side,
