@@ -1,5 +1,6 @@
-"""The one-buffer form of the tcgen05 forward, which serves head dims up to 64 where there are more than two tiles an SM: edge
-shapes of the other tests with as many samples as that takes, against the general kernels."""
+"""The persistent tcgen05 kernels where every CTA walks several tiles (loads and tables run ahead, slots and phases come round), in the
+forward also the one-buffer form of head dims up to 64, which serves more than two tiles an SM: edge shapes of the other tests with
+as many samples as that takes, against the general kernels."""
 import pytest
 import torch
 
@@ -10,12 +11,13 @@ pytestmark = pytest.mark.gpu
 
 
 def samples(size, heads):
-    """Samples for which tiles of 128 rows number more than two an SM however they are cut."""
+    """Samples for which tiles of 128 rows number more than twelve an SM however they are cut: three a CTA of the one-buffer forward,
+    of which four share an SM, and more of the others."""
     rows = heads
     for n in size:
         rows *= n
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    return -(-(2 * sms + 1) * 128 // rows)
+    return -(-(12 * sms + 1) * 128 // rows)
 
 
 def inputs(B, size, hq, hkv, dim, dtype, seed, extra=0):
@@ -25,26 +27,39 @@ def inputs(B, size, hq, hkv, dim, dtype, seed, extra=0):
     return (q, k, v), (dict(extra_k=t(B, extra, hkv, dim), extra_v=t(B, extra, hkv, dim)) if extra else {})
 
 
-def compare(qkv, *geo, **kw):
+def forced(path, run):
     try:
-        _cabi.set_force("simt")
-        want, want_lse = _backend.fused_forward(*qkv, *geo, **kw)
-        _cabi.set_force("tc")
-        got, lse = _backend.fused_forward(*qkv, *geo, **kw)
-        assert _cabi.last_path() == "tcgen05"
+        _cabi.set_force(path)
+        return run()
     finally:
         _cabi.set_force(None)
+
+
+def compare(qkv, *geo, backward=True, **kw):
+    want, want_lse = forced("simt", lambda: _backend.fused_forward(*qkv, *geo, **kw))
+    got, lse = forced("tc", lambda: _backend.fused_forward(*qkv, *geo, **kw))
+    assert _cabi.last_path() == "tcgen05"
+    # the bounds of the same shapes with few tiles (test_gpu_tc.py); among this many outputs some are past 4, where two roundings to
+    # bf16 may differ by 2^-7 of the value
+    assert float(((got.float() - want.float()).abs() / want.float().abs().clamp(min=1.0)).max()) <= 1.6e-2
+    assert float((lse - want_lse).abs().max()) <= 2e-3
+    if backward:
+        g = torch.Generator(device="cuda").manual_seed(11)
+        do = torch.randn(want.shape, device="cuda", generator=g).to(want.dtype)
+        dlse = torch.randn(want_lse.shape, device="cuda", generator=g)
+        run = lambda: _backend.fused_backward(*qkv, want, want_lse, do, *geo, dlse=dlse, **kw)
+        grads, want_grads = forced("tc", run), forced("simt", run)
+        for a, b in zip(grads, want_grads):
+            if b is not None:
+                assert float((a.float() - b.float()).abs().max()) <= 2e-2 * max(1.0, float(b.float().abs().max()))
     torch.cuda.synchronize()
     assert _cabi.device_status() == 0
-    # the bounds of the same shapes with few tiles (test_gpu_tc.py)
-    assert float((got.float() - want.float()).abs().max()) <= 1.6e-2
-    assert float((lse - want_lse).abs().max()) <= 2e-3
     return got, lse
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
-@pytest.mark.parametrize("case", [c for c in few.CASES if few._dim(c) <= 64], ids=few._id)
-def test_forward(case, dtype):
+@pytest.mark.parametrize("case", few.CASES, ids=few._id)
+def test_forward_and_backward(case, dtype):
     size, _, hq, hkv, kernel, dilation, causal, extents = case[:8]
     dim = few._dim(case)
     B = samples(size, hq)
@@ -54,33 +69,35 @@ def test_forward(case, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
-@pytest.mark.parametrize("case", [c for c in few.EXTRA_CASES if c[4] == 64], ids=lambda c: "x".join(map(str, c[0])) + f"_e{c[6]}")
+@pytest.mark.parametrize("case", few.EXTRA_CASES, ids=lambda c: "x".join(map(str, c[0])) + f"_e{c[6]}")
 def test_additional_tokens(case, dtype):
-    size, _, hq, hkv, dim, kernel, extra, _ = case
-    qkv, kw = inputs(samples(size, hq), size, hq, hkv, dim, dtype, 23, extra)
-    compare(qkv, kernel, (1,) * len(size), (1,) * len(size), (False,) * len(size), dim ** -0.5, **kw)
+    size, _, hq, hkv, dim, kernel, extra, extents = case
+    B = samples(size, hq)
+    qkv, kw = inputs(B, size, hq, hkv, dim, dtype, 23, extra)
+    ext = None if extents is None else torch.tensor([extents[b % len(extents)] for b in range(B)], dtype=torch.int32).cuda()
+    compare(qkv, kernel, (1,) * len(size), (1,) * len(size), (False,) * len(size), dim ** -0.5, extents=ext, **kw)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
-@pytest.mark.parametrize("case", [c for c in few.STRIDE_CASES if c[9] == 64], ids=lambda c: "x".join(map(str, c[0])) + f"_s{c[6][-1]}")
+@pytest.mark.parametrize("case", few.STRIDE_CASES, ids=lambda c: "x".join(map(str, c[0])) + f"_s{c[6][-1]}")
 def test_output_stride(case, dtype):
     size, _, hq, hkv, kernel, dilation, stride, causal, extents, dim = case
     B = samples([-(-n // s) for n, s in zip(size, stride)], hq)
     qkv, _ = inputs(B, size, hq, hkv, dim, dtype, 29)
     ext = None if extents is None else torch.tensor([extents[b % len(extents)] for b in range(B)], dtype=torch.int32).cuda()
-    compare(qkv, kernel, stride, dilation, causal, dim ** -0.5, extents=ext)
+    compare(qkv, kernel, stride, dilation, causal, dim ** -0.5, extents=ext, backward=False)
 
 
-@pytest.mark.parametrize("shape", [s for s in tables.SHAPES if s[-1] <= 64], ids=lambda s: "x".join(map(str, s[1] + s[2])) + f"d{s[-1]}")
+@pytest.mark.parametrize("shape", tables.SHAPES, ids=lambda s: "x".join(map(str, s[1] + s[2])) + f"d{s[-1]}")
 @pytest.mark.parametrize("extra", [0, 5])
 def test_tables(shape, extra):
     _, size, kernel, dilation, stride, causal, heads, dim = shape
     B = samples([-(-n // s) for n, s in zip(size, stride)], heads)
     qkv, kw = inputs(B, size, heads, heads, dim, torch.bfloat16, sum(size), extra)
-    compare(qkv, kernel, stride, dilation, tuple(bool(c) for c in causal), dim ** -0.5, **kw)
+    compare(qkv, kernel, stride, dilation, tuple(bool(c) for c in causal), dim ** -0.5, backward=False, **kw)
 
 
-@pytest.mark.parametrize("shape", [s for s in tables.PACKED if s[-1] <= 64], ids=lambda s: "x".join(map(str, s[0] + s[1] + s[3])))
+@pytest.mark.parametrize("shape", tables.PACKED, ids=lambda s: "x".join(map(str, s[0] + s[1] + s[3])))
 def test_grouped_heads_packed(shape):
     size, kernel, causal, (hq, hkv), dim = shape
     qkv, kw = inputs(samples(size, hq), size, hq, hkv, dim, torch.float16, sum(size), 5)
@@ -90,7 +107,7 @@ def test_grouped_heads_packed(shape):
 
 @pytest.mark.parametrize("lens", [(300, 7, 128), (129, 300, 15)])
 def test_lengths(lens):
-    B = samples((7,), 4) // 3 * 3 + 3            # (padding tiles are walked like the others)
+    B = samples((128,), 4) // 3 * 3 + 3          # (a sample has one to three tiles a head, and padding tiles)
     (q, k, v), _ = inputs(B, (300,), 4, 2, 64, torch.float16, 5)
     sizes = torch.tensor([lens[b % 3] for b in range(B)], dtype=torch.int32, device="cuda")
     past = torch.arange(300, device="cuda")[None, :] >= sizes[:, None]
@@ -115,16 +132,11 @@ def test_rescale_when_later_chunks_dominate(size, kernel, slope, axis, dtype):
     q, k, v = [x.to(dtype) for x in (t() * 0.1 + 1.0, t() * 0.1 + ramp / D ** 0.5, t())]
     ones = (1,) * len(size)
     args = (q, k, v, kernel, ones, ones, (False,) * len(size), D ** -0.5)
-    try:
-        _cabi.set_force("simt")
-        want, want_lse = _backend.fused_forward(*args)
-        _cabi.set_force("tc")
-        got, lse = _backend.fused_forward(*args)
-        assert _cabi.last_path() == "tcgen05"
-    finally:
-        _cabi.set_force(None)
+    want, want_lse = forced("simt", lambda: _backend.fused_forward(*args))
+    got, lse = forced("tc", lambda: _backend.fused_forward(*args))
+    assert _cabi.last_path() == "tcgen05"
     torch.cuda.synchronize()
     assert _cabi.device_status() == 0
     assert float(want_lse.max() - want_lse.min()) > 20.0
-    assert float((got.float() - want.float()).abs().max()) <= 2e-2
+    assert float(((got.float() - want.float()).abs() / want.float().abs().clamp(min=1.0)).max()) <= 2e-2      # see compare()
     assert float(((lse - want_lse).abs() / want_lse.abs().clamp(min=1.0)).max()) <= 2e-3
