@@ -528,11 +528,26 @@ inline int make_plan(const Geo& g, Plan& plan, int chunk = kChunk, bool with_str
     if (interleave && !runs) {
         // the first (slowest) axis that needs several chunks is the one along which the warps of a
         // tile differ; tensor maps take element strides up to 8
+        bool skipped = false;
         for (int a = 0; a < 3; ++a) {
-            // (an axis with one row a chunk has nothing to interleave: the forward goes on to the next; 16 x 32 x 32, 3 x 7 x 7, causal
-            // frames, 8 heads of 64, batch 2: 117 -> 104 us.  The backward got slower that way, 129 -> 137 and 166 -> 175)
-            if (p.nchunk[a] <= 1 || (!backward && p.cb[a] == 1)) continue;
-            const int il = p.nchunk[a];
+            if (p.nchunk[a] <= 1) continue;
+            int il = p.nchunk[a];
+            if (!backward) {
+                // An axis with one row a chunk has nothing to interleave.  The forward goes on to the next one where that leaves the row
+                // maps (16-column rows) and there are tiles away from the edges, whose rows do not share their windows: 16 x 32 x 32,
+                // 3 x 7 x 7, causal frames, 8 heads of 64, batch 2, 117 -> 104 us; 10 x 32 x 8, 3 x 7 x 7, 8 heads of 32, batch 6,
+                // 62 -> 54; but 16 x 14 x 20, 3 x 7 x 7 69 -> 75, and 8 x 8 chunks 15 x 20 x 7, 5 x 7 x 7 144 -> 163.  (The backward got
+                // slower that way: 129 -> 137 and 166 -> 175.)
+                if (p.cb[a] == 1) { skipped = true; continue; }
+                if (skipped && (a == 2 || p.cb[2] != 16 || p.ntile[a] <= 2)) break;
+                // Chunks of the longest box that a tensor of this size leaves, not of the tile's nominal one: il chunks are walked
+                // whatever the box.  15 x 7 x 7, 7 x 7 x 5, 4 heads of 32 33 -> 24 us; 8 x 24, 7 x 7, 2 heads of 64, batch 21 11 -> 9.
+                const int lp = (p.L[a] + p.dil[a] - 1) / p.dil[a], nq = (lp + p.qstep[a] - 1) / p.qstep[a];
+                int box = ((p.tile[a] < nq ? p.tile[a] : nq) - 1) * p.qstep[a] + p.K[a];
+                if (!p.causal[a] && box > lp) box = lp > p.K[a] ? lp : p.K[a];       // (a causal window starts in front of the tensor)
+                il = (box + p.cb[a] - 1) / p.cb[a];
+                if (il <= 1) continue;
+            }
             if (p.dil[a] * il <= 8 && p.cb[a] * p.dil[a] * il <= 256) {
                 p.il[a] = il;
                 p.il_mul[a] = (unsigned)((0x100000000ull + il - 1) / il);
