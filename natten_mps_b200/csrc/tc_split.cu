@@ -427,7 +427,7 @@ int launch_scores_inner(const Plan& plan, const CUtensorMap& mx, const CUtensorM
 // ---------------------------------------------------------------------------
 // kThree: three CTAs share an SM, which leaves each one P buffer and 72 registers.  What bounds these kernels is the chain of a tile
 // (geometry, weights, gathering, product), not an issue rate, so at head dim 64 that is the better form wherever the weights of three
-// tiles fit beside each other (101 slots); above it two CTAs with two buffers.  fp16, 8 heads of 64, batch 2, forward and dQ, three
+// tiles fit beside each other (101 slots) and there are more than two tiles an SM; else two CTAs with two buffers.  fp16, 8 heads of 64, batch 2, forward and dQ, three
 // CTAs | two with one buffer | two with two: 61 x 67, 49 slots 48.9 | 51.4 | 50.7 us, 81 slots 58.1 | 60.6 | 60.0, 99 slots
 // 81.5 | 89.0 | 85.9; 121 slots, where a third CTA has no room, 112.7 | 103.6 | 99.3, 147 133.5 | 122.4 | 119.0, 225 175.7 | 168.8 | 162.4.
 template <int DH, bool kThree>
@@ -661,6 +661,19 @@ tc_apply_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_constant__
     }
 }
 
+// Tiles (CTAs) of a launch over `heads` heads.
+inline long long tiles_of(const Plan& plan, const Geo& g, int heads)
+{
+    long long n = plan.p.ntiles;
+    for (int a = 0; a < 3; ++a) n *= plan.p.grp_n[a];
+    return n * heads * g.B;
+}
+// With at most two tiles an SM there is no third for the three-CTA form, which then only lacks the second P buffer and its registers:
+// heads of 64, 16-bit, three | two, gather and the other half of its call: 6 x 29 x 29, 3 x 5 x 7, batch 2 72 | 64 us; 11 x 22 x 22,
+// 3 x 7 x 3, 2 heads, batch 2 122 | 111; apply 42 x 72, 7 x 11, 2 heads, batch 2 13.9 | 12.0.  Of 141 such shapes 0.86 to 1.06 of the
+// time (gathers with few chunks keep the other form's better: 32 x 17, 11 x 11, 8 heads 44 | 47).
+inline bool third_tile(const Plan& plan, const Geo& g, int heads) { return tiles_of(plan, g, heads) > 2 * sm_count(); }
+
 template <int DH, bool BF16, int kInner, bool kThree>
 int launch_apply_as(const Plan& plan, const CUtensorMap& my, const Geo& g, const void* w, void* out, float scale,
                     bool out_by_position, cudaStream_t s)
@@ -687,7 +700,7 @@ int launch_apply_inner(const Plan& plan, const CUtensorMap& my, const Geo& g, co
                        bool out_by_position, cudaStream_t s)
 {
     if constexpr (DH == 64) {
-        if (SmemA<DH, true>::kW + (size_t)kTileRows * g.ktot * 2 <= kThirdOfSm)
+        if (SmemA<DH, true>::kW + (size_t)kTileRows * g.ktot * 2 <= kThirdOfSm && third_tile(plan, g, g.Hq))
             return launch_apply_as<DH, BF16, kInner, true>(plan, my, g, w, out, scale, out_by_position, s);
     }
     return launch_apply_as<DH, BF16, kInner, false>(plan, my, g, w, out, scale, out_by_position, s);
@@ -711,7 +724,7 @@ int launch_apply(const Plan& plan, const CUtensorMap& my, const Geo& g, const vo
 // (lanes of a warp are neighbouring keys, so one load touches one row of w) and acc += P^T X runs on the
 // tensor cores with the X chunk staged by TMA and read MN-major.  The order of accumulation is fixed.
 // ---------------------------------------------------------------------------
-template <int DH>
+template <int DH, bool kThree>
 struct SmemG {
     static constexpr int kHalves = DH / 64;
     static constexpr int kHalf = kTileRows * 128;
@@ -720,16 +733,18 @@ struct SmemG {
     static constexpr int kBar = kX + kStages * kTile;     // barriers, flags: 128 bytes
     static constexpr int kColRow = kBar + 128;            // [2][128] long long: element offset of the column's row of w, -1 = no query
     static constexpr int kTotal = kColRow + 2048;
-    static constexpr int kPBufs = DH == 64 ? 1 : 2, kPerSm = DH == 64 ? 3 : 1;
-    static constexpr uint32_t kColP = 0, kColO = 64 * kPBufs, kTmemCols = kColO + DH;
+    static constexpr int kPBufs = kThree ? 1 : 2, kPerSm = kThree ? 3 : DH == 64 ? 2 : 1;
+    static constexpr uint32_t kColP = 0, kColO = 64 * kPBufs;
+    static constexpr uint32_t kTmemCols = kColO + DH <= 128 ? 128 : 256;       // allocated in powers of two
+    static_assert(kTmemCols * kPerSm <= 512 && kColO + DH <= kTmemCols, "TMEM");
 };
 
-template <int DH, bool BF16>
-__global__ void __launch_bounds__(kThreads, SmemG<DH>::kPerSm)
+template <int DH, bool BF16, bool kThree>
+__global__ void __launch_bounds__(kThreads, SmemG<DH, kThree>::kPerSm)
 tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ TcParams P,
                  const uint16_t* __restrict__ w, uint16_t* __restrict__ dst, float scale, int ktot)
 {
-    using SM = SmemG<DH>;
+    using SM = SmemG<DH, kThree>;
     constexpr int CH = DH / 2;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -938,12 +953,13 @@ tc_gather_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     }
 }
 
-template <int DH, bool BF16>
-int launch_gather(const Plan& plan, const CUtensorMap& mx, const Geo& g, const void* w, void* dst, float scale,
-                  cudaStream_t s)
+template <int DH, bool BF16, bool kThree>
+int launch_gather_as(const Plan& plan, const CUtensorMap& mx, const Geo& g, const void* w, void* dst, float scale,
+                     cudaStream_t s)
 {
-    using SM = SmemG<DH>;
-    cudaError_t err = ensure_dynamic_smem((const void*)tc_gather_kernel<DH, BF16>, SM::kTotal);
+    using SM = SmemG<DH, kThree>;
+    auto* kernel = tc_gather_kernel<DH, BF16, kThree>;
+    cudaError_t err = ensure_dynamic_smem((const void*)kernel, SM::kTotal);
     if (err != cudaSuccess) {
         cudaGetLastError();
         return (int)err;
@@ -951,10 +967,19 @@ int launch_gather(const Plan& plan, const CUtensorMap& mx, const Geo& g, const v
     int ngroups = 1;
     for (int a = 0; a < 3; ++a) ngroups *= plan.p.grp_n[a];
     const dim3 grid((unsigned)(plan.p.ntiles * ngroups), (unsigned)g.Hkv, (unsigned)g.B);
-    tc_gather_kernel<DH, BF16><<<grid, kThreads, SM::kTotal, s>>>(mx, plan.p, (const uint16_t*)w, (uint16_t*)dst, scale, g.ktot);
+    kernel<<<grid, kThreads, SM::kTotal, s>>>(mx, plan.p, (const uint16_t*)w, (uint16_t*)dst, scale, g.ktot);
     tc_count_launch();
     err = cudaGetLastError();
     return err == cudaSuccess ? 0 : (int)err;
+}
+
+template <int DH, bool BF16>
+int launch_gather(const Plan& plan, const CUtensorMap& mx, const Geo& g, const void* w, void* dst, float scale,
+                  cudaStream_t s)
+{
+    if constexpr (DH == 64)
+        if (third_tile(plan, g, g.Hkv)) return launch_gather_as<DH, BF16, true>(plan, mx, g, w, dst, scale, s);
+    return launch_gather_as<DH, BF16, false>(plan, mx, g, w, dst, scale, s);
 }
 
 } // namespace
