@@ -889,7 +889,8 @@ fma_gather_kernel(const __grid_constant__ FmaParams P, const T* __restrict__ w, 
 // dK and dV 80.6, 75.7, 75.5, 72.5, 67.0.  Against 64 KB for all, in nine shapes of ranks 1 to 3: forward and dQ equal or up to 15 %
 // faster at head dim 32, equal to 4 % at 64 and 128; dK and dV 2 to 18 % (head dims 32 | 64 | 128, 56 x 56: 72 -> 65, 114 -> 111,
 // 193 -> 179 us; 12 x 24 x 26, 3 x 3 x 3, 64: 169 -> 127; where the box then fits in one chunk 2 x: 48 x 60, 13 x 13, 128: 544 -> 286).
-// One was slower: 8 x 28 x 28, 3 x 5 x 5, 32: 123 -> 128.
+// Slower: 8 x 28 x 28, 3 x 5 x 5, 32: 123 -> 128; 88 x 106, 5 x 35, dilation 2 x 1, 1 head of 32: 235 -> 270 (undilated 208 -> 180; 3 x 35
+// on 64 x 64, 64: 382 -> 199).
 constexpr int kQueryChunk = 72 * 1024, kKeyChunk = 100 * 1024;
 
 // Rows of a warp are 4 x (256 / D) (rank 1: one row of 1024 / D).  `tensors`: column tensors staged side by side,
